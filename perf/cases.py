@@ -216,11 +216,13 @@ def prepare(case, seed):
         s["f"] = [lat.field(_host(_source(dims, gen)).numpy(), prec=p), lat.field(prec=p), lat.field(prec=p)]
         s["out"] = _pinned(n)
     elif kind == "host":
+        s["ctx"] = wd.Context(0)  # a context keeps one configuration's links for the host-buffer calls
         s["gauge"] = [_host(g, case["pinned"]).numpy() for g in _gauge(dims, gen)]
         s["src"] = _host(_source(dims, gen), case["pinned"])
         s["out"] = _host(torch.zeros(n, dtype=torch.complex128), case["pinned"])
         s["args"] = (wd._dims(dims), wd._gauge_ptrs(s["gauge"]), _ptr(s["src"]), _ptr(s["out"]))
     elif kind == "hostcg":
+        s["ctx"] = wd.Context(0)
         s["gauge"] = [_host(g, False).numpy() for g in _gauge(dims, gen)]
         s["src"] = _host(_source(dims, gen), False).numpy()
         s["out"] = np.empty(n, np.complex128)
