@@ -95,6 +95,31 @@ static void host_cache_drop(wd_context *ctx)
     for (auto &p : ctx->host_gauge_ptr) p = nullptr;
 }
 
+// the fixed-point links of one lattice, if it has them (cudaFree waits for work in flight)
+void wd_drop_fix(wd_lattice *lat)
+{
+    cudaFree(lat->gauge_fix);
+    lat->gauge_fix = nullptr;
+    if (lat->ctx) lat->ctx->fix_lats.erase(lat);
+}
+
+bool wd_release_fix(wd_context *ctx)
+{
+    const bool any = !ctx->fix_lats.empty();
+    while (!ctx->fix_lats.empty()) wd_drop_fix(*ctx->fix_lats.begin());
+    return any;
+}
+
+cudaError_t wd_malloc(wd_context *ctx, void **p, size_t bytes)
+{
+    cudaError_t e = cudaMalloc(p, bytes);
+    if (e == cudaErrorMemoryAllocation && wd_release_fix(ctx)) {
+        cudaGetLastError();
+        e = cudaMalloc(p, bytes);
+    }
+    return e;
+}
+
 wd_status wd_dev_alloc(wd_context *ctx, void **p, size_t bytes)
 {
     if (wd_alloc_fails(ctx)) return wd_fail(ctx, WD_ERR_OOM, "work buffer: injected allocation failure");
@@ -111,7 +136,7 @@ wd_status wd_dev_alloc(wd_context *ctx, void **p, size_t bytes)
     if (e == cudaErrorMemoryAllocation) {
         cudaGetLastError();
         wd_pool_release(ctx);
-        e = cudaMalloc(p, bytes);
+        e = wd_malloc(ctx, p, bytes);
     }
     if (e != cudaSuccess) return wd_cuda_check(ctx, e, "cudaMalloc(work buffer)");
     ctx->pool_used[*p] = bytes;
@@ -143,6 +168,7 @@ extern "C" void wd_context_destroy(wd_context *ctx)
     if (!ctx) return;
     cudaSetDevice(ctx->device);
     host_cache_drop(ctx);
+    for (wd_lattice *lat : ctx->fix_lats) lat->ctx = nullptr;  // a lattice may be destroyed after its context
     wd_pool_release(ctx);
     for (auto &kv : ctx->pool_used) cudaFree(kv.first);
     ctx->pool_used.clear();
@@ -199,7 +225,7 @@ static wd_status ensure_staging(wd_context *ctx, size_t bytes)
     cudaFree(ctx->staging);
     ctx->staging = nullptr;
     ctx->staging_bytes = 0;
-    WD_CUDA(ctx, cudaMalloc(&ctx->staging, bytes));
+    WD_CUDA(ctx, wd_malloc(ctx, &ctx->staging, bytes));
     ctx->staging_bytes = bytes;
     return WD_OK;
 }
@@ -222,36 +248,65 @@ static wd_status make_geom(wd_context *ctx, const int *dims, WdGeom *g, int64_t 
     return WD_OK;
 }
 
+// Allocates the lattice's fixed-point links if it has none: a copy that only
+// makes FP64 hops faster, so it is kept where it leaves at least half of the
+// device's memory free, and given back when a later allocation needs its
+// memory (wd_malloc).  Returns the device flag behind the planes, or null.
+static int *want_fix(wd_context *ctx, wd_lattice *lat)
+{
+    const size_t n = (size_t)lat->volume * 4 * 9 * sizeof(int4);
+    if (!lat->gauge_fix && lat->use_fix) {
+        size_t free_b = 0, total_b = 0;
+        const bool room = n < (64u << 20) || (cudaMemGetInfo(&free_b, &total_b) == cudaSuccess && free_b >= n + total_b / 2);
+        if (!room || cudaMalloc(&lat->gauge_fix, n + sizeof(int4)) != cudaSuccess) {
+            cudaGetLastError();
+            lat->gauge_fix = nullptr;
+            return nullptr;
+        }
+        ctx->fix_lats.insert(lat);
+    }
+    return lat->gauge_fix ? (int *)((char *)lat->gauge_fix + n) : nullptr;
+}
+
 static wd_status upload_gauge(wd_context *ctx, wd_lattice *lat, const double *const gauge[4])
 {
     const WdGeom &g = lat->g;
     const size_t bytes = (size_t)lat->volume * 9 * sizeof(double2);
     wd_status st = ensure_staging(ctx, bytes);
     if (st != WD_OK) return st;
-    for (int mu = 0; mu < 4; ++mu) {
+    for (int mu = 0; mu < 4; ++mu)
         if (!gauge[mu]) return wd_fail(ctx, WD_ERR_BAD_ARG, "gauge pointer is null");
+    int *bad = want_fix(ctx, lat);
+    if (bad) WD_CUDA(ctx, cudaMemsetAsync(bad, 0, sizeof(int), ctx->stream));
+    for (int mu = 0; mu < 4; ++mu) {
         WD_CUDA(ctx, cudaMemcpyAsync(ctx->staging, gauge[mu], bytes, cudaMemcpyHostToDevice, ctx->stream));
-        st = wd_gauge_ref_to_soa(ctx, g, mu, (const double2 *)ctx->staging, lat->gauge);
+        const double2 *ref = (const double2 *)ctx->staging;
+        st = bad ? wd_gauge_ref_to_soa_fix(ctx, g, mu, ref, lat->gauge, lat->gauge_fix, bad)
+                 : wd_gauge_ref_to_soa(ctx, g, mu, ref, lat->gauge);
         if (st != WD_OK) return st;
     }
     wd_lattice_invalidate_derived(lat);
+    int *host_bad = (int *)ctx->state_host;
+    *host_bad = 0;
+    if (bad) WD_CUDA(ctx, cudaMemcpyAsync(host_bad, bad, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
     WD_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+    if (*host_bad) wd_drop_fix(lat);
     return WD_OK;
 }
 
-extern "C" wd_status wd_lattice_create(wd_context *ctx, const int dims[4], const double *const gauge[4],
-                                       wd_lattice **out)
+wd_status wd_lattice_make(wd_context *ctx, const int dims[4], const double *const gauge[4], bool fix, wd_lattice **out)
 {
     if (!ctx || !out || !gauge) return wd_fail(ctx, WD_ERR_BAD_ARG, "null argument");
     *out = nullptr;
     wd_lattice *lat = new wd_lattice();
     lat->ctx = ctx;
+    lat->use_fix = fix;
     wd_status st = make_geom(ctx, dims, &lat->g, &lat->volume);
     if (st != WD_OK) {
         delete lat;
         return st;
     }
-    cudaError_t e = cudaMalloc(&lat->gauge, (size_t)lat->volume * 4 * 9 * sizeof(double2));
+    cudaError_t e = wd_malloc(ctx, (void **)&lat->gauge, (size_t)lat->volume * 4 * 9 * sizeof(double2));
     if (e != cudaSuccess) {
         delete lat;
         return wd_cuda_check(ctx, e, "cudaMalloc(gauge)");
@@ -265,6 +320,12 @@ extern "C" wd_status wd_lattice_create(wd_context *ctx, const int dims[4], const
     return WD_OK;
 }
 
+extern "C" wd_status wd_lattice_create(wd_context *ctx, const int dims[4], const double *const gauge[4],
+                                       wd_lattice **out)
+{
+    return wd_lattice_make(ctx, dims, gauge, true, out);
+}
+
 extern "C" wd_status wd_lattice_update(wd_context *ctx, wd_lattice *lat, const double *const gauge[4])
 {
     if (!ctx || !lat || !gauge) return wd_fail(ctx, WD_ERR_BAD_ARG, "null argument");
@@ -275,6 +336,7 @@ extern "C" void wd_lattice_destroy(wd_lattice *lat)
 {
     if (!lat) return;
     cudaFree(lat->gauge);  // cudaFree waits for work in flight on the device
+    if (lat->gauge_fix) wd_drop_fix(lat);
     wd_lattice_invalidate_derived(lat);
     delete lat;
 }
@@ -299,7 +361,7 @@ extern "C" wd_status wd_field_create_prec(wd_context *ctx, const wd_lattice *lat
     f->lat = lat;
     f->storage = prec;
     const size_t bytes = field_bytes(lat, prec);
-    cudaError_t e = cudaMalloc(&f->data, bytes);
+    cudaError_t e = wd_malloc(ctx, &f->data, bytes);
     if (e != cudaSuccess) {
         delete f;
         return wd_cuda_check(ctx, e, "cudaMalloc(field)");

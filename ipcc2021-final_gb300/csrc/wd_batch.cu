@@ -1077,6 +1077,24 @@ struct wd_server {
 
 static double field_bytes64(const wd_lattice *lat) { return (double)lat->volume * 12 * sizeof(double2); }
 
+// the optional fixed-point links the server's lattices hold now
+static double server_fix_bytes(const wd_server *sv)
+{
+    double b = 0;
+    for (const wd_lattice *l : sv->lats)
+        if (l->gauge_fix) b += (double)l->volume * 4 * 9 * sizeof(int4);
+    return b;
+}
+
+// Gives them up if `bytes` more would not fit the budget beside them: what
+// the server accepts does not depend on them.
+static void server_make_room(wd_server *sv, double bytes)
+{
+    if (sv->gauge_bytes + sv->req_bytes + server_fix_bytes(sv) + bytes <= sv->cfg.hbm_budget_bytes) return;
+    for (wd_lattice *l : sv->lats)
+        if (l->gauge_fix) wd_drop_fix(l);
+}
+
 static double request_bytes(const wd_server *sv, const wd_lattice *lat, int nsrc)
 {
     double per = 2 * field_bytes64(lat);
@@ -1131,7 +1149,9 @@ extern "C" wd_status wd_server_add_lattice(wd_server *sv, const int dims[4], con
 {
     if (!sv || !id) return WD_ERR_BAD_ARG;
     wd_lattice *lat = nullptr;
-    wd_status st = wd_lattice_create(sv->ctx, dims, gauge, &lat);
+    // FP64 hops run in the plain FP64 server and in FP64 reliable updates only
+    const bool fp64 = sv->cfg.prec == WD_PREC_F64 || sv->cfg.prec_reliable != WD_PREC_DF64;
+    wd_status st = wd_lattice_make(sv->ctx, dims, gauge, fp64, &lat);
     if (st != WD_OK) return st;
     // derived link copies the server will use, built now so they count against the budget
     double bytes = (double)lat->volume * 4 * 9 * sizeof(double2);
@@ -1153,6 +1173,7 @@ extern "C" wd_status wd_server_add_lattice(wd_server *sv, const int dims[4], con
     }
     sv->gauge_bytes += bytes;
     sv->lats.push_back(lat);
+    server_make_room(sv, 0);
     *id = (int)sv->lats.size() - 1;
     return WD_OK;
 }
@@ -1228,6 +1249,7 @@ static wd_status server_admit(wd_server *sv, int *completed)
         const double bytes = request_bytes(sv, lat, p.nsrc);
         if (sv->gauge_bytes + sv->req_bytes + bytes > sv->cfg.hbm_budget_bytes) break;
         if (sv->active_systems > 0 && sv->active_systems + p.nsrc > sv->cfg.max_systems) break;
+        server_make_room(sv, bytes);
         wd_server::Req &r = sv->reqs[p.id];
         wd_status st = WD_OK;
         for (int k = 0; k < p.nsrc && st == WD_OK; ++k) {
@@ -1348,6 +1370,6 @@ extern "C" wd_status wd_server_status(const wd_server *sv, int *queued, int *act
     if (!sv) return WD_ERR_BAD_ARG;
     if (queued) *queued = (int)sv->queue.size();
     if (active_systems) *active_systems = sv->active_systems;
-    if (bytes_in_use) *bytes_in_use = sv->gauge_bytes + sv->req_bytes;
+    if (bytes_in_use) *bytes_in_use = sv->gauge_bytes + sv->req_bytes + server_fix_bytes(sv);
     return WD_OK;
 }

@@ -618,6 +618,6 @@ wd_status wd_lattice_gauge_df(wd_context *ctx, const wd_lattice *lat_c)
     wd_lattice *lat = const_cast<wd_lattice *>(lat_c);
     if (lat->gauge_df) return WD_OK;
     const int64_t n = lat->volume * 4 * 9;
-    WD_CUDA(ctx, cudaMalloc(&lat->gauge_df, n * sizeof(float4)));
+    WD_CUDA(ctx, wd_malloc(ctx, (void **)&lat->gauge_df, n * sizeof(float4)));
     return wd_convert_f64_to_df(ctx, lat->gauge, lat->gauge_df, n);
 }

@@ -404,11 +404,11 @@ wd_status wd_lattice_gauge_lp(wd_context *ctx, const wd_lattice *lat_c, wd_preci
     dim3 grid((Vh + 127) / 128, 8);
     if (prec == WD_PREC_F32) {
         if (lat->gauge_f32) return WD_OK;
-        WD_CUDA(ctx, cudaMalloc(&lat->gauge_f32, (size_t)8 * 3 * Vh * sizeof(float4)));
+        WD_CUDA(ctx, wd_malloc(ctx, &lat->gauge_f32, (size_t)8 * 3 * Vh * sizeof(float4)));
         k_gauge_f32<<<grid, 128, 0, ctx->stream>>>(lat->gauge, (float4 *)lat->gauge_f32, Vh);
     } else {
         if (lat->gauge_h12) return WD_OK;
-        WD_CUDA(ctx, cudaMalloc(&lat->gauge_h12, (size_t)8 * Vh * (sizeof(uint4) + sizeof(uint2))));
+        WD_CUDA(ctx, wd_malloc(ctx, &lat->gauge_h12, (size_t)8 * Vh * (sizeof(uint4) + sizeof(uint2))));
         uint4 *a = (uint4 *)lat->gauge_h12;
         k_gauge_f16<<<grid, 128, 0, ctx->stream>>>(lat->gauge, a, (uint2 *)(a + (size_t)8 * Vh), Vh);
     }

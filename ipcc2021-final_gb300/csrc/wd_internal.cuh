@@ -13,6 +13,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 #include <map>
+#include <set>
 #include <string>
 #include <unordered_map>
 #include "../../include/wilson_gb300.h"
@@ -61,6 +62,7 @@ struct wd_context {
     std::multimap<size_t, void *> pool_free;
     std::unordered_map<void *, size_t> pool_used;
     size_t pool_bytes = 0;
+    std::set<wd_lattice *> fix_lats;  // lattices holding fixed-point links (given back when memory runs out)
     // host-side failure injection for tests: after this many more successful
     // field / work-buffer allocations the next ones fail with WD_ERR_OOM
     // (-1: off)
@@ -81,6 +83,10 @@ inline bool wd_alloc_fails(wd_context *ctx)
 wd_status wd_dev_alloc(wd_context *ctx, void **p, size_t bytes);
 void wd_dev_free(wd_context *ctx, void *p);
 void wd_pool_release(wd_context *ctx);
+// cudaMalloc that gives back the context's fixed-point links when memory runs out
+cudaError_t wd_malloc(wd_context *ctx, void **p, size_t bytes);
+// wd_lattice_create; fix = false: without fixed-point links
+wd_status wd_lattice_make(wd_context *ctx, const int dims[4], const double *const gauge[4], bool fix, wd_lattice **out);
 
 struct wd_lattice {
     wd_context *ctx = nullptr;
@@ -88,6 +94,10 @@ struct wd_lattice {
     int64_t volume = 0;
     double2 *gauge = nullptr;     // FP64 [mu][parity][9][Vh]
     float4 *gauge_df = nullptr;   // double-float copy, same shape (lazily built)
+    // fixed-point copy, int4 {re hi, re lo, im hi, im lo}, same shape, written with the FP64 links at
+    // upload; null when they do not fit it or memory is short (FP64 hops then run on the FP64 pipe)
+    void *gauge_fix = nullptr;
+    bool use_fix = true;          // whether FP64 hops are expected on this lattice
     void *gauge_f32 = nullptr;    // FP32 12-real links [mu][parity][3][Vh] float4 (lazily built)
     void *gauge_h12 = nullptr;    // FP16 12-real links: uint4 [8][Vh] then uint2 [8][Vh] (lazily built)
 };

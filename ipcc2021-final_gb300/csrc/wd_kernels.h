@@ -14,6 +14,31 @@ wd_status wd_hop_f64(wd_context *ctx, const wd_lattice *lat, const double2 *in_b
                      double2 *out_block, const double2 *x_block, int cb, int dag, double alpha,
                      double beta);
 
+// ---- the FP64 hop in 64-bit fixed point (wd_dslash_fix.cu)
+// one direction's links from the reference layout into the FP64 planes and
+// the fixed-point planes; *bad (device) is set when they do not fit the latter
+wd_status wd_gauge_ref_to_soa_fix(wd_context *ctx, const WdGeom &g, int mu, const double2 *ref, double2 *soa, void *fix,
+                                  int *bad);
+// Frees every lattice's fixed-point links (their FP64 hops then run on the
+// FP64 pipe); true if there were any.  For allocations that fail otherwise.
+bool wd_release_fix(wd_context *ctx);
+void wd_drop_fix(wd_lattice *lat);
+// a residual hop's outputs: s32 = FP32(bhat - hop), block partials, |s32|^2
+struct WdResSink {
+    const double2 *bhat;
+    float4 *s32;
+    double *partial;
+    unsigned *counter;
+    double *result;
+};
+wd_status wd_hop_fix(wd_context *ctx, const wd_lattice *lat, const double2 *in, double2 *out,
+                     const double2 *x, int cb, int dag, double alpha, double beta, int variant);
+wd_status wd_hop_fix_residual(wd_context *ctx, const wd_lattice *lat, const double2 *in,
+                              const double2 *x, double alpha, double beta, const WdResSink &r, int variant);
+wd_status wd_hop_fix_aos_range(wd_context *ctx, cudaStream_t stream, const wd_lattice *lat, const double2 *in_aos,
+                               double2 *out_aos, const double2 *x_aos, int cb, int dag,
+                               double alpha, double beta, int s_lo, int s_hi);
+
 // ---- layout conversion (reference AoS <-> device SoA), on device buffers
 // spinor: ref[(p*Vh + s)*12 + c]  <->  soa[(p*12 + c)*Vh + s] in the vector's storage format
 wd_status wd_spinor_ref_to_soa(wd_context *ctx, const WdGeom &g, const double2 *ref, WdVec soa);
@@ -103,8 +128,6 @@ wd_status wd_hop_v(wd_context *ctx, const wd_lattice *lat, WdVec in, WdVec out, 
                    double alpha, double beta);
 
 // ---- pipelined host-buffer path: one parity block, output sites [s_lo, s_hi), given stream
-wd_status wd_hop_f64_range(wd_context *ctx, cudaStream_t stream, const wd_lattice *lat, const double2 *in_block,
-                           double2 *out_block, int cb, int dag, double alpha, int s_lo, int s_hi);
 // n 16-byte entries src -> dst by a kernel on `stream` (for host memory the
 // device addresses directly)
 wd_status wd_copy_kernel(wd_context *ctx, cudaStream_t stream, const double2 *src, double2 *dst, int64_t n);
@@ -113,8 +136,3 @@ wd_status wd_copy_kernel(wd_context *ctx, cudaStream_t stream, const double2 *sr
 wd_status wd_hop_f64_aos_range(wd_context *ctx, cudaStream_t stream, const wd_lattice *lat, const double2 *in_aos,
                                double2 *out_aos, const double2 *x_aos, int cb, int dag, double alpha, double beta,
                                int s_lo, int s_hi);
-// aos holds sites [s_lo, s_hi) of one parity block, 12 complex per site; soa_block is the block's planes
-wd_status wd_range_aos_to_soa(wd_context *ctx, cudaStream_t stream, int Vh, const double2 *aos, double2 *soa_block,
-                              int s_lo, int s_hi);
-wd_status wd_range_soa_to_aos(wd_context *ctx, cudaStream_t stream, int Vh, const double2 *soa_block, double2 *aos,
-                              int s_lo, int s_hi);
