@@ -455,19 +455,19 @@ static wd_status check_fields(wd_context *ctx, const wd_lattice *lat, const wd_f
 
 // out_cb = alpha * D_{cb,1-cb} in_{1-cb} + beta * x_cb on blocks of one storage format.
 wd_status wd_hop_v(wd_context *ctx, const wd_lattice *lat, WdVec in, WdVec out, const WdVec *x, int cb, int dag,
-                   double alpha, double beta)
+                   double alpha, double beta, const int *stop)
 {
     if (in.prec != out.prec || (x && x->prec != in.prec))
         return wd_fail(ctx, WD_ERR_BAD_ARG, "hopping term operands have different storage");
     switch (in.prec) {
     case WD_PREC_F64:
         return wd_hop_f64(ctx, lat, (const double2 *)in.p, (double2 *)out.p, x ? (const double2 *)x->p : nullptr, cb,
-                          dag, alpha, beta);
+                          dag, alpha, beta, stop);
     case WD_PREC_DF64:
         return wd_hop_df(ctx, lat, (const float4 *)in.p, (float4 *)out.p, x ? (const float4 *)x->p : nullptr, cb, dag,
-                         alpha, beta);
-    case WD_PREC_F32: return wd_hop_f32(ctx, lat, in, out, x, cb, dag, alpha, beta);
-    case WD_PREC_F16: return wd_hop_f16(ctx, lat, in, out, x, cb, dag, alpha, beta);
+                         alpha, beta, stop);
+    case WD_PREC_F32: return wd_hop_f32(ctx, lat, in, out, x, cb, dag, alpha, beta, stop);
+    case WD_PREC_F16: return wd_hop_f16(ctx, lat, in, out, x, cb, dag, alpha, beta, stop);
     }
     return wd_fail(ctx, WD_ERR_BAD_ARG, "unknown precision");
 }
@@ -541,6 +541,7 @@ extern "C" wd_status wd_dslash_full(wd_context *ctx, const wd_lattice *lat, cons
     if (st != WD_OK) return st;
     const double a = 4.0 + mass;
     return with_arith(ctx, lat, in, out, prec, false, [&](const wd_field *i, wd_field *o) -> wd_status {
+        if (i->storage == WD_PREC_F64 && lat->gauge_fix) return wd_hop_fix_M(ctx, lat, i->d, o->d, mass, dag);
         for (int cb = 0; cb < 2; ++cb) {
             const WdVec x = wd_block(i, cb);
             wd_status s = wd_hop_v(ctx, lat, wd_block(i, 1 - cb), wd_block(o, cb), &x, cb, dag, -0.5, a);

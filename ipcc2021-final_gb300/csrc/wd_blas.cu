@@ -9,6 +9,7 @@
 // FP32 pipe and convert to FP64 once per thread.
 #include "wd_kernels.h"
 #include "wd_df.cuh"
+#include "wd_reduce.cuh"
 
 namespace {
 
@@ -73,34 +74,6 @@ __global__ void __launch_bounds__(256) k_soa_to_aos(const void *__restrict__ soa
 }
 
 // ------------------------------------------------------- reductions
-__device__ __forceinline__ double warp_sum(double v)
-{
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-    return v;
-}
-
-// Block-reduce (a, b) and write one partial per block.
-__device__ __forceinline__ void block_partial(double a, double b, double2 *partial)
-{
-    __shared__ double sa[WD_RED_THREADS / 32], sb[WD_RED_THREADS / 32];
-    a = warp_sum(a);
-    b = warp_sum(b);
-    const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-    if (l == 0) {
-        sa[w] = a;
-        sb[w] = b;
-    }
-    __syncthreads();
-    if (w == 0) {
-        a = l < WD_RED_THREADS / 32 ? sa[l] : 0.0;
-        b = l < WD_RED_THREADS / 32 ? sb[l] : 0.0;
-        a = warp_sum(a);
-        b = warp_sum(b);
-        if (l == 0) partial[blockIdx.x] = make_double2(a, b);
-    }
-}
-
 #define GRID_STRIDE(i, n) \
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < (n); i += (int64_t)gridDim.x * blockDim.x)
 
@@ -113,7 +86,7 @@ __global__ void __launch_bounds__(WD_RED_THREADS) k_norm2(const double2 *__restr
         s = fma(v.x, v.x, s);
         s = fma(v.y, v.y, s);
     }
-    block_partial(s, 0.0, partial);
+    wd_block_partial(s, partial);
 }
 
 __global__ void __launch_bounds__(WD_RED_THREADS) k_dot(const double2 *__restrict__ a, const double2 *__restrict__ b,
@@ -128,7 +101,7 @@ __global__ void __launch_bounds__(WD_RED_THREADS) k_dot(const double2 *__restric
         im = fma(u.x, v.y, im);
         im = fma(-u.y, v.x, im);
     }
-    block_partial(re, im, partial);
+    wd_block_partial(re, im, partial);
 }
 
 __global__ void __launch_bounds__(WD_RED_THREADS) k_norm2_df(const float4 *__restrict__ a, int64_t n, double2 *partial)
@@ -139,7 +112,7 @@ __global__ void __launch_bounds__(WD_RED_THREADS) k_norm2_df(const float4 *__res
         const dfc v = df_from_f4(a[i]);
         s = df_madd(df_madd(s, v.re, v.re), v.im, v.im);
     }
-    block_partial(df_value(s), 0.0, partial);
+    wd_block_partial(df_value(s), partial);
 }
 
 __global__ void __launch_bounds__(WD_RED_THREADS) k_dot_df(const float4 *__restrict__ a, const float4 *__restrict__ b,
@@ -147,7 +120,7 @@ __global__ void __launch_bounds__(WD_RED_THREADS) k_dot_df(const float4 *__restr
 {
     dfc s = c_zero(dfc());
     GRID_STRIDE(i, n) { s = c_maddc(s, df_from_f4(a[i]), df_from_f4(b[i])); }
-    block_partial(df_value(s.re), df_value(s.im), partial);
+    wd_block_partial(df_value(s.re), df_value(s.im), partial);
 }
 
 // One block of 1024 threads folds WD_RED_BLOCKS partials into *result.
@@ -159,8 +132,8 @@ __global__ void __launch_bounds__(1024) k_red_finish(const double2 *__restrict__
         a += partial[i].x;
         b += partial[i].y;
     }
-    a = warp_sum(a);
-    b = warp_sum(b);
+    a = wd_warp_sum(a);
+    b = wd_warp_sum(b);
     const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
     if (l == 0) {
         sa[w] = a;
@@ -170,8 +143,8 @@ __global__ void __launch_bounds__(1024) k_red_finish(const double2 *__restrict__
     if (w == 0) {
         a = l < (int)(blockDim.x >> 5) ? sa[l] : 0.0;
         b = l < (int)(blockDim.x >> 5) ? sb[l] : 0.0;
-        a = warp_sum(a);
-        b = warp_sum(b);
+        a = wd_warp_sum(a);
+        b = wd_warp_sum(b);
         if (l == 0) *result = make_double2(a, b);
     }
 }
@@ -210,32 +183,7 @@ __global__ void k_scale(double a, const double2 *__restrict__ x, double2 *__rest
     }
 }
 
-// x += alpha p; r -= alpha q; partial |r|^2  (src/invert.cpp:89-107 fused)
-__global__ void __launch_bounds__(WD_RED_THREADS) k_cg_update(double2 alpha, const double2 *__restrict__ p,
-                                                              const double2 *__restrict__ q, double2 *__restrict__ x,
-                                                              double2 *__restrict__ r, int64_t n, double2 *partial)
-{
-    double s = 0.0;
-    GRID_STRIDE(i, n)
-    {
-        const double2 pv = p[i], qv = q[i];
-        double2 xv = x[i], rv = r[i];
-        const double2 ap = cmul(alpha, pv), aq = cmul(alpha, qv);
-        xv.x += ap.x;
-        xv.y += ap.y;
-        rv.x -= aq.x;
-        rv.y -= aq.y;
-        x[i] = xv;
-        r[i] = rv;
-        s = fma(rv.x, rv.x, s);
-        s = fma(rv.y, rv.y, s);
-    }
-    block_partial(s, 0.0, partial);
-}
-
-// Real-scalar forms for the even-odd CG, whose alpha and beta are real
-// (ratios of norms): one FMA per real instead of a complex product.
-// y = x + b y
+// y = x + b y, b real
 __global__ void k_xpby_real(const double2 *__restrict__ x, double b, double2 *__restrict__ y, int64_t n)
 {
     GRID_STRIDE(i, n)
@@ -243,27 +191,6 @@ __global__ void k_xpby_real(const double2 *__restrict__ x, double b, double2 *__
         const double2 u = x[i], v = y[i];
         y[i] = make_double2(fma(b, v.x, u.x), fma(b, v.y, u.y));
     }
-}
-
-// x += alpha p; r -= alpha q; partial |r|^2
-__global__ void __launch_bounds__(WD_RED_THREADS) k_cg_update_real(double alpha, const double2 *__restrict__ p,
-                                                                   const double2 *__restrict__ q,
-                                                                   double2 *__restrict__ x, double2 *__restrict__ r,
-                                                                   int64_t n, double2 *partial)
-{
-    double s = 0.0;
-    GRID_STRIDE(i, n)
-    {
-        const double2 pv = p[i], qv = q[i];
-        double2 xv = x[i], rv = r[i];
-        xv = make_double2(fma(alpha, pv.x, xv.x), fma(alpha, pv.y, xv.y));
-        rv = make_double2(fma(-alpha, qv.x, rv.x), fma(-alpha, qv.y, rv.y));
-        x[i] = xv;
-        r[i] = rv;
-        s = fma(rv.x, rv.x, s);
-        s = fma(rv.y, rv.y, s);
-    }
-    block_partial(s, 0.0, partial);
 }
 
 // ----------------------------------------------------- double-float BLAS
@@ -286,42 +213,6 @@ __global__ void k_xpby_real_df(const float4 *__restrict__ x, dfr b, float4 *__re
         const dfc u = df_from_f4(x[i]), v = df_from_f4(y[i]);
         y[i] = df_to_f4(dfc{df_madd(u.re, b, v.re), df_madd(u.im, b, v.im)});
     }
-}
-
-__global__ void __launch_bounds__(WD_RED_THREADS) k_cg_update_real_df(dfr alpha, dfr malpha,
-                                                                      const float4 *__restrict__ p,
-                                                                      const float4 *__restrict__ q,
-                                                                      float4 *__restrict__ x, float4 *__restrict__ r,
-                                                                      int64_t n, double2 *partial)
-{
-    dfr s{0.f, 0.f};
-    GRID_STRIDE(i, n)
-    {
-        const dfc pv = df_from_f4(p[i]), qv = df_from_f4(q[i]);
-        dfc xv = df_from_f4(x[i]), rv = df_from_f4(r[i]);
-        xv = dfc{df_madd(xv.re, alpha, pv.re), df_madd(xv.im, alpha, pv.im)};
-        rv = dfc{df_madd(rv.re, malpha, qv.re), df_madd(rv.im, malpha, qv.im)};
-        x[i] = df_to_f4(xv);
-        r[i] = df_to_f4(rv);
-        s = df_madd(df_madd(s, rv.re, rv.re), rv.im, rv.im);
-    }
-    block_partial(df_value(s), 0.0, partial);
-}
-
-__global__ void __launch_bounds__(WD_RED_THREADS) k_cg_update_df(dfc alpha, dfc malpha, const float4 *__restrict__ p,
-                                                                 const float4 *__restrict__ q, float4 *__restrict__ x,
-                                                                 float4 *__restrict__ r, int64_t n, double2 *partial)
-{
-    dfr s{0.f, 0.f};
-    GRID_STRIDE(i, n)
-    {
-        const dfc xv = c_madd(df_from_f4(x[i]), alpha, df_from_f4(p[i]));
-        const dfc rv = c_madd(df_from_f4(r[i]), malpha, df_from_f4(q[i]));
-        x[i] = df_to_f4(xv);
-        r[i] = df_to_f4(rv);
-        s = df_madd(df_madd(s, rv.re, rv.re), rv.im, rv.im);
-    }
-    block_partial(df_value(s), 0.0, partial);
 }
 
 inline int blas_blocks(int64_t n)
@@ -445,14 +336,6 @@ wd_status wd_blas_scale(wd_context *ctx, double a, const double2 *x, double2 *y,
     return WD_OK;
 }
 
-wd_status wd_blas_cg_update(wd_context *ctx, double2 alpha, const double2 *p, const double2 *q, double2 *x,
-                            double2 *r, int64_t n, int slot)
-{
-    k_cg_update<<<WD_RED_BLOCKS, WD_RED_THREADS, 0, ctx->stream>>>(alpha, p, q, x, r, n, (double2 *)ctx->red_partial);
-    WD_LAUNCHED(ctx);
-    return wd_red_finish(ctx, slot);
-}
-
 // ------------------------------------------- precision-dispatched BLAS
 static wd_status same_prec(wd_context *ctx, std::initializer_list<WdVec> v)
 {
@@ -507,20 +390,6 @@ wd_status wd_v_xpayz(wd_context *ctx, WdVec x, double2 a, WdVec y, WdVec z, int6
     return WD_OK;
 }
 
-wd_status wd_v_cg_update(wd_context *ctx, double2 alpha, WdVec p, WdVec q, WdVec x, WdVec r, int64_t n, int slot)
-{
-    wd_status st = same_prec(ctx, {p, q, x, r});
-    if (st != WD_OK) return st;
-    if (p.prec == WD_PREC_F64)
-        return wd_blas_cg_update(ctx, alpha, (const double2 *)p.p, (const double2 *)q.p, (double2 *)x.p,
-                                 (double2 *)r.p, n, slot);
-    k_cg_update_df<<<WD_RED_BLOCKS, WD_RED_THREADS, 0, ctx->stream>>>(
-        dfc_split(alpha), dfc_split(make_double2(-alpha.x, -alpha.y)), (const float4 *)p.p, (const float4 *)q.p,
-        (float4 *)x.p, (float4 *)r.p, n, (double2 *)ctx->red_partial);
-    WD_LAUNCHED(ctx);
-    return wd_red_finish(ctx, slot);
-}
-
 wd_status wd_v_xpby(wd_context *ctx, WdVec x, double b, WdVec y, int64_t n)
 {
     wd_status st = same_prec(ctx, {x, y});
@@ -531,22 +400,6 @@ wd_status wd_v_xpby(wd_context *ctx, WdVec x, double b, WdVec y, int64_t n)
         k_xpby_real_df<<<blas_blocks(n), 256, 0, ctx->stream>>>((const float4 *)x.p, df_split(b), (float4 *)y.p, n);
     WD_LAUNCHED(ctx);
     return WD_OK;
-}
-
-wd_status wd_v_cg_update_real(wd_context *ctx, double alpha, WdVec p, WdVec q, WdVec x, WdVec r, int64_t n, int slot)
-{
-    wd_status st = same_prec(ctx, {p, q, x, r});
-    if (st != WD_OK) return st;
-    double2 *part = (double2 *)ctx->red_partial;
-    if (p.prec == WD_PREC_F64)
-        k_cg_update_real<<<WD_RED_BLOCKS, WD_RED_THREADS, 0, ctx->stream>>>(
-            alpha, (const double2 *)p.p, (const double2 *)q.p, (double2 *)x.p, (double2 *)r.p, n, part);
-    else
-        k_cg_update_real_df<<<WD_RED_BLOCKS, WD_RED_THREADS, 0, ctx->stream>>>(
-            df_split(alpha), df_split(-alpha), (const float4 *)p.p, (const float4 *)q.p, (float4 *)x.p,
-            (float4 *)r.p, n, part);
-    WD_LAUNCHED(ctx);
-    return wd_red_finish(ctx, slot);
 }
 
 wd_status wd_v_copy(wd_context *ctx, WdVec dst, WdVec src, int64_t n)

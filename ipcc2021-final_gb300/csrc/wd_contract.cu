@@ -46,7 +46,7 @@ __global__ void __launch_bounds__(WD_RED_THREADS) k_slice_density(Props P, WdGeo
             }
         }
     }
-    wd_block_partial(acc, 0.0, partial);
+    wd_block_partial(acc, partial);
 }
 
 __global__ void k_slice_finish(const double2 *partial, int Lt, int per_slice, double *ct)

@@ -48,6 +48,7 @@ struct SplitDF {
     const float4 *__restrict__ x;
     float4 *__restrict__ out;
     dfr alpha, beta;
+    const int *stop = nullptr;  // device gate: the launch is a no-op while *stop != 0
 };
 
 __device__ __forceinline__ dfc shfl_dfc(const dfc &v, int src)
@@ -136,6 +137,7 @@ __device__ __forceinline__ SplitCtx split_ctx(const SplitDF &p)
 template <bool DAG, int WARPS>
 __global__ void __launch_bounds__(32 * WARPS) k_hop_df_pipe(const SplitDF p)
 {
+    if (p.stop && *p.stop) return;
     const SplitCtx x = split_ctx<WARPS>(p);
     dfc acc[4];
 #pragma unroll
@@ -313,6 +315,7 @@ __device__ __forceinline__ void df_staged_site(const SplitDF &p, const SplitCtx 
 template <bool DAG, int WARPS, int LOOK, int NS, bool LCG>
 __global__ void __launch_bounds__(32 * WARPS) k_hop_df_staged(const SplitDF p)
 {
+    if (p.stop && *p.stop) return;
     const SplitCtx x = split_ctx<WARPS>(p);
     dfp acc[4];
     df_staged_site<DAG, WARPS, LOOK, NS, LCG>(p, x, acc);
@@ -414,6 +417,7 @@ __device__ __forceinline__ void df_group_site(const SplitDF &p, const SplitCtx &
 template <bool DAG, int GROUPS, bool LCG, int MINB>
 __global__ void __launch_bounds__(96 * GROUPS, MINB) k_hop_df_grouped(const SplitDF p)
 {
+    if (p.stop && *p.stop) return;
     const SplitCtx x = group_ctx<GROUPS>(p);
     dfp acc[4];
     df_group_site<DAG, GROUPS, LCG>(p, x, acc);
@@ -482,7 +486,7 @@ int conv_blocks(int64_t n)
 }  // namespace
 
 wd_status wd_hop_df(wd_context *ctx, const wd_lattice *lat, const float4 *in_block, float4 *out_block,
-                    const float4 *x_block, int cb, int dag, double alpha, double beta)
+                    const float4 *x_block, int cb, int dag, double alpha, double beta, const int *stop)
 {
     wd_status st = wd_lattice_gauge_df(ctx, lat);
     if (st != WD_OK) return st;
@@ -495,6 +499,7 @@ wd_status wd_hop_df(wd_context *ctx, const wd_lattice *lat, const float4 *in_blo
     p.out = out_block;
     p.alpha = df_split(alpha);
     p.beta = df_split(beta);
+    p.stop = stop;
     auto run_pipe = [&](auto warps) -> wd_status {
         constexpr int W = decltype(warps)::value;
         const int sites_per_block = kSitesPerWarp * W;

@@ -66,8 +66,7 @@ wd_status wd_hop_hi_residual(wd_context *ctx, const wd_lattice *lat, WdVec in, W
     if (in.prec != WD_PREC_F64) return wd_fail(ctx, WD_ERR_BAD_ARG, "residual hop: FP64 or double-float storage");
     const WdResSink r{(const double2 *)bhat.p, (float4 *)s32.p, partial, counter, result};
     if (lat->gauge_fix)
-        return wd_hop_fix_residual(ctx, lat, (const double2 *)in.p, (const double2 *)x.p, -0.25 / a, a, r,
-                                   wd_tune_choice(ctx, "hop_f64", lat->g.Vh));
+        return wd_hop_fix_residual(ctx, lat, (const double2 *)in.p, (const double2 *)x.p, -0.25 / a, a, r);
     auto run = [&](auto tag) -> wd_status {
         using P = HopF64<decltype(tag)::value>;
         P p;
@@ -120,13 +119,9 @@ wd_status wd_hop_f64_aos_range(wd_context *ctx, cudaStream_t stream, const wd_la
 
 wd_status wd_hop_f64(wd_context *ctx, const wd_lattice *lat, const double2 *in_block,
                      double2 *out_block, const double2 *x_block, int cb, int dag, double alpha,
-                     double beta)
+                     double beta, const int *stop)
 {
-    // fixed point where the links allow it; variants: 128, 64, 32 threads per block
-    if (lat->gauge_fix)
-        return wd_tune_launch(ctx, "hop_f64", lat->g.Vh, 3, [&](int v) {
-            return wd_hop_fix(ctx, lat, in_block, out_block, x_block, cb, dag, alpha, beta, v);
-        });
+    if (lat->gauge_fix) return wd_hop_fix(ctx, lat, in_block, out_block, x_block, cb, dag, alpha, beta, stop);
     auto run = [&](auto tag) -> wd_status {
         using P = HopF64<decltype(tag)::value>;
         P p;
@@ -139,6 +134,7 @@ wd_status wd_hop_f64(wd_context *ctx, const wd_lattice *lat, const double2 *in_b
         p.alpha = alpha;
         p.beta = beta;
         p.scale = F64Scale::make(alpha);
+        p.stop = stop;
         const int blocks = (lat->g.Vh + P::kThreads - 1) / P::kThreads;
         if (dag) wd_hop_kernel<true><<<blocks, P::kThreads, 0, ctx->stream>>>(p);
         else wd_hop_kernel<false><<<blocks, P::kThreads, 0, ctx->stream>>>(p);

@@ -3,6 +3,8 @@
 #include "wd_fix.cuh"
 #include "wd_kernels.h"
 #include "wd_reduce.cuh"
+#include "wd_solver.h"
+#include "wd_tune.h"
 
 namespace {
 
@@ -48,87 +50,230 @@ __global__ void __launch_bounds__(256) k_gauge_in(const double2 *__restrict__ ao
     }
 }
 
-template <class Base>
-struct HopFix : Base {
-    const int4 *__restrict__ links;
+struct FixArgs {
+    WdGeom g;
+    int cb;                // output parity (of the first blocks when both parities run)
+    const double2 *in;     // source parity block; whole field when both parities run, as x and out
+    const double2 *gauge;  // FP64 links, for the sites that need them
+    const double2 *x;
+    double2 *out;
+    const int4 *links;
+    double alpha, beta;
+    F64Scale scale;
+    const int *stop;
+};
+// One block's parity: its operand pointers
+struct FixView {
+    int cb;
+    const double2 *in, *x;
+    double2 *out;
 };
 
 // The FP64-pipe arithmetic for a site whose values do not fit a block scale
-template <bool DAG, class P>
-__device__ __noinline__ void f64_route(const P &p, int s)
+template <bool DAG, bool AOS>
+__device__ __noinline__ void f64_route(const FixArgs &a, const FixView &w, int s, double2 *acc)
 {
-    double2 acc[12];
+    std::conditional_t<AOS, HopF64AoS<128>, HopF64<128>> p;
+    p.g = a.g;
+    p.cb = w.cb;
+    p.in = w.in;
+    p.gauge = a.gauge;
     wd_hop_site<DAG>(p, s, acc);
-    p.epilogue(s, acc);
 }
 
-// Output sites [s_lo, s_hi), two threads a site
-template <bool DAG, class P, int T>
-__global__ void __launch_bounds__(T, 512 / T) k_hop_fix(const __grid_constant__ P p, int s_lo, int s_hi)
+template <bool AOS>
+__device__ __forceinline__ size_t entry(const FixArgs &a, int c, int s)
 {
-    extern __shared__ __align__(16) char smem[];
-    const int id = blockIdx.x * T + threadIdx.x, half = id & 1;
-    const int s0 = s_lo + (id >> 1), s = s0 < s_hi ? s0 : s_hi - 1;
-    double2 up[3], low[3];
-    const bool ok = wd_fix::site<DAG>(p, *reinterpret_cast<wd_fix::Stage<T> *>(smem), s, half, up, low);
-    if (s0 >= s_hi) return;
-    if (ok) {
-        p.store_spin(s, half, up);
-        p.store_spin(s, 3 - half, low);
-    } else if (half == 0) {
-        f64_route<DAG>(p, s);
+    return AOS ? (size_t)s * 12 + c : (size_t)c * a.g.Vh + s;
+}
+// alpha v + beta x; a power-of-two alpha is exact on the exponent, which
+// leaves one FP64 operation per real (and one rounding) instead of two
+__device__ __forceinline__ double2 hop_value(const FixArgs &a, const FixView &w, size_t i, double2 v)
+{
+    if (!w.x) return a.scale.apply(v);
+    const double2 x = w.x[i];
+    if (a.scale.mode == 0) return c_axpby(a.alpha, v, a.beta, x);
+    v = a.scale.apply(v);
+    return make_double2(fma(a.beta, x.x, v.x), fma(a.beta, x.y, v.y));
+}
+
+// ---- epilogues: put() takes each component's hopping sum v at entry i of the
+// output parity block, finish() the sums of what put() returned in n
+template <bool AOS_>
+struct EpiStore {
+    static constexpr bool AOS = AOS_;
+    static constexpr int N = 0;
+    __device__ __forceinline__ void put(const FixArgs &a, const FixView &w, int c, int s, double2 v, double *) const
+    {
+        const size_t i = entry<AOS>(a, c, s);
+        w.out[i] = hop_value(a, w, i, v);
     }
-}
-
-template <class P>
-__device__ __noinline__ void f64_route_acc(const P &p, int s, double2 *acc)
-{
-    wd_hop_site<false>(p, s, acc);
-}
-
+};
+// t stored, |t|^2 -> alpha
+struct EpiNorm {
+    static constexpr bool AOS = false;
+    static constexpr int N = 1;
+    WdCgDev *dev;
+    double *partial;
+    __device__ __forceinline__ unsigned *counter() const { return &dev->count_a; }
+    __device__ __forceinline__ void put(const FixArgs &a, const FixView &w, int c, int s, double2 v, double *n) const
+    {
+        const size_t i = entry<false>(a, c, s);
+        const double2 o = hop_value(a, w, i, v);
+        w.out[i] = o;
+        n[0] = fma(o.x, o.x, fma(o.y, o.y, n[0]));
+    }
+    __device__ __forceinline__ void finish(const double *t) const { wd_cg_set_alpha(dev, t[0], 0.0, false); }
+};
+// q not stored: r -= alpha q, y += alpha p, |r|^2 -> beta or the gate
+struct EpiUpdate {
+    static constexpr bool AOS = false;
+    static constexpr int N = 1;
+    WdCgDev *dev;
+    double *partial;
+    const double2 *p;
+    double2 *r, *y;
+    __device__ __forceinline__ unsigned *counter() const { return &dev->count_r; }
+    __device__ __forceinline__ void put(const FixArgs &a, const FixView &w, int c, int s, double2 v, double *n) const
+    {
+        const size_t i = entry<false>(a, c, s);
+        const double al = dev->are;
+        const double2 q = hop_value(a, w, i, v), pv = p[i];
+        double2 rv = r[i], yv = y[i];
+        rv = make_double2(fma(-al, q.x, rv.x), fma(-al, q.y, rv.y));
+        yv = make_double2(fma(al, pv.x, yv.x), fma(al, pv.y, yv.y));
+        r[i] = rv;
+        y[i] = yv;
+        n[0] = fma(rv.x, rv.x, fma(rv.y, rv.y, n[0]));
+    }
+    __device__ __forceinline__ void finish(const double *t) const { wd_cg_set_beta(dev, t[0]); }
+};
+// q stored, (p, q) -> alpha; p is a whole field
+struct EpiDot {
+    static constexpr bool AOS = false;
+    static constexpr int N = 2;
+    WdCgDev *dev;
+    double *partial;
+    const double2 *p;
+    __device__ __forceinline__ unsigned *counter() const { return &dev->count_a; }
+    __device__ __forceinline__ void put(const FixArgs &a, const FixView &w, int c, int s, double2 v, double *n) const
+    {
+        const size_t i = entry<false>(a, c, s);
+        const double2 q = hop_value(a, w, i, v), u = p[(size_t)w.cb * 12 * a.g.Vh + i];
+        w.out[i] = q;
+        n[0] = fma(u.x, q.x, fma(u.y, q.y, n[0]));
+        n[1] = fma(u.x, q.y, fma(-u.y, q.x, n[1]));
+    }
+    __device__ __forceinline__ void finish(const double *t) const { wd_cg_set_alpha(dev, t[0], t[1], true); }
+};
 // The reliable update's second Schur hop fused with the true residual (as
 // k_hop_f64_res): s = bhat - (alpha acc + beta x) in FP64, rounded to FP32
-// into s32 (plane c/2, half c&1 of the float4 for component c), |s32|^2
-// reduced over the grid.
-template <class P, int T>
-__global__ void __launch_bounds__(T, 512 / T) k_hop_fix_res(const __grid_constant__ P p, const WdResSink r)
+// into s32 (plane c/2, half c&1 of the float4 for component c), |s32|^2.
+struct EpiRes {
+    static constexpr bool AOS = false;
+    static constexpr int N = 1;
+    WdResSink r;
+    double *partial;
+    __device__ __forceinline__ unsigned *counter() const { return r.counter; }
+    __device__ __forceinline__ void put(const FixArgs &a, const FixView &w, int c, int s, double2 v, double *n) const
+    {
+        const size_t i = entry<false>(a, c, s);
+        const double2 o = hop_value(a, w, i, v), b = r.bhat[i];
+        const float2 f = make_float2((float)(b.x - o.x), (float)(b.y - o.y));
+        reinterpret_cast<float2 *>(r.s32 + (size_t)(c >> 1) * a.g.Vh + s)[c & 1] = f;
+        n[0] += (double)fmaf(f.x, f.x, f.y * f.y);
+    }
+    __device__ __forceinline__ void finish(const double *t) const { *r.result = t[0]; }
+};
+
+// 512 threads per SM (128 registers each).  Output sites [s_lo, s_hi).  T > 0: T threads a block, two a site; T = 0: the
+// form with a direction pair per warp, 16 sites a block.  gridDim.y = 2 runs
+// both parities (s_lo = 0, s_hi = Vh).
+constexpr int block_threads(int T) { return T ? T : 128; }
+template <bool DAG, int T, class Epi>
+__global__ void __launch_bounds__(block_threads(T), 512 / block_threads(T))
+    k_hop_fix(const __grid_constant__ FixArgs a, const __grid_constant__ Epi epi, int s_lo, int s_hi)
 {
+    if (a.stop && *a.stop) return;
+    constexpr bool AOS = Epi::AOS;
+    constexpr int B = block_threads(T);
     extern __shared__ __align__(16) char smem[];
-    const int id = blockIdx.x * T + threadIdx.x, half = id & 1;
-    const int s0 = id >> 1, Vh = p.g.Vh, s = s0 < Vh ? s0 : Vh - 1;
+    FixView w{a.cb, a.in, a.x, a.out};
+    if (gridDim.y == 2) {
+        const size_t half_field = (size_t)12 * a.g.Vh;
+        w.cb = a.cb ^ blockIdx.y;
+        w.in += (1 - w.cb) * half_field;
+        w.x += w.cb * half_field;
+        w.out += w.cb * half_field;
+    }
+    const wd_fix::Operands<AOS> p{a.g, w.cb, w.in, a.links};
+    const int l = threadIdx.x & 31, half = l & 1;
+    const int s0 = s_lo + (T ? (int)(blockIdx.x * B + threadIdx.x) >> 1 : (int)blockIdx.x * 16 + (l >> 1));
+    const int s = s0 < s_hi ? s0 : s_hi - 1;
     double2 v[6];
-    const bool ok = wd_fix::site<false>(p, *reinterpret_cast<wd_fix::Stage<T> *>(smem), s, half, v, v + 3);
-    float n = 0.f;
-    if (s0 < Vh) {
+    bool ok;
+    if constexpr (T > 0) ok = wd_fix::site<DAG>(p, *reinterpret_cast<wd_fix::Stage<B> *>(smem), s, half, v);
+    else ok = wd_fix::site_split<DAG>(p, *reinterpret_cast<wd_fix::Split *>(smem), s, half, v);
+    double n[Epi::N ? Epi::N : 1] = {};
+    const int warp = threadIdx.x >> 5;  // split form: warps 0-2 hold colour `warp` of the two spins
+    if (s0 < s_hi && (T > 0 || warp < 3)) {
         if (!ok) {
             double2 acc[12];
-            f64_route_acc(p, s, acc);
-            for (int k = 0; k < 3; ++k) {
-                v[k] = acc[half * 3 + k];
-                v[3 + k] = acc[(3 - half) * 3 + k];
+            f64_route<DAG, AOS>(a, w, s, acc);
+#pragma unroll
+            for (int k = 0; k < (T ? 6 : 2); ++k) {
+                const int spin = k < (T ? 3 : 1) ? half : 3 - half;
+                v[k] = acc[spin * 3 + (T ? k % 3 : warp)];
             }
         }
 #pragma unroll
-        for (int k = 0; k < 6; ++k) {
-            const int c = (k < 3 ? half : 3 - half) * 3 + k % 3;
-            const size_t i = (size_t)c * Vh + s;
-            const double2 o = c_axpby(p.alpha, v[k], p.beta, p.x[i]), b = r.bhat[i];
-            const float2 f = make_float2((float)(b.x - o.x), (float)(b.y - o.y));
-            reinterpret_cast<float2 *>(r.s32 + (size_t)(c >> 1) * Vh + s)[c & 1] = f;
-            n = fmaf(f.x, f.x, fmaf(f.y, f.y, n));
+        for (int k = 0; k < (T ? 6 : 2); ++k) {
+            const int spin = k < (T ? 3 : 1) ? half : 3 - half;
+            epi.put(a, w, spin * 3 + (T ? k % 3 : warp), s, v[k], n);
         }
     }
-    double tot;
-    if (wd_grid_sum<T>((double)n, r.partial, r.counter, &tot)) *r.result = tot;
+    if constexpr (Epi::N > 0) {
+        double t[Epi::N];
+        if (wd_grid_sum_n<B, Epi::N>(n, epi.partial, epi.counter(), t)) epi.finish(t);
+    }
 }
 
-// launch shapes of the plain and the residual hop: threads per block
-template <class Run>
-wd_status with_threads(int variant, Run run)
+// A launch over up to this many output sites takes the form with a direction
+// pair per warp: there the chip has warps to spare and the time is one
+// thread's chain (us per hop, split / not: 6.2 / 10.3 up to 512 sites, 8.2 /
+// 10.3 at 2048 and 4096, 10.3 / 10.3 at 8192, 16.4 / 14.3 at 16384).
+constexpr int kSplitSites = 8192;
+
+template <bool DAG, int T, class Epi>
+void launch_fix(cudaStream_t stream, const FixArgs &a, const Epi &epi, bool both, int s_lo, int s_hi)
 {
-    if (variant == 1) return run(std::integral_constant<int, 64>());
-    if (variant == 2) return run(std::integral_constant<int, 32>());
-    return run(std::integral_constant<int, 128>());
+    constexpr int B = T ? T / 2 : 16;  // sites a block
+    constexpr size_t sm = T ? sizeof(wd_fix::Stage<T ? T : 128>) : sizeof(wd_fix::Split);
+    const dim3 grid((unsigned)((s_hi - s_lo + B - 1) / B), both ? 2 : 1);
+    k_hop_fix<DAG, T, Epi><<<grid, T ? T : 128, sm, stream>>>(a, epi, s_lo, s_hi);
+}
+
+// launch shapes of the form with two threads a site: 128, 64, 32 threads a
+// block; 128 with a reduction (fewest block sums: at 16^3x32 the update hop
+// took 56 us with 32)
+template <bool DAG, class Epi>
+wd_status run_fix(wd_context *ctx, const FixArgs &a, const Epi &epi, bool both, int variant)
+{
+    const int Vh = a.g.Vh;
+    if ((both ? 2 : 1) * Vh <= kSplitSites) launch_fix<DAG, 0>(ctx->stream, a, epi, both, 0, Vh);
+    else if (Epi::N > 0) launch_fix<DAG, 128>(ctx->stream, a, epi, both, 0, Vh);
+    else if (variant == 1) launch_fix<DAG, 64>(ctx->stream, a, epi, both, 0, Vh);
+    else if (variant == 2) launch_fix<DAG, 32>(ctx->stream, a, epi, both, 0, Vh);
+    else launch_fix<DAG, 128>(ctx->stream, a, epi, both, 0, Vh);
+    WD_LAUNCHED(ctx);
+    return WD_OK;
+}
+
+FixArgs fix_args(const wd_lattice *lat, const void *in, void *out, const void *x, int cb, double alpha, double beta,
+                 const int *stop = nullptr)
+{
+    return FixArgs{lat->g, cb, (const double2 *)in, lat->gauge, (const double2 *)x, (double2 *)out,
+                   (const int4 *)lat->gauge_fix, alpha, beta, F64Scale::make(alpha), stop};
 }
 
 }  // namespace
@@ -142,65 +287,74 @@ wd_status wd_gauge_ref_to_soa_fix(wd_context *ctx, const WdGeom &g, int mu, cons
     return WD_OK;
 }
 
-template <class Base>
-static HopFix<Base> make_fix(const wd_lattice *lat, const double2 *in, double2 *out, const double2 *x,
-                             int cb, double alpha, double beta)
+wd_status wd_hop_fix(wd_context *ctx, const wd_lattice *lat, const double2 *in, double2 *out, const double2 *x, int cb,
+                     int dag, double alpha, double beta, const int *stop)
 {
-    HopFix<Base> p;
-    p.g = lat->g;
-    p.cb = cb;
-    p.in = in;
-    p.gauge = lat->gauge;
-    p.x = x;
-    p.out = out;
-    p.alpha = alpha;
-    p.beta = beta;
-    p.scale = F64Scale::make(alpha);
-    p.links = (const int4 *)lat->gauge_fix;
-    return p;
+    const FixArgs a = fix_args(lat, in, out, x, cb, alpha, beta, stop);
+    auto run = [&](int v) {
+        return dag ? run_fix<true>(ctx, a, EpiStore<false>(), false, v) : run_fix<false>(ctx, a, EpiStore<false>(), false, v);
+    };
+    if (lat->g.Vh <= kSplitSites) {
+        wd_tune_note("hop_f64", 3);
+        return run(0);
+    }
+    return wd_tune_launch(ctx, "hop_f64", lat->g.Vh, 3, run);
 }
 
-wd_status wd_hop_fix(wd_context *ctx, const wd_lattice *lat, const double2 *in, double2 *out,
-                     const double2 *x, int cb, int dag, double alpha, double beta, int variant)
+wd_status wd_hop_fix_M(wd_context *ctx, const wd_lattice *lat, const double2 *in, double2 *out, double mass, int dag,
+                       const int *stop)
 {
-    const auto p = make_fix<HopF64<128>>(lat, in, out, x, cb, alpha, beta);
-    using P = std::decay_t<decltype(p)>;
-    return with_threads(variant, [&](auto t) -> wd_status {
-        constexpr int T = decltype(t)::value;
-        constexpr size_t sm = sizeof(wd_fix::Stage<T>);
-        const int blocks = (int)(((int64_t)lat->g.Vh * 2 + T - 1) / T);
-        if (dag) k_hop_fix<true, P, T><<<blocks, T, sm, ctx->stream>>>(p, 0, lat->g.Vh);
-        else k_hop_fix<false, P, T><<<blocks, T, sm, ctx->stream>>>(p, 0, lat->g.Vh);
-        WD_LAUNCHED(ctx);
-        return WD_OK;
-    });
+    const FixArgs a = fix_args(lat, in, out, in, 0, -0.5, 4.0 + mass, stop);
+    const int v = wd_tune_choice(ctx, "hop_f64", lat->g.Vh);
+    return dag ? run_fix<true>(ctx, a, EpiStore<false>(), true, v) : run_fix<false>(ctx, a, EpiStore<false>(), true, v);
 }
 
-wd_status wd_hop_fix_residual(wd_context *ctx, const wd_lattice *lat, const double2 *in,
-                              const double2 *x, double alpha, double beta, const WdResSink &r, int variant)
+wd_status wd_hop_fix_residual(wd_context *ctx, const wd_lattice *lat, const double2 *in, const double2 *x, double alpha,
+                              double beta, const WdResSink &r)
 {
-    const auto p = make_fix<HopF64<128>>(lat, in, nullptr, x, 0, alpha, beta);
-    using P = std::decay_t<decltype(p)>;
-    return with_threads(variant, [&](auto t) -> wd_status {
-        constexpr int T = decltype(t)::value;
-        const int blocks = (int)(((int64_t)lat->g.Vh * 2 + T - 1) / T);
-        k_hop_fix_res<P, T><<<blocks, T, sizeof(wd_fix::Stage<T>), ctx->stream>>>(p, r);
-        WD_LAUNCHED(ctx);
-        return WD_OK;
-    });
+    return run_fix<false>(ctx, fix_args(lat, in, nullptr, x, 0, alpha, beta), EpiRes{r, r.partial}, false,
+                          wd_tune_choice(ctx, "hop_f64", lat->g.Vh));
+}
+
+size_t wd_hop_fix_partials(const wd_lattice *lat) { return 2 * (2 * (size_t)lat->g.Vh / 16 + 2); }
+
+wd_status wd_hop_fix_norm(wd_context *ctx, const wd_lattice *lat, WdVec in, WdVec t, WdVec p, double mass, WdCgDev *dev,
+                          double *partial)
+{
+    const double a = 4.0 + mass;
+    return run_fix<false>(ctx, fix_args(lat, in.p, t.p, p.p, 0, -0.25 / a, a, &dev->stop), EpiNorm{dev, partial}, false,
+                          wd_tune_choice(ctx, "hop_f64", lat->g.Vh));
+}
+
+wd_status wd_hop_fix_update(wd_context *ctx, const wd_lattice *lat, WdVec in, WdVec t, WdVec p, WdVec r, WdVec x,
+                            double mass, WdCgDev *dev, double *partial)
+{
+    const double a = 4.0 + mass;
+    return run_fix<true>(ctx, fix_args(lat, in.p, nullptr, t.p, 0, -0.25 / a, a, &dev->stop),
+                         EpiUpdate{dev, partial, (const double2 *)p.p, (double2 *)r.p, (double2 *)x.p}, false,
+                         wd_tune_choice(ctx, "hop_f64", lat->g.Vh));
+}
+
+wd_status wd_hop_fix_M_dot(wd_context *ctx, const wd_lattice *lat, WdVec in, WdVec q, WdVec p, double mass, WdCgDev *dev,
+                           double *partial)
+{
+    return run_fix<true>(ctx, fix_args(lat, in.p, q.p, in.p, 0, -0.5, 4.0 + mass, &dev->stop),
+                         EpiDot{dev, partial, (const double2 *)p.p}, true,
+                         wd_tune_choice(ctx, "hop_f64", lat->g.Vh));
 }
 
 wd_status wd_hop_fix_aos_range(wd_context *ctx, cudaStream_t stream, const wd_lattice *lat, const double2 *in_aos,
-                               double2 *out_aos, const double2 *x_aos, int cb, int dag,
-                               double alpha, double beta, int s_lo, int s_hi)
+                               double2 *out_aos, const double2 *x_aos, int cb, int dag, double alpha, double beta,
+                               int s_lo, int s_hi)
 {
-    constexpr int T = 64;
-    constexpr size_t sm = sizeof(wd_fix::Stage<T>);
-    const auto p = make_fix<HopF64AoS<T>>(lat, in_aos, out_aos, x_aos, cb, alpha, beta);
-    using P = std::decay_t<decltype(p)>;
-    const int blocks = (int)(((int64_t)(s_hi - s_lo) * 2 + T - 1) / T);
-    if (dag) k_hop_fix<true, P, T><<<blocks, T, sm, stream>>>(p, s_lo, s_hi);
-    else k_hop_fix<false, P, T><<<blocks, T, sm, stream>>>(p, s_lo, s_hi);
+    const FixArgs a = fix_args(lat, in_aos, out_aos, x_aos, cb, alpha, beta);
+    auto run = [&](auto d) {
+        constexpr bool D = decltype(d)::value;
+        if (s_hi - s_lo <= kSplitSites) launch_fix<D, 0>(stream, a, EpiStore<true>(), false, s_lo, s_hi);
+        else launch_fix<D, 64>(stream, a, EpiStore<true>(), false, s_lo, s_hi);
+    };
+    if (dag) run(std::true_type());
+    else run(std::false_type());
     WD_LAUNCHED(ctx);
     return WD_OK;
 }

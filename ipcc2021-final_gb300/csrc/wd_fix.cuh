@@ -131,8 +131,23 @@ struct Stage {
     int4 link[2][9][T / 2];  // one link matrix per site
 };
 
-template <int MU, bool FWD, int T, class P>
-__device__ __forceinline__ void stage(const P &p, Stage<T> &sm, int slot, int s, const WdSite &c, int half)
+// What a hop reads: the source parity block (SoA planes, or the reference's
+// site-major layout) and the fixed-point links
+template <bool AOS>
+struct Operands {
+    WdGeom g;
+    int cb;             // output parity
+    const double2 *in;  // parity 1 - cb
+    const int4 *links;
+    __device__ __forceinline__ const double2 *spin(int s, int k) const
+    {
+        return AOS ? in + (size_t)s * 12 + k * 3 : in + (size_t)(k * 3) * g.Vh + s;
+    }
+    __device__ __forceinline__ size_t colour_stride() const { return AOS ? 1 : (size_t)g.Vh; }
+};
+
+template <int MU, bool FWD, int T, bool AOS>
+__device__ __forceinline__ void stage(const Operands<AOS> &p, Stage<T> &sm, int slot, int s, const WdSite &c, int half)
 {
     const int nb = wd_neighbour(p.g, s, c, MU, FWD), i = threadIdx.x;
     const double2 *a = p.spin(nb, half), *b = p.spin(nb, MU < 2 ? 3 - half : 2 + half);
@@ -175,8 +190,9 @@ __device__ __forceinline__ void dir(const Stage<T> &sm, int slot, int half, doub
     const uint32_t e = mb >> 20;
     if (mb < ((uint32_t)kExpTiny << 20)) {
 #pragma unroll
-        for (int k = 0; k < 3; ++k) A.tiny |= (uint32_t)(__double2hiint(h[k].x) << 1) | __double2loint(h[k].x) | (uint32_t)(__double2hiint(h[k].y) << 1) |
-                      __double2loint(h[k].y);
+        for (int k = 0; k < 3; ++k)
+            A.tiny |= (uint32_t)(__double2hiint(h[k].x) << 1) | (uint32_t)__double2loint(h[k].x) |
+                      (uint32_t)(__double2hiint(h[k].y) << 1) | (uint32_t)__double2loint(h[k].y);
     }
     if constexpr (FIRST) {
         A.E = e > (uint32_t)kExpTiny ? e : kExpTiny;
@@ -254,51 +270,128 @@ __device__ __forceinline__ double value(long long T, uint32_t E)
     return hi ? __hiloint2double(hi + (((int)E - kUnit) << 20), __double2loint(v)) : 0.0;
 }
 
-// The hopping term at site s for the thread pair (half = 0, 1): upper[] is
-// spin `half`, lower[] spin 3 - half.  Returns false when the site's values
-// need the FP64 route (then upper and lower are not to be used).
-template <bool DAG, int T, class P>
-__device__ __forceinline__ bool site(const P &p, Stage<T> &sm, int s, int half, double2 *upper, double2 *lower)
+__device__ __forceinline__ bool in_range(uint32_t E, uint32_t tiny)
+{
+    return E <= (uint32_t)kExpHigh && !(tiny && E < (uint32_t)kExpLow);
+}
+
+__device__ __forceinline__ void clear(Acc &A)
+{
+#pragma unroll
+    for (int k = 0; k < 6; ++k) A.o[k] = A.P[k] = A.Q[k] = 0;
+    A.tiny = 0;
+    A.E = kExpTiny;
+}
+
+// The hopping term at site s for the thread pair (half = 0, 1): v[0..2] is
+// spin `half`, v[3..5] spin 3 - half.  Returns false when the site's values
+// need the FP64 route (then v is not to be used).
+template <bool DAG, int T, bool AOS>
+__device__ __forceinline__ bool site(const Operands<AOS> &p, Stage<T> &sm, int s, int half, double2 *v)
 {
     const WdSite c = wd_site(p.g, s, p.cb);
     const double sigma = half ? -1.0 : 1.0;
     Acc A;
-#pragma unroll
-    for (int k = 0; k < 6; ++k) A.Q[k] = 0;
-    A.tiny = 0;
+    clear(A);
     stage<0, true, T>(p, sm, 0, s, c, half);
     // the copies of this direction have landed, and every lane has read the
     // other slot, before the next direction's copies go into it
-    auto step = [&](auto mu, auto fwd, auto slot) {
-        constexpr int MU = decltype(mu)::value, S = decltype(slot)::value;
+    auto step = [&](auto mu, auto fwd) {
+        constexpr int MU = decltype(mu)::value;
         constexpr bool FWD = decltype(fwd)::value;
+        constexpr int S = FWD ? 0 : 1;
         wd_cp_async_wait<0>();
         __syncwarp();
-        if constexpr (FWD) stage<MU, false, T>(p, sm, 1 - S, s, c, half);
-        else if constexpr (MU < 3) stage<(MU + 1) & 3, true, T>(p, sm, 1 - S, s, c, half);
+        if constexpr (FWD) stage<MU, false, T>(p, sm, 1, s, c, half);
+        else if constexpr (MU < 3) stage<(MU + 1) & 3, true, T>(p, sm, 0, s, c, half);
         dir<MU, FWD, DAG, MU == 0 && FWD, T>(sm, S, half, sigma, A);
     };
-    using F = std::true_type;
-    using B = std::false_type;
-    using S0 = std::integral_constant<int, 0>;
-    using S1 = std::integral_constant<int, 1>;
-    step(std::integral_constant<int, 0>(), F(), S0());
-    step(std::integral_constant<int, 0>(), B(), S1());
-    step(std::integral_constant<int, 1>(), F(), S0());
-    step(std::integral_constant<int, 1>(), B(), S1());
-    step(std::integral_constant<int, 2>(), F(), S0());
-    step(std::integral_constant<int, 2>(), B(), S1());
-    step(std::integral_constant<int, 3>(), F(), S0());
-    step(std::integral_constant<int, 3>(), B(), S1());
+    auto both = [&](auto mu) {
+        step(mu, std::true_type());
+        step(mu, std::false_type());
+    };
+    both(std::integral_constant<int, 0>());
+    both(std::integral_constant<int, 1>());
+    both(std::integral_constant<int, 2>());
+    both(std::integral_constant<int, 3>());
     const uint32_t tiny = A.tiny | __shfl_xor_sync(0xffffffffu, A.tiny, 1);
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
         const long long lr = A.P[2 * k] + __shfl_xor_sync(0xffffffffu, A.Q[2 * k], 1);
         const long long li = A.P[2 * k + 1] + __shfl_xor_sync(0xffffffffu, A.Q[2 * k + 1], 1);
-        upper[k] = make_double2(value(A.o[2 * k], A.E), value(A.o[2 * k + 1], A.E));
-        lower[k] = make_double2(value(lr, A.E), value(li, A.E));
+        v[k] = make_double2(value(A.o[2 * k], A.E), value(A.o[2 * k + 1], A.E));
+        v[3 + k] = make_double2(value(lr, A.E), value(li, A.E));
     }
-    return A.E <= (uint32_t)kExpHigh && !(tiny && A.E < (uint32_t)kExpLow);
+    return in_range(A.E, tiny);
+}
+
+// The same with a direction pair per warp, for lattices too small to fill the
+// chip with two threads a site: the block's four warps take mu = 0..3 of its
+// 16 sites, leave their integer sums in shared memory, and warps 0-2 add up
+// colour 0-2 of the two spins: v[0] of spin `half`, v[1] of spin 3 - half.
+struct Split {
+    Stage<128> st;
+    uint32_t E[4][32], tiny[4][32];
+    // a thread's sums (re, im): of its own spin's colour c (k = c) and lower share (k = 3 + c), in
+    // the place of its spinor copies once it has read them
+    __device__ __forceinline__ longlong2 &sum(int warp, int k, int lane)
+    {
+        return reinterpret_cast<longlong2 &>(st.spin[0][k][warp * 32 + lane]);
+    }
+};
+
+template <bool DAG, bool AOS>
+__device__ __forceinline__ bool site_split(const Operands<AOS> &p, Split &sm, int s, int half, double2 *v)
+{
+    const WdSite c = wd_site(p.g, s, p.cb);
+    const double sigma = half ? -1.0 : 1.0;
+    const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
+    auto pair = [&](auto mu) {
+        constexpr int MU = decltype(mu)::value;
+        Acc A;
+        clear(A);
+        stage<MU, true, 128>(p, sm.st, 0, s, c, half);
+        stage<MU, false, 128>(p, sm.st, 1, s, c, half);
+        wd_cp_async_wait<0>();
+        __syncwarp();
+        dir<MU, true, DAG, false, 128>(sm.st, 0, half, sigma, A);
+        dir<MU, false, DAG, false, 128>(sm.st, 1, half, sigma, A);
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            const long long *d = MU < 2 ? A.P : A.Q;
+            sm.sum(MU, k, l) = make_longlong2(A.o[2 * k], A.o[2 * k + 1]);
+            sm.sum(MU, 3 + k, l) = make_longlong2(d[2 * k], d[2 * k + 1]);
+        }
+        sm.E[MU][l] = A.E;
+        sm.tiny[MU][l] = A.tiny;
+    };
+    if (w == 0) pair(std::integral_constant<int, 0>());
+    else if (w == 1) pair(std::integral_constant<int, 1>());
+    else if (w == 2) pair(std::integral_constant<int, 2>());
+    else pair(std::integral_constant<int, 3>());
+    __syncthreads();
+    uint32_t E = 0, tiny = 0;
+#pragma unroll
+    for (int m = 0; m < 4; ++m) {
+        E = max(E, sm.E[m][l]);  // the pair's two lanes hold the same exponent
+        tiny |= sm.tiny[m][l] | sm.tiny[m][l ^ 1];
+    }
+    if (w < 3) {
+        long long t[4] = {0, 0, 0, 0};
+#pragma unroll
+        for (int m = 0; m < 4; ++m) {
+            const uint32_t d = min(E - sm.E[m][l], 63u);
+            const int j = m < 2 ? l : l ^ 1;  // the lower share of mu = 2, 3 is the partner's
+            const longlong2 a = sm.sum(m, w, l), b = sm.sum(m, 3 + w, j);
+            t[0] += a.x >> d;
+            t[1] += a.y >> d;
+            t[2] += b.x >> d;
+            t[3] += b.y >> d;
+        }
+        v[0] = make_double2(value(t[0], E), value(t[1], E));
+        v[1] = make_double2(value(t[2], E), value(t[3], E));
+    }
+    return in_range(E, tiny);
 }
 
 }  // namespace wd_fix

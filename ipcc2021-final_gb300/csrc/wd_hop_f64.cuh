@@ -57,6 +57,7 @@ struct HopF64 {
     double2 *__restrict__ out;          // parity cb block
     double alpha, beta;
     F64Scale scale;                     // alpha, applied when there is no x
+    const int *stop = nullptr;          // device gate (wd_gate_closed)
 
     __device__ __forceinline__ void load_in(int s, C *v) const
     {
@@ -68,18 +69,6 @@ struct HopF64 {
         const double2 *b = gauge + (size_t)((mu * 2 + par) * 9) * g.Vh + s;
 #pragma unroll
         for (int k = 0; k < 9; ++k) U[k] = b[(size_t)k * g.Vh];
-    }
-    // one spin's colours: the first, and the distance to the next
-    __device__ __forceinline__ const C *spin(int s, int k) const { return in + (size_t)(k * 3) * g.Vh + s; }
-    __device__ __forceinline__ size_t colour_stride() const { return (size_t)g.Vh; }
-    // one spin's three output colours from the hop's v
-    __device__ __forceinline__ void store_spin(int s, int spin, const C *v) const
-    {
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-            const size_t i = (size_t)(spin * 3 + c) * g.Vh + s;
-            out[i] = x ? c_axpby(alpha, v[c], beta, x[i]) : scale.apply(v[c]);
-        }
     }
     __device__ __forceinline__ void epilogue(int s, const C *acc) const
     {
@@ -108,16 +97,6 @@ struct HopF64AoS : HopF64<THREADS> {
         const double2 *b = this->in + (size_t)s * 12;
 #pragma unroll
         for (int c = 0; c < 12; ++c) v[c] = b[c];
-    }
-    __device__ __forceinline__ const double2 *spin(int s, int k) const { return this->in + (size_t)s * 12 + k * 3; }
-    __device__ __forceinline__ size_t colour_stride() const { return 1; }
-    __device__ __forceinline__ void store_spin(int s, int spin, const double2 *v) const
-    {
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-            const size_t i = (size_t)s * 12 + spin * 3 + c;
-            this->out[i] = this->x ? c_axpby(this->alpha, v[c], this->beta, this->x[i]) : this->scale.apply(v[c]);
-        }
     }
     __device__ __forceinline__ void epilogue(int s, const double2 *acc) const
     {

@@ -12,7 +12,7 @@
 // ---- hopping term: out_cb = alpha * D_{cb,1-cb} in_{1-cb} + beta * x_cb
 wd_status wd_hop_f64(wd_context *ctx, const wd_lattice *lat, const double2 *in_block,
                      double2 *out_block, const double2 *x_block, int cb, int dag, double alpha,
-                     double beta);
+                     double beta, const int *stop = nullptr);
 
 // ---- the FP64 hop in 64-bit fixed point (wd_dslash_fix.cu)
 // one direction's links from the reference layout into the FP64 planes and
@@ -31,13 +31,17 @@ struct WdResSink {
     unsigned *counter;
     double *result;
 };
-wd_status wd_hop_fix(wd_context *ctx, const wd_lattice *lat, const double2 *in, double2 *out,
-                     const double2 *x, int cb, int dag, double alpha, double beta, int variant);
-wd_status wd_hop_fix_residual(wd_context *ctx, const wd_lattice *lat, const double2 *in,
-                              const double2 *x, double alpha, double beta, const WdResSink &r, int variant);
+// (the lattice has gauge_fix; stop as for the other hops)
+wd_status wd_hop_fix(wd_context *ctx, const wd_lattice *lat, const double2 *in, double2 *out, const double2 *x, int cb,
+                     int dag, double alpha, double beta, const int *stop = nullptr);
+// M (or M^dag) on whole fields in one launch
+wd_status wd_hop_fix_M(wd_context *ctx, const wd_lattice *lat, const double2 *in, double2 *out, double mass, int dag,
+                       const int *stop = nullptr);
+wd_status wd_hop_fix_residual(wd_context *ctx, const wd_lattice *lat, const double2 *in, const double2 *x, double alpha,
+                              double beta, const WdResSink &r);
 wd_status wd_hop_fix_aos_range(wd_context *ctx, cudaStream_t stream, const wd_lattice *lat, const double2 *in_aos,
-                               double2 *out_aos, const double2 *x_aos, int cb, int dag,
-                               double alpha, double beta, int s_lo, int s_hi);
+                               double2 *out_aos, const double2 *x_aos, int cb, int dag, double alpha, double beta,
+                               int s_lo, int s_hi);
 
 // ---- layout conversion (reference AoS <-> device SoA), on device buffers
 // spinor: ref[(p*Vh + s)*12 + c]  <->  soa[(p*12 + c)*Vh + s] in the vector's storage format
@@ -61,15 +65,12 @@ wd_status wd_blas_axpby(wd_context *ctx, double2 a, const double2 *x, double2 b,
 // z = x + a*y     (a complex)
 wd_status wd_blas_xpayz(wd_context *ctx, const double2 *x, double2 a, const double2 *y,
                         double2 *z, int64_t n);
-// x += alpha p; r -= alpha q; slot <- |r|^2
-wd_status wd_blas_cg_update(wd_context *ctx, double2 alpha, const double2 *p, const double2 *q,
-                            double2 *x, double2 *r, int64_t n, int slot);
 // y = a*x (real a)
 wd_status wd_blas_scale(wd_context *ctx, double a, const double2 *x, double2 *y, int64_t n);
 
 // ---- double-float (df64) storage: float4 {re.h, im.h, re.l, im.l} per complex
 wd_status wd_hop_df(wd_context *ctx, const wd_lattice *lat, const float4 *in_block, float4 *out_block,
-                    const float4 *x_block, int cb, int dag, double alpha, double beta);
+                    const float4 *x_block, int cb, int dag, double alpha, double beta, const int *stop = nullptr);
 wd_status wd_convert_f64_to_df(wd_context *ctx, const double2 *in, float4 *out, int64_t n);
 wd_status wd_convert_df_to_f64(wd_context *ctx, const float4 *in, double2 *out, int64_t n);
 wd_status wd_lattice_gauge_df(wd_context *ctx, const wd_lattice *lat);
@@ -80,10 +81,8 @@ wd_status wd_v_norm2(wd_context *ctx, WdVec a, int64_t n, int slot);
 wd_status wd_v_dot(wd_context *ctx, WdVec a, WdVec b, int64_t n, int slot);
 wd_status wd_v_axpby(wd_context *ctx, double2 a, WdVec x, double2 b, WdVec y, int64_t n);
 wd_status wd_v_xpayz(wd_context *ctx, WdVec x, double2 a, WdVec y, WdVec z, int64_t n);
-wd_status wd_v_cg_update(wd_context *ctx, double2 alpha, WdVec p, WdVec q, WdVec x, WdVec r, int64_t n, int slot);
-// real-scalar forms (even-odd CG): y = x + b y; x += alpha p, r -= alpha q, |r|^2 -> slot
+// y = x + b y, b real
 wd_status wd_v_xpby(wd_context *ctx, WdVec x, double b, WdVec y, int64_t n);
-wd_status wd_v_cg_update_real(wd_context *ctx, double alpha, WdVec p, WdVec q, WdVec x, WdVec r, int64_t n, int slot);
 wd_status wd_v_copy(wd_context *ctx, WdVec dst, WdVec src, int64_t n);
 wd_status wd_v_zero(wd_context *ctx, WdVec v, int64_t n);
 
@@ -125,7 +124,7 @@ wd_status wd_spinor_ref_to_h16(wd_context *ctx, const WdGeom &g, const double2 *
 wd_status wd_spinor_h16_to_ref(wd_context *ctx, const WdGeom &g, WdVec f, double2 *ref);
 // out_cb = alpha * D_{cb,1-cb} in_{1-cb} + beta * x_cb, dispatched on the storage
 wd_status wd_hop_v(wd_context *ctx, const wd_lattice *lat, WdVec in, WdVec out, const WdVec *x, int cb, int dag,
-                   double alpha, double beta);
+                   double alpha, double beta, const int *stop = nullptr);
 
 // ---- pipelined host-buffer path: one parity block, output sites [s_lo, s_hi), given stream
 // n 16-byte entries src -> dst by a kernel on `stream` (for host memory the

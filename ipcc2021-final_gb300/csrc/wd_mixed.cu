@@ -111,7 +111,7 @@ __global__ void __launch_bounds__(WD_RED_THREADS) k_mx_norm2(SpL t, int Vh, doub
 #pragma unroll
         for (int c = 0; c < 12; ++c) acc = df_sq_acc(acc, v[c]);
     }
-    wd_block_partial(df_value(acc), 0.0, partial);
+    wd_block_partial(df_value(acc), partial);
 }
 
 // high precision -> low precision (two outputs: FP32 r_s and kernel-storage p)

@@ -11,9 +11,9 @@
 // Both run in FP64 or in double-float (prec = WD_PREC_DF64: the same
 // recurrences on float-pair vectors, ~5x faster on GB300's narrow FP64
 // pipe).  Mixed precision (FP32 / FP16 inner) lives in wd_mixed.cu.
+#include <algorithm>
 #include <chrono>
 #include <cmath>
-#include <vector>
 #include "wd_kernels.h"
 #include "wd_solver.h"
 
@@ -42,12 +42,16 @@ void WdVecBuf::release()
 static inline WdVec par_half(WdVec v, int par, int Vh) { return wd_offset(v, (int64_t)par * 12 * Vh, (int64_t)par * Vh); }
 
 // ---------------------------------------------------------------- operators
-wd_status wd_apply_M_v(wd_context *ctx, const wd_lattice *lat, WdVec in, WdVec out, double mass, int dag)
+wd_status wd_apply_M_v(wd_context *ctx, const wd_lattice *lat, WdVec in, WdVec out, double mass, int dag,
+                       const int *stop)
 {
+    if (in.prec == WD_PREC_F64 && lat->gauge_fix)
+        return wd_hop_fix_M(ctx, lat, (const double2 *)in.p, (double2 *)out.p, mass, dag, stop);
     const int Vh = lat->g.Vh;
     for (int cb = 0; cb < 2; ++cb) {
         const WdVec x = par_half(in, cb, Vh);
-        wd_status st = wd_hop_v(ctx, lat, par_half(in, 1 - cb, Vh), par_half(out, cb, Vh), &x, cb, dag, -0.5, 4.0 + mass);
+        wd_status st = wd_hop_v(ctx, lat, par_half(in, 1 - cb, Vh), par_half(out, cb, Vh), &x, cb, dag, -0.5, 4.0 + mass,
+                                stop);
         if (st != WD_OK) return st;
     }
     return WD_OK;
@@ -80,13 +84,72 @@ wd_status wd_true_residual(wd_context *ctx, const wd_lattice *lat, const double2
     return WD_OK;
 }
 
-static double2 cdiv(double2 a, double2 b)
-{
-    const double d = b.x * b.x + b.y * b.y;
-    return make_double2((a.x * b.x + a.y * b.y) / d, (a.y * b.x - a.x * b.y) / d);
-}
+namespace {
 
-static wd_status fetch1(wd_context *ctx, double2 *v) { return wd_red_fetch(ctx, 1, v); }
+// CG iterations on device scalars, queued ahead of the host.  The host
+// enqueues a few iterations, asks for a copy of the scalars, and looks at the
+// copy before last while the device works on; iterations queued past the one
+// that closed the gate are no-ops.
+struct CgLoop {
+    wd_context *ctx;
+    WdCgDev *dev = nullptr;  // device
+    WdCgDev *host;           // three pinned copies: two in flight, one for uploads
+    double *partial = nullptr;
+    void *blk = nullptr;
+    int chunk;               // iterations per look
+
+    CgLoop(wd_context *c, int Vh) : ctx(c), host((WdCgDev *)c->state_host), chunk(Vh <= 32768 ? 4 : Vh <= 524288 ? 2 : 1)
+    {
+    }
+    ~CgLoop() { wd_dev_free(ctx, blk); }
+    wd_status alloc(size_t partials)
+    {
+        wd_status st = wd_dev_alloc(ctx, &blk, 256 + partials * sizeof(double));
+        dev = (WdCgDev *)blk;
+        partial = (double *)((char *)blk + 256);
+        return st;
+    }
+    wd_status start(double rr, double target, bool strict, int iters)
+    {
+        static_assert(sizeof(WdCgDev) <= 256 && 3 * sizeof(WdCgDev) <= WD_STATE_HOST_BYTES, "device scalars");
+        host[2] = WdCgDev{};
+        host[2].rr = rr;
+        host[2].target2 = target * target;
+        host[2].strict = strict;
+        host[2].iters = iters;
+        WD_CUDA(ctx, cudaMemcpyAsync(dev, &host[2], sizeof(WdCgDev), cudaMemcpyHostToDevice, ctx->stream));
+        return WD_OK;
+    }
+    // up to `left` iterations; on return every queued one is done and *end holds the scalars
+    template <class Iteration>
+    wd_status run(int left, Iteration iteration, WdCgDev *end)
+    {
+        int looks = 0, seen = 0;  // copies asked for, and looked at
+        bool stop = false;
+        wd_status st = WD_OK;
+        while (!stop && left > 0 && st == WD_OK) {
+            const int k = chunk < left ? chunk : left;
+            for (int i = 0; i < k && st == WD_OK; ++i) st = iteration();
+            if (st != WD_OK) break;
+            left -= k;
+            WD_CUDA(ctx, cudaMemcpyAsync(&host[looks & 1], dev, sizeof(WdCgDev), cudaMemcpyDeviceToHost, ctx->stream));
+            WD_CUDA(ctx, cudaEventRecord(ctx->chunk_done[looks & 1], ctx->stream));
+            ++looks;
+            if (looks - seen == 2) {
+                WD_CUDA(ctx, cudaEventSynchronize(ctx->chunk_done[seen & 1]));
+                stop = host[seen & 1].stop != 0;
+                ++seen;
+            }
+        }
+        WD_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+        if (st == WD_OK && looks > 0) *end = host[(looks - 1) & 1];
+        return st;
+    }
+};
+
+wd_status fetch1(wd_context *ctx, double2 *v) { return wd_red_fetch(ctx, 1, v); }
+
+}  // namespace
 
 // ------------------------------------------------------- reference CGNR
 // src/invert.cpp:25-121 on full-lattice vectors of one storage (FP64 or df).
@@ -95,13 +158,17 @@ static wd_status cgnr_ref_core(wd_context *ctx, const wd_lattice *lat, WdVec src
 {
     const int64_t n = lat->volume * 12;
     const double m = prm->mass;
+    const bool fused = src.prec == WD_PREC_F64 && lat->gauge_fix;
     WdVecBuf b[5];
     for (auto &v : b) {
         wd_status s = wd_vec_alloc(ctx, v, src.prec, n);
         if (s != WD_OK) return s;
     }
     WdVec r0 = b[0].v, q = b[1].v, qq = b[2].v, p = b[3].v, Mdb = b[4].v;
-    wd_status st;
+    CgLoop loop(ctx, lat->g.Vh);
+    wd_status st = loop.alloc(std::max((size_t)2 * WD_RED_BLOCKS, wd_hop_fix_partials(lat)));
+    if (st != WD_OK) return st;
+    WdCgDev *dev = loop.dev;
     // Mdb = M^dag src; r0 = Mdb - M^dag M x   (src/invert.cpp:41-58)
     if ((st = wd_apply_M_v(ctx, lat, src, Mdb, m, 1)) != WD_OK) return st;
     if ((st = wd_apply_M_v(ctx, lat, x, qq, m, 0)) != WD_OK) return st;
@@ -110,41 +177,29 @@ static wd_status cgnr_ref_core(wd_context *ctx, const wd_lattice *lat, WdVec src
     if ((st = wd_v_norm2(ctx, r0, n, 0)) != WD_OK) return st;
     double2 red;
     if ((st = fetch1(ctx, &red)) != WD_OK) return st;
-    double rr = red.x, r1 = rr, rsd = std::sqrt(rr);
-    int iters = 0;
-    bool converged = false;
-    for (int f = 1; f < prm->max_iter; ++f) {
-        if (f == 1) {
-            if ((st = wd_v_copy(ctx, p, r0, n)) != WD_OK) return st;
+    if ((st = wd_v_copy(ctx, p, r0, n)) != WD_OK) return st;
+    if ((st = loop.start(red.x, prm->tol, true, 0)) != WD_OK) return st;
+    // qq = M p, q = M^dag qq, alpha = (r,r) / (p,q); dest += alpha p; r0 -= alpha q; |r0|^2
+    // (src/invert.cpp:77-107); beta = (r,r)_new / (r,r), p = r + beta p (:67-76)
+    auto iteration = [&]() -> wd_status {
+        wd_status e;
+        if ((e = wd_apply_M_v(ctx, lat, p, qq, m, 0, &dev->stop)) != WD_OK) return e;
+        if (fused) {
+            if ((e = wd_hop_fix_M_dot(ctx, lat, qq, q, p, m, dev, loop.partial)) != WD_OK) return e;
         } else {
-            // beta = (r,r)/r1; p = r + beta p   (src/invert.cpp:67-76)
-            if ((st = wd_v_axpby(ctx, make_double2(1.0, 0.0), r0, make_double2(rr / r1, 0.0), p, n)) != WD_OK)
-                return st;
+            if ((e = wd_apply_M_v(ctx, lat, qq, q, m, 1, &dev->stop)) != WD_OK) return e;
+            if ((e = wd_cgd_dot(ctx, p, q, n, dev, loop.partial)) != WD_OK) return e;
         }
-        if ((st = wd_apply_M_v(ctx, lat, p, qq, m, 0)) != WD_OK) return st;
-        if ((st = wd_apply_M_v(ctx, lat, qq, q, m, 1)) != WD_OK) return st;
-        r1 = rr;
-        if ((st = wd_v_dot(ctx, p, q, n, 0)) != WD_OK) return st;
-        if ((st = fetch1(ctx, &red)) != WD_OK) return st;
-        const double2 alpha = cdiv(make_double2(r1, 0.0), red);
-        // dest += alpha p; r0 -= alpha q; |r0|^2   (src/invert.cpp:84-107)
-        if ((st = wd_v_cg_update(ctx, alpha, p, q, x, r0, n, 0)) != WD_OK) return st;
-        if ((st = fetch1(ctx, &red)) != WD_OK) return st;
-        rr = red.x;
-        rsd = std::sqrt(rr);
-        iters = f;
-        if (!std::isfinite(rsd)) {
-            stats->iterations = iters;
-            return wd_fail(ctx, WD_ERR_NAN, "CG residual is not finite");
-        }
-        if (rsd < prm->tol) {
-            converged = true;
-            break;
-        }
-    }
-    stats->iterations = iters;
-    stats->residual = rsd;
-    stats->converged = converged;
+        if ((e = wd_cgd_update(ctx, true, p, q, x, r0, n, dev, loop.partial)) != WD_OK) return e;
+        return wd_cgd_xpby(ctx, r0, p, n, dev);
+    };
+    WdCgDev end{};
+    end.rr = end.rr_new = red.x;
+    if ((st = loop.run(prm->max_iter - 1, iteration, &end)) != WD_OK) return st;
+    stats->iterations = end.iters;
+    if (end.stop == 2) return wd_fail(ctx, WD_ERR_NAN, "CG residual is not finite");
+    stats->residual = std::sqrt(end.rr_new);
+    stats->converged = end.stop == 1;
     return WD_OK;
 }
 
@@ -155,6 +210,7 @@ static wd_status cg_eo_core(wd_context *ctx, const wd_lattice *lat, WdVec src, W
     const int Vh = lat->g.Vh;
     const int64_t nh = (int64_t)12 * Vh;
     const double m = prm->mass, a = 4.0 + m;
+    const bool fused = src.prec == WD_PREC_F64 && lat->gauge_fix;
     WdVecBuf b[7];
     for (auto &v : b) {
         wd_status s = wd_vec_alloc(ctx, v, src.prec, nh);
@@ -163,7 +219,10 @@ static wd_status cg_eo_core(wd_context *ctx, const wd_lattice *lat, WdVec src, W
     WdVec bhat = b[0].v, r = b[1].v, p = b[2].v, t = b[3].v, q = b[4].v, tmp_o = b[5].v, s_e = b[6].v;
     const WdVec b_e = par_half(src, 0, Vh), b_o = par_half(src, 1, Vh);
     WdVec x_e = par_half(x, 0, Vh), x_o = par_half(x, 1, Vh);
-    wd_status st;
+    CgLoop loop(ctx, Vh);
+    wd_status st = loop.alloc(std::max((size_t)2 * WD_RED_BLOCKS, wd_hop_fix_partials(lat)));
+    if (st != WD_OK) return st;
+    WdCgDev *dev = loop.dev;
 
     // bhat_e = b_e + D_eo b_o / (2a)
     if ((st = wd_hop_v(ctx, lat, b_o, bhat, &b_e, 0, 0, 0.5 / a, 1.0)) != WD_OK) return st;
@@ -189,6 +248,25 @@ static wd_status cg_eo_core(wd_context *ctx, const wd_lattice *lat, WdVec src, W
         ss = v[1].x;
         return WD_OK;
     };
+    // t = Mhat p, alpha = rr / |t|^2, q = Mhat^dag t, the update with |r|^2, p = r + beta p
+    auto iteration = [&]() -> wd_status {
+        wd_status e;
+        if ((e = wd_hop_v(ctx, lat, p, tmp_o, nullptr, 1, 0, 1.0, 0.0, &dev->stop)) != WD_OK) return e;
+        if (fused) {
+            if ((e = wd_hop_fix_norm(ctx, lat, tmp_o, t, p, m, dev, loop.partial)) != WD_OK) return e;
+        } else {
+            if ((e = wd_hop_v(ctx, lat, tmp_o, t, &p, 0, 0, -0.25 / a, a, &dev->stop)) != WD_OK) return e;
+            if ((e = wd_cgd_norm(ctx, t, nh, dev, loop.partial)) != WD_OK) return e;
+        }
+        if ((e = wd_hop_v(ctx, lat, t, tmp_o, nullptr, 1, 1, 1.0, 0.0, &dev->stop)) != WD_OK) return e;
+        if (fused) {
+            if ((e = wd_hop_fix_update(ctx, lat, tmp_o, t, p, r, x_e, m, dev, loop.partial)) != WD_OK) return e;
+        } else {
+            if ((e = wd_hop_v(ctx, lat, tmp_o, q, &t, 0, 1, -0.25 / a, a, &dev->stop)) != WD_OK) return e;
+            if ((e = wd_cgd_update(ctx, false, p, q, x_e, r, nh, dev, loop.partial)) != WD_OK) return e;
+        }
+        return wd_cgd_xpby(ctx, r, p, nh, dev);
+    };
 
     double rr;
     if ((st = residuals(&rr)) != WD_OK) return st;
@@ -200,36 +278,28 @@ static wd_status cg_eo_core(wd_context *ctx, const wd_lattice *lat, WdVec src, W
     int iters = 0;
     bool converged = true_res <= prm->tol;
     while (!converged && iters < prm->max_iter) {
-        // t = Mhat p, q = Mhat^dag t, alpha = rr / |t|^2
-        if ((st = wd_apply_Mhat_v(ctx, lat, p, t, tmp_o, m, 0)) != WD_OK) return st;
-        if ((st = wd_apply_Mhat_v(ctx, lat, t, q, tmp_o, m, 1)) != WD_OK) return st;
-        if ((st = wd_v_norm2(ctx, t, nh, 0)) != WD_OK) return st;
-        if ((st = fetch1(ctx, red)) != WD_OK) return st;
-        const double alpha = rr / red[0].x;
-        if ((st = wd_v_cg_update_real(ctx, alpha, p, q, x_e, r, nh, 0)) != WD_OK) return st;
-        if ((st = fetch1(ctx, red)) != WD_OK) return st;
-        double rr_new = red[0].x;
-        ++iters;
-        if (!std::isfinite(rr_new)) {
+        WdCgDev end{};
+        if ((st = loop.start(rr, target, false, iters)) != WD_OK) return st;
+        if ((st = loop.run(prm->max_iter - iters, iteration, &end)) != WD_OK) return st;
+        iters = end.iters;
+        if (end.stop == 2) {
             stats->iterations = iters;
             return wd_fail(ctx, WD_ERR_NAN, "CG residual is not finite");
         }
-        if (std::sqrt(rr_new) <= target) {
-            // check the true residual; replace r by the recomputed one
-            if ((st = residuals(&rr_new)) != WD_OK) return st;
-            stats->reliable_updates++;
-            true_res = std::sqrt(ss) / norm_b;
-            if (true_res <= prm->tol) {
-                converged = true;
-                rr = rr_new;
-                break;
-            }
-            ratio = ss > 0 ? std::sqrt(rr_new / ss) : ratio;
-            target = std::fmin(target * 0.5, prm->tol * norm_b * ratio * 0.5);
+        if (end.stop != 1) break;  // out of iterations
+        // check the true residual; replace r by the recomputed one
+        double rr_new;
+        if ((st = residuals(&rr_new)) != WD_OK) return st;
+        stats->reliable_updates++;
+        true_res = std::sqrt(ss) / norm_b;
+        if (true_res <= prm->tol) {
+            converged = true;
+            break;
         }
-        const double beta = rr_new / rr;
+        ratio = ss > 0 ? std::sqrt(rr_new / ss) : ratio;
+        target = std::fmin(target * 0.5, prm->tol * norm_b * ratio * 0.5);
+        if ((st = wd_v_xpby(ctx, r, rr_new / end.rr, p, nh)) != WD_OK) return st;
         rr = rr_new;
-        if ((st = wd_v_xpby(ctx, r, beta, p, nh)) != WD_OK) return st;
     }
     // x_o = (b_o + D_oe x_e / 2) / a
     if ((st = wd_hop_v(ctx, lat, x_e, x_o, &b_o, 1, 0, 0.5 / a, 1.0 / a)) != WD_OK) return st;

@@ -15,7 +15,8 @@ struct WdVecBuf {
 wd_status wd_vec_alloc(wd_context *ctx, WdVecBuf &b, wd_precision prec, int64_t n_complex);
 
 // M (dag=0) or M^dag on full-lattice vectors of one storage
-wd_status wd_apply_M_v(wd_context *ctx, const wd_lattice *lat, WdVec in, WdVec out, double mass, int dag);
+wd_status wd_apply_M_v(wd_context *ctx, const wd_lattice *lat, WdVec in, WdVec out, double mass, int dag,
+                       const int *stop = nullptr);
 // Schur operator a - D_eo D_oe/(4a) (or its adjoint) on even blocks; tmp_o is an odd block
 wd_status wd_apply_Mhat_v(wd_context *ctx, const wd_lattice *lat, WdVec v, WdVec out, WdVec tmp_o, double mass,
                           int dag);
@@ -77,3 +78,70 @@ struct WdMxDev {
     int iters;        // iterations completed on the device
     unsigned count_t, count_r;  // last-block counters of the two reductions
 };
+
+// Device-side scalars of the FP64 / double-float CG solvers (wd_solver.cu):
+// the reductions' last blocks set alpha and beta and close the stop gate, so
+// iterations run back to back with no host wait.
+struct WdCgDev {
+    double rr;        // |r|^2 of the current iterate (the previous one once stop is set)
+    double rr_new;    // |r|^2 after the running iteration's update
+    double target2;   // stop once |r|^2 <= target2 (strict: < target2)
+    double are, aim;  // alpha
+    double beta;
+    int strict;
+    int stop;         // 0 iterate; 1 target reached; 2 non-finite |r|^2
+    int iters;        // iterations completed
+    unsigned count_a, count_r;  // last-block counters of the two reductions
+};
+
+#ifdef __CUDACC__
+// alpha = |r|^2 / d, d complex (src/invert.cpp:79-83); real d for the even-odd CG
+__device__ __forceinline__ void wd_cg_set_alpha(WdCgDev *d, double re, double im, bool cplx)
+{
+    if (cplx) {
+        const double n = re * re + im * im;
+        d->are = (d->rr * re) / n;
+        d->aim = (0.0 - d->rr * im) / n;
+    } else {
+        d->are = d->rr / re;
+        d->aim = 0.0;
+    }
+}
+// after the update of r: beta, or the stop gate
+__device__ __forceinline__ void wd_cg_set_beta(WdCgDev *d, double rr_new)
+{
+    d->iters++;
+    d->rr_new = rr_new;
+    if (!isfinite(rr_new)) d->stop = 2;
+    else if (d->strict ? rr_new < d->target2 : rr_new <= d->target2) d->stop = 1;
+    else {
+        d->beta = rr_new / d->rr;
+        d->rr = rr_new;
+    }
+}
+#endif
+
+// One iteration's pieces on n complex entries of one storage (FP64 or
+// double-float), all no-ops while dev->stop != 0 (wd_cg.cu).  partial: at
+// least 2 * WD_RED_BLOCKS doubles.
+// alpha from |t|^2, or from the complex (p, q)
+wd_status wd_cgd_norm(wd_context *ctx, WdVec t, int64_t n, WdCgDev *dev, double *partial);
+wd_status wd_cgd_dot(wd_context *ctx, WdVec p, WdVec q, int64_t n, WdCgDev *dev, double *partial);
+// x += alpha p, r -= alpha q, |r|^2 -> beta or the gate
+wd_status wd_cgd_update(wd_context *ctx, bool cplx, WdVec p, WdVec q, WdVec x, WdVec r, int64_t n, WdCgDev *dev,
+                        double *partial);
+// p = r + beta p
+wd_status wd_cgd_xpby(wd_context *ctx, WdVec r, WdVec p, int64_t n, const WdCgDev *dev);
+
+// The same fused into the fixed-point FP64 hops (wd_dslash_fix.cu; the
+// lattice has gauge_fix).  partial: wd_hop_fix_partials(lat) doubles.
+size_t wd_hop_fix_partials(const wd_lattice *lat);
+//   t = -D_eo in / (4a) + a p on even blocks (a = 4 + mass), |t|^2 -> alpha
+wd_status wd_hop_fix_norm(wd_context *ctx, const wd_lattice *lat, WdVec in, WdVec t, WdVec p, double mass, WdCgDev *dev,
+                          double *partial);
+//   q = -D_eo^dag in / (4a) + a t, not stored: r -= alpha q, x += alpha p, |r|^2 -> beta or the gate
+wd_status wd_hop_fix_update(wd_context *ctx, const wd_lattice *lat, WdVec in, WdVec t, WdVec p, WdVec r, WdVec x,
+                            double mass, WdCgDev *dev, double *partial);
+//   q = M^dag in on the whole lattice, (p, q) -> alpha
+wd_status wd_hop_fix_M_dot(wd_context *ctx, const wd_lattice *lat, WdVec in, WdVec q, WdVec p, double mass, WdCgDev *dev,
+                           double *partial);

@@ -133,6 +133,13 @@ int wd_tune_choice(wd_context *ctx, const char *kernel, int Vh)
     return T.on() ? -1 : 0;
 }
 
+void wd_tune_note(const char *kernel, int nvariants)
+{
+    Tuner &T = tuner();
+    std::lock_guard<std::mutex> lock(T.mu);
+    T.variants[kernel] = nvariants;
+}
+
 extern "C" int wd_tune_report(char *buf, int len)
 {
     Tuner &T = tuner();

@@ -14,3 +14,7 @@ wd_status wd_tune_launch(wd_context *ctx, const char *kernel, int Vh, int nvaria
 // a tuned kernel's epilogue (and so cannot be timed repeatedly) take the
 // plain kernel's shape.
 int wd_tune_choice(wd_context *ctx, const char *kernel, int Vh);
+
+// Records that `kernel` has nvariants launch variants, for a launch whose
+// shape needs no timing.
+void wd_tune_note(const char *kernel, int nvariants);
