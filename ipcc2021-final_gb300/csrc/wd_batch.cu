@@ -39,7 +39,7 @@
 namespace {
 
 constexpr int kSites = 32;  // sites per warp (one system per warp)
-constexpr int kChunk = 8192;     // sites per xpay chunk (one block each)
+constexpr int kChunk = 512;      // sites per xpay chunk (one block each; 8192 left 12 x 16^3x32 with 96 blocks: 60 us)
 constexpr int kBatchHopVariants = 7;
 constexpr int kMaxPerGraph = 8;  // iterations queued per graph launch at most
 
@@ -47,8 +47,15 @@ struct BGroup {
     WdGeom g;
     const void *gauge;  // 12-real links of the group's lattice in the kernel storage
     int first_sys, nsys;
-    int block_start;    // first blockIdx.x of this group
+    // Shape of the group's blocks for kernels of 2, 4 and 8 warps a block
+    // (index log2(warps) - 1): a block's warps are `sys` systems x (warps /
+    // sys) runs of 32 sites, `ny` blocks cover the group's systems, and they
+    // follow one another in the grid (y fastest), so that the blocks that
+    // read the same links run together.  A group with few systems gives its
+    // warps more sites instead of leaving them idle.
+    int sys[3], ny[3], block_start[3];
 };
+constexpr int warps_index(int warps) { return warps == 2 ? 0 : warps == 4 ? 1 : 2; }
 
 // one operand set per system for one batched hop launch
 struct BSys {
@@ -109,12 +116,13 @@ struct BatchHop {
     __device__ __forceinline__ void load_link(int mu, int par, int s, C *U) const { link.load(mu, par, s, U); }
 };
 
+template <int W>
 __device__ __forceinline__ int find_group(const BGroup *groups, int ngroups, int block)
 {
     int lo = 0, hi = ngroups - 1;
     while (lo < hi) {
         const int mid = (lo + hi + 1) >> 1;
-        if (groups[mid].block_start <= block) lo = mid;
+        if (groups[mid].block_start[W] <= block) lo = mid;
         else hi = mid - 1;
     }
     return lo;
@@ -200,33 +208,37 @@ __device__ __forceinline__ auto batch_policy(const BTable &t, const BGroup &G, c
     }
 }
 
-// SYS systems (warps) per block sharing the block's 32 sites; MINB blocks per
-// SM (0: no bound) bound the registers.  A warp is one system's 32
-// consecutive sites, so a reducing epilogue writes one partial per warp.
+// SYS warps per block: that many systems sharing the block's 32 sites, or
+// fewer systems and more sites (BGroup); MINB blocks per SM (0: no bound)
+// bound the registers.  A warp is one system's 32 consecutive sites, so a
+// reducing epilogue writes one partial per warp.
 // R2 (FP16 storage): row 2 of the block's links is rebuilt once per site and
 // direction into shared memory by all the block's warps together, and every
-// system reads it there instead of rebuilding it (the same values).
+// system reads it there instead of rebuilding it (the same values); blocks
+// whose warps hold different sites rebuild it themselves.
 template <bool DAG, bool F16, int SYS, int MINB, int EPI, bool R2 = false>
 __global__ void __launch_bounds__(kSites * SYS, MINB) k_batch_hop(const BTable t)
 {
-    const int gi = find_group(t.groups, t.ngroups, blockIdx.x);
+    constexpr int W = SYS == 2 ? 0 : SYS == 4 ? 1 : 2;
+    const int gi = find_group<W>(t.groups, t.ngroups, blockIdx.x);
     const BGroup &G = t.groups[gi];
-    const int r = blockIdx.y * SYS + (threadIdx.x / kSites);
-    const int blk = blockIdx.x - G.block_start;
-    const int lane = threadIdx.x % kSites;
+    const int warp = threadIdx.x / kSites, lane = threadIdx.x % kSites;
+    const int b = blockIdx.x - G.block_start[W], gs = G.sys[W], ny = G.ny[W];
+    const int r = (b % ny) * gs + warp % gs;           // system of the group
+    const int blk = (b / ny) * (SYS / gs) + warp / gs;  // its run of 32 sites
     const int s = blk * kSites + lane;
     static_assert(!R2 || F16, "the shared row-2 table is for 12-real FP16 links");
     __shared__ unsigned r2[R2 ? 8 : 1][3][kSites];
     if constexpr (R2) {
         // every warp takes part, whether or not its system iterates
-        if (s < G.g.Vh) {
+        if (gs == SYS && s < G.g.Vh) {
             const uint4 *a = (const uint4 *)G.gauge;
             const LinkF16 lk{a, (const uint2 *)(a + (size_t)8 * G.g.Vh), G.g.Vh};
-            h16_fill_row2<SYS>(G.g, t.cb, lk, s, r2, threadIdx.x / kSites, lane);
+            h16_fill_row2<SYS>(G.g, t.cb, lk, s, r2, warp, lane);
         }
         __syncthreads();
     }
-    if (r >= G.nsys) return;  // whole warps
+    if (r >= G.nsys || blk * kSites >= G.g.Vh) return;  // whole warps
     const int sys = G.first_sys + r;
     if (!t.sc[sys].active) return;
     const BSys &S = t.sys[sys];
@@ -234,8 +246,10 @@ __global__ void __launch_bounds__(kSites * SYS, MINB) k_batch_hop(const BTable t
     if (s < G.g.Vh) {
         float2 acc[12];
         // FP16 storage: the FP16-operand arithmetic of the solo FP16 kernel
-        if constexpr (R2) h16_hop_site_r2<DAG>(batch_policy<F16>(t, G, S), s, r2, lane, acc);
-        else if constexpr (F16) h16_hop_site<DAG>(batch_policy<F16>(t, G, S), s, acc);
+        if constexpr (R2) {
+            if (gs == SYS) h16_hop_site_r2<DAG>(batch_policy<F16>(t, G, S), s, r2, lane, acc);
+            else h16_hop_site<DAG>(batch_policy<F16>(t, G, S), s, acc);
+        } else if constexpr (F16) h16_hop_site<DAG>(batch_policy<F16>(t, G, S), s, acc);
         else wd_hop_site<DAG>(batch_policy<F16>(t, G, S), s, acc);
         v = batch_epilogue<F16, EPI>(t, S, sys, s, G.g.Vh, acc);
     }
@@ -280,23 +294,20 @@ __global__ void __launch_bounds__(WD_RED_THREADS) k_batch_xpay(const BVec *v, co
 // mode 1 (|r_s|^2 after the update): the reliable-update rule -- mask the
 // system and flag it when |r_s|^2 < delta2 rr_max or <= target2, else
 // beta = rr_new / rr, rr = rr_new.
-constexpr int kScalThreads = 128;
+// (a 24^3x48 system has 10,368 partials: 13 us with 128 threads)
+constexpr int kScalThreads = 512;
 __global__ void __launch_bounds__(kScalThreads) k_batch_scalars(const BSys *sys_tab, BScal *sc, const double *partial,
                                                                 int mode, double delta2)
 {
     const int sys = blockIdx.x;
     if (!sc[sys].active) return;  // the whole block
     const BSys &S = sys_tab[sys];
-    double v = 0.0;
-    for (int i = threadIdx.x; i < S.nparts; i += kScalThreads) v += partial[S.part0 + i];
-    v = wd_warp_sum(v);
-    __shared__ double sw[kScalThreads / 32];
-    if ((threadIdx.x & 31) == 0) sw[threadIdx.x >> 5] = v;
-    __syncthreads();
+    double p[1] = {0.0}, tot[1];
+#pragma unroll 4
+    for (int i = threadIdx.x; i < S.nparts; i += kScalThreads) p[0] += partial[S.part0 + i];
+    wd_block_sum<kScalThreads, 1>(p, tot);
     if (threadIdx.x != 0) return;
-    v = 0.0;
-#pragma unroll
-    for (int w = 0; w < kScalThreads / 32; ++w) v += sw[w];
+    const double v = tot[0];
     BScal &c = sc[sys];
     if (mode == 0) {
         c.tt = v;
@@ -463,7 +474,7 @@ class BatchEngine {
     DevArray<double> d_partial_, d_rel_;
     DevArray<int> d_chunk_sys_;
     std::vector<BScal> h_sc_;
-    int grid_x_ = 0, nchunks_ = 0, ngroups_ = 0, max_group_sys_ = 1;
+    int grid_[3] = {}, nchunks_ = 0, ngroups_ = 0;  // blocks of a batched hop with 2, 4, 8 warps a block
     int hop_variant_ = 0;  // launch shape of the batched hop (tuned in rebuild)
     std::map<int, cudaGraphExec_t> graphs_;  // K -> K captured iterations
     uint64_t kernels_per_iter_ = 0;
@@ -622,7 +633,6 @@ wd_status BatchEngine::rebuild()
     const bool f16 = L_ == WD_PREC_F16;
     std::vector<BGroup> groups;
     std::vector<int> sys_group(nsys);
-    int blocks = 0;
     for (int k = 0; k < nsys; ++k) {
         if (k == 0 || sys_[k]->lat != sys_[k - 1]->lat) {
             BGroup G{};
@@ -630,16 +640,25 @@ wd_status BatchEngine::rebuild()
             G.gauge = f16 ? sys_[k]->lat->gauge_h12 : sys_[k]->lat->gauge_f32;
             G.first_sys = k;
             G.nsys = 0;
-            G.block_start = blocks;
-            blocks += (G.g.Vh + kSites - 1) / kSites;
             groups.push_back(G);
         }
         groups.back().nsys++;
         sys_group[k] = (int)groups.size() - 1;
     }
-    grid_x_ = blocks;
-    max_group_sys_ = 1;
-    for (const BGroup &G : groups) max_group_sys_ = std::max(max_group_sys_, G.nsys);
+    for (int w = 0; w < 3; ++w) {
+        const int warps = 2 << w;
+        int64_t blocks = 0;
+        for (BGroup &G : groups) {
+            G.sys[w] = 1;
+            while (G.sys[w] < warps && G.sys[w] < G.nsys) G.sys[w] *= 2;
+            G.ny[w] = (G.nsys + G.sys[w] - 1) / G.sys[w];
+            G.block_start[w] = (int)blocks;
+            const int runs = (G.g.Vh + kSites - 1) / kSites, per = warps / G.sys[w];
+            blocks += (int64_t)((runs + per - 1) / per) * G.ny[w];
+        }
+        if (blocks > 0x7fffffff) return wd_fail(ctx_, WD_ERR_BAD_DIMS, "batch too large for one launch");
+        grid_[w] = (int)blocks;
+    }
     ngroups_ = (int)groups.size();
     std::vector<BVec> bvec(nsys);
     std::vector<int> chunk_sys;
@@ -755,7 +774,7 @@ wd_status BatchEngine::hop(int h, int cb, int dag, int v, int epi)
     const BTable t{d_groups_.p, ngroups_, d_sys_[h].p, d_alpha_[h].p, d_beta_[h].p, d_sc_.p, d_partial_.p, cb};
     auto run = [&](auto sys, auto minb, auto share) -> wd_status {
         constexpr int S = decltype(sys)::value, M = decltype(minb)::value;
-        const dim3 grid(grid_x_, (max_group_sys_ + S - 1) / S);
+        const int grid = grid_[warps_index(S)];
         auto go = [&](auto f16, auto e) {
             constexpr bool F = decltype(f16)::value;
             constexpr int E = decltype(e)::value;

@@ -97,12 +97,15 @@ __device__ __forceinline__ double2 hop_value(const FixArgs &a, const FixView &w,
     return make_double2(fma(a.beta, x.x, v.x), fma(a.beta, x.y, v.y));
 }
 
-// ---- epilogues: put() takes each component's hopping sum v at entry i of the
-// output parity block, finish() the sums of what put() returned in n
+// ---- epilogues: put() takes each component's hopping sum v, finish() the
+// grid's sums of what put() added up in n.  The FP64 pipe has little room
+// beside the hop's own 132 operations per site, so products are merged
+// (r - al (alpha v + beta x) in two multiply-adds).
 template <bool AOS_>
 struct EpiStore {
     static constexpr bool AOS = AOS_;
     static constexpr int N = 0;
+    using Num = double;
     __device__ __forceinline__ void put(const FixArgs &a, const FixView &w, int c, int s, double2 v, double *) const
     {
         const size_t i = entry<AOS>(a, c, s);
@@ -113,6 +116,7 @@ struct EpiStore {
 struct EpiNorm {
     static constexpr bool AOS = false;
     static constexpr int N = 1;
+    using Num = double;
     WdCgDev *dev;
     double *partial;
     __device__ __forceinline__ unsigned *counter() const { return &dev->count_a; }
@@ -129,6 +133,7 @@ struct EpiNorm {
 struct EpiUpdate {
     static constexpr bool AOS = false;
     static constexpr int N = 1;
+    using Num = double;
     WdCgDev *dev;
     double *partial;
     const double2 *p;
@@ -137,10 +142,10 @@ struct EpiUpdate {
     __device__ __forceinline__ void put(const FixArgs &a, const FixView &w, int c, int s, double2 v, double *n) const
     {
         const size_t i = entry<false>(a, c, s);
-        const double al = dev->are;
-        const double2 q = hop_value(a, w, i, v), pv = p[i];
+        const double al = dev->are, av = -al * a.alpha, ax = -al * a.beta;
+        const double2 x = w.x[i], pv = p[i];
         double2 rv = r[i], yv = y[i];
-        rv = make_double2(fma(-al, q.x, rv.x), fma(-al, q.y, rv.y));
+        rv = make_double2(fma(av, v.x, fma(ax, x.x, rv.x)), fma(av, v.y, fma(ax, x.y, rv.y)));
         yv = make_double2(fma(al, pv.x, yv.x), fma(al, pv.y, yv.y));
         r[i] = rv;
         y[i] = yv;
@@ -152,6 +157,7 @@ struct EpiUpdate {
 struct EpiDot {
     static constexpr bool AOS = false;
     static constexpr int N = 2;
+    using Num = double;
     WdCgDev *dev;
     double *partial;
     const double2 *p;
@@ -172,16 +178,18 @@ struct EpiDot {
 struct EpiRes {
     static constexpr bool AOS = false;
     static constexpr int N = 1;
+    using Num = float;
     WdResSink r;
     double *partial;
     __device__ __forceinline__ unsigned *counter() const { return r.counter; }
-    __device__ __forceinline__ void put(const FixArgs &a, const FixView &w, int c, int s, double2 v, double *n) const
+    __device__ __forceinline__ void put(const FixArgs &a, const FixView &w, int c, int s, double2 v, float *n) const
     {
         const size_t i = entry<false>(a, c, s);
-        const double2 o = hop_value(a, w, i, v), b = r.bhat[i];
-        const float2 f = make_float2((float)(b.x - o.x), (float)(b.y - o.y));
+        const double2 x = w.x[i], b = r.bhat[i];
+        const float2 f = make_float2((float)fma(-a.alpha, v.x, fma(-a.beta, x.x, b.x)),
+                                     (float)fma(-a.alpha, v.y, fma(-a.beta, x.y, b.y)));
         reinterpret_cast<float2 *>(r.s32 + (size_t)(c >> 1) * a.g.Vh + s)[c & 1] = f;
-        n[0] += (double)fmaf(f.x, f.x, f.y * f.y);
+        n[0] = fmaf(f.x, f.x, fmaf(f.y, f.y, n[0]));
     }
     __device__ __forceinline__ void finish(const double *t) const { *r.result = t[0]; }
 };
@@ -214,7 +222,7 @@ __global__ void __launch_bounds__(block_threads(T), 512 / block_threads(T))
     bool ok;
     if constexpr (T > 0) ok = wd_fix::site<DAG>(p, *reinterpret_cast<wd_fix::Stage<B> *>(smem), s, half, v);
     else ok = wd_fix::site_split<DAG>(p, *reinterpret_cast<wd_fix::Split *>(smem), s, half, v);
-    double n[Epi::N ? Epi::N : 1] = {};
+    typename Epi::Num n[Epi::N ? Epi::N : 1] = {};
     const int warp = threadIdx.x >> 5;  // split form: warps 0-2 hold colour `warp` of the two spins
     if (s0 < s_hi && (T > 0 || warp < 3)) {
         if (!ok) {
@@ -233,8 +241,10 @@ __global__ void __launch_bounds__(block_threads(T), 512 / block_threads(T))
         }
     }
     if constexpr (Epi::N > 0) {
-        double t[Epi::N];
-        if (wd_grid_sum_n<B, Epi::N>(n, epi.partial, epi.counter(), t)) epi.finish(t);
+        double d[Epi::N], t[Epi::N];
+#pragma unroll
+        for (int k = 0; k < Epi::N; ++k) d[k] = (double)n[k];
+        if (wd_grid_sum_n<B, Epi::N>(d, epi.partial, epi.counter(), t)) epi.finish(t);
     }
 }
 

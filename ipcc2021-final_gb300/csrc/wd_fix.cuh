@@ -76,12 +76,14 @@ __device__ __forceinline__ void limbs(uint32_t hi, uint32_t lo, uint32_t ekey, i
 
 // c + a b.  Written as the carry pair: ptxas makes one wide multiply-add of
 // it, where mad.wide.s32 costs an extra ALU operation (measured).
-__device__ __forceinline__ void macw(long long &c, int a, int b)
+__device__ __forceinline__ long long macw(long long c, int a, int b)
 {
-    asm("{\n\t.reg .u32 l, h;\n\tmov.b64 {l, h}, %0;\n\tmad.lo.cc.s32 l, %1, %2, l;\n\tmadc.hi.s32 h, %1, %2, h;\n\t"
+    long long d;
+    asm("{\n\t.reg .u32 l, h;\n\tmov.b64 {l, h}, %1;\n\tmad.lo.cc.s32 l, %2, %3, l;\n\tmadc.hi.s32 h, %2, %3, h;\n\t"
         "mov.b64 %0, {l, h};\n\t}"
-        : "+l"(c)
-        : "r"(a), "r"(b));
+        : "=l"(d)
+        : "l"(c), "r"(a), "r"(b));
+    return d;
 }
 
 // (re, im) of sum_b U[a][b] h_b (forward) or sum_b conj(U[b][a]) h_b
@@ -92,25 +94,25 @@ template <bool FWD, int T>
 __device__ __forceinline__ void su3_row(const int4 (*link)[T / 2], const int *x1, const int *x0, const int *q1,
                                         const int *q0, const int *v1, const int *v0, int a, long long &re, long long &im)
 {
-    long long k = 0, m = 1ll << 29;
+    long long k, m;
     int4 u[3];
 #pragma unroll
     for (int b = 0; b < 3; ++b) {
         u[b] = link[FWD ? a * 3 + b : b * 3 + a][threadIdx.x >> 1];
         const int s1 = FWD ? u[b].x + u[b].z : u[b].x - u[b].z, s0 = FWD ? u[b].y + u[b].w : u[b].y - u[b].w;
-        macw(k, s1, x1[b]);
-        macw(m, s1, x0[b]);
-        macw(m, s0, x1[b]);
+        k = b == 0 ? (long long)s1 * x1[b] : macw(k, s1, x1[b]);
+        m = macw(b == 0 ? 1ll << 29 : m, s1, x0[b]);
+        m = macw(m, s0, x1[b]);
     }
     long long rk = k, rm = m, ik = k, im_ = m;
 #pragma unroll
     for (int b = 0; b < 3; ++b) {
-        macw(rk, u[b].z, q1[b]);
-        macw(rm, u[b].z, q0[b]);
-        macw(rm, u[b].w, q1[b]);
-        macw(ik, u[b].x, v1[b]);
-        macw(im_, u[b].x, v0[b]);
-        macw(im_, u[b].y, v1[b]);
+        rk = macw(rk, u[b].z, q1[b]);
+        rm = macw(rm, u[b].z, q0[b]);
+        rm = macw(rm, u[b].w, q1[b]);
+        ik = macw(ik, u[b].x, v1[b]);
+        im_ = macw(im_, u[b].x, v0[b]);
+        im_ = macw(im_, u[b].y, v1[b]);
     }
     re = rk + (rm >> 30);
     im = ik + (im_ >> 30);

@@ -109,3 +109,39 @@ def test_batch_hop_variants_bit_identical(wd, ctx, prec, kernel):
                     assert np.array_equal(a, b), f"{kernel} variant {v}"
     finally:
         wd.tune_pin(kernel, bucket, -1)
+
+
+@pytest.mark.parametrize("prec,kernel", [("F32", "batch_hop_f32"), ("F16", "batch_hop_f16")])
+@pytest.mark.parametrize("counts", [(1, 1), (3, 1), (5, 2), (9, 1)])
+def test_block_shapes_of_uneven_groups(wd, ctx, oracle, prec, kernel, counts):
+    """A batched hop's blocks hold several systems of a lattice, or several
+    runs of 32 sites where a lattice has few systems: every launch variant
+    (2, 4 or 8 warps a block) gives the same bits, and the oracle's solution.
+    Vh = 1080 and 96 leave partial runs and partial blocks."""
+    dims = [(10, 6, 6, 6), (4, 4, 2, 6)]
+    lats, gauges = [], []
+    for i, d in enumerate(dims):
+        gauges.append(wd.gen_gauge(d, seed=60 + i))
+        lats.append(ctx.lattice(d, gauges[-1]))
+    jobs = [(i, wd.gen_source(dims[i], seed=70 + 10 * i + k), 0.08 + 0.02 * k) for i, n in enumerate(counts)
+            for k in range(n)]
+    params = wd.solver_params(kind=wd.CG_EO, tol=1e-10, max_iter=2000, prec=getattr(wd, prec), prec_reliable=wd.DF64)
+    sites = sum(int(np.prod(dims[i])) // 2 for i, _, _ in jobs)
+    bucket = 1
+    while bucket < sites:
+        bucket *= 2
+    sols = {}
+    try:
+        for v in range(7):
+            wd.tune_pin(kernel, bucket, v)
+            systems = [(lats[i], lats[i].field(s), lats[i].field(), m) for i, s, m in jobs]
+            stats = ctx.solve_batch(systems, params)
+            assert all(st.converged and st.true_residual <= 1e-10 for st in stats)
+            sols[v] = [x.download() for _, _, x, _ in systems]
+            for a, b in zip(sols[v], sols[0]):
+                assert np.array_equal(a, b), v
+    finally:
+        wd.tune_pin(kernel, bucket, -1)
+    for (i, s, m), x in zip(jobs, sols[0]):
+        want, _, _ = oracle.cg_eo(s, gauges[i], dims[i], m, tol=1e-13)
+        assert np.linalg.norm(x - want) <= 1e-9 * np.linalg.norm(want)
