@@ -61,6 +61,7 @@ struct FixArgs {
     double alpha, beta;
     F64Scale scale;
     const int *stop;
+    double2 *zero;         // a parity block to clear beside out, or null
 };
 // One block's parity: its operand pointers
 struct FixView {
@@ -110,6 +111,7 @@ struct EpiStore {
     {
         const size_t i = entry<AOS>(a, c, s);
         w.out[i] = hop_value(a, w, i, v);
+        if (a.zero) a.zero[i] = make_double2(0.0, 0.0);
     }
 };
 // t stored, |t|^2 -> alpha
@@ -283,7 +285,7 @@ FixArgs fix_args(const wd_lattice *lat, const void *in, void *out, const void *x
                  const int *stop = nullptr)
 {
     return FixArgs{lat->g, cb, (const double2 *)in, lat->gauge, (const double2 *)x, (double2 *)out,
-                   (const int4 *)lat->gauge_fix, alpha, beta, F64Scale::make(alpha), stop};
+                   (const int4 *)lat->gauge_fix, alpha, beta, F64Scale::make(alpha), stop, nullptr};
 }
 
 }  // namespace
@@ -298,9 +300,10 @@ wd_status wd_gauge_ref_to_soa_fix(wd_context *ctx, const WdGeom &g, int mu, cons
 }
 
 wd_status wd_hop_fix(wd_context *ctx, const wd_lattice *lat, const double2 *in, double2 *out, const double2 *x, int cb,
-                     int dag, double alpha, double beta, const int *stop)
+                     int dag, double alpha, double beta, const int *stop, double2 *zero)
 {
-    const FixArgs a = fix_args(lat, in, out, x, cb, alpha, beta, stop);
+    FixArgs a = fix_args(lat, in, out, x, cb, alpha, beta, stop);
+    a.zero = zero;
     auto run = [&](int v) {
         return dag ? run_fix<true>(ctx, a, EpiStore<false>(), false, v) : run_fix<false>(ctx, a, EpiStore<false>(), false, v);
     };

@@ -31,9 +31,10 @@ struct WdResSink {
     unsigned *counter;
     double *result;
 };
-// (the lattice has gauge_fix; stop as for the other hops)
+// (the lattice has gauge_fix; stop as for the other hops; zero: a parity block
+// that the launch also clears)
 wd_status wd_hop_fix(wd_context *ctx, const wd_lattice *lat, const double2 *in, double2 *out, const double2 *x, int cb,
-                     int dag, double alpha, double beta, const int *stop = nullptr);
+                     int dag, double alpha, double beta, const int *stop = nullptr, double2 *zero = nullptr);
 // M (or M^dag) on whole fields in one launch
 wd_status wd_hop_fix_M(wd_context *ctx, const wd_lattice *lat, const double2 *in, double2 *out, double mass, int dag,
                        const int *stop = nullptr);
