@@ -244,6 +244,9 @@ static wd_status make_geom(wd_context *ctx, const int *dims, WdGeom *g, int64_t 
     if (v > WD_MAX_SITES) return wd_fail(ctx, WD_ERR_BAD_DIMS, "lattice too large");
     g->Lxh = dims[0] / 2;
     g->Vh = (int)(v / 2);
+    g->dx = WdDiv(g->Lxh);
+    g->dy = WdDiv(dims[1]);
+    g->dz = WdDiv(dims[2]);
     *vol = v;
     return WD_OK;
 }

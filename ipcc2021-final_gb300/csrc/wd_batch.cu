@@ -1005,10 +1005,7 @@ extern "C" wd_status wd_solve_batch(wd_context *ctx, int nsys, const wd_lattice 
         s.seconds = secs;
         if (stats) {
             // FP64 true residual of each returned solution (a check, after the timed solve)
-            WdVecBuf tmp;
-            if ((st = wd_vec_alloc(ctx, tmp, WD_PREC_F64, lats[i]->volume * 12)) != WD_OK) return st;
-            st = wd_true_residual(ctx, lats[i], srcs[i]->d, dests[i]->d, (double2 *)tmp.v.p, masses[i],
-                                  &s.true_residual);
+            st = wd_true_residual(ctx, lats[i], srcs[i]->d, dests[i]->d, masses[i], &s.true_residual);
             if (st != WD_OK) return st;
             stats[i] = s;
         }

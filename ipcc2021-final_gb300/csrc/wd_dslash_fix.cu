@@ -58,8 +58,10 @@ struct FixArgs {
     const double2 *x;
     double2 *out;
     const int4 *links;
-    double alpha, beta;
-    F64Scale scale;
+    double alpha, beta;    // alpha = pre * post: what the integer sums take on their exponent, and the rest
+    wd_fix::Pow2 pre;
+    double post;           // 1, or alpha where that is no power of two (scaled = 1)
+    int scaled;
     const int *stop;
     double2 *zero;         // a parity block to clear beside out, or null
 };
@@ -87,22 +89,34 @@ __device__ __forceinline__ size_t entry(const FixArgs &a, int c, int s)
 {
     return AOS ? (size_t)s * 12 + c : (size_t)c * a.g.Vh + s;
 }
-// alpha v + beta x; a power-of-two alpha is exact on the exponent, which
-// leaves one FP64 operation per real (and one rounding) instead of two
+__device__ __noinline__ double2 scale_rare(double2 v, double f) { return c_scale(v, f); }
+
+// alpha acc + beta x from v = pre acc.  The forms are separate kernels: FP64
+// operations that a condition turns off still hold the FP64 pipe for their
+// 16 cycles (with one kernel for all, D_eo at 32^3x64 took 0.391 ms, not 0.370).
+enum Form {
+    kPlain,   // no x (a factor that is no power of two is met by no solver)
+    kPow2X,   // x, alpha a power of two: one operation per real, one rounding
+    kScaledX  // x, any alpha
+};
+template <Form F>
 __device__ __forceinline__ double2 hop_value(const FixArgs &a, const FixView &w, size_t i, double2 v)
 {
-    if (!w.x) return a.scale.apply(v);
-    const double2 x = w.x[i];
-    if (a.scale.mode == 0) return c_axpby(a.alpha, v, a.beta, x);
-    v = a.scale.apply(v);
-    return make_double2(fma(a.beta, x.x, v.x), fma(a.beta, x.y, v.y));
+    if constexpr (F == kPlain) {
+        if (a.scaled) v = scale_rare(v, a.post);
+        return v;
+    } else {
+        const double2 x = w.x[i];
+        if constexpr (F == kScaledX) v = c_scale(v, a.post);
+        return make_double2(fma(a.beta, x.x, v.x), fma(a.beta, x.y, v.y));
+    }
 }
 
 // ---- epilogues: put() takes each component's hopping sum v, finish() the
 // grid's sums of what put() added up in n.  The FP64 pipe has little room
 // beside the hop's own 132 operations per site, so products are merged
 // (r - al (alpha v + beta x) in two multiply-adds).
-template <bool AOS_>
+template <bool AOS_, Form F>
 struct EpiStore {
     static constexpr bool AOS = AOS_;
     static constexpr int N = 0;
@@ -110,8 +124,8 @@ struct EpiStore {
     __device__ __forceinline__ void put(const FixArgs &a, const FixView &w, int c, int s, double2 v, double *) const
     {
         const size_t i = entry<AOS>(a, c, s);
-        w.out[i] = hop_value(a, w, i, v);
-        if (a.zero) a.zero[i] = make_double2(0.0, 0.0);
+        w.out[i] = hop_value<F>(a, w, i, v);
+        if (F == kPlain && a.zero) a.zero[i] = make_double2(0.0, 0.0);
     }
 };
 // t stored, |t|^2 -> alpha
@@ -125,7 +139,7 @@ struct EpiNorm {
     __device__ __forceinline__ void put(const FixArgs &a, const FixView &w, int c, int s, double2 v, double *n) const
     {
         const size_t i = entry<false>(a, c, s);
-        const double2 o = hop_value(a, w, i, v);
+        const double2 o = hop_value<kScaledX>(a, w, i, v);
         w.out[i] = o;
         n[0] = fma(o.x, o.x, fma(o.y, o.y, n[0]));
     }
@@ -144,7 +158,7 @@ struct EpiUpdate {
     __device__ __forceinline__ void put(const FixArgs &a, const FixView &w, int c, int s, double2 v, double *n) const
     {
         const size_t i = entry<false>(a, c, s);
-        const double al = dev->are, av = -al * a.alpha, ax = -al * a.beta;
+        const double al = dev->are, av = -al * a.post, ax = -al * a.beta;
         const double2 x = w.x[i], pv = p[i];
         double2 rv = r[i], yv = y[i];
         rv = make_double2(fma(av, v.x, fma(ax, x.x, rv.x)), fma(av, v.y, fma(ax, x.y, rv.y)));
@@ -167,7 +181,7 @@ struct EpiDot {
     __device__ __forceinline__ void put(const FixArgs &a, const FixView &w, int c, int s, double2 v, double *n) const
     {
         const size_t i = entry<false>(a, c, s);
-        const double2 q = hop_value(a, w, i, v), u = p[(size_t)w.cb * 12 * a.g.Vh + i];
+        const double2 q = hop_value<kPow2X>(a, w, i, v), u = p[(size_t)w.cb * 12 * a.g.Vh + i];
         w.out[i] = q;
         n[0] = fma(u.x, q.x, fma(u.y, q.y, n[0]));
         n[1] = fma(u.x, q.y, fma(-u.y, q.x, n[1]));
@@ -188,12 +202,37 @@ struct EpiRes {
     {
         const size_t i = entry<false>(a, c, s);
         const double2 x = w.x[i], b = r.bhat[i];
-        const float2 f = make_float2((float)fma(-a.alpha, v.x, fma(-a.beta, x.x, b.x)),
-                                     (float)fma(-a.alpha, v.y, fma(-a.beta, x.y, b.y)));
+        const float2 f = make_float2((float)fma(-a.post, v.x, fma(-a.beta, x.x, b.x)),
+                                     (float)fma(-a.post, v.y, fma(-a.beta, x.y, b.y)));
         reinterpret_cast<float2 *>(r.s32 + (size_t)(c >> 1) * a.g.Vh + s)[c & 1] = f;
         n[0] = fmaf(f.x, f.x, fmaf(f.y, f.y, n[0]));
     }
     __device__ __forceinline__ void finish(const double *t) const { *r.result = t[0]; }
+};
+
+// |b - M x|^2 and |b|^2 -> result[0], result[1]; nothing stored
+struct EpiTrueRes {
+    static constexpr bool AOS = false;
+    static constexpr int N = 2;
+    using Num = double;
+    double *partial;
+    unsigned *count;
+    const double2 *b;
+    double *result;
+    __device__ __forceinline__ unsigned *counter() const { return count; }
+    __device__ __forceinline__ void put(const FixArgs &a, const FixView &w, int c, int s, double2 v, double *n) const
+    {
+        const size_t i = entry<false>(a, c, s);
+        const double2 x = w.x[i], bv = b[(size_t)w.cb * 12 * a.g.Vh + i];
+        const double2 d = make_double2(bv.x - fma(a.beta, x.x, v.x), bv.y - fma(a.beta, x.y, v.y));
+        n[0] = fma(d.x, d.x, fma(d.y, d.y, n[0]));
+        n[1] = fma(bv.x, bv.x, fma(bv.y, bv.y, n[1]));
+    }
+    __device__ __forceinline__ void finish(const double *t) const
+    {
+        result[0] = t[0];
+        result[1] = t[1];
+    }
 };
 
 // 512 threads per SM (128 registers each).  Output sites [s_lo, s_hi).  T > 0: T threads a block, two a site; T = 0: the
@@ -222,18 +261,19 @@ __global__ void __launch_bounds__(block_threads(T), 512 / block_threads(T))
     const int s = s0 < s_hi ? s0 : s_hi - 1;
     double2 v[6];
     bool ok;
-    if constexpr (T > 0) ok = wd_fix::site<DAG>(p, *reinterpret_cast<wd_fix::Stage<B> *>(smem), s, half, v);
-    else ok = wd_fix::site_split<DAG>(p, *reinterpret_cast<wd_fix::Split *>(smem), s, half, v);
+    if constexpr (T > 0) ok = wd_fix::site<DAG>(p, *reinterpret_cast<wd_fix::Stage<B> *>(smem), s, half, a.pre, v);
+    else ok = wd_fix::site_split<DAG>(p, *reinterpret_cast<wd_fix::Split *>(smem), s, half, a.pre, v);
     typename Epi::Num n[Epi::N ? Epi::N : 1] = {};
     const int warp = threadIdx.x >> 5;  // split form: warps 0-2 hold colour `warp` of the two spins
     if (s0 < s_hi && (T > 0 || warp < 3)) {
         if (!ok) {
             double2 acc[12];
             f64_route<DAG, AOS>(a, w, s, acc);
+            const double pre = a.scaled ? 1.0 : a.alpha;
 #pragma unroll
             for (int k = 0; k < (T ? 6 : 2); ++k) {
                 const int spin = k < (T ? 3 : 1) ? half : 3 - half;
-                v[k] = acc[spin * 3 + (T ? k % 3 : warp)];
+                v[k] = c_scale(acc[spin * 3 + (T ? k % 3 : warp)], pre);
             }
         }
 #pragma unroll
@@ -265,27 +305,40 @@ void launch_fix(cudaStream_t stream, const FixArgs &a, const Epi &epi, bool both
     k_hop_fix<DAG, T, Epi><<<grid, T ? T : 128, sm, stream>>>(a, epi, s_lo, s_hi);
 }
 
-// launch shapes of the form with two threads a site: 128, 64, 32 threads a
-// block; 128 with a reduction (fewest block sums: at 16^3x32 the update hop
-// took 56 us with 32)
 template <bool DAG, class Epi>
-wd_status run_fix(wd_context *ctx, const FixArgs &a, const Epi &epi, bool both, int variant)
+wd_status run_fix(wd_context *ctx, cudaStream_t stream, const FixArgs &a, const Epi &epi, bool both, int s_lo, int s_hi)
 {
-    const int Vh = a.g.Vh;
-    if ((both ? 2 : 1) * Vh <= kSplitSites) launch_fix<DAG, 0>(ctx->stream, a, epi, both, 0, Vh);
-    else if (Epi::N > 0) launch_fix<DAG, 128>(ctx->stream, a, epi, both, 0, Vh);
-    else if (variant == 1) launch_fix<DAG, 64>(ctx->stream, a, epi, both, 0, Vh);
-    else if (variant == 2) launch_fix<DAG, 32>(ctx->stream, a, epi, both, 0, Vh);
-    else launch_fix<DAG, 128>(ctx->stream, a, epi, both, 0, Vh);
+    if ((both ? 2 : 1) * (s_hi - s_lo) <= kSplitSites) launch_fix<DAG, 0>(stream, a, epi, both, s_lo, s_hi);
+    else launch_fix<DAG, 128>(stream, a, epi, both, s_lo, s_hi);
     WD_LAUNCHED(ctx);
     return WD_OK;
+}
+template <bool DAG, class Epi>
+wd_status run_fix(wd_context *ctx, const FixArgs &a, const Epi &epi, bool both = false)
+{
+    return run_fix<DAG>(ctx, ctx->stream, a, epi, both, 0, a.g.Vh);
+}
+
+// stored hops, in the form their x and alpha ask for
+template <bool AOS>
+wd_status store_fix(wd_context *ctx, cudaStream_t stream, const FixArgs &a, int dag, bool both, int s_lo, int s_hi)
+{
+    auto run = [&](auto epi) {
+        return dag ? run_fix<true>(ctx, stream, a, epi, both, s_lo, s_hi) : run_fix<false>(ctx, stream, a, epi, both, s_lo, s_hi);
+    };
+    if (!a.x) return run(EpiStore<AOS, kPlain>());
+    if (!a.scaled) return run(EpiStore<AOS, kPow2X>());
+    return run(EpiStore<AOS, kScaledX>());
 }
 
 FixArgs fix_args(const wd_lattice *lat, const void *in, void *out, const void *x, int cb, double alpha, double beta,
                  const int *stop = nullptr)
 {
+    const F64Scale f = F64Scale::make(alpha);
+    const bool pow2 = f.mode == 1 || (f.mode == 2 && f.shift >= -60 && f.shift <= 60);
+    const wd_fix::Pow2 pre{pow2 ? f.shift : 0, pow2 && alpha < 0 ? 0x80000000u : 0u};
     return FixArgs{lat->g, cb, (const double2 *)in, lat->gauge, (const double2 *)x, (double2 *)out,
-                   (const int4 *)lat->gauge_fix, alpha, beta, F64Scale::make(alpha), stop, nullptr};
+                   (const int4 *)lat->gauge_fix, alpha, beta, pre, pow2 ? 1.0 : alpha, !pow2, stop, nullptr};
 }
 
 }  // namespace
@@ -304,29 +357,23 @@ wd_status wd_hop_fix(wd_context *ctx, const wd_lattice *lat, const double2 *in, 
 {
     FixArgs a = fix_args(lat, in, out, x, cb, alpha, beta, stop);
     a.zero = zero;
-    auto run = [&](int v) {
-        return dag ? run_fix<true>(ctx, a, EpiStore<false>(), false, v) : run_fix<false>(ctx, a, EpiStore<false>(), false, v);
-    };
-    if (lat->g.Vh <= kSplitSites) {
-        wd_tune_note("hop_f64", 3);
-        return run(0);
-    }
-    return wd_tune_launch(ctx, "hop_f64", lat->g.Vh, 3, run);
+    // one shape (64 and 32 threads a block run within 0.3 % of 128): the
+    // tuner's variants are the FP64-pipe kernel's
+    wd_tune_note("hop_f64", 3);
+    return store_fix<false>(ctx, ctx->stream, a, dag, false, 0, lat->g.Vh);
 }
 
 wd_status wd_hop_fix_M(wd_context *ctx, const wd_lattice *lat, const double2 *in, double2 *out, double mass, int dag,
                        const int *stop)
 {
-    const FixArgs a = fix_args(lat, in, out, in, 0, -0.5, 4.0 + mass, stop);
-    const int v = wd_tune_choice(ctx, "hop_f64", lat->g.Vh);
-    return dag ? run_fix<true>(ctx, a, EpiStore<false>(), true, v) : run_fix<false>(ctx, a, EpiStore<false>(), true, v);
+    return store_fix<false>(ctx, ctx->stream, fix_args(lat, in, out, in, 0, -0.5, 4.0 + mass, stop), dag, true, 0,
+                            lat->g.Vh);
 }
 
 wd_status wd_hop_fix_residual(wd_context *ctx, const wd_lattice *lat, const double2 *in, const double2 *x, double alpha,
                               double beta, const WdResSink &r)
 {
-    return run_fix<false>(ctx, fix_args(lat, in, nullptr, x, 0, alpha, beta), EpiRes{r, r.partial}, false,
-                          wd_tune_choice(ctx, "hop_f64", lat->g.Vh));
+    return run_fix<false>(ctx, fix_args(lat, in, nullptr, x, 0, alpha, beta), EpiRes{r, r.partial});
 }
 
 size_t wd_hop_fix_partials(const wd_lattice *lat) { return 2 * (2 * (size_t)lat->g.Vh / 16 + 2); }
@@ -335,8 +382,7 @@ wd_status wd_hop_fix_norm(wd_context *ctx, const wd_lattice *lat, WdVec in, WdVe
                           double *partial)
 {
     const double a = 4.0 + mass;
-    return run_fix<false>(ctx, fix_args(lat, in.p, t.p, p.p, 0, -0.25 / a, a, &dev->stop), EpiNorm{dev, partial}, false,
-                          wd_tune_choice(ctx, "hop_f64", lat->g.Vh));
+    return run_fix<false>(ctx, fix_args(lat, in.p, t.p, p.p, 0, -0.25 / a, a, &dev->stop), EpiNorm{dev, partial});
 }
 
 wd_status wd_hop_fix_update(wd_context *ctx, const wd_lattice *lat, WdVec in, WdVec t, WdVec p, WdVec r, WdVec x,
@@ -344,30 +390,26 @@ wd_status wd_hop_fix_update(wd_context *ctx, const wd_lattice *lat, WdVec in, Wd
 {
     const double a = 4.0 + mass;
     return run_fix<true>(ctx, fix_args(lat, in.p, nullptr, t.p, 0, -0.25 / a, a, &dev->stop),
-                         EpiUpdate{dev, partial, (const double2 *)p.p, (double2 *)r.p, (double2 *)x.p}, false,
-                         wd_tune_choice(ctx, "hop_f64", lat->g.Vh));
+                         EpiUpdate{dev, partial, (const double2 *)p.p, (double2 *)r.p, (double2 *)x.p});
 }
 
 wd_status wd_hop_fix_M_dot(wd_context *ctx, const wd_lattice *lat, WdVec in, WdVec q, WdVec p, double mass, WdCgDev *dev,
                            double *partial)
 {
     return run_fix<true>(ctx, fix_args(lat, in.p, q.p, in.p, 0, -0.5, 4.0 + mass, &dev->stop),
-                         EpiDot{dev, partial, (const double2 *)p.p}, true,
-                         wd_tune_choice(ctx, "hop_f64", lat->g.Vh));
+                         EpiDot{dev, partial, (const double2 *)p.p}, true);
+}
+
+wd_status wd_hop_fix_M_residual(wd_context *ctx, const wd_lattice *lat, const double2 *b, const double2 *x, double mass,
+                                double *partial, unsigned *counter, double *result)
+{
+    return run_fix<false>(ctx, fix_args(lat, x, nullptr, x, 0, -0.5, 4.0 + mass),
+                          EpiTrueRes{partial, counter, b, result}, true);
 }
 
 wd_status wd_hop_fix_aos_range(wd_context *ctx, cudaStream_t stream, const wd_lattice *lat, const double2 *in_aos,
                                double2 *out_aos, const double2 *x_aos, int cb, int dag, double alpha, double beta,
                                int s_lo, int s_hi)
 {
-    const FixArgs a = fix_args(lat, in_aos, out_aos, x_aos, cb, alpha, beta);
-    auto run = [&](auto d) {
-        constexpr bool D = decltype(d)::value;
-        if (s_hi - s_lo <= kSplitSites) launch_fix<D, 0>(stream, a, EpiStore<true>(), false, s_lo, s_hi);
-        else launch_fix<D, 64>(stream, a, EpiStore<true>(), false, s_lo, s_hi);
-    };
-    if (dag) run(std::true_type());
-    else run(std::false_type());
-    WD_LAUNCHED(ctx);
-    return WD_OK;
+    return store_fix<true>(ctx, stream, fix_args(lat, in_aos, out_aos, x_aos, cb, alpha, beta), dag, false, s_lo, s_hi);
 }

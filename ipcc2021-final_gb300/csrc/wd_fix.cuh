@@ -32,14 +32,16 @@
 // are multiplied (0.472 -> 0.386 ms at 32^3x64); a row's links are read
 // from there when the row is due (0.377).  Complex products take three real
 // ones (Gauss): additions are cheaper than wide multiply-adds here.
-// Measured at 32^3x64: 0.372 ms (FP64 form 1.453 ms), 4.33 TB/s of
-// compulsory bytes, 65 % of measured HBM.  What bounds it now is issue and the
-// integer pipes together (fma-heavy 56 %, FP64 54 %, issue slots 46 % busy at
-// 24^3x48); with every load served by L1 it is no faster.  Dropped:
-// converting with F2I.S64.F64 (0.67 ms: it occupies the FP64 pipe), projecting
-// after conversion on integers (0.458 ms before staging), 20 warps per SM at
-// 96 registers (0.395 ms: the second slot set takes the L1), the next
-// direction's projection ahead of the current product (0.381 ms).
+// Measured at 32^3x64: 0.357 ms (FP64 form 1.453 ms), 4.52 TB/s of
+// compulsory bytes, 68 % of measured HBM; 0.372 ms before the power-of-two
+// factor moved into the final conversion and the site coordinates lost their
+// divisions.  What bounds it now is issue and the integer pipes together
+// (fma-heavy 57 %, FP64 56 %, issue slots 46 % busy at 24^3x48); with every
+// load served by L1 it is no faster.  Dropped: converting with F2I.S64.F64
+// (0.67 ms: it occupies the FP64 pipe), projecting after conversion on
+// integers (0.458 ms before staging), 20 warps per SM at 96 registers (0.395
+// ms against 0.372), the next direction's projection ahead of the current
+// product (0.381 ms).
 #pragma once
 #include "wd_async.cuh"
 #include "wd_hop_f64.cuh"
@@ -264,13 +266,21 @@ __device__ __forceinline__ void dir(const Stage<T> &sm, int slot, int half, doub
     }
 }
 
-// T 2^(E - kUnit) as FP64, T rounded once
-__device__ __forceinline__ double value(long long T, uint32_t E)
+// sign * T 2^(E - kUnit + shift) as FP64, T rounded once; kexp = (E - kUnit +
+// shift) << 20, sign = 0 or the sign bit (exponents here are far from FP64's
+// limits: see the ranges above)
+__device__ __forceinline__ double value(long long T, int kexp, uint32_t sign)
 {
     const double v = (double)T;
     const int hi = __double2hiint(v);
-    return hi ? __hiloint2double(hi + (((int)E - kUnit) << 20), __double2loint(v)) : 0.0;
+    return hi ? __hiloint2double((int)((uint32_t)(hi + kexp) ^ sign), __double2loint(v)) : 0.0;
 }
+
+// a power-of-two factor of the result, applied on the exponent: sign 2^shift
+struct Pow2 {
+    int shift;      // |shift| <= 60
+    uint32_t sign;
+};
 
 __device__ __forceinline__ bool in_range(uint32_t E, uint32_t tiny)
 {
@@ -285,11 +295,11 @@ __device__ __forceinline__ void clear(Acc &A)
     A.E = kExpTiny;
 }
 
-// The hopping term at site s for the thread pair (half = 0, 1): v[0..2] is
-// spin `half`, v[3..5] spin 3 - half.  Returns false when the site's values
+// f times the hopping term at site s for the thread pair (half = 0, 1):
+// v[0..2] is spin `half`, v[3..5] spin 3 - half.  Returns false when the site's values
 // need the FP64 route (then v is not to be used).
 template <bool DAG, int T, bool AOS>
-__device__ __forceinline__ bool site(const Operands<AOS> &p, Stage<T> &sm, int s, int half, double2 *v)
+__device__ __forceinline__ bool site(const Operands<AOS> &p, Stage<T> &sm, int s, int half, Pow2 f, double2 *v)
 {
     const WdSite c = wd_site(p.g, s, p.cb);
     const double sigma = half ? -1.0 : 1.0;
@@ -317,12 +327,13 @@ __device__ __forceinline__ bool site(const Operands<AOS> &p, Stage<T> &sm, int s
     both(std::integral_constant<int, 2>());
     both(std::integral_constant<int, 3>());
     const uint32_t tiny = A.tiny | __shfl_xor_sync(0xffffffffu, A.tiny, 1);
+    const int kexp = ((int)A.E - kUnit + f.shift) << 20;
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
         const long long lr = A.P[2 * k] + __shfl_xor_sync(0xffffffffu, A.Q[2 * k], 1);
         const long long li = A.P[2 * k + 1] + __shfl_xor_sync(0xffffffffu, A.Q[2 * k + 1], 1);
-        v[k] = make_double2(value(A.o[2 * k], A.E), value(A.o[2 * k + 1], A.E));
-        v[3 + k] = make_double2(value(lr, A.E), value(li, A.E));
+        v[k] = make_double2(value(A.o[2 * k], kexp, f.sign), value(A.o[2 * k + 1], kexp, f.sign));
+        v[3 + k] = make_double2(value(lr, kexp, f.sign), value(li, kexp, f.sign));
     }
     return in_range(A.E, tiny);
 }
@@ -343,7 +354,7 @@ struct Split {
 };
 
 template <bool DAG, bool AOS>
-__device__ __forceinline__ bool site_split(const Operands<AOS> &p, Split &sm, int s, int half, double2 *v)
+__device__ __forceinline__ bool site_split(const Operands<AOS> &p, Split &sm, int s, int half, Pow2 f, double2 *v)
 {
     const WdSite c = wd_site(p.g, s, p.cb);
     const double sigma = half ? -1.0 : 1.0;
@@ -390,8 +401,9 @@ __device__ __forceinline__ bool site_split(const Operands<AOS> &p, Split &sm, in
             t[2] += b.x >> d;
             t[3] += b.y >> d;
         }
-        v[0] = make_double2(value(t[0], E), value(t[1], E));
-        v[1] = make_double2(value(t[2], E), value(t[3], E));
+        const int kexp = ((int)E - kUnit + f.shift) << 20;
+        v[0] = make_double2(value(t[0], kexp, f.sign), value(t[1], kexp, f.sign));
+        v[1] = make_double2(value(t[2], kexp, f.sign), value(t[3], kexp, f.sign));
     }
     return in_range(E, tiny);
 }

@@ -27,10 +27,30 @@ constexpr size_t WD_STATE_HOST_BYTES = 4096;
 constexpr int WD_MAX_CHUNKS = 16;
 constexpr int WD_MAX_UPLOADS = 32;
 
+// n / d for 0 <= n < 2^29 without a division: m = ceil(2^(31+c) / d), c the
+// smallest with d <= 2^c, n / d = (2n m) >> (32 + c).  Exact: m d - 2^(31+c)
+// < d <= 2^c, so n times that stays below 2^(31+c).
+struct WdDiv {
+    uint32_t m = 1u << 31;
+    int c = 0;
+    int d = 1;
+    WdDiv() = default;
+    explicit WdDiv(int div) : d(div)
+    {
+        while ((int64_t(1) << c) < d) ++c;
+        m = (uint32_t)(((uint64_t(1) << (31 + c)) + d - 1) / d);
+    }
+#ifdef __CUDACC__
+    __device__ __forceinline__ int div(int n) const { return (int)(__umulhi(2u * (uint32_t)n, m) >> c); }
+#endif
+};
+
 struct WdGeom {
     int L[4];  // Lx, Ly, Lz, Lt
     int Lxh;   // Lx / 2
     int Vh;    // sites per parity
+    WdDiv dx, dy, dz;  // by Lxh, Ly, Lz: four instructions each of the hop kernels' site coordinates
+                       // instead of about twenty (the FP16 hop issues 1622 per site)
 };
 
 struct wd_context {
@@ -183,12 +203,11 @@ struct WdSite {
 __device__ __forceinline__ WdSite wd_site(const WdGeom &g, int s, int p)
 {
     WdSite c;
-    c.xh = s % g.Lxh;
-    int r = s / g.Lxh;
-    c.y = r % g.L[1];
-    r /= g.L[1];
-    c.z = r % g.L[2];
-    c.t = r / g.L[2];
+    const int ry = g.dx.div(s), rz = g.dy.div(ry);
+    c.xh = s - ry * g.Lxh;
+    c.y = ry - rz * g.L[1];
+    c.t = g.dz.div(rz);
+    c.z = rz - c.t * g.L[2];
     c.xodd = (c.y + c.z + c.t + p) & 1;
     return c;
 }

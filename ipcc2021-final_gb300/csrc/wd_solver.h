@@ -21,8 +21,8 @@ wd_status wd_apply_M_v(wd_context *ctx, const wd_lattice *lat, WdVec in, WdVec o
 wd_status wd_apply_Mhat_v(wd_context *ctx, const wd_lattice *lat, WdVec v, WdVec out, WdVec tmp_o, double mass,
                           int dag);
 // |b - M x| / |b| in FP64
-wd_status wd_true_residual(wd_context *ctx, const wd_lattice *lat, const double2 *b, const double2 *x, double2 *tmp,
-                           double mass, double *rel);
+wd_status wd_true_residual(wd_context *ctx, const wd_lattice *lat, const double2 *b, const double2 *x, double mass,
+                           double *rel);
 // mixed-precision (FP32 / FP16 inner) even-odd CG with reliable updates
 wd_status wd_solve_cg_eo_mixed(wd_context *ctx, const wd_lattice *lat, const double2 *src, double2 *x,
                                const wd_solver_params *prm, wd_solver_stats *stats);
@@ -142,6 +142,9 @@ wd_status wd_hop_fix_norm(wd_context *ctx, const wd_lattice *lat, WdVec in, WdVe
 //   q = -D_eo^dag in / (4a) + a t, not stored: r -= alpha q, x += alpha p, |r|^2 -> beta or the gate
 wd_status wd_hop_fix_update(wd_context *ctx, const wd_lattice *lat, WdVec in, WdVec t, WdVec p, WdVec r, WdVec x,
                             double mass, WdCgDev *dev, double *partial);
+//   |b - M x|^2 and |b|^2 -> result[0], result[1] (device); counter: zero at launch
+wd_status wd_hop_fix_M_residual(wd_context *ctx, const wd_lattice *lat, const double2 *b, const double2 *x, double mass,
+                                double *partial, unsigned *counter, double *result);
 //   q = M^dag in on the whole lattice, (p, q) -> alpha
 wd_status wd_hop_fix_M_dot(wd_context *ctx, const wd_lattice *lat, WdVec in, WdVec q, WdVec p, double mass, WdCgDev *dev,
                            double *partial);
