@@ -553,7 +553,7 @@ wd_status BatchEngine::add(int tag, const wd_lattice *lat, const double2 *src, d
         if ((st = wd_vec_alloc(ctx_, *b, H_, nh)) != WD_OK) return st;
     for (WdVecBuf *b : {&B.hs, &B.hx})
         if ((st = wd_vec_alloc(ctx_, *b, H_, 2 * nh)) != WD_OK) return st;
-    if ((st = wd_vec_alloc(ctx_, B.rel, WD_PREC_F64, (int64_t)(wd_mx_reliable_scratch_doubles(Vh) + 1) / 2)) != WD_OK)
+    if ((st = wd_vec_alloc(ctx_, B.rel, WD_PREC_F64, (int64_t)(wd_red_doubles(wd_red_blocks(Vh), 1) + 1) / 2)) != WD_OK)
         return st;
     if ((st = wd_lattice_gauge_lp(ctx_, lat, L_)) != WD_OK) return st;
     if (H_ == WD_PREC_DF64) {

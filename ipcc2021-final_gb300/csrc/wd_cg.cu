@@ -58,19 +58,19 @@ __device__ __forceinline__ typename V::R norm_acc(typename V::R s, typename V::C
 
 template <class V>
 __global__ void __launch_bounds__(WD_RED_THREADS) k_cgd_norm(const typename V::E *__restrict__ t, int64_t n, WdCgDev *dev,
-                                                             double *partial)
+                                                             WdRed red)
 {
     if (dev->stop) return;
     typename V::R s = V::zero();
     GRID_STRIDE(i, n) s = norm_acc<V>(s, V::load(t[i]));
     double tot;
-    if (wd_grid_sum<WD_RED_THREADS>(V::value(s), partial, &dev->count_a, &tot)) wd_cg_set_alpha(dev, tot, 0.0, false);
+    if (wd_grid_sum<WD_RED_THREADS>(V::value(s), red, &tot)) wd_cg_set_alpha(dev, tot, 0.0, false);
 }
 
 template <class V>
 __global__ void __launch_bounds__(WD_RED_THREADS) k_cgd_dot(const typename V::E *__restrict__ p,
                                                             const typename V::E *__restrict__ q, int64_t n, WdCgDev *dev,
-                                                            double *partial)
+                                                            WdRed red)
 {
     if (dev->stop) return;
     typename V::R re = V::zero(), im = V::zero();
@@ -81,7 +81,7 @@ __global__ void __launch_bounds__(WD_RED_THREADS) k_cgd_dot(const typename V::E 
         im = V::madd(V::madd(im, V::re(u), V::im(v)), V::neg(V::im(u)), V::re(v));
     }
     double t[2];
-    if (wd_grid_sum_n<WD_RED_THREADS, 2>({V::value(re), V::value(im)}, partial, &dev->count_a, t))
+    if (wd_grid_sum_n<WD_RED_THREADS, 2>({V::value(re), V::value(im)}, red, t))
         wd_cg_set_alpha(dev, t[0], t[1], true);
 }
 
@@ -90,7 +90,7 @@ __global__ void __launch_bounds__(WD_RED_THREADS) k_cgd_update(const typename V:
                                                                const typename V::E *__restrict__ q,
                                                                typename V::E *__restrict__ x,
                                                                typename V::E *__restrict__ r, int64_t n, WdCgDev *dev,
-                                                               double *partial)
+                                                               WdRed red)
 {
     if (dev->stop) return;
     const typename V::R re = V::real(dev->are), im = V::real(dev->aim), mre = V::neg(re), mim = V::neg(im);
@@ -106,7 +106,7 @@ __global__ void __launch_bounds__(WD_RED_THREADS) k_cgd_update(const typename V:
         s = norm_acc<V>(s, rv);
     }
     double tot;
-    if (wd_grid_sum<WD_RED_THREADS>(V::value(s), partial, &dev->count_r, &tot)) wd_cg_set_beta(dev, tot);
+    if (wd_grid_sum<WD_RED_THREADS>(V::value(s), red, &tot)) wd_cg_set_beta(dev, tot);
 }
 
 template <class V>
@@ -139,33 +139,33 @@ wd_status typed(wd_context *ctx, WdVec v, F f)
 
 }  // namespace
 
-wd_status wd_cgd_norm(wd_context *ctx, WdVec t, int64_t n, WdCgDev *dev, double *partial)
+wd_status wd_cgd_norm(wd_context *ctx, WdVec t, int64_t n, WdCgDev *dev, WdRed red)
 {
     return typed(ctx, t, [&](auto v) {
         using V = decltype(v);
-        k_cgd_norm<V><<<red_blocks(n), WD_RED_THREADS, 0, ctx->stream>>>((const typename V::E *)t.p, n, dev, partial);
+        k_cgd_norm<V><<<red_blocks(n), WD_RED_THREADS, 0, ctx->stream>>>((const typename V::E *)t.p, n, dev, red);
     });
 }
 
-wd_status wd_cgd_dot(wd_context *ctx, WdVec p, WdVec q, int64_t n, WdCgDev *dev, double *partial)
+wd_status wd_cgd_dot(wd_context *ctx, WdVec p, WdVec q, int64_t n, WdCgDev *dev, WdRed red)
 {
     return typed(ctx, p, [&](auto v) {
         using V = decltype(v);
         using E = typename V::E;
-        k_cgd_dot<V><<<red_blocks(n), WD_RED_THREADS, 0, ctx->stream>>>((const E *)p.p, (const E *)q.p, n, dev, partial);
+        k_cgd_dot<V><<<red_blocks(n), WD_RED_THREADS, 0, ctx->stream>>>((const E *)p.p, (const E *)q.p, n, dev, red);
     });
 }
 
 wd_status wd_cgd_update(wd_context *ctx, bool cplx, WdVec p, WdVec q, WdVec x, WdVec r, int64_t n, WdCgDev *dev,
-                        double *partial)
+                        WdRed red)
 {
     return typed(ctx, p, [&](auto v) {
         using V = decltype(v);
         using E = typename V::E;
         const E *pp = (const E *)p.p, *qq = (const E *)q.p;
         E *xx = (E *)x.p, *rr = (E *)r.p;
-        if (cplx) k_cgd_update<V, true><<<red_blocks(n), WD_RED_THREADS, 0, ctx->stream>>>(pp, qq, xx, rr, n, dev, partial);
-        else k_cgd_update<V, false><<<red_blocks(n), WD_RED_THREADS, 0, ctx->stream>>>(pp, qq, xx, rr, n, dev, partial);
+        if (cplx) k_cgd_update<V, true><<<red_blocks(n), WD_RED_THREADS, 0, ctx->stream>>>(pp, qq, xx, rr, n, dev, red);
+        else k_cgd_update<V, false><<<red_blocks(n), WD_RED_THREADS, 0, ctx->stream>>>(pp, qq, xx, rr, n, dev, red);
     });
 }
 

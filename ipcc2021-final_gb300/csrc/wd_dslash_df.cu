@@ -431,8 +431,7 @@ __global__ void __launch_bounds__(96 * GROUPS, MINB) k_hop_df_grouped(const Spli
 struct ResSinkDF {
     const float4 *bhat;
     float4 *s32;
-    double *partial;
-    unsigned *counter;
+    WdRed red;
     double *result;
 };
 
@@ -462,7 +461,7 @@ __global__ void __launch_bounds__(32 * WARPS, MINB) k_hop_df_res(const SplitDF p
         }
     }
     double tot;
-    if (wd_grid_sum<32 * WARPS>((double)n, r.partial, r.counter, &tot)) *r.result = tot;
+    if (wd_grid_sum<32 * WARPS>((double)n, r.red, &tot)) *r.result = tot;
 }
 
 __global__ void k_f64_to_df(const double2 *__restrict__ in, float4 *__restrict__ out, int64_t n)
@@ -566,7 +565,7 @@ wd_status wd_hop_df(wd_context *ctx, const wd_lattice *lat, const float4 *in_blo
 }
 
 wd_status wd_hop_df_residual(wd_context *ctx, const wd_lattice *lat, const float4 *in_block, const float4 *x_block,
-                             const float4 *bhat, float4 *s32, double mass, double *partial, unsigned *counter,
+                             const float4 *bhat, float4 *s32, double mass, WdRed red,
                              double *result)
 {
     wd_status st = wd_lattice_gauge_df(ctx, lat);
@@ -581,7 +580,7 @@ wd_status wd_hop_df_residual(wd_context *ctx, const wd_lattice *lat, const float
     p.out = nullptr;
     p.alpha = df_split(-0.25 / a);
     p.beta = df_split(a);
-    const ResSinkDF r{bhat, s32, partial, counter, result};
+    const ResSinkDF r{bhat, s32, red, result};
     auto run = [&](auto warps, auto lcg) -> wd_status {
         constexpr int W = decltype(warps)::value;
         const int sites_per_block = kSitesPerWarp * W;

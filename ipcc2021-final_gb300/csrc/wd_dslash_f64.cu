@@ -45,26 +45,26 @@ __global__ void __launch_bounds__(P::kThreads) k_hop_f64_res(const P p, const Wd
         }
     }
     double tot;
-    if (wd_grid_sum<P::kThreads>((double)n, r.partial, r.counter, &tot)) *r.result = tot;
+    if (wd_grid_sum<P::kThreads>((double)n, r.red, &tot)) *r.result = tot;
 }
 
 }  // namespace
 
 wd_status wd_hop_df_residual(wd_context *ctx, const wd_lattice *lat, const float4 *in_block, const float4 *x_block,
-                             const float4 *bhat, float4 *s32, double mass, double *partial, unsigned *counter,
+                             const float4 *bhat, float4 *s32, double mass, WdRed red,
                              double *result);
 
 wd_status wd_hop_hi_residual(wd_context *ctx, const wd_lattice *lat, WdVec in, WdVec x, WdVec bhat, WdVec s32,
-                             double mass, double *partial, unsigned *counter, double *result)
+                             double mass, WdRed red, double *result)
 {
     if (in.prec != x.prec || in.prec != bhat.prec || s32.prec != WD_PREC_F32)
         return wd_fail(ctx, WD_ERR_BAD_ARG, "residual hop: in, x, bhat of one storage, s32 FP32");
     const double a = 4.0 + mass;
     if (in.prec == WD_PREC_DF64)
         return wd_hop_df_residual(ctx, lat, (const float4 *)in.p, (const float4 *)x.p, (const float4 *)bhat.p,
-                                  (float4 *)s32.p, mass, partial, counter, result);
+                                  (float4 *)s32.p, mass, red, result);
     if (in.prec != WD_PREC_F64) return wd_fail(ctx, WD_ERR_BAD_ARG, "residual hop: FP64 or double-float storage");
-    const WdResSink r{(const double2 *)bhat.p, (float4 *)s32.p, partial, counter, result};
+    const WdResSink r{(const double2 *)bhat.p, (float4 *)s32.p, red, result};
     if (lat->gauge_fix)
         return wd_hop_fix_residual(ctx, lat, (const double2 *)in.p, (const double2 *)x.p, -0.25 / a, a, r);
     auto run = [&](auto tag) -> wd_status {

@@ -134,8 +134,7 @@ struct EpiNorm {
     static constexpr int N = 1;
     using Num = double;
     WdCgDev *dev;
-    double *partial;
-    __device__ __forceinline__ unsigned *counter() const { return &dev->count_a; }
+    WdRed red;
     __device__ __forceinline__ void put(const FixArgs &a, const FixView &w, int c, int s, double2 v, double *n) const
     {
         const size_t i = entry<false>(a, c, s);
@@ -151,10 +150,9 @@ struct EpiUpdate {
     static constexpr int N = 1;
     using Num = double;
     WdCgDev *dev;
-    double *partial;
+    WdRed red;
     const double2 *p;
     double2 *r, *y;
-    __device__ __forceinline__ unsigned *counter() const { return &dev->count_r; }
     __device__ __forceinline__ void put(const FixArgs &a, const FixView &w, int c, int s, double2 v, double *n) const
     {
         const size_t i = entry<false>(a, c, s);
@@ -175,9 +173,8 @@ struct EpiDot {
     static constexpr int N = 2;
     using Num = double;
     WdCgDev *dev;
-    double *partial;
+    WdRed red;
     const double2 *p;
-    __device__ __forceinline__ unsigned *counter() const { return &dev->count_a; }
     __device__ __forceinline__ void put(const FixArgs &a, const FixView &w, int c, int s, double2 v, double *n) const
     {
         const size_t i = entry<false>(a, c, s);
@@ -195,9 +192,8 @@ struct EpiRes {
     static constexpr bool AOS = false;
     static constexpr int N = 1;
     using Num = float;
+    WdRed red;
     WdResSink r;
-    double *partial;
-    __device__ __forceinline__ unsigned *counter() const { return r.counter; }
     __device__ __forceinline__ void put(const FixArgs &a, const FixView &w, int c, int s, double2 v, float *n) const
     {
         const size_t i = entry<false>(a, c, s);
@@ -215,11 +211,9 @@ struct EpiTrueRes {
     static constexpr bool AOS = false;
     static constexpr int N = 2;
     using Num = double;
-    double *partial;
-    unsigned *count;
+    WdRed red;
     const double2 *b;
     double *result;
-    __device__ __forceinline__ unsigned *counter() const { return count; }
     __device__ __forceinline__ void put(const FixArgs &a, const FixView &w, int c, int s, double2 v, double *n) const
     {
         const size_t i = entry<false>(a, c, s);
@@ -286,7 +280,7 @@ __global__ void __launch_bounds__(block_threads(T), 512 / block_threads(T))
         double d[Epi::N], t[Epi::N];
 #pragma unroll
         for (int k = 0; k < Epi::N; ++k) d[k] = (double)n[k];
-        if (wd_grid_sum_n<B, Epi::N>(d, epi.partial, epi.counter(), t)) epi.finish(t);
+        if (wd_grid_sum_n<B, Epi::N>(d, epi.red, t)) epi.finish(t);
     }
 }
 
@@ -373,38 +367,36 @@ wd_status wd_hop_fix_M(wd_context *ctx, const wd_lattice *lat, const double2 *in
 wd_status wd_hop_fix_residual(wd_context *ctx, const wd_lattice *lat, const double2 *in, const double2 *x, double alpha,
                               double beta, const WdResSink &r)
 {
-    return run_fix<false>(ctx, fix_args(lat, in, nullptr, x, 0, alpha, beta), EpiRes{r, r.partial});
+    return run_fix<false>(ctx, fix_args(lat, in, nullptr, x, 0, alpha, beta), EpiRes{r.red, r});
 }
 
-size_t wd_hop_fix_partials(const wd_lattice *lat) { return 2 * (2 * (size_t)lat->g.Vh / 16 + 2); }
-
 wd_status wd_hop_fix_norm(wd_context *ctx, const wd_lattice *lat, WdVec in, WdVec t, WdVec p, double mass, WdCgDev *dev,
-                          double *partial)
+                          WdRed red)
 {
     const double a = 4.0 + mass;
-    return run_fix<false>(ctx, fix_args(lat, in.p, t.p, p.p, 0, -0.25 / a, a, &dev->stop), EpiNorm{dev, partial});
+    return run_fix<false>(ctx, fix_args(lat, in.p, t.p, p.p, 0, -0.25 / a, a, &dev->stop), EpiNorm{dev, red});
 }
 
 wd_status wd_hop_fix_update(wd_context *ctx, const wd_lattice *lat, WdVec in, WdVec t, WdVec p, WdVec r, WdVec x,
-                            double mass, WdCgDev *dev, double *partial)
+                            double mass, WdCgDev *dev, WdRed red)
 {
     const double a = 4.0 + mass;
     return run_fix<true>(ctx, fix_args(lat, in.p, nullptr, t.p, 0, -0.25 / a, a, &dev->stop),
-                         EpiUpdate{dev, partial, (const double2 *)p.p, (double2 *)r.p, (double2 *)x.p});
+                         EpiUpdate{dev, red, (const double2 *)p.p, (double2 *)r.p, (double2 *)x.p});
 }
 
 wd_status wd_hop_fix_M_dot(wd_context *ctx, const wd_lattice *lat, WdVec in, WdVec q, WdVec p, double mass, WdCgDev *dev,
-                           double *partial)
+                           WdRed red)
 {
     return run_fix<true>(ctx, fix_args(lat, in.p, q.p, in.p, 0, -0.5, 4.0 + mass, &dev->stop),
-                         EpiDot{dev, partial, (const double2 *)p.p}, true);
+                         EpiDot{dev, red, (const double2 *)p.p}, true);
 }
 
 wd_status wd_hop_fix_M_residual(wd_context *ctx, const wd_lattice *lat, const double2 *b, const double2 *x, double mass,
-                                double *partial, unsigned *counter, double *result)
+                                WdRed red, double *result)
 {
     return run_fix<false>(ctx, fix_args(lat, x, nullptr, x, 0, -0.5, 4.0 + mass),
-                          EpiTrueRes{partial, counter, b, result}, true);
+                          EpiTrueRes{red, b, result}, true);
 }
 
 wd_status wd_hop_fix_aos_range(wd_context *ctx, cudaStream_t stream, const wd_lattice *lat, const double2 *in_aos,

@@ -494,10 +494,9 @@ wd_status wd_spinor_h16_to_ref(wd_context *ctx, const WdGeom &g, WdVec f, double
 // ===================================================================
 // Reducing operator steps of the mixed-precision CG (wd_mixed.cu): the
 // second hop of t = Mhat p also reduces |t|^2, the second hop of
-// q = Mhat^dag t applies the CG update instead of storing q.  One block
-// partial per block; the last block to finish (a one-shot atomic counter, no
-// waiting) folds the partials in a fixed order -- the result does not depend
-// on which block finishes last -- and updates the solver's device scalars.
+// q = Mhat^dag t applies the CG update instead of storing q.  The last block
+// of the grid sum (wd_grid_sum: no waiting, fixed order) updates the solver's
+// device scalars.
 namespace {
 
 // kEpiNorm / kEpiUpdate: the CG iteration's steps (device scalars in dev);
@@ -507,8 +506,7 @@ enum { kEpiNorm = 0, kEpiUpdate = 1, kEpiNormResult = 2 };
 template <class Sp, class Lk, int THREADS, int MINB, int EPI>
 struct HopLPRed : HopLP<Sp, Lk, THREADS, MINB> {
     WdMxDev *dev;
-    double *partial;
-    unsigned *counter;  // kEpiNormResult
+    WdRed red;
     double *result;     // kEpiNormResult
     Sp pvec;       // update: p at the output site (x_s += alpha p)
     SpF32 rs, xs;  // update: iterated residual and solution increment
@@ -606,9 +604,8 @@ __global__ void __launch_bounds__(P::kThreads, wd_min_blocks<P>::value) k_hop_lp
     if (EPI != kEpiNormResult && p.dev->stop) return;  // the same value in every block of the launch
     const int s = blockIdx.x * T + threadIdx.x;
     const float v = red_site<DAG, STAGED, EPI>(p, s);
-    unsigned *counter = EPI == kEpiNorm ? &p.dev->count_t : EPI == kEpiUpdate ? &p.dev->count_r : p.counter;
     double tot;
-    if (!wd_grid_sum<T>((double)v, p.partial, counter, &tot)) return;
+    if (!wd_grid_sum<T>((double)v, p.red, &tot)) return;
     if constexpr (EPI == kEpiNorm) mx_fin_norm(p.dev, tot);
     else if constexpr (EPI == kEpiUpdate) mx_fin_update(p.dev, tot);
     else *p.result = tot;
@@ -619,8 +616,7 @@ __global__ void __launch_bounds__(P::kThreads, wd_min_blocks<P>::value) k_hop_lp
 // reduction partials and bits; mixed FP16 solves 0.8-1.2 % faster with it)
 template <int EPI, class Sp, class Lk>
 wd_status launch_red(wd_context *ctx, const char *name, const HopLP<Sp, Lk> &b, int dag, WdMxDev *dev,
-                     double *partial, Sp pvec, SpF32 rs, SpF32 xs, unsigned *counter = nullptr,
-                     double *result = nullptr)
+                     WdRed red, Sp pvec, SpF32 rs, SpF32 xs, double *result = nullptr)
 {
     constexpr bool kF16 = std::is_same_v<Sp, SpF16>;
     int v = wd_tune_choice(ctx, name, b.g.Vh);
@@ -631,8 +627,8 @@ wd_status launch_red(wd_context *ctx, const char *name, const HopLP<Sp, Lk> &b, 
         HopLPRed<Sp, Lk, TH, MB, EPI> q;
         q.g = b.g, q.cb = b.cb, q.in = b.in, q.out = b.out, q.x = b.x, q.link = b.link;
         q.has_x = true, q.alpha = b.alpha, q.beta = b.beta;
-        q.dev = dev, q.partial = partial, q.pvec = pvec, q.rs = rs, q.xs = xs;
-        q.counter = counter, q.result = result;
+        q.dev = dev, q.red = red, q.pvec = pvec, q.rs = rs, q.xs = xs;
+        q.result = result;
         const int blocks = (b.g.Vh + TH - 1) / TH;
         if (dag) k_hop_lp_red<true, ST, EPI><<<blocks, TH, 0, ctx->stream>>>(q);
         else k_hop_lp_red<false, ST, EPI><<<blocks, TH, 0, ctx->stream>>>(q);
@@ -673,7 +669,7 @@ HopLP<Sp, Lk> red_base(const wd_lattice *lat, Sp in, Sp out, Sp x, Lk link, doub
 
 template <int EPI>
 wd_status hop_lp_red(wd_context *ctx, const wd_lattice *lat, WdVec in, WdVec out, WdVec x, WdVec p, WdVec rs,
-                     WdVec xs, double mass, int dag, WdMxDev *dev, double *partial)
+                     WdVec xs, double mass, int dag, WdMxDev *dev, WdRed red)
 {
     const int Vh = lat->g.Vh;
     if (in.prec != x.prec || in.prec != p.prec || (in.prec != WD_PREC_F32 && in.prec != WD_PREC_F16))
@@ -684,33 +680,33 @@ wd_status hop_lp_red(wd_context *ctx, const wd_lattice *lat, WdVec in, WdVec out
     if (in.prec == WD_PREC_F32) {
         const LinkF32 lk{(const float4 *)lat->gauge_f32, Vh};
         return launch_red<EPI>(ctx, "hop_f32", red_base(lat, sp_f32(in, Vh), sp_f32(out, Vh), sp_f32(x, Vh), lk, mass),
-                               dag, dev, partial, sp_f32(p, Vh), r32, x32);
+                               dag, dev, red, sp_f32(p, Vh), r32, x32);
     }
     const uint4 *a = (const uint4 *)lat->gauge_h12;
     const LinkF16 lk{a, (const uint2 *)(a + (size_t)8 * Vh), Vh};
     return launch_red<EPI>(ctx, "hop_f16", red_base(lat, sp_f16(in, Vh), sp_f16(out, Vh), sp_f16(x, Vh), lk, mass), dag,
-                           dev, partial, sp_f16(p, Vh), r32, x32);
+                           dev, red, sp_f16(p, Vh), r32, x32);
 }
 
 }  // namespace
 
 wd_status wd_hop_lp_norm(wd_context *ctx, const wd_lattice *lat, WdVec in, WdVec t, WdVec p, double mass,
-                         WdMxDev *dev, double *partial)
+                         WdMxDev *dev, WdRed red)
 {
     WdVec none;
     none.prec = WD_PREC_F32;
-    return hop_lp_red<kEpiNorm>(ctx, lat, in, t, p, p, none, none, mass, 0, dev, partial);
+    return hop_lp_red<kEpiNorm>(ctx, lat, in, t, p, p, none, none, mass, 0, dev, red);
 }
 
 wd_status wd_hop_lp_update(wd_context *ctx, const wd_lattice *lat, WdVec in, WdVec t, WdVec p, WdVec rs, WdVec xs,
-                           double mass, WdMxDev *dev, double *partial)
+                           double mass, WdMxDev *dev, WdRed red)
 {
     // out is not written by the update epilogue
-    return hop_lp_red<kEpiUpdate>(ctx, lat, in, t, t, p, rs, xs, mass, 1, dev, partial);
+    return hop_lp_red<kEpiUpdate>(ctx, lat, in, t, t, p, rs, xs, mass, 1, dev, red);
 }
 
 wd_status wd_hop_f32_norm(wd_context *ctx, const wd_lattice *lat, WdVec in, WdVec out, WdVec x, double mass, int dag,
-                          double *partial, unsigned *counter, double *result)
+                          WdRed red, double *result)
 {
     const int Vh = lat->g.Vh;
     if (in.prec != WD_PREC_F32 || out.prec != WD_PREC_F32 || x.prec != WD_PREC_F32)
@@ -721,5 +717,5 @@ wd_status wd_hop_f32_norm(wd_context *ctx, const wd_lattice *lat, WdVec in, WdVe
     const SpF32 none = sp_f32(out, Vh);
     return launch_red<kEpiNormResult>(ctx, "hop_f32",
                                       red_base(lat, sp_f32(in, Vh), sp_f32(out, Vh), sp_f32(x, Vh), lk, mass), dag,
-                                      nullptr, partial, none, none, none, counter, result);
+                                      nullptr, red, none, none, none, result);
 }

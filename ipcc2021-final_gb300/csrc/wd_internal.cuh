@@ -130,6 +130,28 @@ struct wd_field {
     double2 *d = nullptr;     // == data for FP64 storage, else null
 };
 
+// Work space of a grid reduction (wd_grid_sum_n): the blocks' partials, then
+// the groups', and one counter per group of blocks after one for the groups.
+// The counters are zero before the first launch and every launch leaves them
+// zero.
+constexpr int kRedGroup = 1024;  // blocks per group (256 gave 8^3x16 launches a second level: 1 us each)
+struct WdRed {
+    double *partial = nullptr;
+    unsigned *counters = nullptr;
+};
+// doubles of a work space for up to `blocks` blocks of `n` sums each, and the view of one
+inline size_t wd_red_counters(int64_t blocks) { return (size_t)(blocks / kRedGroup + 3); }
+inline size_t wd_red_doubles(int64_t blocks, int n)
+{
+    return (wd_red_counters(blocks) + 1) / 2 + (size_t)n * (blocks + blocks / kRedGroup + 1);
+}
+inline WdRed wd_red_view(void *mem, int64_t blocks)
+{
+    return WdRed{(double *)mem + (wd_red_counters(blocks) + 1) / 2, (unsigned *)mem};
+}
+// blocks of any reducing hop kernel on a lattice (16 sites each, both parities), or of the vector passes
+inline int64_t wd_red_blocks(int Vh) { return Vh / 8 + 2 > 1216 ? Vh / 8 + 2 : 1216; }
+
 // A typed view of a spinor array (one parity block or a whole field).
 struct WdVec {
     void *p = nullptr;

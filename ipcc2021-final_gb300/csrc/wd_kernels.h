@@ -23,12 +23,11 @@ wd_status wd_gauge_ref_to_soa_fix(wd_context *ctx, const WdGeom &g, int mu, cons
 // FP64 pipe); true if there were any.  For allocations that fail otherwise.
 bool wd_release_fix(wd_context *ctx);
 void wd_drop_fix(wd_lattice *lat);
-// a residual hop's outputs: s32 = FP32(bhat - hop), block partials, |s32|^2
+// a residual hop's outputs: s32 = FP32(bhat - hop), |s32|^2
 struct WdResSink {
     const double2 *bhat;
     float4 *s32;
-    double *partial;
-    unsigned *counter;
+    WdRed red;
     double *result;
 };
 // (the lattice has gauge_fix; stop as for the other hops; zero: a parity block
@@ -102,22 +101,21 @@ struct WdMxDev;
 //  * update: q = -D_eo^dag in / (4a) + a t (in = D_oe^dag t), not stored:
 //            rs -= alpha q, xs += alpha p, and |rs|^2 reduced; the last block
 //            applies the reliable-update rule (wd_solver.h).
-// partial: at least Vh/64 + 1 doubles.  Both are no-ops while dev->stop != 0.
+// Both are no-ops while dev->stop != 0.
 wd_status wd_hop_lp_norm(wd_context *ctx, const wd_lattice *lat, WdVec in, WdVec t, WdVec p, double mass,
-                         WdMxDev *dev, double *partial);
+                         WdMxDev *dev, WdRed red);
 wd_status wd_hop_lp_update(wd_context *ctx, const wd_lattice *lat, WdVec in, WdVec t, WdVec p, WdVec rs, WdVec xs,
-                           double mass, WdMxDev *dev, double *partial);
+                           double mass, WdMxDev *dev, WdRed red);
 // The reliable update's reducing steps (even outputs, Schur operator second
-// hops).  partial: at least Vh/16 + 1 doubles; counter: zero at launch (the
-// last block resets it).
+// hops).
 //  * FP32: out = a x - D_eo in / (4a) (D^dag with dag), stored; |out|^2 -> *result
 wd_status wd_hop_f32_norm(wd_context *ctx, const wd_lattice *lat, WdVec in, WdVec out, WdVec x, double mass, int dag,
-                          double *partial, unsigned *counter, double *result);
+                          WdRed red, double *result);
 //  * high precision (FP64 or double-float storage of in, x, bhat): the true
 //    residual s = bhat - (a x - D_eo in / (4a)) of the Schur system, rounded
 //    to FP32 into s32 (FP32 storage), and |s32|^2 -> *result
 wd_status wd_hop_hi_residual(wd_context *ctx, const wd_lattice *lat, WdVec in, WdVec x, WdVec bhat, WdVec s32,
-                             double mass, double *partial, unsigned *counter, double *result);
+                             double mass, WdRed red, double *result);
 // FP64 block [12][Vh] <-> low-precision block; accumulate != 0 adds into out
 wd_status wd_lp_from_f64(wd_context *ctx, int Vh, const double2 *in, WdVec out);
 wd_status wd_lp_to_f64(wd_context *ctx, int Vh, WdVec in, double2 *out, int accumulate);

@@ -307,8 +307,6 @@ wd_status wd_mx_reliable(wd_context *ctx, const wd_lattice *lat, double mass, wd
     return WD_OK;
 }
 
-size_t wd_mx_reliable_scratch_doubles(int Vh) { return (size_t)Vh / 16 + 3; }
-
 wd_status wd_mx_reliable_enqueue(wd_context *ctx, const wd_lattice *lat, double mass, wd_precision L, wd_precision H,
                                  const WdMxReliable &v, const WdVec *p_restart, double *rr_dev, double *ss_dev,
                                  double *scratch)
@@ -320,24 +318,20 @@ wd_status wd_mx_reliable_enqueue(wd_context *ctx, const wd_lattice *lat, double 
     s32.prec = tmp32.prec = WD_PREC_F32;
     s32.p = v.scratch_h.p;
     tmp32.p = (char *)v.scratch_h.p + (size_t)nh * sizeof(float2);
-    // block partials of the two reductions, then their two counters: the
-    // caller's scratch, or a block from the work-buffer cache
-    const size_t nparts = wd_mx_reliable_scratch_doubles(Vh) - 1;
+    // the two reductions' work space: the caller's scratch, or a block from the work-buffer cache
+    const int64_t rb = wd_red_blocks(Vh);
     DevBlock blk;
     wd_status e;
-    if (!scratch && (e = blk.alloc(ctx, (nparts + 1) * sizeof(double))) != WD_OK) return e;
-    double *partial = scratch ? scratch : (double *)blk.p;
-    unsigned *count = (unsigned *)(partial + nparts);
-    WD_CUDA(ctx, cudaMemsetAsync(count, 0, 2 * sizeof(unsigned), ctx->stream));
+    if (!scratch && (e = blk.alloc(ctx, wd_red_doubles(rb, 1) * sizeof(double))) != WD_OK) return e;
+    const WdRed red = wd_red_view(scratch ? scratch : blk.p, rb);
+    WD_CUDA(ctx, cudaMemsetAsync(red.counters, 0, wd_red_counters(rb) * sizeof(unsigned), ctx->stream));
     if ((e = mx.accum(v.xs, v.x_e)) != WD_OK) return e;
     // s = bhat - Mhat x_e (high precision, rounded to FP32 as stored), |s|^2 -> slot + 1
     if ((e = wd_hop_v(ctx, lat, v.x_e, v.tmp_oh, nullptr, 1, 0, 1.0, 0.0)) != WD_OK) return e;
-    if ((e = wd_hop_hi_residual(ctx, lat, v.tmp_oh, v.x_e, v.bhat, s32, mass, partial, count, ss_dev)) != WD_OK)
-        return e;
+    if ((e = wd_hop_hi_residual(ctx, lat, v.tmp_oh, v.x_e, v.bhat, s32, mass, red, ss_dev)) != WD_OK) return e;
     // r_s = Mhat^dag s (FP32), |r_s|^2 -> slot
     if ((e = wd_hop_v(ctx, lat, s32, tmp32, nullptr, 1, 1, 1.0, 0.0)) != WD_OK) return e;
-    if ((e = wd_hop_f32_norm(ctx, lat, tmp32, v.rs, s32, mass, 1, partial, count + 1, rr_dev)) != WD_OK)
-        return e;
+    if ((e = wd_hop_f32_norm(ctx, lat, tmp32, v.rs, s32, mass, 1, red, rr_dev)) != WD_OK) return e;
     return p_restart ? mx.f32_to(v.rs, *p_restart) : WD_OK;
 }
 
@@ -406,9 +400,11 @@ wd_status wd_solve_cg_eo_mixed(wd_context *ctx, const wd_lattice *lat, const dou
     // asked for an update are no-ops.
     DevBlock dev_blk, part_blk;
     if ((st = dev_blk.alloc(ctx, sizeof(WdMxDev))) != WD_OK) return st;
-    if ((st = part_blk.alloc(ctx, sizeof(double) * ((size_t)Vh / 64 + 2))) != WD_OK) return st;
+    const int64_t rb = wd_red_blocks(Vh);
+    if ((st = part_blk.alloc(ctx, wd_red_doubles(rb, 1) * sizeof(double))) != WD_OK) return st;
+    const WdRed red_it = wd_red_view(part_blk.p, rb);
+    WD_CUDA(ctx, cudaMemsetAsync(red_it.counters, 0, wd_red_counters(rb) * sizeof(unsigned), ctx->stream));
     WdMxDev *dev = (WdMxDev *)dev_blk.p;
-    double *partial = (double *)part_blk.p;
     WdMxDev *sc = (WdMxDev *)ctx->state_host;
     *sc = WdMxDev{};
     sc->rr = sc->rr_max = rr;
@@ -421,9 +417,9 @@ wd_status wd_solve_cg_eo_mixed(wd_context *ctx, const wd_lattice *lat, const dou
         for (int i = 0; i < k; ++i) {
             // t = Mhat p with |t|^2 -> alpha; q = Mhat^dag t applied as the update; p = r_s + beta p
             if ((st = hop_oe_gated(ctx, lat, p.v, tmp_ol.v, 0, &dev->stop)) != WD_OK) return st;
-            if ((st = wd_hop_lp_norm(ctx, lat, tmp_ol.v, t.v, p.v, m, dev, partial)) != WD_OK) return st;
+            if ((st = wd_hop_lp_norm(ctx, lat, tmp_ol.v, t.v, p.v, m, dev, red_it)) != WD_OK) return st;
             if ((st = hop_oe_gated(ctx, lat, t.v, tmp_ol.v, 1, &dev->stop)) != WD_OK) return st;
-            if ((st = wd_hop_lp_update(ctx, lat, tmp_ol.v, t.v, p.v, rs.v, xs.v, m, dev, partial)) != WD_OK)
+            if ((st = wd_hop_lp_update(ctx, lat, tmp_ol.v, t.v, p.v, rs.v, xs.v, m, dev, red_it)) != WD_OK)
                 return st;
             if ((st = mx.xpay_dev(rs.v, dev, p.v)) != WD_OK) return st;
         }

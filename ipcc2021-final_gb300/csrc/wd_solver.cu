@@ -11,7 +11,6 @@
 // Both run in FP64 or in double-float (prec = WD_PREC_DF64: the same
 // recurrences on float-pair vectors, ~5x faster on GB300's narrow FP64
 // pipe).  Mixed precision (FP32 / FP16 inner) lives in wd_mixed.cu.
-#include <algorithm>
 #include <chrono>
 #include <cmath>
 #include "wd_kernels.h"
@@ -77,14 +76,13 @@ wd_status wd_true_residual(wd_context *ctx, const wd_lattice *lat, const double2
     double2 r[2];
     wd_status st;
     if (lat->gauge_fix) {
-        const size_t parts = wd_hop_fix_partials(lat);
+        const int64_t rb = wd_red_blocks(lat->g.Vh);
         WdVecBuf buf;
-        if ((st = wd_vec_alloc(ctx, buf, WD_PREC_F64, (int64_t)(parts + 4) / 2 + 1)) != WD_OK) return st;
-        double *partial = (double *)buf.v.p;
-        unsigned *counter = (unsigned *)(partial + parts);
+        if ((st = wd_vec_alloc(ctx, buf, WD_PREC_F64, (int64_t)wd_red_doubles(rb, 2) / 2 + 1)) != WD_OK) return st;
+        const WdRed red = wd_red_view(buf.v.p, rb);
         double2 *res = (double2 *)ctx->red_partial + WD_RED_BLOCKS;
-        WD_CUDA(ctx, cudaMemsetAsync(counter, 0, sizeof(unsigned), ctx->stream));
-        if ((st = wd_hop_fix_M_residual(ctx, lat, b, x, mass, partial, counter, &res[0].x)) != WD_OK) return st;
+        WD_CUDA(ctx, cudaMemsetAsync(red.counters, 0, wd_red_counters(rb) * sizeof(unsigned), ctx->stream));
+        if ((st = wd_hop_fix_M_residual(ctx, lat, b, x, mass, red, &res[0].x)) != WD_OK) return st;
         if ((st = wd_red_fetch(ctx, 1, r)) != WD_OK) return st;
         r[1].x = r[0].y;
     } else {
@@ -111,20 +109,22 @@ struct CgLoop {
     wd_context *ctx;
     WdCgDev *dev = nullptr;  // device
     WdCgDev *host;           // three pinned copies: two in flight, one for uploads
-    double *partial = nullptr;
+    WdRed red;
     void *blk = nullptr;
-    int chunk;               // iterations per look
+    int chunk = 1;           // iterations per look
 
-    CgLoop(wd_context *c, int Vh) : ctx(c), host((WdCgDev *)c->state_host), chunk(Vh <= 32768 ? 4 : Vh <= 524288 ? 2 : 1)
-    {
-    }
+    CgLoop(wd_context *c) : ctx(c), host((WdCgDev *)c->state_host) {}
     ~CgLoop() { wd_dev_free(ctx, blk); }
-    wd_status alloc(size_t partials)
+    wd_status alloc(int Vh)
     {
-        wd_status st = wd_dev_alloc(ctx, &blk, 256 + partials * sizeof(double));
+        chunk = Vh <= 32768 ? 4 : Vh <= 524288 ? 2 : 1;
+        const int64_t rb = wd_red_blocks(Vh);
+        wd_status st = wd_dev_alloc(ctx, &blk, 256 + wd_red_doubles(rb, 2) * sizeof(double));
+        if (st != WD_OK) return st;
         dev = (WdCgDev *)blk;
-        partial = (double *)((char *)blk + 256);
-        return st;
+        red = wd_red_view((char *)blk + 256, rb);
+        WD_CUDA(ctx, cudaMemsetAsync(red.counters, 0, wd_red_counters(rb) * sizeof(unsigned), ctx->stream));
+        return WD_OK;
     }
     wd_status start(double rr, double target, bool strict, int iters)
     {
@@ -182,8 +182,8 @@ static wd_status cgnr_ref_core(wd_context *ctx, const wd_lattice *lat, WdVec src
         if (s != WD_OK) return s;
     }
     WdVec r0 = b[0].v, q = b[1].v, qq = b[2].v, p = b[3].v, Mdb = b[4].v;
-    CgLoop loop(ctx, lat->g.Vh);
-    wd_status st = loop.alloc(std::max((size_t)2 * WD_RED_BLOCKS, wd_hop_fix_partials(lat)));
+    CgLoop loop(ctx);
+    wd_status st = loop.alloc(lat->g.Vh);
     if (st != WD_OK) return st;
     WdCgDev *dev = loop.dev;
     // Mdb = M^dag src; r0 = Mdb - M^dag M x   (src/invert.cpp:41-58)
@@ -202,12 +202,12 @@ static wd_status cgnr_ref_core(wd_context *ctx, const wd_lattice *lat, WdVec src
         wd_status e;
         if ((e = wd_apply_M_v(ctx, lat, p, qq, m, 0, &dev->stop)) != WD_OK) return e;
         if (fused) {
-            if ((e = wd_hop_fix_M_dot(ctx, lat, qq, q, p, m, dev, loop.partial)) != WD_OK) return e;
+            if ((e = wd_hop_fix_M_dot(ctx, lat, qq, q, p, m, dev, loop.red)) != WD_OK) return e;
         } else {
             if ((e = wd_apply_M_v(ctx, lat, qq, q, m, 1, &dev->stop)) != WD_OK) return e;
-            if ((e = wd_cgd_dot(ctx, p, q, n, dev, loop.partial)) != WD_OK) return e;
+            if ((e = wd_cgd_dot(ctx, p, q, n, dev, loop.red)) != WD_OK) return e;
         }
-        if ((e = wd_cgd_update(ctx, true, p, q, x, r0, n, dev, loop.partial)) != WD_OK) return e;
+        if ((e = wd_cgd_update(ctx, true, p, q, x, r0, n, dev, loop.red)) != WD_OK) return e;
         return wd_cgd_xpby(ctx, r0, p, n, dev);
     };
     WdCgDev end{};
@@ -236,8 +236,8 @@ static wd_status cg_eo_core(wd_context *ctx, const wd_lattice *lat, WdVec src, W
     WdVec bhat = b[0].v, r = b[1].v, p = b[2].v, t = b[3].v, q = b[4].v, tmp_o = b[5].v, s_e = b[6].v;
     const WdVec b_e = par_half(src, 0, Vh), b_o = par_half(src, 1, Vh);
     WdVec x_e = par_half(x, 0, Vh), x_o = par_half(x, 1, Vh);
-    CgLoop loop(ctx, Vh);
-    wd_status st = loop.alloc(std::max((size_t)2 * WD_RED_BLOCKS, wd_hop_fix_partials(lat)));
+    CgLoop loop(ctx);
+    wd_status st = loop.alloc(Vh);
     if (st != WD_OK) return st;
     WdCgDev *dev = loop.dev;
 
@@ -270,17 +270,17 @@ static wd_status cg_eo_core(wd_context *ctx, const wd_lattice *lat, WdVec src, W
         wd_status e;
         if ((e = wd_hop_v(ctx, lat, p, tmp_o, nullptr, 1, 0, 1.0, 0.0, &dev->stop)) != WD_OK) return e;
         if (fused) {
-            if ((e = wd_hop_fix_norm(ctx, lat, tmp_o, t, p, m, dev, loop.partial)) != WD_OK) return e;
+            if ((e = wd_hop_fix_norm(ctx, lat, tmp_o, t, p, m, dev, loop.red)) != WD_OK) return e;
         } else {
             if ((e = wd_hop_v(ctx, lat, tmp_o, t, &p, 0, 0, -0.25 / a, a, &dev->stop)) != WD_OK) return e;
-            if ((e = wd_cgd_norm(ctx, t, nh, dev, loop.partial)) != WD_OK) return e;
+            if ((e = wd_cgd_norm(ctx, t, nh, dev, loop.red)) != WD_OK) return e;
         }
         if ((e = wd_hop_v(ctx, lat, t, tmp_o, nullptr, 1, 1, 1.0, 0.0, &dev->stop)) != WD_OK) return e;
         if (fused) {
-            if ((e = wd_hop_fix_update(ctx, lat, tmp_o, t, p, r, x_e, m, dev, loop.partial)) != WD_OK) return e;
+            if ((e = wd_hop_fix_update(ctx, lat, tmp_o, t, p, r, x_e, m, dev, loop.red)) != WD_OK) return e;
         } else {
             if ((e = wd_hop_v(ctx, lat, tmp_o, q, &t, 0, 1, -0.25 / a, a, &dev->stop)) != WD_OK) return e;
-            if ((e = wd_cgd_update(ctx, false, p, q, x_e, r, nh, dev, loop.partial)) != WD_OK) return e;
+            if ((e = wd_cgd_update(ctx, false, p, q, x_e, r, nh, dev, loop.red)) != WD_OK) return e;
         }
         return wd_cgd_xpby(ctx, r, p, nh, dev);
     };

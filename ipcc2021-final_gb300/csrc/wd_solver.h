@@ -48,14 +48,13 @@ wd_status wd_mx_reliable(wd_context *ctx, const wd_lattice *lat, double mass, wd
 // the same with no host wait: |rs|^2 and |s|^2 land in the device doubles
 // rr_dev and ss_dev, for the caller to fetch (several systems per fetch).
 // Its kernels go to ctx->stream.  scratch (device, optional): the
-// reductions' work space of wd_mx_reliable_scratch_doubles(Vh) doubles,
+// reductions' work space of wd_red_doubles(wd_red_blocks(Vh), 1) doubles,
 // owned by the caller -- needed when updates of several systems run on
 // different streams at once; without it a block from the context's
 // work-buffer cache (stream-ordered on ctx->stream) is used.
 wd_status wd_mx_reliable_enqueue(wd_context *ctx, const wd_lattice *lat, double mass, wd_precision L, wd_precision H,
                                  const WdMxReliable &v, const WdVec *p_restart, double *rr_dev, double *ss_dev,
                                  double *scratch = nullptr);
-size_t wd_mx_reliable_scratch_doubles(int Vh);
 // p (storage L) = rs (FP32) + beta p
 wd_status wd_mx_xpay(wd_context *ctx, int Vh, wd_precision L, WdVec rs, double beta, WdVec p);
 
@@ -76,7 +75,6 @@ struct WdMxDev {
     float alpha, beta;
     int stop;         // 0 iterate; 1 reliable update due; 2 non-finite scalar
     int iters;        // iterations completed on the device
-    unsigned count_t, count_r;  // last-block counters of the two reductions
 };
 
 // Device-side scalars of the FP64 / double-float CG solvers (wd_solver.cu):
@@ -91,7 +89,6 @@ struct WdCgDev {
     int strict;
     int stop;         // 0 iterate; 1 target reached; 2 non-finite |r|^2
     int iters;        // iterations completed
-    unsigned count_a, count_r;  // last-block counters of the two reductions
 };
 
 #ifdef __CUDACC__
@@ -122,29 +119,28 @@ __device__ __forceinline__ void wd_cg_set_beta(WdCgDev *d, double rr_new)
 #endif
 
 // One iteration's pieces on n complex entries of one storage (FP64 or
-// double-float), all no-ops while dev->stop != 0 (wd_cg.cu).  partial: at
-// least 2 * WD_RED_BLOCKS doubles.
+// double-float), all no-ops while dev->stop != 0 (wd_cg.cu).  red: for
+// wd_red_blocks(Vh) blocks of two sums.
 // alpha from |t|^2, or from the complex (p, q)
-wd_status wd_cgd_norm(wd_context *ctx, WdVec t, int64_t n, WdCgDev *dev, double *partial);
-wd_status wd_cgd_dot(wd_context *ctx, WdVec p, WdVec q, int64_t n, WdCgDev *dev, double *partial);
+wd_status wd_cgd_norm(wd_context *ctx, WdVec t, int64_t n, WdCgDev *dev, WdRed red);
+wd_status wd_cgd_dot(wd_context *ctx, WdVec p, WdVec q, int64_t n, WdCgDev *dev, WdRed red);
 // x += alpha p, r -= alpha q, |r|^2 -> beta or the gate
 wd_status wd_cgd_update(wd_context *ctx, bool cplx, WdVec p, WdVec q, WdVec x, WdVec r, int64_t n, WdCgDev *dev,
-                        double *partial);
+                        WdRed red);
 // p = r + beta p
 wd_status wd_cgd_xpby(wd_context *ctx, WdVec r, WdVec p, int64_t n, const WdCgDev *dev);
 
 // The same fused into the fixed-point FP64 hops (wd_dslash_fix.cu; the
-// lattice has gauge_fix).  partial: wd_hop_fix_partials(lat) doubles.
-size_t wd_hop_fix_partials(const wd_lattice *lat);
+// lattice has gauge_fix).
 //   t = -D_eo in / (4a) + a p on even blocks (a = 4 + mass), |t|^2 -> alpha
 wd_status wd_hop_fix_norm(wd_context *ctx, const wd_lattice *lat, WdVec in, WdVec t, WdVec p, double mass, WdCgDev *dev,
-                          double *partial);
+                          WdRed red);
 //   q = -D_eo^dag in / (4a) + a t, not stored: r -= alpha q, x += alpha p, |r|^2 -> beta or the gate
 wd_status wd_hop_fix_update(wd_context *ctx, const wd_lattice *lat, WdVec in, WdVec t, WdVec p, WdVec r, WdVec x,
-                            double mass, WdCgDev *dev, double *partial);
-//   |b - M x|^2 and |b|^2 -> result[0], result[1] (device); counter: zero at launch
+                            double mass, WdCgDev *dev, WdRed red);
+//   |b - M x|^2 and |b|^2 -> result[0], result[1] (device)
 wd_status wd_hop_fix_M_residual(wd_context *ctx, const wd_lattice *lat, const double2 *b, const double2 *x, double mass,
-                                double *partial, unsigned *counter, double *result);
+                                WdRed red, double *result);
 //   q = M^dag in on the whole lattice, (p, q) -> alpha
 wd_status wd_hop_fix_M_dot(wd_context *ctx, const wd_lattice *lat, WdVec in, WdVec q, WdVec p, double mass, WdCgDev *dev,
-                           double *partial);
+                           WdRed red);
