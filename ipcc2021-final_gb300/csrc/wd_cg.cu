@@ -3,6 +3,7 @@
 // FP64 pipe); what they save over host scalars is the two host waits an
 // iteration (about 30 us of an 8^3x16 iteration's 146).  Reductions: fixed
 // grid, fixed fold order.
+#include <type_traits>
 #include "wd_async.cuh"
 #include "wd_df.cuh"
 #include "wd_reduce.cuh"
@@ -131,6 +132,17 @@ inline int red_blocks(int64_t n)
     return (int)(b < WD_RED_BLOCKS ? b : WD_RED_BLOCKS);
 }
 
+// An early launch leaves a one-wave grid unevenly spread over the SMs, which
+// the FP64 update pays for (FP64 pipe: 8.7 against 8.3 ms a reference CG at
+// 16^4, 17.7 against 16.6 at 16^3x32); below a block per SM it gains (2.02
+// against 2.28 ms at 4^4), and the double-float passes gain at every size
+// (3.3 against 3.6 ms a double-float CG at 16^4)
+template <class V>
+bool early_update(int64_t n)
+{
+    return std::is_same_v<V, VDF> || red_blocks(n) <= 152;
+}
+
 // runs f(V()) for the vectors' storage
 template <class F>
 wd_status typed(wd_context *ctx, WdVec v, F f)
@@ -169,8 +181,8 @@ wd_status wd_cgd_update(wd_context *ctx, bool cplx, WdVec p, WdVec q, WdVec x, W
         using E = typename V::E;
         const E *pp = (const E *)p.p, *qq = (const E *)q.p;
         E *xx = (E *)x.p, *rr = (E *)r.p;
-        if (cplx) wd_launch_pdl(true, k_cgd_update<V, true>, red_blocks(n), WD_RED_THREADS, 0, ctx->stream, pp, qq, xx, rr, n, dev, red);
-        else wd_launch_pdl(true, k_cgd_update<V, false>, red_blocks(n), WD_RED_THREADS, 0, ctx->stream, pp, qq, xx, rr, n, dev, red);
+        if (cplx) wd_launch_pdl(early_update<V>(n), k_cgd_update<V, true>, red_blocks(n), WD_RED_THREADS, 0, ctx->stream, pp, qq, xx, rr, n, dev, red);
+        else wd_launch_pdl(early_update<V>(n), k_cgd_update<V, false>, red_blocks(n), WD_RED_THREADS, 0, ctx->stream, pp, qq, xx, rr, n, dev, red);
     });
 }
 
