@@ -528,7 +528,8 @@ wd_status BatchEngine::reliable_enqueue(EngineSys &s, bool reset_p, double *rr_d
     SysBufs &B = s.B;
     WdVec b_e, b_o, x_e, x_o;
     slices(s, b_e, b_o, x_e, x_o);
-    const WdMxReliable rv{B.xs.v, x_e, B.bhat.v, B.tmp_oh.v, B.r_h.v, B.rs.v};
+    // the restart is the set-up's, from x = 0
+    const WdMxReliable rv{B.xs.v, x_e, B.bhat.v, B.tmp_oh.v, B.r_h.v, B.rs.v, reset_p};
     return wd_mx_reliable_enqueue(ctx_, s.lat, s.mass, L_, H_, rv, reset_p ? &B.p.v : nullptr, rr_dev, ss_dev,
                                   (double *)B.rel.v.p);
 }

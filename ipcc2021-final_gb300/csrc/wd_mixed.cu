@@ -141,6 +141,26 @@ __global__ void k_mx_to_f32(H in, SpF32 a, int Vh)
     }
 }
 
+// s = bhat rounded to FP32, |s|^2: the residual of x = 0, in one pass over bhat
+// where the general update takes two high-precision hops
+template <class H>
+__global__ void __launch_bounds__(WD_RED_THREADS) k_mx_seed(H bhat, SpF32 s32, int Vh, WdRed red, double *result)
+{
+    dfr acc{0.f, 0.f};
+    SITE_STRIDE(s, Vh)
+    {
+        float2 v[12];
+#pragma unroll
+        for (int c = 0; c < 12; ++c) {
+            v[c] = bhat.load_f32(c, s);
+            acc = df_sq_acc(acc, v[c]);
+        }
+        s32.store(s, v);
+    }
+    double tot;
+    if (wd_grid_sum<WD_RED_THREADS>(df_value(acc), red, &tot)) *result = tot;
+}
+
 // FP32 -> kernel storage
 template <class SpL>
 __global__ void k_mx_f32_to(SpF32 a, SpL b, int Vh)
@@ -232,6 +252,14 @@ struct Mixed {
         k_mx_norm2<<<site_grid(Vh), WD_RED_THREADS, 0, ctx->stream>>>(sp_f32(t, Vh), Vh, (double2 *)ctx->red_partial);
         WD_LAUNCHED(ctx);
         return wd_red_finish(ctx, slot);
+    }
+    wd_status seed(WdVec bhat, WdVec s32, const WdRed &red, double *result) const
+    {
+        const int b = (Vh + WD_RED_THREADS - 1) / WD_RED_THREADS, g = b < WD_RED_BLOCKS ? b : WD_RED_BLOCKS;
+        if (H == WD_PREC_F64) k_mx_seed<<<g, WD_RED_THREADS, 0, ctx->stream>>>(HF64{(double2 *)bhat.p, Vh}, sp_f32(s32, Vh), Vh, red, result);
+        else k_mx_seed<<<g, WD_RED_THREADS, 0, ctx->stream>>>(HDF{(float4 *)bhat.p, Vh}, sp_f32(s32, Vh), Vh, red, result);
+        WD_LAUNCHED(ctx);
+        return WD_OK;
     }
     wd_status accum(WdVec xs, WdVec xh) const
     {
@@ -325,10 +353,14 @@ wd_status wd_mx_reliable_enqueue(wd_context *ctx, const wd_lattice *lat, double 
     if (!scratch && (e = blk.alloc(ctx, wd_red_doubles(rb, 1) * sizeof(double))) != WD_OK) return e;
     const WdRed red = wd_red_view(scratch ? scratch : blk.p, rb);
     WD_CUDA(ctx, cudaMemsetAsync(red.counters, 0, wd_red_counters(rb) * sizeof(unsigned), ctx->stream));
-    if ((e = mx.accum(v.xs, v.x_e)) != WD_OK) return e;
-    // s = bhat - Mhat x_e (high precision, rounded to FP32 as stored), |s|^2 -> slot + 1
-    if ((e = wd_hop_v(ctx, lat, v.x_e, v.tmp_oh, nullptr, 1, 0, 1.0, 0.0)) != WD_OK) return e;
-    if ((e = wd_hop_hi_residual(ctx, lat, v.tmp_oh, v.x_e, v.bhat, s32, mass, red, ss_dev)) != WD_OK) return e;
+    if (v.x_zero) {
+        if ((e = mx.seed(v.bhat, s32, red, ss_dev)) != WD_OK) return e;
+    } else {
+        if ((e = mx.accum(v.xs, v.x_e)) != WD_OK) return e;
+        // s = bhat - Mhat x_e (high precision, rounded to FP32 as stored), |s|^2 -> slot + 1
+        if ((e = wd_hop_v(ctx, lat, v.x_e, v.tmp_oh, nullptr, 1, 0, 1.0, 0.0)) != WD_OK) return e;
+        if ((e = wd_hop_hi_residual(ctx, lat, v.tmp_oh, v.x_e, v.bhat, s32, mass, red, ss_dev)) != WD_OK) return e;
+    }
     // r_s = Mhat^dag s (FP32), |r_s|^2 -> slot
     if ((e = wd_hop_v(ctx, lat, s32, tmp32, nullptr, 1, 1, 1.0, 0.0)) != WD_OK) return e;
     if ((e = wd_hop_f32_norm(ctx, lat, tmp32, v.rs, s32, mass, 1, red, rr_dev)) != WD_OK) return e;
@@ -380,9 +412,11 @@ wd_status wd_solve_cg_eo_mixed(wd_context *ctx, const wd_lattice *lat, const dou
 
     // reliable update: x_e += x_s; s = bhat - Mhat x_e; r_s = Mhat^dag s (p <- r_s only on a restart)
     double rr = 0, ss = 0;
-    const WdMxReliable rv{xs.v, x_e, bhat.v, tmp_oh.v, r_h.v, rs.v};
+    WdMxReliable rv{xs.v, x_e, bhat.v, tmp_oh.v, r_h.v, rs.v, !prm->use_initial_guess};
     auto reliable = [&](bool reset_p) -> wd_status {
-        return wd_mx_reliable(ctx, lat, m, prm->prec, H, rv, reset_p ? &p.v : nullptr, &rr, &ss);
+        const wd_status e = wd_mx_reliable(ctx, lat, m, prm->prec, H, rv, reset_p ? &p.v : nullptr, &rr, &ss);
+        rv.x_zero = false;
+        return e;
     };
 
     if ((st = reliable(true)) != WD_OK) return st;

@@ -252,13 +252,16 @@ static wd_status cg_eo_core(wd_context *ctx, const wd_lattice *lat, WdVec src, W
     // s = bhat - Mhat x (its norm is the full-system true residual |b - M x|
     // once x_o = (b_o + D_oe x_e / 2)/a), r = Mhat^dag s
     double ss = 0.0;
-    auto residuals = [&](double *rr) -> wd_status {
-        wd_status e = wd_apply_Mhat_v(ctx, lat, x_e, t, tmp_o, m, 0);
-        if (e != WD_OK) return e;
-        if ((e = wd_v_xpayz(ctx, bhat, make_double2(-1.0, 0.0), t, s_e, nh)) != WD_OK) return e;
-        if ((e = wd_apply_Mhat_v(ctx, lat, s_e, r, tmp_o, m, 1)) != WD_OK) return e;
+    auto residuals = [&](double *rr, bool x_zero) -> wd_status {
+        wd_status e;
+        const WdVec s = x_zero ? bhat : s_e;
+        if (!x_zero) {
+            if ((e = wd_apply_Mhat_v(ctx, lat, x_e, t, tmp_o, m, 0)) != WD_OK) return e;
+            if ((e = wd_v_xpayz(ctx, bhat, make_double2(-1.0, 0.0), t, s, nh)) != WD_OK) return e;
+        }
+        if ((e = wd_apply_Mhat_v(ctx, lat, s, r, tmp_o, m, 1)) != WD_OK) return e;
         if ((e = wd_v_norm2(ctx, r, nh, 0)) != WD_OK) return e;
-        if ((e = wd_v_norm2(ctx, s_e, nh, 1)) != WD_OK) return e;
+        if ((e = wd_v_norm2(ctx, s, nh, 1)) != WD_OK) return e;
         double2 v[2];
         if ((e = wd_red_fetch(ctx, 2, v)) != WD_OK) return e;
         *rr = v[0].x;
@@ -286,7 +289,7 @@ static wd_status cg_eo_core(wd_context *ctx, const wd_lattice *lat, WdVec src, W
     };
 
     double rr;
-    if ((st = residuals(&rr)) != WD_OK) return st;
+    if ((st = residuals(&rr, !prm->use_initial_guess)) != WD_OK) return st;
     if ((st = wd_v_copy(ctx, p, r, nh)) != WD_OK) return st;
     // normal-residual target from the observed ratio |r| / |s|
     double ratio = ss > 0 ? std::sqrt(rr / ss) : 1.0;
@@ -306,7 +309,7 @@ static wd_status cg_eo_core(wd_context *ctx, const wd_lattice *lat, WdVec src, W
         if (end.stop != 1) break;  // out of iterations
         // check the true residual; replace r by the recomputed one
         double rr_new;
-        if ((st = residuals(&rr_new)) != WD_OK) return st;
+        if ((st = residuals(&rr_new, false)) != WD_OK) return st;
         stats->reliable_updates++;
         true_res = std::sqrt(ss) / norm_b;
         if (true_res <= prm->tol) {

@@ -39,6 +39,7 @@ struct WdMxReliable {
     WdVec tmp_oh;     // high-precision odd-parity work
     WdVec scratch_h;  // high-precision work, used as two FP32 blocks
     WdVec rs;         // FP32 iterated residual, receives Mhat^dag s
+    bool x_zero = false;  // x_e and xs are zero: s is bhat
 };
 // x_e += xs; s = bhat - Mhat x_e (high precision, kept only as FP32);
 // rs = Mhat^dag s (FP32); rr = |rs|^2, ss = |s|^2; p_restart (storage L) <- rs
