@@ -1271,10 +1271,10 @@ static wd_status server_admit(wd_server *sv, int *completed)
         wd_status st = WD_OK;
         for (int k = 0; k < p.nsrc && st == WD_OK; ++k) {
             wd_field *fs = nullptr, *fd = nullptr;
-            st = wd_field_create(sv->ctx, lat, &fs);
+            st = wd_field_create_work(sv->ctx, lat, &fs);
             if (st == WD_OK) {
                 r.src.push_back(fs);
-                st = wd_field_create(sv->ctx, lat, &fd);
+                st = wd_field_create_work(sv->ctx, lat, &fd);
             }
             if (st == WD_OK) {
                 r.dest.push_back(fd);

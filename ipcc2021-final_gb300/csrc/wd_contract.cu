@@ -114,7 +114,7 @@ extern "C" wd_status wd_propagator(wd_context *ctx, const wd_lattice *lat, const
     std::vector<wd_field *> srcs(12, nullptr);
     wd_status st = WD_OK;
     for (int k = 0; k < 12 && st == WD_OK; ++k) {
-        st = wd_field_create(ctx, lat, &srcs[k]);
+        st = wd_field_create_work(ctx, lat, &srcs[k]);
         if (st == WD_OK) st = wd_point_source(ctx, srcs[k], x_src, k / 3, k % 3);
     }
     if (st == WD_OK) {

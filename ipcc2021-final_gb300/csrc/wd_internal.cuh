@@ -98,13 +98,15 @@ inline bool wd_alloc_fails(wd_context *ctx)
     return false;
 }
 
-// Work-buffer allocation through the context's cache (stream-ordered reuse;
-// on allocation failure the cached blocks are released and the call retried).
+// Work-buffer allocation through the context's cache (stream-ordered reuse)
 wd_status wd_dev_alloc(wd_context *ctx, void **p, size_t bytes);
 void wd_dev_free(wd_context *ctx, void *p);
 void wd_pool_release(wd_context *ctx);
-// cudaMalloc that gives back the context's fixed-point links when memory runs out
+// cudaMalloc that gives back the context's cached work buffers, then its
+// fixed-point links, when memory runs out
 cudaError_t wd_malloc(wd_context *ctx, void **p, size_t bytes);
+// a library-internal FP64 field, from the work-buffer cache if it is small
+wd_status wd_field_create_work(wd_context *ctx, const wd_lattice *lat, wd_field **out);
 // wd_lattice_create; fix = false: without fixed-point links
 wd_status wd_lattice_make(wd_context *ctx, const int dims[4], const double *const gauge[4], bool fix, wd_lattice **out);
 
@@ -128,6 +130,7 @@ struct wd_field {
     void *data = nullptr;     // [parity][12][Vh] entries of the storage type
     float *scale = nullptr;   // FP16 storage: [parity][Vh] per-site scales (inside data)
     double2 *d = nullptr;     // == data for FP64 storage, else null
+    wd_context *pool = nullptr;  // owns data in its work-buffer cache, else null
 };
 
 // Work space of a grid reduction (wd_grid_sum_n): the blocks' partials, then
