@@ -34,14 +34,19 @@ __device__ __forceinline__ void wd_cp_async_wait()
 // Programmatic dependent launch: a kernel launched with wd_launch_pdl may start
 // while its predecessor in the stream finishes.  It calls wd_pdl_wait before it
 // touches memory (a no-op under an ordinary launch), which returns once the
-// predecessor has completed, and at that point lets its own successor start
-// the same way (pdl = false: an ordinary launch).  It hides the launch itself:
-// a fixed-point hop at 4^4 takes 3.5 us in a row of them instead of 6.2, at
-// 8^3x16 6.7 instead of 8.2, at 16^3x32 25.8 instead of 28.7.
-__device__ __forceinline__ void wd_pdl_wait()
+// predecessor has completed, and from that point lets its own successor start
+// the same way (pdl = false: an ordinary launch).  ahead: the successor may
+// start before the wait already.  That piles up kernels ahead of the running
+// one, which spread unevenly over the SMs where a grid does not fill them (a
+// fixed-point hop at 8^4: 6.5 us instead of 4.9), but is the better order for
+// the FP64 solver's full grids (CG at 16^3x32: 7.07 ms instead of 7.26).
+// It hides the launch itself: a fixed-point hop at 4^4 takes 3.4 us in a row of
+// them instead of 6.2, at 8^3x16 5.8 instead of 8.2, at 16^3x32 25.8 instead of 28.7.
+__device__ __forceinline__ void wd_pdl_wait(bool ahead = false)
 {
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    if (ahead) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");
+    if (!ahead) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 template <class... P, class... A>
 inline void wd_launch_pdl(bool pdl, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
@@ -58,4 +63,17 @@ inline void wd_launch_pdl(bool pdl, void (*kernel)(P...), dim3 grid, dim3 block,
     cfg.attrs = &attr;
     cfg.numAttrs = pdl ? 1 : 0;
     cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
+// The same for the other hops, by the number of their blocks.  Up to a block
+// per SM (FP32 hop at 8^3x16 3.6 instead of 6.2 us) and from several waves on
+// (24^4 16.4 instead of 18.4 us; double-float at 16^3x32 25.2 instead of 27.5)
+// the early launch gains; in between it is unevenly spread (double-float CG at
+// 12^3x16 2.45 instead of 2.19 ms), and the largest grids lose by it (82,944
+// blocks: an FP16 solve at 48^3x96 145.7 instead of 140.8 ms).
+inline bool wd_pdl_early(int blocks) { return blocks <= 152 || (blocks >= 1000 && blocks <= 10000); }
+template <class... P, class... A>
+inline void wd_launch_early(void (*kernel)(P...), int blocks, int threads, cudaStream_t stream, A... args)
+{
+    wd_launch_pdl(wd_pdl_early(blocks), kernel, blocks, threads, 0, stream, args...);
 }

@@ -28,6 +28,7 @@
 #include <memory>
 #include <type_traits>
 #include <vector>
+#include "wd_async.cuh"
 #include "wd_df.cuh"
 #include "wd_hop.cuh"
 #include "wd_lp.cuh"
@@ -219,6 +220,7 @@ __device__ __forceinline__ auto batch_policy(const BTable &t, const BGroup &G, c
 template <bool DAG, bool F16, int SYS, int MINB, int EPI, bool R2 = false>
 __global__ void __launch_bounds__(kSites * SYS, MINB) k_batch_hop(const BTable t)
 {
+    wd_pdl_wait();
     constexpr int W = SYS == 2 ? 0 : SYS == 4 ? 1 : 2;
     const int gi = find_group<W>(t.groups, t.ngroups, blockIdx.x);
     const BGroup &G = t.groups[gi];
@@ -272,6 +274,7 @@ struct BVec {
 template <bool F16>
 __global__ void __launch_bounds__(WD_RED_THREADS) k_batch_xpay(const BVec *v, const int *chunk_sys, const BScal *sc)
 {
+    wd_pdl_wait();
     const int c = blockIdx.x;
     const int sys = chunk_sys[c];
     if (!sc[sys].active) return;
@@ -299,6 +302,7 @@ constexpr int kScalThreads = 512;
 __global__ void __launch_bounds__(kScalThreads) k_batch_scalars(const BSys *sys_tab, BScal *sc, const double *partial,
                                                                 int mode, double delta2)
 {
+    wd_pdl_wait();
     const int sys = blockIdx.x;
     if (!sc[sys].active) return;  // the whole block
     const BSys &S = sys_tab[sys];
@@ -780,8 +784,8 @@ wd_status BatchEngine::hop(int h, int cb, int dag, int v, int epi)
             constexpr bool F = decltype(f16)::value;
             constexpr int E = decltype(e)::value;
             constexpr bool R = F && decltype(share)::value;  // the shared row-2 table: FP16 links only
-            if (dag) k_batch_hop<true, F, S, M, E, R><<<grid, kSites * S, 0, ctx_->stream>>>(t);
-            else k_batch_hop<false, F, S, M, E, R><<<grid, kSites * S, 0, ctx_->stream>>>(t);
+            if (dag) wd_launch_early(k_batch_hop<true, F, S, M, E, R>, grid, kSites * S, ctx_->stream, t);
+            else wd_launch_early(k_batch_hop<false, F, S, M, E, R>, grid, kSites * S, ctx_->stream, t);
         };
         using E0 = std::integral_constant<int, kBEpiPlain>;
         using E1 = std::integral_constant<int, kBEpiNorm>;
@@ -822,14 +826,18 @@ wd_status BatchEngine::iteration()
     wd_status e;
     // t = Mhat p with |t|^2 -> alpha
     if ((e = hop(0, 1, 0, v, kBEpiPlain)) != WD_OK || (e = hop(1, 0, 0, v, kBEpiNorm)) != WD_OK) return e;
-    k_batch_scalars<<<nsys, kScalThreads, 0, ctx_->stream>>>(d_sys_[1].p, d_sc_.p, d_partial_.p, 0, 0.0);
+    const auto scalars = [&](int h, int mode) {
+        wd_launch_pdl(true, k_batch_scalars, nsys, kScalThreads, 0, ctx_->stream, d_sys_[h].p, d_sc_.p, d_partial_.p,
+                      mode, delta_ * delta_);
+    };
+    scalars(1, 0);
     WD_LAUNCHED(ctx_);
     // q = Mhat^dag t applied as the update, |r_s|^2 -> beta (or a reliable update due)
     if ((e = hop(2, 1, 1, v, kBEpiPlain)) != WD_OK || (e = hop(3, 0, 1, v, kBEpiUpdate)) != WD_OK) return e;
-    k_batch_scalars<<<nsys, kScalThreads, 0, ctx_->stream>>>(d_sys_[3].p, d_sc_.p, d_partial_.p, 1, delta_ * delta_);
+    scalars(3, 1);
     WD_LAUNCHED(ctx_);
-    if (f16) k_batch_xpay<true><<<nchunks_, WD_RED_THREADS, 0, ctx_->stream>>>(d_vec_.p, d_chunk_sys_.p, d_sc_.p);
-    else k_batch_xpay<false><<<nchunks_, WD_RED_THREADS, 0, ctx_->stream>>>(d_vec_.p, d_chunk_sys_.p, d_sc_.p);
+    wd_launch_pdl(true, f16 ? k_batch_xpay<true> : k_batch_xpay<false>, nchunks_, WD_RED_THREADS, 0, ctx_->stream,
+                  d_vec_.p, d_chunk_sys_.p, d_sc_.p);
     WD_LAUNCHED(ctx_);
     return WD_OK;
 }

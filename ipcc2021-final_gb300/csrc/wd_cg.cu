@@ -62,7 +62,7 @@ template <class V>
 __global__ void __launch_bounds__(WD_RED_THREADS) k_cgd_norm(const typename V::E *__restrict__ t, int64_t n, WdCgDev *dev,
                                                              WdRed red)
 {
-    wd_pdl_wait();
+    wd_pdl_wait(gridDim.x > 152);
     if (dev->stop) return;
     typename V::R s = V::zero();
     GRID_STRIDE(i, n) s = norm_acc<V>(s, V::load(t[i]));
@@ -75,7 +75,7 @@ __global__ void __launch_bounds__(WD_RED_THREADS) k_cgd_dot(const typename V::E 
                                                             const typename V::E *__restrict__ q, int64_t n, WdCgDev *dev,
                                                             WdRed red)
 {
-    wd_pdl_wait();
+    wd_pdl_wait(gridDim.x > 152);
     if (dev->stop) return;
     typename V::R re = V::zero(), im = V::zero();
     GRID_STRIDE(i, n)
@@ -96,7 +96,7 @@ __global__ void __launch_bounds__(WD_RED_THREADS) k_cgd_update(const typename V:
                                                                typename V::E *__restrict__ r, int64_t n, WdCgDev *dev,
                                                                WdRed red)
 {
-    wd_pdl_wait();
+    wd_pdl_wait(gridDim.x > 152);
     if (dev->stop) return;
     const typename V::R re = V::real(dev->are), im = V::real(dev->aim), mre = V::neg(re), mim = V::neg(im);
     typename V::R s = V::zero();
@@ -118,7 +118,7 @@ template <class V>
 __global__ void k_cgd_xpby(const typename V::E *__restrict__ r, typename V::E *__restrict__ p, int64_t n,
                            const WdCgDev *dev)
 {
-    wd_pdl_wait();
+    wd_pdl_wait(gridDim.x > 152);
     if (dev->stop) return;
     const typename V::R b = V::real(dev->beta);
     GRID_STRIDE(i, n) p[i] = V::store(V::axpy(b, V::load(p[i]), V::load(r[i])));
@@ -133,14 +133,15 @@ inline int red_blocks(int64_t n)
 }
 
 // An early launch leaves a one-wave grid unevenly spread over the SMs, which
-// the FP64 update pays for (FP64 pipe: 8.7 against 8.3 ms a reference CG at
-// 16^4, 17.7 against 16.6 at 16^3x32); below a block per SM it gains (2.02
-// against 2.28 ms at 4^4), and the double-float passes gain at every size
-// (3.3 against 3.6 ms a double-float CG at 16^4)
+// the FP64 passes pay for (FP64 pipe: 17.7 against 16.6 ms a reference CG at
+// 16^3x32) and the double-float passes where their threads loop (59.8 against
+// 57.7 ms a CG at 32^3x64).  Up to a block per SM the former gain (2.02 against
+// 2.28 ms at 4^4), and up to the full grid the latter (1.88 against 2.03 at
+// 8^3x32)
 template <class V>
-bool early_update(int64_t n)
+bool early_reduce(int64_t n)
 {
-    return std::is_same_v<V, VDF> || red_blocks(n) <= 152;
+    return red_blocks(n) <= (std::is_same_v<V, VDF> ? WD_RED_BLOCKS - 1 : 152);
 }
 
 // runs f(V()) for the vectors' storage
@@ -160,7 +161,7 @@ wd_status wd_cgd_norm(wd_context *ctx, WdVec t, int64_t n, WdCgDev *dev, WdRed r
 {
     return typed(ctx, t, [&](auto v) {
         using V = decltype(v);
-        wd_launch_pdl(true, k_cgd_norm<V>, red_blocks(n), WD_RED_THREADS, 0, ctx->stream, (const typename V::E *)t.p, n, dev, red);
+        wd_launch_pdl(early_reduce<V>(n), k_cgd_norm<V>, red_blocks(n), WD_RED_THREADS, 0, ctx->stream, (const typename V::E *)t.p, n, dev, red);
     });
 }
 
@@ -169,7 +170,7 @@ wd_status wd_cgd_dot(wd_context *ctx, WdVec p, WdVec q, int64_t n, WdCgDev *dev,
     return typed(ctx, p, [&](auto v) {
         using V = decltype(v);
         using E = typename V::E;
-        wd_launch_pdl(true, k_cgd_dot<V>, red_blocks(n), WD_RED_THREADS, 0, ctx->stream, (const E *)p.p, (const E *)q.p, n, dev, red);
+        wd_launch_pdl(early_reduce<V>(n), k_cgd_dot<V>, red_blocks(n), WD_RED_THREADS, 0, ctx->stream, (const E *)p.p, (const E *)q.p, n, dev, red);
     });
 }
 
@@ -181,8 +182,8 @@ wd_status wd_cgd_update(wd_context *ctx, bool cplx, WdVec p, WdVec q, WdVec x, W
         using E = typename V::E;
         const E *pp = (const E *)p.p, *qq = (const E *)q.p;
         E *xx = (E *)x.p, *rr = (E *)r.p;
-        if (cplx) wd_launch_pdl(early_update<V>(n), k_cgd_update<V, true>, red_blocks(n), WD_RED_THREADS, 0, ctx->stream, pp, qq, xx, rr, n, dev, red);
-        else wd_launch_pdl(early_update<V>(n), k_cgd_update<V, false>, red_blocks(n), WD_RED_THREADS, 0, ctx->stream, pp, qq, xx, rr, n, dev, red);
+        if (cplx) wd_launch_pdl(early_reduce<V>(n), k_cgd_update<V, true>, red_blocks(n), WD_RED_THREADS, 0, ctx->stream, pp, qq, xx, rr, n, dev, red);
+        else wd_launch_pdl(early_reduce<V>(n), k_cgd_update<V, false>, red_blocks(n), WD_RED_THREADS, 0, ctx->stream, pp, qq, xx, rr, n, dev, red);
     });
 }
 
@@ -192,6 +193,6 @@ wd_status wd_cgd_xpby(wd_context *ctx, WdVec r, WdVec p, int64_t n, const WdCgDe
     return typed(ctx, p, [&](auto v) {
         using V = decltype(v);
         using E = typename V::E;
-        wd_launch_pdl(true, k_cgd_xpby<V>, (int)(b < 152 * 16 ? b : 152 * 16), 256, 0, ctx->stream, (const E *)r.p, (E *)p.p, n, dev);
+        wd_launch_pdl(std::is_same_v<V, VF64> || b <= 152 * 16, k_cgd_xpby<V>, (int)(b < 152 * 16 ? b : 152 * 16), 256, 0, ctx->stream, (const E *)r.p, (E *)p.p, n, dev);
     });
 }

@@ -137,6 +137,7 @@ __device__ __forceinline__ SplitCtx split_ctx(const SplitDF &p)
 template <bool DAG, int WARPS>
 __global__ void __launch_bounds__(32 * WARPS) k_hop_df_pipe(const SplitDF p)
 {
+    wd_pdl_wait();
     if (p.stop && *p.stop) return;
     const SplitCtx x = split_ctx<WARPS>(p);
     dfc acc[4];
@@ -315,6 +316,7 @@ __device__ __forceinline__ void df_staged_site(const SplitDF &p, const SplitCtx 
 template <bool DAG, int WARPS, int LOOK, int NS, bool LCG>
 __global__ void __launch_bounds__(32 * WARPS) k_hop_df_staged(const SplitDF p)
 {
+    wd_pdl_wait();
     if (p.stop && *p.stop) return;
     const SplitCtx x = split_ctx<WARPS>(p);
     dfp acc[4];
@@ -417,6 +419,7 @@ __device__ __forceinline__ void df_group_site(const SplitDF &p, const SplitCtx &
 template <bool DAG, int GROUPS, bool LCG, int MINB>
 __global__ void __launch_bounds__(96 * GROUPS, MINB) k_hop_df_grouped(const SplitDF p)
 {
+    wd_pdl_wait();
     if (p.stop && *p.stop) return;
     const SplitCtx x = group_ctx<GROUPS>(p);
     dfp acc[4];
@@ -440,6 +443,7 @@ struct ResSinkDF {
 template <int WARPS, bool LCG, bool GROUPED = false, int MINB = 0>
 __global__ void __launch_bounds__(32 * WARPS, MINB) k_hop_df_res(const SplitDF p, const ResSinkDF r)
 {
+    wd_pdl_wait();
     const SplitCtx x = GROUPED ? group_ctx<WARPS / 3>(p) : split_ctx<WARPS>(p);
     dfp acc[4];
     if constexpr (GROUPED) df_group_site<false, WARPS / 3, LCG>(p, x, acc);
@@ -503,8 +507,8 @@ wd_status wd_hop_df(wd_context *ctx, const wd_lattice *lat, const float4 *in_blo
         constexpr int W = decltype(warps)::value;
         const int sites_per_block = kSitesPerWarp * W;
         const int blocks = (lat->g.Vh + sites_per_block - 1) / sites_per_block;
-        if (dag) k_hop_df_pipe<true, W><<<blocks, 32 * W, 0, ctx->stream>>>(p);
-        else k_hop_df_pipe<false, W><<<blocks, 32 * W, 0, ctx->stream>>>(p);
+        if (dag) wd_launch_early(k_hop_df_pipe<true, W>, blocks, 32 * W, ctx->stream, p);
+        else wd_launch_early(k_hop_df_pipe<false, W>, blocks, 32 * W, ctx->stream, p);
         WD_LAUNCHED(ctx);
         return WD_OK;
     };
@@ -513,8 +517,8 @@ wd_status wd_hop_df(wd_context *ctx, const wd_lattice *lat, const float4 *in_blo
         constexpr bool LCG = decltype(lcg)::value;
         const int sites_per_block = kSitesPerWarp * W;
         const int blocks = (lat->g.Vh + sites_per_block - 1) / sites_per_block;
-        if (dag) k_hop_df_staged<true, W, 1, 2, LCG><<<blocks, 32 * W, 0, ctx->stream>>>(p);
-        else k_hop_df_staged<false, W, 1, 2, LCG><<<blocks, 32 * W, 0, ctx->stream>>>(p);
+        if (dag) wd_launch_early(k_hop_df_staged<true, W, 1, 2, LCG>, blocks, 32 * W, ctx->stream, p);
+        else wd_launch_early(k_hop_df_staged<false, W, 1, 2, LCG>, blocks, 32 * W, ctx->stream, p);
         WD_LAUNCHED(ctx);
         return WD_OK;
     };
@@ -545,8 +549,8 @@ wd_status wd_hop_df(wd_context *ctx, const wd_lattice *lat, const float4 *in_blo
     // the grouped split: 2 groups (192 threads), registers capped for 4 blocks per SM
     auto run_grouped = [&]() -> wd_status {
         const int blocks = (lat->g.Vh + 63) / 64;
-        if (dag) k_hop_df_grouped<true, 2, true, 4><<<blocks, 192, 0, ctx->stream>>>(p);
-        else k_hop_df_grouped<false, 2, true, 4><<<blocks, 192, 0, ctx->stream>>>(p);
+        if (dag) wd_launch_early(k_hop_df_grouped<true, 2, true, 4>, blocks, 192, ctx->stream, p);
+        else wd_launch_early(k_hop_df_grouped<false, 2, true, 4>, blocks, 192, ctx->stream, p);
         WD_LAUNCHED(ctx);
         return WD_OK;
     };
@@ -585,7 +589,7 @@ wd_status wd_hop_df_residual(wd_context *ctx, const wd_lattice *lat, const float
         constexpr int W = decltype(warps)::value;
         const int sites_per_block = kSitesPerWarp * W;
         const int blocks = (lat->g.Vh + sites_per_block - 1) / sites_per_block;
-        k_hop_df_res<W, decltype(lcg)::value><<<blocks, 32 * W, 0, ctx->stream>>>(p, r);
+        wd_launch_early(k_hop_df_res<W, decltype(lcg)::value>, blocks, 32 * W, ctx->stream, p, r);
         WD_LAUNCHED(ctx);
         return WD_OK;
     };
@@ -593,7 +597,7 @@ wd_status wd_hop_df_residual(wd_context *ctx, const wd_lattice *lat, const float
     // variants 3 and 4 take variant 0's)
     const int v = wd_tune_choice(ctx, "hop_df64", lat->g.Vh);
     if (v == 5) {  // the grouped split (2 groups, 4 blocks per SM)
-        k_hop_df_res<6, true, true, 4><<<(lat->g.Vh + 63) / 64, 192, 0, ctx->stream>>>(p, r);
+        wd_launch_early(k_hop_df_res<6, true, true, 4>, (lat->g.Vh + 63) / 64, 192, ctx->stream, p, r);
         WD_LAUNCHED(ctx);
         return WD_OK;
     }

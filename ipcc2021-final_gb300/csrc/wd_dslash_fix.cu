@@ -237,7 +237,7 @@ template <bool DAG, int T, class Epi>
 __global__ void __launch_bounds__(block_threads(T), 512 / block_threads(T))
     k_hop_fix(const __grid_constant__ FixArgs a, const __grid_constant__ Epi epi, int s_lo, int s_hi)
 {
-    wd_pdl_wait();
+    wd_pdl_wait(T > 0);
     if (a.stop && *a.stop) return;
     constexpr bool AOS = Epi::AOS;
     constexpr int B = block_threads(T);

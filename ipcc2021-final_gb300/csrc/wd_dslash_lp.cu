@@ -158,8 +158,8 @@ template <class P>
 wd_status launch_hop(wd_context *ctx, const P &p, int dag)
 {
     const int blocks = (p.g.Vh + P::kThreads - 1) / P::kThreads;
-    if (dag) wd_hop_kernel<true><<<blocks, P::kThreads, 0, ctx->stream>>>(p);
-    else wd_hop_kernel<false><<<blocks, P::kThreads, 0, ctx->stream>>>(p);
+    if (dag) wd_launch_early(wd_hop_kernel<true, P>, blocks, P::kThreads, ctx->stream, p);
+    else wd_launch_early(wd_hop_kernel<false, P>, blocks, P::kThreads, ctx->stream, p);
     WD_LAUNCHED(ctx);
     return WD_OK;
 }
@@ -171,6 +171,7 @@ __global__ void __launch_bounds__(P::kThreads, wd_min_blocks<P>::value) k_hop_h1
     using Sp = decltype(p.in);
     using Lk = decltype(p.link);
     __shared__ LpStage<Sp, Lk, P::kThreads> st;
+    wd_pdl_wait();
     if (wd_gate_closed(p)) return;
     const int s = blockIdx.x * P::kThreads + threadIdx.x;
     if (s >= p.g.Vh) return;
@@ -183,8 +184,8 @@ template <class P>
 wd_status launch_hop_h16m(wd_context *ctx, const P &p, int dag)
 {
     const int blocks = (p.g.Vh + P::kThreads - 1) / P::kThreads;
-    if (dag) k_hop_h16m<true><<<blocks, P::kThreads, 0, ctx->stream>>>(p);
-    else k_hop_h16m<false><<<blocks, P::kThreads, 0, ctx->stream>>>(p);
+    if (dag) wd_launch_early(k_hop_h16m<true, P>, blocks, P::kThreads, ctx->stream, p);
+    else wd_launch_early(k_hop_h16m<false, P>, blocks, P::kThreads, ctx->stream, p);
     WD_LAUNCHED(ctx);
     return WD_OK;
 }
@@ -601,6 +602,7 @@ template <bool DAG, bool STAGED, int EPI, class P>
 __global__ void __launch_bounds__(P::kThreads, wd_min_blocks<P>::value) k_hop_lp_red(const P p)
 {
     constexpr int T = P::kThreads;
+    wd_pdl_wait();
     if (EPI != kEpiNormResult && p.dev->stop) return;  // the same value in every block of the launch
     const int s = blockIdx.x * T + threadIdx.x;
     const float v = red_site<DAG, STAGED, EPI>(p, s);
@@ -630,8 +632,9 @@ wd_status launch_red(wd_context *ctx, const char *name, const HopLP<Sp, Lk> &b, 
         q.dev = dev, q.red = red, q.pvec = pvec, q.rs = rs, q.xs = xs;
         q.result = result;
         const int blocks = (b.g.Vh + TH - 1) / TH;
-        if (dag) k_hop_lp_red<true, ST, EPI><<<blocks, TH, 0, ctx->stream>>>(q);
-        else k_hop_lp_red<false, ST, EPI><<<blocks, TH, 0, ctx->stream>>>(q);
+        using Q = decltype(q);
+        if (dag) wd_launch_early(k_hop_lp_red<true, ST, EPI, Q>, blocks, TH, ctx->stream, q);
+        else wd_launch_early(k_hop_lp_red<false, ST, EPI, Q>, blocks, TH, ctx->stream, q);
         WD_LAUNCHED(ctx);
         return WD_OK;
     };

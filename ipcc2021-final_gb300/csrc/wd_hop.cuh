@@ -20,6 +20,7 @@
 #pragma once
 #include <type_traits>
 #include "wd_internal.cuh"
+#include "wd_async.cuh"
 #include "wd_complex.cuh"
 
 template <class P, class = void>
@@ -339,6 +340,7 @@ __device__ __forceinline__ bool wd_gate_closed(const P &p)
 template <bool DAG, class P>
 __global__ void __launch_bounds__(P::kThreads, wd_min_blocks<P>::value) wd_hop_kernel(const P p)
 {
+    wd_pdl_wait();
     if (wd_gate_closed(p)) return;
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= p.g.Vh) return;

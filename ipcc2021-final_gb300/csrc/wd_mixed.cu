@@ -15,6 +15,7 @@
 #include <algorithm>
 #include <chrono>
 #include <cmath>
+#include "wd_async.cuh"
 #include "wd_df.cuh"
 #include "wd_lp.cuh"
 #include "wd_reduce.cuh"
@@ -71,6 +72,7 @@ __device__ __forceinline__ dfr df_sq_acc(dfr acc, float2 v)
 template <class SpL>
 __global__ void k_mx_xpay(SpF32 rs, float beta, SpL p, int Vh)
 {
+    wd_pdl_wait();
     SITE_STRIDE(s, Vh)
     {
         float2 rv[12], pv[12];
@@ -87,6 +89,7 @@ __global__ void k_mx_xpay(SpF32 rs, float beta, SpL p, int Vh)
 template <class SpL>
 __global__ void k_mx_xpay_dev(SpF32 rs, const WdMxDev *d, SpL p, int Vh)
 {
+    wd_pdl_wait();
     if (d->stop) return;
     const float beta = d->beta;
     SITE_STRIDE(s, Vh)
@@ -100,52 +103,12 @@ __global__ void k_mx_xpay_dev(SpF32 rs, const WdMxDev *d, SpL p, int Vh)
     }
 }
 
-template <class SpL>
-__global__ void __launch_bounds__(WD_RED_THREADS) k_mx_norm2(SpL t, int Vh, double2 *partial)
-{
-    dfr acc{0.f, 0.f};
-    SITE_STRIDE(s, Vh)
-    {
-        float2 v[12];
-        t.load(s, v);
-#pragma unroll
-        for (int c = 0; c < 12; ++c) acc = df_sq_acc(acc, v[c]);
-    }
-    wd_block_partial(df_value(acc), partial);
-}
-
-// high precision -> low precision (two outputs: FP32 r_s and kernel-storage p)
-template <class H, class SpL>
-__global__ void k_mx_from_h(H in, SpF32 a, SpL b, int Vh)
-{
-    SITE_STRIDE(s, Vh)
-    {
-        float2 v[12];
-#pragma unroll
-        for (int c = 0; c < 12; ++c) v[c] = in.load_f32(c, s);
-        a.store(s, v);
-        b.store(s, v);
-    }
-}
-
-// high precision -> FP32
-template <class H>
-__global__ void k_mx_to_f32(H in, SpF32 a, int Vh)
-{
-    SITE_STRIDE(s, Vh)
-    {
-        float2 v[12];
-#pragma unroll
-        for (int c = 0; c < 12; ++c) v[c] = in.load_f32(c, s);
-        a.store(s, v);
-    }
-}
-
 // s = bhat rounded to FP32, |s|^2: the residual of x = 0, in one pass over bhat
 // where the general update takes two high-precision hops
 template <class H>
 __global__ void __launch_bounds__(WD_RED_THREADS) k_mx_seed(H bhat, SpF32 s32, int Vh, WdRed red, double *result)
 {
+    wd_pdl_wait();
     dfr acc{0.f, 0.f};
     SITE_STRIDE(s, Vh)
     {
@@ -165,6 +128,7 @@ __global__ void __launch_bounds__(WD_RED_THREADS) k_mx_seed(H bhat, SpF32 s32, i
 template <class SpL>
 __global__ void k_mx_f32_to(SpF32 a, SpL b, int Vh)
 {
+    wd_pdl_wait();
     SITE_STRIDE(s, Vh)
     {
         float2 v[12];
@@ -177,6 +141,7 @@ __global__ void k_mx_f32_to(SpF32 a, SpL b, int Vh)
 template <class H>
 __global__ void k_mx_accum(SpF32 xs, H x, int Vh)
 {
+    wd_pdl_wait();
     SITE_STRIDE(s, Vh)
     {
         float2 v[12];
@@ -190,50 +155,29 @@ __global__ void k_mx_accum(SpF32 xs, H x, int Vh)
     }
 }
 
-// Reduction kernels always run the fixed grid of WD_RED_BLOCKS blocks (idle
-// blocks write zero partials): wd_red_finish folds exactly that many.
-inline int site_grid(int) { return WD_RED_BLOCKS; }
-
 // Typed launchers over (kernel storage L) x (high precision H)
 struct Mixed {
     wd_context *ctx;
     int Vh;
     wd_precision L, H;
 
+    // a pass over the sites: memory-bound, so an early launch gains at every size
+    template <class... P, class... A>
+    void launch(void (*kernel)(P...), A... args) const
+    {
+        wd_launch_pdl(true, kernel, (Vh + WD_RED_THREADS - 1) / WD_RED_THREADS, WD_RED_THREADS, 0, ctx->stream, args...);
+    }
     wd_status xpay(WdVec rs, float beta, WdVec p) const
     {
-        if (L == WD_PREC_F32) k_mx_xpay<<<site_grid(Vh), WD_RED_THREADS, 0, ctx->stream>>>(sp_f32(rs, Vh), beta, sp_f32(p, Vh), Vh);
-        else k_mx_xpay<<<site_grid(Vh), WD_RED_THREADS, 0, ctx->stream>>>(sp_f32(rs, Vh), beta, sp_f16(p, Vh), Vh);
+        if (L == WD_PREC_F32) launch(k_mx_xpay<SpF32>, sp_f32(rs, Vh), beta, sp_f32(p, Vh), Vh);
+        else launch(k_mx_xpay<SpF16>, sp_f32(rs, Vh), beta, sp_f16(p, Vh), Vh);
         WD_LAUNCHED(ctx);
         return WD_OK;
     }
     wd_status xpay_dev(WdVec rs, const WdMxDev *d, WdVec p) const
     {
-        if (L == WD_PREC_F32) k_mx_xpay_dev<<<site_grid(Vh), WD_RED_THREADS, 0, ctx->stream>>>(sp_f32(rs, Vh), d, sp_f32(p, Vh), Vh);
-        else k_mx_xpay_dev<<<site_grid(Vh), WD_RED_THREADS, 0, ctx->stream>>>(sp_f32(rs, Vh), d, sp_f16(p, Vh), Vh);
-        WD_LAUNCHED(ctx);
-        return WD_OK;
-    }
-    wd_status from_h(WdVec h, WdVec rs, WdVec p) const
-    {
-        const int g = site_grid(Vh);
-        if (H == WD_PREC_F64) {
-            const HF64 in{(double2 *)h.p, Vh};
-            if (L == WD_PREC_F32) k_mx_from_h<<<g, WD_RED_THREADS, 0, ctx->stream>>>(in, sp_f32(rs, Vh), sp_f32(p, Vh), Vh);
-            else k_mx_from_h<<<g, WD_RED_THREADS, 0, ctx->stream>>>(in, sp_f32(rs, Vh), sp_f16(p, Vh), Vh);
-        } else {
-            const HDF in{(float4 *)h.p, Vh};
-            if (L == WD_PREC_F32) k_mx_from_h<<<g, WD_RED_THREADS, 0, ctx->stream>>>(in, sp_f32(rs, Vh), sp_f32(p, Vh), Vh);
-            else k_mx_from_h<<<g, WD_RED_THREADS, 0, ctx->stream>>>(in, sp_f32(rs, Vh), sp_f16(p, Vh), Vh);
-        }
-        WD_LAUNCHED(ctx);
-        return WD_OK;
-    }
-    wd_status to_f32(WdVec h, WdVec a) const
-    {
-        const int g = site_grid(Vh);
-        if (H == WD_PREC_F64) k_mx_to_f32<<<g, WD_RED_THREADS, 0, ctx->stream>>>(HF64{(double2 *)h.p, Vh}, sp_f32(a, Vh), Vh);
-        else k_mx_to_f32<<<g, WD_RED_THREADS, 0, ctx->stream>>>(HDF{(float4 *)h.p, Vh}, sp_f32(a, Vh), Vh);
+        if (L == WD_PREC_F32) launch(k_mx_xpay_dev<SpF32>, sp_f32(rs, Vh), d, sp_f32(p, Vh), Vh);
+        else launch(k_mx_xpay_dev<SpF16>, sp_f32(rs, Vh), d, sp_f16(p, Vh), Vh);
         WD_LAUNCHED(ctx);
         return WD_OK;
     }
@@ -243,29 +187,21 @@ struct Mixed {
             WD_CUDA(ctx, cudaMemcpyAsync(p.p, a.p, (size_t)12 * Vh * sizeof(float2), cudaMemcpyDeviceToDevice, ctx->stream));
             return WD_OK;
         }
-        k_mx_f32_to<<<site_grid(Vh), WD_RED_THREADS, 0, ctx->stream>>>(sp_f32(a, Vh), sp_f16(p, Vh), Vh);
+        launch(k_mx_f32_to<SpF16>, sp_f32(a, Vh), sp_f16(p, Vh), Vh);
         WD_LAUNCHED(ctx);
         return WD_OK;
     }
-    wd_status norm2_f32(WdVec t, int slot) const
-    {
-        k_mx_norm2<<<site_grid(Vh), WD_RED_THREADS, 0, ctx->stream>>>(sp_f32(t, Vh), Vh, (double2 *)ctx->red_partial);
-        WD_LAUNCHED(ctx);
-        return wd_red_finish(ctx, slot);
-    }
     wd_status seed(WdVec bhat, WdVec s32, const WdRed &red, double *result) const
     {
-        const int b = (Vh + WD_RED_THREADS - 1) / WD_RED_THREADS, g = b < WD_RED_BLOCKS ? b : WD_RED_BLOCKS;
-        if (H == WD_PREC_F64) k_mx_seed<<<g, WD_RED_THREADS, 0, ctx->stream>>>(HF64{(double2 *)bhat.p, Vh}, sp_f32(s32, Vh), Vh, red, result);
-        else k_mx_seed<<<g, WD_RED_THREADS, 0, ctx->stream>>>(HDF{(float4 *)bhat.p, Vh}, sp_f32(s32, Vh), Vh, red, result);
+        if (H == WD_PREC_F64) launch(k_mx_seed<HF64>, HF64{(double2 *)bhat.p, Vh}, sp_f32(s32, Vh), Vh, red, result);
+        else launch(k_mx_seed<HDF>, HDF{(float4 *)bhat.p, Vh}, sp_f32(s32, Vh), Vh, red, result);
         WD_LAUNCHED(ctx);
         return WD_OK;
     }
     wd_status accum(WdVec xs, WdVec xh) const
     {
-        const int g = site_grid(Vh);
-        if (H == WD_PREC_F64) k_mx_accum<<<g, WD_RED_THREADS, 0, ctx->stream>>>(sp_f32(xs, Vh), HF64{(double2 *)xh.p, Vh}, Vh);
-        else k_mx_accum<<<g, WD_RED_THREADS, 0, ctx->stream>>>(sp_f32(xs, Vh), HDF{(float4 *)xh.p, Vh}, Vh);
+        if (H == WD_PREC_F64) launch(k_mx_accum<HF64>, sp_f32(xs, Vh), HF64{(double2 *)xh.p, Vh}, Vh);
+        else launch(k_mx_accum<HDF>, sp_f32(xs, Vh), HDF{(float4 *)xh.p, Vh}, Vh);
         WD_LAUNCHED(ctx);
         return WD_OK;
     }
@@ -300,11 +236,6 @@ struct DevBlock {
 wd_status wd_mx_accum(wd_context *ctx, int Vh, wd_precision H, WdVec xs, WdVec xh)
 {
     return Mixed{ctx, Vh, WD_PREC_F32, H}.accum(xs, xh);
-}
-
-wd_status wd_mx_from_h(wd_context *ctx, int Vh, wd_precision L, wd_precision H, WdVec h, WdVec rs, WdVec p)
-{
-    return Mixed{ctx, Vh, L, H}.from_h(h, rs, p);
 }
 
 // Reliable update shared by the solo and batched mixed solvers:

@@ -29,8 +29,6 @@ wd_status wd_solve_cg_eo_mixed(wd_context *ctx, const wd_lattice *lat, const dou
 // reliable-update pieces shared by the mixed solvers (wd_mixed.cu):
 // xh (FP64 or double-float) += xs (FP32), xs = 0
 wd_status wd_mx_accum(wd_context *ctx, int Vh, wd_precision H, WdVec xs, WdVec xh);
-// rs (FP32) <- h and p (storage L) <- h
-wd_status wd_mx_from_h(wd_context *ctx, int Vh, wd_precision L, wd_precision H, WdVec h, WdVec rs, WdVec p);
 // one system's buffers for a reliable update (even-parity half-lattice blocks)
 struct WdMxReliable {
     WdVec xs;         // FP32 solution increment (zeroed)
