@@ -120,13 +120,43 @@ __host__ __device__ __forceinline__ dfr df_split(double x)
     const float h = (float)x;
     return dfr{h, (float)(x - (double)h)};
 }
+// A conversion between the float types is an FP64-pipe operation, which holds
+// that pipe for 16 cycles per warp; the passes that convert whole vectors were
+// bound by it (48^3x96: f64 -> df 1.82 ms with four operations a real, df -> f64
+// 1.35 ms with three).  The forms below give the same bits with one each: 0.59
+// and 0.62 ms, the time of the bytes.
+
+// (double)f on integers: the exponent is rebiased, a subnormal first scaled
+// into the normal range
+__device__ __forceinline__ double df_widen(float f)
+{
+    const bool sub = (__float_as_uint(f) & 0x7f800000u) == 0;
+    const unsigned b = __float_as_uint(sub ? __fmul_rn(f, 16777216.f) : f), mag = b & 0x7fffffffu;
+    const unsigned hi = (mag >> 3) + (sub ? 0x36800000u : mag >= 0x7f800000u ? 0x70000000u : 0x38000000u);
+    return __hiloint2double((int)((mag ? hi : 0u) | (b & 0x80000000u)), (int)(b << 29));
+}
+// df_split with x - h on integers: it is at most 2^28 units of x's last place,
+// so the low words hold it, and it rounds to l as an integer does, while h and
+// l are normal; other values (but zero) take the general form, in warps that
+// have any (a call, so that it is not predicated into the others' path)
+static __device__ __noinline__ float df_split_low(double x, float h) { return (float)(x - (double)h); }
+__device__ __forceinline__ dfr df_split_vec(double x)
+{
+    const float h = (float)x;
+    const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x), e = hi >> 20 & 0x7ffu;
+    const int d = (int)(lo - (__float_as_uint(h) << 29));
+    const bool zero = ((hi << 1) | lo) == 0, normal = e - 949u <= 200u;
+    float l = zero ? 0.f : __fmul_rn(__int2float_rn((int)hi < 0 ? -d : d), __uint_as_float((e - 948u) << 23));
+    if (!zero && !normal) l = df_split_low(x, h);
+    return dfr{h, l};
+}
 __device__ __forceinline__ double df_value(dfr a) { return (double)a.h + (double)a.l; }
 __device__ __forceinline__ float4 df_pack(double2 v)
 {
-    const dfr r = df_split(v.x), i = df_split(v.y);
+    const dfr r = df_split_vec(v.x), i = df_split_vec(v.y);
     return make_float4(r.h, i.h, r.l, i.l);
 }
 __device__ __forceinline__ double2 df_unpack(float4 v)
 {
-    return make_double2((double)v.x + (double)v.z, (double)v.y + (double)v.w);
+    return make_double2(df_widen(v.x) + df_widen(v.z), df_widen(v.y) + df_widen(v.w));
 }

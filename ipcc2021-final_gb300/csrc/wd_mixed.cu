@@ -37,8 +37,8 @@ struct HF64 {
     __device__ void add_f32(int c, int s, float2 v) const
     {
         double2 d = load(c, s);
-        d.x += (double)v.x;
-        d.y += (double)v.y;
+        d.x += df_widen(v.x);
+        d.y += df_widen(v.y);
         store(c, s, d);
     }
 };
