@@ -495,7 +495,6 @@ class BatchEngine {
         for (auto &kv : graphs_) cudaGraphExecDestroy(kv.second);
         graphs_.clear();
     }
-    wd_status reliable(EngineSys &s, bool reset_p, double *rr, double *ss);
     wd_status reliable_enqueue(EngineSys &s, bool reset_p, double *rr_dev, double *ss_dev);
     wd_status finish(EngineSys &s);
     wd_status rebuild();
@@ -515,18 +514,6 @@ static inline void slices(EngineSys &s, WdVec &b_e, WdVec &b_o, WdVec &x_e, WdVe
 }
 
 // reliable update: x_e += x_s; s = bhat - Mhat x_e; r_s = Mhat^dag s (FP32); p <- r_s on a restart
-wd_status BatchEngine::reliable(EngineSys &s, bool reset_p, double *rr, double *ss)
-{
-    double2 *res = (double2 *)ctx_->red_partial + WD_RED_BLOCKS;
-    wd_status e = reliable_enqueue(s, reset_p, &res[0].x, &res[1].x);
-    if (e != WD_OK) return e;
-    double2 red[2];
-    if ((e = wd_red_fetch(ctx_, 2, red)) != WD_OK) return e;
-    *rr = red[0].x;
-    *ss = red[1].x;
-    return WD_OK;
-}
-
 wd_status BatchEngine::reliable_enqueue(EngineSys &s, bool reset_p, double *rr_dev, double *ss_dev)
 {
     SysBufs &B = s.B;
@@ -571,12 +558,13 @@ wd_status BatchEngine::add(int tag, const wd_lattice *lat, const double2 *src, d
     if ((st = wd_hop_v(ctx_, lat, b_o, B.bhat.v, &b_e, 0, 0, 0.5 / a, 1.0)) != WD_OK) return st;
     if ((st = wd_v_zero(ctx_, B.hx.v, 2 * nh)) != WD_OK) return st;
     if ((st = wd_v_zero(ctx_, B.xs.v, nh)) != WD_OK) return st;
-    if ((st = wd_red_norm2(ctx_, src, 2 * nh, 0)) != WD_OK) return st;
-    double2 v;
-    if ((st = wd_red_fetch(ctx_, 1, &v)) != WD_OK) return st;
-    s.norm_b = v.x > 0 ? std::sqrt(v.x) : 1.0;
-    double rr, ss;
-    if ((st = reliable(s, true, &rr, &ss)) != WD_OK) return st;
+    // |b|^2 and the first residual's norms with one wait
+    double2 *res = (double2 *)ctx_->red_partial + WD_RED_BLOCKS, red[3];
+    if ((st = wd_red_norm2(ctx_, src, 2 * nh, 2)) != WD_OK) return st;
+    if ((st = reliable_enqueue(s, true, &res[0].x, &res[1].x)) != WD_OK) return st;
+    if ((st = wd_red_fetch(ctx_, 3, red)) != WD_OK) return st;
+    const double rr = red[0].x, ss = red[1].x;
+    s.norm_b = red[2].x > 0 ? std::sqrt(red[2].x) : 1.0;
     s.true_res = std::sqrt(ss) / s.norm_b;
     s.ratio = ss > 0 ? std::sqrt(rr / ss) : 1.0;
     s.target = tol * s.norm_b * s.ratio * 0.5;
@@ -1239,11 +1227,8 @@ static wd_status server_source(wd_server *sv, const wd_server::Pending &p, int k
     k_gen_source<<<152 * 8, 256, 0, ctx->stream>>>(gen_mix(p.seeds[k] ^ 0xA5A5A5A5ull), Vh, f->d);
     WD_LAUNCHED(ctx);
     const int64_t n = f->lat->volume * 12;
-    wd_status st = wd_red_norm2(ctx, f->d, n, 0);
-    if (st != WD_OK) return st;
-    double2 v;
-    if ((st = wd_red_fetch(ctx, 1, &v)) != WD_OK) return st;
-    return wd_blas_scale(ctx, v.x > 0 ? 1.0 / std::sqrt(v.x) : 1.0, f->d, f->d, n);
+    const wd_status st = wd_red_norm2(ctx, f->d, n, 0);
+    return st == WD_OK ? wd_blas_unit(ctx, f->d, n, 0) : st;
 }
 
 // systems k0.. of request r that could not be admitted complete as failed

@@ -183,6 +183,21 @@ __global__ void k_scale(double a, const double2 *__restrict__ x, double2 *__rest
     }
 }
 
+// x /= |x| with the sum |x|^2 on the device, where it was just left; one
+// thread's square root and quotient a block (FP64 pipe)
+__global__ void k_unit(double2 *__restrict__ x, int64_t n, const double2 *norm2)
+{
+    __shared__ double f;
+    if (threadIdx.x == 0) f = norm2->x > 0 ? 1.0 / sqrt(norm2->x) : 1.0;
+    __syncthreads();
+    const double a = f;
+    GRID_STRIDE(i, n)
+    {
+        const double2 u = x[i];
+        x[i] = make_double2(a * u.x, a * u.y);
+    }
+}
+
 // y = x + b y, b real
 __global__ void k_xpby_real(const double2 *__restrict__ x, double b, double2 *__restrict__ y, int64_t n)
 {
@@ -332,6 +347,13 @@ wd_status wd_blas_xpayz(wd_context *ctx, const double2 *x, double2 a, const doub
 wd_status wd_blas_scale(wd_context *ctx, double a, const double2 *x, double2 *y, int64_t n)
 {
     k_scale<<<blas_blocks(n), 256, 0, ctx->stream>>>(a, x, y, n);
+    WD_LAUNCHED(ctx);
+    return WD_OK;
+}
+
+wd_status wd_blas_unit(wd_context *ctx, double2 *x, int64_t n, int slot)
+{
+    k_unit<<<blas_blocks(n), 256, 0, ctx->stream>>>(x, n, (const double2 *)ctx->red_partial + WD_RED_BLOCKS + slot);
     WD_LAUNCHED(ctx);
     return WD_OK;
 }

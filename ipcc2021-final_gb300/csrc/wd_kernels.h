@@ -67,6 +67,8 @@ wd_status wd_blas_xpayz(wd_context *ctx, const double2 *x, double2 a, const doub
                         double2 *z, int64_t n);
 // y = a*x (real a)
 wd_status wd_blas_scale(wd_context *ctx, double a, const double2 *x, double2 *y, int64_t n);
+// x /= |x| (|x|^2 in result slot `slot`; a zero x stays)
+wd_status wd_blas_unit(wd_context *ctx, double2 *x, int64_t n, int slot);
 
 // ---- double-float (df64) storage: float4 {re.h, im.h, re.l, im.l} per complex
 wd_status wd_hop_df(wd_context *ctx, const wd_lattice *lat, const float4 *in_block, float4 *out_block,
