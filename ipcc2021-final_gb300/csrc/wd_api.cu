@@ -283,14 +283,17 @@ static void *pinned_view(const void *p)
 
 // Allocates the lattice's fixed-point links if it has none: a copy that only
 // makes FP64 hops faster, so it is kept where it leaves at least half of the
-// device's memory free, and given back when a later allocation needs its
-// memory (wd_malloc).  Returns the device flag behind the planes, or null.
+// device's memory free or in the context's work-buffer cache (an eighth free),
+// and given back when a later allocation needs its memory (wd_malloc).  Returns the device flag behind the planes, or null.
 static int *want_fix(wd_context *ctx, wd_lattice *lat)
 {
     const size_t n = (size_t)lat->volume * 4 * 9 * sizeof(int4);
     if (!lat->gauge_fix && lat->use_fix) {
         size_t free_b = 0, total_b = 0;
-        const bool room = n < (64u << 20) || (cudaMemGetInfo(&free_b, &total_b) == cudaSuccess && free_b >= n + total_b / 2);
+        size_t cached = 0;
+        for (const auto &kv : ctx->pool_free) cached += kv.first;
+        const bool room = n < (64u << 20) || (cudaMemGetInfo(&free_b, &total_b) == cudaSuccess &&
+                                              free_b + cached >= n + total_b / 2 && free_b >= n + total_b / 8);
         if (!room || cudaMalloc(&lat->gauge_fix, n + sizeof(int4)) != cudaSuccess) {
             cudaGetLastError();
             lat->gauge_fix = nullptr;

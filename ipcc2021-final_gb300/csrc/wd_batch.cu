@@ -1257,7 +1257,10 @@ static wd_status server_admit(wd_server *sv, int *completed)
         wd_server::Pending &p = sv->queue.front();
         const wd_lattice *lat = sv->lats[p.lat];
         const double bytes = request_bytes(sv, lat, p.nsrc);
-        if (sv->gauge_bytes + sv->req_bytes + bytes > sv->cfg.hbm_budget_bytes) break;
+        // FP64 mode solves one system at a time: admitting a request early is not
+        // worth the fixed-point links (a quarter of the hop's time)
+        const double keep = !sv->eng && sv->active_systems > 0 ? server_fix_bytes(sv) : 0.0;
+        if (sv->gauge_bytes + sv->req_bytes + keep + bytes > sv->cfg.hbm_budget_bytes) break;
         if (sv->active_systems > 0 && sv->active_systems + p.nsrc > sv->cfg.max_systems) break;
         server_make_room(sv, bytes);
         wd_server::Req &r = sv->reqs[p.id];
