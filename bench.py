@@ -145,7 +145,7 @@ def measured_peak_hbm() -> tuple[float, str]:
 # at 32^3x64, from one ncu capture of each kernel at 24^3x48 scaled by the
 # number of output sites (traffic per site is constant across volumes for
 # these kernels); not measured by this run.
-TRAFFIC_PER_LAUNCH = {"f64": 1.595e9, "df64": 1.592e9, "f32": 5.660e8, "f16": 2.706e8}
+TRAFFIC_PER_LAUNCH = {"f64": 1.590e9, "df64": 1.592e9, "f32": 5.660e8, "f16": 2.706e8}
 TRAFFIC_SOURCE = ("ncu capture at 24^3x48 of the same kernel (dram__bytes_read.sum + dram__bytes_write.sum), "
                   "scaled to 32^3x64 by output sites; a recorded constant, not measured in this run")
 
@@ -670,7 +670,8 @@ def run_ours(args) -> None:
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                          "frac": achieved / peak, "traffic": traffic, "traffic_source": TRAFFIC_SOURCE,
                          "peak_source": peak_src,
-                         "note": "FP64 kernels are bounded by the FP64 pipe on GB300; see compute"},
+                         "note": "the FP64 hop computes in fixed point on the integer pipe, which bounds it with the FP64 pipe's "
+                                 "share; compute.fp64_frac is against the FP64 FMA peak and can exceed 1"},
             "compute": {"bound": "fp64" if args.prec == "f64" else "fp32",
                         "achieved_tflops": gflops / 1e3,
                         "fp64_peak_tflops": fp64_peak, "fp32_peak_tflops": fp32_peak,

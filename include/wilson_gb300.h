@@ -43,7 +43,7 @@ typedef enum wd_status {
 
 /* Arithmetic used by the hopping kernels. */
 typedef enum wd_precision {
-    WD_PREC_F64 = 0,  /* native FP64 */
+    WD_PREC_F64 = 0,  /* FP64 (links of unitary size: fixed point on the integer pipe, same accuracy) */
     WD_PREC_DF64 = 1, /* double-float: FP32 hi/lo pairs, ~48-bit mantissa, FP64-class results */
     WD_PREC_F32 = 2,  /* FP32 storage and arithmetic */
     WD_PREC_F16 = 3   /* FP16 spinors with a per-site FP32 scale, 12-real links, FP32 arithmetic */
