@@ -32,7 +32,7 @@
 // are multiplied (0.472 -> 0.386 ms at 32^3x64); a row's links are read
 // from there when the row is due (0.377).  Complex products take three real
 // ones (Gauss): additions are cheaper than wide multiply-adds here.
-// Measured at 32^3x64: 0.357 ms (FP64 form 1.453 ms), 4.52 TB/s of
+// Measured at 32^3x64: 0.354 ms (FP64 form 1.453 ms), 4.55 TB/s of
 // compulsory bytes, 68 % of measured HBM; 0.372 ms before the power-of-two
 // factor moved into the final conversion and the site coordinates lost their
 // divisions.  What bounds it now is issue and the integer pipes together
