@@ -76,6 +76,12 @@ wd_status wd_context_device_check(wd_context *ctx);
  * WD_ERR_OOM; n < 0 turns it off (the default).  Returns the previous
  * setting (the allocations left before failing, or -1). */
 int wd_debug_fail_allocations_after(wd_context *ctx, int n);
+/* The same for device memory that runs short: after n more requests to CUDA
+ * for memory on this context, one finds none free until the lattices' second
+ * copies of their links, held for speed only, have been given back
+ * (WD_ERR_OOM if there are none).  Acts once; n < 0 turns it off (the default).  Returns the previous
+ * setting (the requests left, or -1). */
+int wd_debug_exhaust_memory_after(wd_context *ctx, int n);
 /* Testing aid for the bounded device waits: one warp waits on a shared-memory
  * barrier that nothing completes; the wait gives up after its bound (0.5 s)
  * and sets the device error flag, as a kernel whose copies never landed

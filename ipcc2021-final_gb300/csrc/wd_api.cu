@@ -112,11 +112,14 @@ bool wd_release_fix(wd_context *ctx)
 
 cudaError_t wd_malloc(wd_context *ctx, void **p, size_t bytes)
 {
-    cudaError_t e = cudaMalloc(p, bytes);
+    // injected exhaustion: as if only what the steps below give back made room
+    const bool full = ctx->exhaust_after == 0;
+    if (ctx->exhaust_after >= 0) --ctx->exhaust_after;
+    cudaError_t e = full ? cudaErrorMemoryAllocation : cudaMalloc(p, bytes);
     if (e == cudaErrorMemoryAllocation && !ctx->pool_free.empty()) {
         cudaGetLastError();
         wd_pool_release(ctx);
-        e = cudaMalloc(p, bytes);
+        if (!full) e = cudaMalloc(p, bytes);
     }
     if (e == cudaErrorMemoryAllocation && wd_release_fix(ctx)) {
         cudaGetLastError();
@@ -214,6 +217,14 @@ extern "C" int wd_debug_fail_allocations_after(wd_context *ctx, int n)
     if (!ctx) return -1;
     const int prev = ctx->fail_alloc_after;
     ctx->fail_alloc_after = n < 0 ? -1 : n;
+    return prev;
+}
+
+extern "C" int wd_debug_exhaust_memory_after(wd_context *ctx, int n)
+{
+    if (!ctx) return -1;
+    const int prev = ctx->exhaust_after;
+    ctx->exhaust_after = n < 0 ? -1 : n;
     return prev;
 }
 extern "C" uint64_t wd_context_launches(const wd_context *ctx) { return ctx ? ctx->launches : 0; }

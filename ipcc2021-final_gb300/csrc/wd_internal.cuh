@@ -87,6 +87,7 @@ struct wd_context {
     // field / work-buffer allocations the next ones fail with WD_ERR_OOM
     // (-1: off)
     int fail_alloc_after = -1;
+    int exhaust_after = -1;  // after this many more device memory requests one finds memory exhausted (-1: off)
 };
 
 // true when the injected allocation failure applies to this allocation

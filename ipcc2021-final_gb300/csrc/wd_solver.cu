@@ -75,10 +75,13 @@ wd_status wd_true_residual(wd_context *ctx, const wd_lattice *lat, const double2
     const int64_t n = lat->volume * 12;
     double2 r[2];
     wd_status st;
+    const int64_t rb = wd_red_blocks(lat->g.Vh);
+    WdVecBuf buf;
+    // an allocation may give the fixed-point links back: looked for after it
+    if (lat->gauge_fix &&
+        (st = wd_vec_alloc(ctx, buf, WD_PREC_F64, (int64_t)wd_red_doubles(rb, 2) / 2 + 1)) != WD_OK)
+        return st;
     if (lat->gauge_fix) {
-        const int64_t rb = wd_red_blocks(lat->g.Vh);
-        WdVecBuf buf;
-        if ((st = wd_vec_alloc(ctx, buf, WD_PREC_F64, (int64_t)wd_red_doubles(rb, 2) / 2 + 1)) != WD_OK) return st;
         const WdRed red = wd_red_view(buf.v.p, rb);
         double2 *res = (double2 *)ctx->red_partial + WD_RED_BLOCKS;
         WD_CUDA(ctx, cudaMemsetAsync(red.counters, 0, wd_red_counters(rb) * sizeof(unsigned), ctx->stream));
@@ -175,7 +178,8 @@ static wd_status cgnr_ref_core(wd_context *ctx, const wd_lattice *lat, WdVec src
 {
     const int64_t n = lat->volume * 12;
     const double m = prm->mass;
-    const bool fused = src.prec == WD_PREC_F64 && lat->gauge_fix;
+    // looked for at each launch: any allocation may give the fixed-point links back
+    const auto fused = [&] { return src.prec == WD_PREC_F64 && lat->gauge_fix; };
     WdVecBuf b[5];
     for (auto &v : b) {
         wd_status s = wd_vec_alloc(ctx, v, src.prec, n);
@@ -201,7 +205,7 @@ static wd_status cgnr_ref_core(wd_context *ctx, const wd_lattice *lat, WdVec src
     auto iteration = [&]() -> wd_status {
         wd_status e;
         if ((e = wd_apply_M_v(ctx, lat, p, qq, m, 0, &dev->stop)) != WD_OK) return e;
-        if (fused) {
+        if (fused()) {
             if ((e = wd_hop_fix_M_dot(ctx, lat, qq, q, p, m, dev, loop.red)) != WD_OK) return e;
         } else {
             if ((e = wd_apply_M_v(ctx, lat, qq, q, m, 1, &dev->stop)) != WD_OK) return e;
@@ -227,7 +231,7 @@ static wd_status cg_eo_core(wd_context *ctx, const wd_lattice *lat, WdVec src, W
     const int Vh = lat->g.Vh;
     const int64_t nh = (int64_t)12 * Vh;
     const double m = prm->mass, a = 4.0 + m;
-    const bool fused = src.prec == WD_PREC_F64 && lat->gauge_fix;
+    const auto fused = [&] { return src.prec == WD_PREC_F64 && lat->gauge_fix; };  // as in cgnr_ref_core
     WdVecBuf b[7];
     for (auto &v : b) {
         wd_status s = wd_vec_alloc(ctx, v, src.prec, nh);
@@ -272,14 +276,14 @@ static wd_status cg_eo_core(wd_context *ctx, const wd_lattice *lat, WdVec src, W
     auto iteration = [&]() -> wd_status {
         wd_status e;
         if ((e = wd_hop_v(ctx, lat, p, tmp_o, nullptr, 1, 0, 1.0, 0.0, &dev->stop)) != WD_OK) return e;
-        if (fused) {
+        if (fused()) {
             if ((e = wd_hop_fix_norm(ctx, lat, tmp_o, t, p, m, dev, loop.red)) != WD_OK) return e;
         } else {
             if ((e = wd_hop_v(ctx, lat, tmp_o, t, &p, 0, 0, -0.25 / a, a, &dev->stop)) != WD_OK) return e;
             if ((e = wd_cgd_norm(ctx, t, nh, dev, loop.red)) != WD_OK) return e;
         }
         if ((e = wd_hop_v(ctx, lat, t, tmp_o, nullptr, 1, 1, 1.0, 0.0, &dev->stop)) != WD_OK) return e;
-        if (fused) {
+        if (fused()) {
             if ((e = wd_hop_fix_update(ctx, lat, tmp_o, t, p, r, x_e, m, dev, loop.red)) != WD_OK) return e;
         } else {
             if ((e = wd_hop_v(ctx, lat, tmp_o, q, &t, 0, 1, -0.25 / a, a, &dev->stop)) != WD_OK) return e;

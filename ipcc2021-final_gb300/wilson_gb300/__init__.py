@@ -76,6 +76,7 @@ def _load() -> C.CDLL:
         "wd_context_device_check": (C.c_int, [vp]),
         "wd_debug_expire_wait": (C.c_int, [vp, C.POINTER(C.c_double)]),
         "wd_debug_fail_allocations_after": (C.c_int, [vp, C.c_int]),
+        "wd_debug_exhaust_memory_after": (C.c_int, [vp, C.c_int]),
         "wd_lattice_create": (C.c_int, [vp, ip, d4, C.POINTER(vp)]),
         "wd_lattice_update": (C.c_int, [vp, vp, d4]),
         "wd_lattice_destroy": (None, [vp]),
@@ -273,6 +274,12 @@ class Context:
         """Testing aid: the next allocations after n more successful ones fail
         with OOM (n < 0: off).  Returns the previous setting."""
         return int(lib.wd_debug_fail_allocations_after(self.handle, int(n)))
+
+    def exhaust_memory_after(self, n: int) -> int:
+        """Testing aid: after n more device memory requests one finds memory
+        exhausted and gives back what is held for speed only (n < 0: off).
+        Returns the previous setting (-1 once it has acted)."""
+        return int(lib.wd_debug_exhaust_memory_after(self.handle, int(n)))
 
     def fma_peak(self) -> tuple[float, float]:
         """Measured (FP64, FP32) FMA throughput of the device in TFLOP/s."""
