@@ -4,6 +4,7 @@
 #include <cstring>
 #include <cstdio>
 #include <string>
+#include "wd_fix_links.h"
 #include "wd_kernels.h"
 #include "wd_precision.h"
 #include "wd_solver.h"
@@ -95,19 +96,58 @@ static void host_cache_drop(wd_context *ctx)
     for (auto &p : ctx->host_gauge_ptr) p = nullptr;
 }
 
-// the fixed-point links of one lattice, if it has them (cudaFree waits for work in flight)
-void wd_drop_fix(wd_lattice *lat)
+// ------------------------------------------- fixed-point links (wd_fix_links.h)
+static wd_lattice *fix_list = nullptr;
+
+std::shared_mutex &wd_fix_mutex()
 {
-    cudaFree(lat->gauge_fix);
-    lat->gauge_fix = nullptr;
-    if (lat->ctx) lat->ctx->fix_lats.erase(lat);
+    static auto *m = new std::shared_mutex;  // never destroyed: lattices may outlive static objects
+    return *m;
 }
 
-bool wd_release_fix(wd_context *ctx)
+void wd_fix_enter(wd_lattice *lat, void *links)
 {
-    const bool any = !ctx->fix_lats.empty();
-    while (!ctx->fix_lats.empty()) wd_drop_fix(*ctx->fix_lats.begin());
+    lat->gauge_fix = links;
+    lat->fix_prev = nullptr;
+    lat->fix_next = fix_list;
+    if (fix_list) fix_list->fix_prev = lat;
+    fix_list = lat;
+}
+
+void wd_fix_free(wd_lattice *lat)
+{
+    if (!lat->gauge_fix) return;
+    cudaDeviceSynchronize();  // launches of any context may still read them
+    cudaFree(lat->gauge_fix);
+    lat->gauge_fix = nullptr;
+    (lat->fix_prev ? lat->fix_prev->fix_next : fix_list) = lat->fix_next;
+    if (lat->fix_next) lat->fix_next->fix_prev = lat->fix_prev;
+    lat->fix_prev = lat->fix_next = nullptr;
+}
+
+void wd_drop_fix(wd_lattice *lat)
+{
+    const WdFixAlone lock(wd_fix_mutex());
+    wd_fix_free(lat);
+}
+
+bool wd_release_fix(int device)
+{
+    const WdFixAlone lock(wd_fix_mutex());
+    bool any = false;
+    for (wd_lattice *lat = fix_list, *next; lat; lat = next) {
+        next = lat->fix_next;
+        if (lat->device != device) continue;
+        wd_fix_free(lat);
+        any = true;
+    }
     return any;
+}
+
+size_t wd_fix_bytes(const wd_lattice *lat)
+{
+    const WdFixShared lock(wd_fix_mutex());
+    return lat->gauge_fix ? (size_t)lat->volume * 4 * 9 * sizeof(int4) : 0;
 }
 
 cudaError_t wd_malloc(wd_context *ctx, void **p, size_t bytes)
@@ -121,7 +161,7 @@ cudaError_t wd_malloc(wd_context *ctx, void **p, size_t bytes)
         wd_pool_release(ctx);
         if (!full) e = cudaMalloc(p, bytes);
     }
-    if (e == cudaErrorMemoryAllocation && wd_release_fix(ctx)) {
+    if (e == cudaErrorMemoryAllocation && wd_release_fix(ctx->device)) {
         cudaGetLastError();
         e = cudaMalloc(p, bytes);
     }
@@ -171,7 +211,6 @@ extern "C" void wd_context_destroy(wd_context *ctx)
     if (!ctx) return;
     cudaSetDevice(ctx->device);
     host_cache_drop(ctx);
-    for (wd_lattice *lat : ctx->fix_lats) lat->ctx = nullptr;  // a lattice may be destroyed after its context
     wd_pool_release(ctx);
     for (auto &kv : ctx->pool_used) cudaFree(kv.first);
     ctx->pool_used.clear();
@@ -295,7 +334,8 @@ static void *pinned_view(const void *p)
 // Allocates the lattice's fixed-point links if it has none: a copy that only
 // makes FP64 hops faster, so it is kept where it leaves at least half of the
 // device's memory free or in the context's work-buffer cache (an eighth free),
-// and given back when a later allocation needs its memory (wd_malloc).  Returns the device flag behind the planes, or null.
+// and given back when a later allocation needs its memory (wd_malloc).  The
+// caller holds the lock alone.  Returns the device flag behind the planes, or null.
 static int *want_fix(wd_context *ctx, wd_lattice *lat)
 {
     const size_t n = (size_t)lat->volume * 4 * 9 * sizeof(int4);
@@ -305,12 +345,12 @@ static int *want_fix(wd_context *ctx, wd_lattice *lat)
         for (const auto &kv : ctx->pool_free) cached += kv.first;
         const bool room = n < (64u << 20) || (cudaMemGetInfo(&free_b, &total_b) == cudaSuccess &&
                                               free_b + cached >= n + total_b / 2 && free_b >= n + total_b / 8);
-        if (!room || cudaMalloc(&lat->gauge_fix, n + sizeof(int4)) != cudaSuccess) {
+        void *links = nullptr;
+        if (!room || cudaMalloc(&links, n + sizeof(int4)) != cudaSuccess) {
             cudaGetLastError();
-            lat->gauge_fix = nullptr;
             return nullptr;
         }
-        ctx->fix_lats.insert(lat);
+        wd_fix_enter(lat, links);
     }
     return lat->gauge_fix ? (int *)((char *)lat->gauge_fix + n) : nullptr;
 }
@@ -328,6 +368,7 @@ static wd_status upload_gauge(wd_context *ctx, wd_lattice *lat, const double *co
     }
     wd_status st = stage ? ensure_staging(ctx, bytes) : WD_OK;
     if (st != WD_OK) return st;
+    const WdFixAlone lock(wd_fix_mutex());  // no other context may take the copy while it is written
     int *bad = want_fix(ctx, lat);
     if (bad) WD_CUDA(ctx, cudaMemsetAsync(bad, 0, sizeof(int), ctx->stream));
     for (int mu = 0; mu < 4; ++mu) {
@@ -348,7 +389,7 @@ static wd_status upload_gauge(wd_context *ctx, wd_lattice *lat, const double *co
     *host_bad = 0;
     if (bad) WD_CUDA(ctx, cudaMemcpyAsync(host_bad, bad, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
     WD_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-    if (*host_bad) wd_drop_fix(lat);
+    if (*host_bad) wd_fix_free(lat);
     return WD_OK;
 }
 
@@ -357,7 +398,7 @@ wd_status wd_lattice_make(wd_context *ctx, const int dims[4], const double *cons
     if (!ctx || !out || !gauge) return wd_fail(ctx, WD_ERR_BAD_ARG, "null argument");
     *out = nullptr;
     wd_lattice *lat = new wd_lattice();
-    lat->ctx = ctx;
+    lat->device = ctx->device;
     lat->use_fix = fix;
     wd_status st = make_geom(ctx, dims, &lat->g, &lat->volume);
     if (st != WD_OK) {
@@ -394,7 +435,7 @@ extern "C" void wd_lattice_destroy(wd_lattice *lat)
 {
     if (!lat) return;
     cudaFree(lat->gauge);  // cudaFree waits for work in flight on the device
-    if (lat->gauge_fix) wd_drop_fix(lat);
+    wd_drop_fix(lat);
     wd_lattice_invalidate_derived(lat);
     delete lat;
 }
@@ -583,10 +624,11 @@ extern "C" wd_status wd_dslash_offd(wd_context *ctx, const wd_lattice *lat, cons
     if (cb != 0 && cb != 1) return wd_fail(ctx, WD_ERR_BAD_ARG, "cb must be 0 or 1");
     return with_arith(ctx, lat, in, out, prec, false, [&](const wd_field *i, wd_field *o) -> wd_status {
         // the reference zeroes the whole destination (src/dslash_new.cpp:1398)
-        if (i->storage == WD_PREC_F64 && lat->gauge_fix) {
+        if (i->storage == WD_PREC_F64) {
             const int64_t half = (int64_t)12 * lat->g.Vh;
-            return wd_hop_fix(ctx, lat, i->d + (1 - cb) * half, o->d + cb * half, nullptr, cb, dag, -0.5, 0.0, nullptr,
-                              o->d + (1 - cb) * half);
+            if (const WdTried r = wd_hop_fix(ctx, lat, i->d + (1 - cb) * half, o->d + cb * half, nullptr, cb, dag, -0.5,
+                                             0.0, nullptr, o->d + (1 - cb) * half))
+                return *r;
         }
         wd_status s = wd_v_zero(ctx, wd_block(o, 1 - cb), (int64_t)12 * lat->g.Vh);
         if (s != WD_OK) return s;
@@ -627,7 +669,8 @@ extern "C" wd_status wd_dslash_full(wd_context *ctx, const wd_lattice *lat, cons
     if (st != WD_OK) return st;
     const double a = 4.0 + mass;
     return with_arith(ctx, lat, in, out, prec, false, [&](const wd_field *i, wd_field *o) -> wd_status {
-        if (i->storage == WD_PREC_F64 && lat->gauge_fix) return wd_hop_fix_M(ctx, lat, i->d, o->d, mass, dag);
+        if (i->storage == WD_PREC_F64)
+            if (const WdTried r = wd_hop_fix_M(ctx, lat, i->d, o->d, mass, dag)) return *r;
         for (int cb = 0; cb < 2; ++cb) {
             const WdVec x = wd_block(i, cb);
             wd_status s = wd_hop_v(ctx, lat, wd_block(i, 1 - cb), wd_block(o, cb), &x, cb, dag, -0.5, a);

@@ -30,6 +30,7 @@
 #include <vector>
 #include "wd_async.cuh"
 #include "wd_df.cuh"
+#include "wd_fix_links.h"
 #include "wd_hop.cuh"
 #include "wd_lp.cuh"
 #include "wd_h16m.cuh"
@@ -1095,7 +1096,7 @@ static double server_fix_bytes(const wd_server *sv)
 {
     double b = 0;
     for (const wd_lattice *l : sv->lats)
-        if (l->gauge_fix) b += (double)l->volume * 4 * 9 * sizeof(int4);
+        b += (double)wd_fix_bytes(l);
     return b;
 }
 
@@ -1105,7 +1106,7 @@ static void server_make_room(wd_server *sv, double bytes)
 {
     if (sv->gauge_bytes + sv->req_bytes + server_fix_bytes(sv) + bytes <= sv->cfg.hbm_budget_bytes) return;
     for (wd_lattice *l : sv->lats)
-        if (l->gauge_fix) wd_drop_fix(l);
+        wd_drop_fix(l);
 }
 
 static double request_bytes(const wd_server *sv, const wd_lattice *lat, int nsrc)

@@ -65,8 +65,8 @@ wd_status wd_hop_hi_residual(wd_context *ctx, const wd_lattice *lat, WdVec in, W
                                   (float4 *)s32.p, mass, red, result);
     if (in.prec != WD_PREC_F64) return wd_fail(ctx, WD_ERR_BAD_ARG, "residual hop: FP64 or double-float storage");
     const WdResSink r{(const double2 *)bhat.p, (float4 *)s32.p, red, result};
-    if (lat->gauge_fix)
-        return wd_hop_fix_residual(ctx, lat, (const double2 *)in.p, (const double2 *)x.p, -0.25 / a, a, r);
+    if (const WdTried t = wd_hop_fix_residual(ctx, lat, (const double2 *)in.p, (const double2 *)x.p, -0.25 / a, a, r))
+        return *t;
     auto run = [&](auto tag) -> wd_status {
         using P = HopF64<decltype(tag)::value>;
         P p;
@@ -96,8 +96,8 @@ wd_status wd_hop_f64_aos_range(wd_context *ctx, cudaStream_t stream, const wd_la
                                int s_lo, int s_hi)
 {
     if (s_hi <= s_lo) return WD_OK;
-    if (lat->gauge_fix)
-        return wd_hop_fix_aos_range(ctx, stream, lat, in_aos, out_aos, x_aos, cb, dag, alpha, beta, s_lo, s_hi);
+    if (const WdTried t = wd_hop_fix_aos_range(ctx, stream, lat, in_aos, out_aos, x_aos, cb, dag, alpha, beta, s_lo, s_hi))
+        return *t;
     using P = HopF64AoS<64>;
     P p;
     p.g = lat->g;
@@ -121,7 +121,7 @@ wd_status wd_hop_f64(wd_context *ctx, const wd_lattice *lat, const double2 *in_b
                      double2 *out_block, const double2 *x_block, int cb, int dag, double alpha,
                      double beta, const int *stop)
 {
-    if (lat->gauge_fix) return wd_hop_fix(ctx, lat, in_block, out_block, x_block, cb, dag, alpha, beta, stop);
+    if (const WdTried t = wd_hop_fix(ctx, lat, in_block, out_block, x_block, cb, dag, alpha, beta, stop)) return *t;
     auto run = [&](auto tag) -> wd_status {
         using P = HopF64<decltype(tag)::value>;
         P p;

@@ -1,6 +1,7 @@
 // wd_dslash_fix.cu -- the FP64 hopping term computed in 64-bit fixed point.
 #include <type_traits>
 #include "wd_fix.cuh"
+#include "wd_fix_links.h"
 #include "wd_kernels.h"
 #include "wd_reduce.cuh"
 #include "wd_solver.h"
@@ -340,12 +341,6 @@ FixArgs fix_args(const wd_lattice *lat, const void *in, void *out, const void *x
                    (const int4 *)lat->gauge_fix, alpha, beta, pre, pow2 ? 1.0 : alpha, !pow2, stop, nullptr};
 }
 
-// the links are there (a kernel must not start on a null pointer)
-wd_status need_links(wd_context *ctx, const wd_lattice *lat)
-{
-    return lat->gauge_fix ? WD_OK : wd_fail(ctx, WD_ERR_BAD_ARG, "the lattice has no fixed-point links");
-}
-
 }  // namespace
 
 wd_status wd_gauge_ref_to_soa_fix(wd_context *ctx, const WdGeom &g, int mu, const double2 *ref, double2 *soa, void *fix,
@@ -357,10 +352,11 @@ wd_status wd_gauge_ref_to_soa_fix(wd_context *ctx, const WdGeom &g, int mu, cons
     return WD_OK;
 }
 
-wd_status wd_hop_fix(wd_context *ctx, const wd_lattice *lat, const double2 *in, double2 *out, const double2 *x, int cb,
-                     int dag, double alpha, double beta, const int *stop, double2 *zero)
+WdTried wd_hop_fix(wd_context *ctx, const wd_lattice *lat, const double2 *in, double2 *out, const double2 *x, int cb,
+                   int dag, double alpha, double beta, const int *stop, double2 *zero)
 {
-    if (wd_status st = need_links(ctx, lat)) return st;
+    const WdFixShared lock(wd_fix_mutex());
+    if (!lat->gauge_fix) return {};
     FixArgs a = fix_args(lat, in, out, x, cb, alpha, beta, stop);
     a.zero = zero;
     // one shape (64 and 32 threads a block run within 0.3 % of 128): the
@@ -369,58 +365,65 @@ wd_status wd_hop_fix(wd_context *ctx, const wd_lattice *lat, const double2 *in, 
     return store_fix<false>(ctx, ctx->stream, a, dag, false, 0, lat->g.Vh);
 }
 
-wd_status wd_hop_fix_M(wd_context *ctx, const wd_lattice *lat, const double2 *in, double2 *out, double mass, int dag,
-                       const int *stop)
+WdTried wd_hop_fix_M(wd_context *ctx, const wd_lattice *lat, const double2 *in, double2 *out, double mass, int dag,
+                     const int *stop)
 {
-    if (wd_status st = need_links(ctx, lat)) return st;
+    const WdFixShared lock(wd_fix_mutex());
+    if (!lat->gauge_fix) return {};
     return store_fix<false>(ctx, ctx->stream, fix_args(lat, in, out, in, 0, -0.5, 4.0 + mass, stop), dag, true, 0,
                             lat->g.Vh);
 }
 
-wd_status wd_hop_fix_residual(wd_context *ctx, const wd_lattice *lat, const double2 *in, const double2 *x, double alpha,
-                              double beta, const WdResSink &r)
+WdTried wd_hop_fix_residual(wd_context *ctx, const wd_lattice *lat, const double2 *in, const double2 *x, double alpha,
+                            double beta, const WdResSink &r)
 {
-    if (wd_status st = need_links(ctx, lat)) return st;
+    const WdFixShared lock(wd_fix_mutex());
+    if (!lat->gauge_fix) return {};
     return run_fix<false>(ctx, fix_args(lat, in, nullptr, x, 0, alpha, beta), EpiRes{r.red, r});
 }
 
-wd_status wd_hop_fix_norm(wd_context *ctx, const wd_lattice *lat, WdVec in, WdVec t, WdVec p, double mass, WdCgDev *dev,
-                          WdRed red)
+WdTried wd_hop_fix_norm(wd_context *ctx, const wd_lattice *lat, WdVec in, WdVec t, WdVec p, double mass, WdCgDev *dev,
+                        WdRed red)
 {
-    if (wd_status st = need_links(ctx, lat)) return st;
+    const WdFixShared lock(wd_fix_mutex());
+    if (!lat->gauge_fix) return {};
     const double a = 4.0 + mass;
     return run_fix<false>(ctx, fix_args(lat, in.p, t.p, p.p, 0, -0.25 / a, a, &dev->stop), EpiNorm{dev, red});
 }
 
-wd_status wd_hop_fix_update(wd_context *ctx, const wd_lattice *lat, WdVec in, WdVec t, WdVec p, WdVec r, WdVec x,
-                            double mass, WdCgDev *dev, WdRed red)
+WdTried wd_hop_fix_update(wd_context *ctx, const wd_lattice *lat, WdVec in, WdVec t, WdVec p, WdVec r, WdVec x,
+                          double mass, WdCgDev *dev, WdRed red)
 {
-    if (wd_status st = need_links(ctx, lat)) return st;
+    const WdFixShared lock(wd_fix_mutex());
+    if (!lat->gauge_fix) return {};
     const double a = 4.0 + mass;
     return run_fix<true>(ctx, fix_args(lat, in.p, nullptr, t.p, 0, -0.25 / a, a, &dev->stop),
                          EpiUpdate{dev, red, (const double2 *)p.p, (double2 *)r.p, (double2 *)x.p});
 }
 
-wd_status wd_hop_fix_M_dot(wd_context *ctx, const wd_lattice *lat, WdVec in, WdVec q, WdVec p, double mass, WdCgDev *dev,
-                           WdRed red)
+WdTried wd_hop_fix_M_dot(wd_context *ctx, const wd_lattice *lat, WdVec in, WdVec q, WdVec p, double mass, WdCgDev *dev,
+                         WdRed red)
 {
-    if (wd_status st = need_links(ctx, lat)) return st;
+    const WdFixShared lock(wd_fix_mutex());
+    if (!lat->gauge_fix) return {};
     return run_fix<true>(ctx, fix_args(lat, in.p, q.p, in.p, 0, -0.5, 4.0 + mass, &dev->stop),
                          EpiDot{dev, red, (const double2 *)p.p}, true);
 }
 
-wd_status wd_hop_fix_M_residual(wd_context *ctx, const wd_lattice *lat, const double2 *b, const double2 *x, double mass,
-                                WdRed red, double *result)
+WdTried wd_hop_fix_M_residual(wd_context *ctx, const wd_lattice *lat, const double2 *b, const double2 *x, double mass,
+                              WdRed red, double *result)
 {
-    if (wd_status st = need_links(ctx, lat)) return st;
+    const WdFixShared lock(wd_fix_mutex());
+    if (!lat->gauge_fix) return {};
     return run_fix<false>(ctx, fix_args(lat, x, nullptr, x, 0, -0.5, 4.0 + mass),
                           EpiTrueRes{red, b, result}, true);
 }
 
-wd_status wd_hop_fix_aos_range(wd_context *ctx, cudaStream_t stream, const wd_lattice *lat, const double2 *in_aos,
-                               double2 *out_aos, const double2 *x_aos, int cb, int dag, double alpha, double beta,
-                               int s_lo, int s_hi)
+WdTried wd_hop_fix_aos_range(wd_context *ctx, cudaStream_t stream, const wd_lattice *lat, const double2 *in_aos,
+                             double2 *out_aos, const double2 *x_aos, int cb, int dag, double alpha, double beta,
+                             int s_lo, int s_hi)
 {
-    if (wd_status st = need_links(ctx, lat)) return st;
+    const WdFixShared lock(wd_fix_mutex());
+    if (!lat->gauge_fix) return {};
     return store_fix<true>(ctx, stream, fix_args(lat, in_aos, out_aos, x_aos, cb, alpha, beta), dag, false, s_lo, s_hi);
 }

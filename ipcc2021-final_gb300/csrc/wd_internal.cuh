@@ -13,7 +13,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 #include <map>
-#include <set>
+#include <optional>
 #include <string>
 #include <unordered_map>
 #include "../../include/wilson_gb300.h"
@@ -82,7 +82,6 @@ struct wd_context {
     std::multimap<size_t, void *> pool_free;
     std::unordered_map<void *, size_t> pool_used;
     size_t pool_bytes = 0;
-    std::set<wd_lattice *> fix_lats;  // lattices holding fixed-point links (given back when memory runs out)
     // host-side failure injection for tests: after this many more successful
     // field / work-buffer allocations the next ones fail with WD_ERR_OOM
     // (-1: off)
@@ -99,12 +98,16 @@ inline bool wd_alloc_fails(wd_context *ctx)
     return false;
 }
 
+// The status of a launch on a lattice's fixed-point links, or nothing if it has
+// none now (then nothing was launched)
+using WdTried = std::optional<wd_status>;
+
 // Work-buffer allocation through the context's cache (stream-ordered reuse)
 wd_status wd_dev_alloc(wd_context *ctx, void **p, size_t bytes);
 void wd_dev_free(wd_context *ctx, void *p);
 void wd_pool_release(wd_context *ctx);
-// cudaMalloc that gives back the context's cached work buffers, then its
-// fixed-point links, when memory runs out
+// cudaMalloc that gives back the context's cached work buffers, then the
+// fixed-point links of the device's lattices, when memory runs out
 cudaError_t wd_malloc(wd_context *ctx, void **p, size_t bytes);
 // a library-internal FP64 field, from the work-buffer cache if it is small
 wd_status wd_field_create_work(wd_context *ctx, const wd_lattice *lat, wd_field **out);
@@ -112,14 +115,16 @@ wd_status wd_field_create_work(wd_context *ctx, const wd_lattice *lat, wd_field 
 wd_status wd_lattice_make(wd_context *ctx, const int dims[4], const double *const gauge[4], bool fix, wd_lattice **out);
 
 struct wd_lattice {
-    wd_context *ctx = nullptr;
+    int device = 0;
     WdGeom g;
     int64_t volume = 0;
     double2 *gauge = nullptr;     // FP64 [mu][parity][9][Vh]
     float4 *gauge_df = nullptr;   // double-float copy, same shape (lazily built)
     // fixed-point copy, int4 {re hi, re lo, im hi, im lo}, same shape, written with the FP64 links at
     // upload; null when they do not fit it or memory is short (FP64 hops then run on the FP64 pipe)
+    // (gauge_fix and the list are read and written under the lock of wd_fix_links.h only)
     void *gauge_fix = nullptr;
+    wd_lattice *fix_prev = nullptr, *fix_next = nullptr;  // list of the lattices that hold one
     bool use_fix = true;          // whether FP64 hops are expected on this lattice
     void *gauge_f32 = nullptr;    // FP32 12-real links [mu][parity][3][Vh] float4 (lazily built)
     void *gauge_h12 = nullptr;    // FP16 12-real links: uint4 [8][Vh] then uint2 [8][Vh] (lazily built)

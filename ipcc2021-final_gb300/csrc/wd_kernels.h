@@ -19,10 +19,6 @@ wd_status wd_hop_f64(wd_context *ctx, const wd_lattice *lat, const double2 *in_b
 // the fixed-point planes; *bad (device) is set when they do not fit the latter
 wd_status wd_gauge_ref_to_soa_fix(wd_context *ctx, const WdGeom &g, int mu, const double2 *ref, double2 *soa, void *fix,
                                   int *bad);
-// Frees every lattice's fixed-point links (their FP64 hops then run on the
-// FP64 pipe); true if there were any.  For allocations that fail otherwise.
-bool wd_release_fix(wd_context *ctx);
-void wd_drop_fix(wd_lattice *lat);
 // a residual hop's outputs: s32 = FP32(bhat - hop), |s32|^2
 struct WdResSink {
     const double2 *bhat;
@@ -30,18 +26,17 @@ struct WdResSink {
     WdRed red;
     double *result;
 };
-// (the lattice has gauge_fix; stop as for the other hops; zero: a parity block
-// that the launch also clears)
-wd_status wd_hop_fix(wd_context *ctx, const wd_lattice *lat, const double2 *in, double2 *out, const double2 *x, int cb,
-                     int dag, double alpha, double beta, const int *stop = nullptr, double2 *zero = nullptr);
+// stop as for the other hops; zero: a parity block that the launch also clears
+WdTried wd_hop_fix(wd_context *ctx, const wd_lattice *lat, const double2 *in, double2 *out, const double2 *x, int cb,
+                   int dag, double alpha, double beta, const int *stop = nullptr, double2 *zero = nullptr);
 // M (or M^dag) on whole fields in one launch
-wd_status wd_hop_fix_M(wd_context *ctx, const wd_lattice *lat, const double2 *in, double2 *out, double mass, int dag,
-                       const int *stop = nullptr);
-wd_status wd_hop_fix_residual(wd_context *ctx, const wd_lattice *lat, const double2 *in, const double2 *x, double alpha,
-                              double beta, const WdResSink &r);
-wd_status wd_hop_fix_aos_range(wd_context *ctx, cudaStream_t stream, const wd_lattice *lat, const double2 *in_aos,
-                               double2 *out_aos, const double2 *x_aos, int cb, int dag, double alpha, double beta,
-                               int s_lo, int s_hi);
+WdTried wd_hop_fix_M(wd_context *ctx, const wd_lattice *lat, const double2 *in, double2 *out, double mass, int dag,
+                     const int *stop = nullptr);
+WdTried wd_hop_fix_residual(wd_context *ctx, const wd_lattice *lat, const double2 *in, const double2 *x, double alpha,
+                            double beta, const WdResSink &r);
+WdTried wd_hop_fix_aos_range(wd_context *ctx, cudaStream_t stream, const wd_lattice *lat, const double2 *in_aos,
+                             double2 *out_aos, const double2 *x_aos, int cb, int dag, double alpha, double beta,
+                             int s_lo, int s_hi);
 
 // ---- layout conversion (reference AoS <-> device SoA), on device buffers
 // spinor: ref[(p*Vh + s)*12 + c]  <->  soa[(p*12 + c)*Vh + s] in the vector's storage format

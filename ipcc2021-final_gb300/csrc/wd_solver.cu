@@ -13,6 +13,7 @@
 // pipe).  Mixed precision (FP32 / FP16 inner) lives in wd_mixed.cu.
 #include <chrono>
 #include <cmath>
+#include "wd_fix_links.h"
 #include "wd_kernels.h"
 #include "wd_solver.h"
 
@@ -44,8 +45,8 @@ static inline WdVec par_half(WdVec v, int par, int Vh) { return wd_offset(v, (in
 wd_status wd_apply_M_v(wd_context *ctx, const wd_lattice *lat, WdVec in, WdVec out, double mass, int dag,
                        const int *stop)
 {
-    if (in.prec == WD_PREC_F64 && lat->gauge_fix)
-        return wd_hop_fix_M(ctx, lat, (const double2 *)in.p, (double2 *)out.p, mass, dag, stop);
+    if (in.prec == WD_PREC_F64)
+        if (const WdTried r = wd_hop_fix_M(ctx, lat, (const double2 *)in.p, (double2 *)out.p, mass, dag, stop)) return *r;
     const int Vh = lat->g.Vh;
     for (int cb = 0; cb < 2; ++cb) {
         const WdVec x = par_half(in, cb, Vh);
@@ -77,15 +78,16 @@ wd_status wd_true_residual(wd_context *ctx, const wd_lattice *lat, const double2
     wd_status st;
     const int64_t rb = wd_red_blocks(lat->g.Vh);
     WdVecBuf buf;
-    // an allocation may give the fixed-point links back: looked for after it
-    if (lat->gauge_fix &&
-        (st = wd_vec_alloc(ctx, buf, WD_PREC_F64, (int64_t)wd_red_doubles(rb, 2) / 2 + 1)) != WD_OK)
-        return st;
-    if (lat->gauge_fix) {
+    WdTried one;
+    if (wd_fix_bytes(lat)) {  // (the allocation may give the links back)
+        if ((st = wd_vec_alloc(ctx, buf, WD_PREC_F64, (int64_t)wd_red_doubles(rb, 2) / 2 + 1)) != WD_OK) return st;
         const WdRed red = wd_red_view(buf.v.p, rb);
         double2 *res = (double2 *)ctx->red_partial + WD_RED_BLOCKS;
         WD_CUDA(ctx, cudaMemsetAsync(red.counters, 0, wd_red_counters(rb) * sizeof(unsigned), ctx->stream));
-        if ((st = wd_hop_fix_M_residual(ctx, lat, b, x, mass, red, &res[0].x)) != WD_OK) return st;
+        one = wd_hop_fix_M_residual(ctx, lat, b, x, mass, red, &res[0].x);
+    }
+    if (one) {
+        if (*one != WD_OK) return *one;
         if ((st = wd_red_fetch(ctx, 1, r)) != WD_OK) return st;
         r[1].x = r[0].y;
     } else {
@@ -178,8 +180,7 @@ static wd_status cgnr_ref_core(wd_context *ctx, const wd_lattice *lat, WdVec src
 {
     const int64_t n = lat->volume * 12;
     const double m = prm->mass;
-    // looked for at each launch: any allocation may give the fixed-point links back
-    const auto fused = [&] { return src.prec == WD_PREC_F64 && lat->gauge_fix; };
+    const bool f64 = src.prec == WD_PREC_F64;
     WdVecBuf b[5];
     for (auto &v : b) {
         wd_status s = wd_vec_alloc(ctx, v, src.prec, n);
@@ -205,8 +206,10 @@ static wd_status cgnr_ref_core(wd_context *ctx, const wd_lattice *lat, WdVec src
     auto iteration = [&]() -> wd_status {
         wd_status e;
         if ((e = wd_apply_M_v(ctx, lat, p, qq, m, 0, &dev->stop)) != WD_OK) return e;
-        if (fused()) {
-            if ((e = wd_hop_fix_M_dot(ctx, lat, qq, q, p, m, dev, loop.red)) != WD_OK) return e;
+        WdTried fused;
+        if (f64) fused = wd_hop_fix_M_dot(ctx, lat, qq, q, p, m, dev, loop.red);
+        if (fused) {
+            if (*fused != WD_OK) return *fused;
         } else {
             if ((e = wd_apply_M_v(ctx, lat, qq, q, m, 1, &dev->stop)) != WD_OK) return e;
             if ((e = wd_cgd_dot(ctx, p, q, n, dev, loop.red)) != WD_OK) return e;
@@ -231,7 +234,7 @@ static wd_status cg_eo_core(wd_context *ctx, const wd_lattice *lat, WdVec src, W
     const int Vh = lat->g.Vh;
     const int64_t nh = (int64_t)12 * Vh;
     const double m = prm->mass, a = 4.0 + m;
-    const auto fused = [&] { return src.prec == WD_PREC_F64 && lat->gauge_fix; };  // as in cgnr_ref_core
+    const bool f64 = src.prec == WD_PREC_F64;
     WdVecBuf b[7];
     for (auto &v : b) {
         wd_status s = wd_vec_alloc(ctx, v, src.prec, nh);
@@ -276,15 +279,19 @@ static wd_status cg_eo_core(wd_context *ctx, const wd_lattice *lat, WdVec src, W
     auto iteration = [&]() -> wd_status {
         wd_status e;
         if ((e = wd_hop_v(ctx, lat, p, tmp_o, nullptr, 1, 0, 1.0, 0.0, &dev->stop)) != WD_OK) return e;
-        if (fused()) {
-            if ((e = wd_hop_fix_norm(ctx, lat, tmp_o, t, p, m, dev, loop.red)) != WD_OK) return e;
+        WdTried fused;
+        if (f64) fused = wd_hop_fix_norm(ctx, lat, tmp_o, t, p, m, dev, loop.red);
+        if (fused) {
+            if (*fused != WD_OK) return *fused;
         } else {
             if ((e = wd_hop_v(ctx, lat, tmp_o, t, &p, 0, 0, -0.25 / a, a, &dev->stop)) != WD_OK) return e;
             if ((e = wd_cgd_norm(ctx, t, nh, dev, loop.red)) != WD_OK) return e;
         }
         if ((e = wd_hop_v(ctx, lat, t, tmp_o, nullptr, 1, 1, 1.0, 0.0, &dev->stop)) != WD_OK) return e;
-        if (fused()) {
-            if ((e = wd_hop_fix_update(ctx, lat, tmp_o, t, p, r, x_e, m, dev, loop.red)) != WD_OK) return e;
+        fused.reset();
+        if (f64) fused = wd_hop_fix_update(ctx, lat, tmp_o, t, p, r, x_e, m, dev, loop.red);
+        if (fused) {
+            if (*fused != WD_OK) return *fused;
         } else {
             if ((e = wd_hop_v(ctx, lat, tmp_o, q, &t, 0, 1, -0.25 / a, a, &dev->stop)) != WD_OK) return e;
             if ((e = wd_cgd_update(ctx, false, p, q, x_e, r, nh, dev, loop.red)) != WD_OK) return e;

@@ -129,17 +129,16 @@ wd_status wd_cgd_update(wd_context *ctx, bool cplx, WdVec p, WdVec q, WdVec x, W
 // p = r + beta p
 wd_status wd_cgd_xpby(wd_context *ctx, WdVec r, WdVec p, int64_t n, const WdCgDev *dev);
 
-// The same fused into the fixed-point FP64 hops (wd_dslash_fix.cu; the
-// lattice has gauge_fix).
+// The same fused into the fixed-point FP64 hops (wd_dslash_fix.cu).
 //   t = -D_eo in / (4a) + a p on even blocks (a = 4 + mass), |t|^2 -> alpha
-wd_status wd_hop_fix_norm(wd_context *ctx, const wd_lattice *lat, WdVec in, WdVec t, WdVec p, double mass, WdCgDev *dev,
-                          WdRed red);
+WdTried wd_hop_fix_norm(wd_context *ctx, const wd_lattice *lat, WdVec in, WdVec t, WdVec p, double mass, WdCgDev *dev,
+                        WdRed red);
 //   q = -D_eo^dag in / (4a) + a t, not stored: r -= alpha q, x += alpha p, |r|^2 -> beta or the gate
-wd_status wd_hop_fix_update(wd_context *ctx, const wd_lattice *lat, WdVec in, WdVec t, WdVec p, WdVec r, WdVec x,
-                            double mass, WdCgDev *dev, WdRed red);
+WdTried wd_hop_fix_update(wd_context *ctx, const wd_lattice *lat, WdVec in, WdVec t, WdVec p, WdVec r, WdVec x,
+                          double mass, WdCgDev *dev, WdRed red);
 //   |b - M x|^2 and |b|^2 -> result[0], result[1] (device)
-wd_status wd_hop_fix_M_residual(wd_context *ctx, const wd_lattice *lat, const double2 *b, const double2 *x, double mass,
-                                WdRed red, double *result);
+WdTried wd_hop_fix_M_residual(wd_context *ctx, const wd_lattice *lat, const double2 *b, const double2 *x, double mass,
+                              WdRed red, double *result);
 //   q = M^dag in on the whole lattice, (p, q) -> alpha
-wd_status wd_hop_fix_M_dot(wd_context *ctx, const wd_lattice *lat, WdVec in, WdVec q, WdVec p, double mass, WdCgDev *dev,
-                           WdRed red);
+WdTried wd_hop_fix_M_dot(wd_context *ctx, const wd_lattice *lat, WdVec in, WdVec q, WdVec p, double mass, WdCgDev *dev,
+                         WdRed red);
