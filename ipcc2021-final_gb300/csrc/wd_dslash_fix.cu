@@ -341,6 +341,16 @@ FixArgs fix_args(const wd_lattice *lat, const void *in, void *out, const void *x
                    (const int4 *)lat->gauge_fix, alpha, beta, pre, pow2 ? 1.0 : alpha, !pow2, stop, nullptr};
 }
 
+// Whether a launch on `stream` may use the lattice's fixed-point links (under
+// the lock).  A stream that is being captured may not: the graph would keep
+// their address past the moment they are freed or replaced, while the FP64
+// links stay where they are as long as the lattice.
+bool links_for(const wd_lattice *lat, cudaStream_t stream)
+{
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    return lat->gauge_fix && cudaStreamIsCapturing(stream, &cs) == cudaSuccess && cs == cudaStreamCaptureStatusNone;
+}
+
 }  // namespace
 
 wd_status wd_gauge_ref_to_soa_fix(wd_context *ctx, const WdGeom &g, int mu, const double2 *ref, double2 *soa, void *fix,
@@ -356,7 +366,7 @@ WdTried wd_hop_fix(wd_context *ctx, const wd_lattice *lat, const double2 *in, do
                    int dag, double alpha, double beta, const int *stop, double2 *zero)
 {
     const WdFixShared lock(wd_fix_mutex());
-    if (!lat->gauge_fix) return {};
+    if (!links_for(lat, ctx->stream)) return {};
     FixArgs a = fix_args(lat, in, out, x, cb, alpha, beta, stop);
     a.zero = zero;
     // one shape (64 and 32 threads a block run within 0.3 % of 128): the
@@ -369,7 +379,7 @@ WdTried wd_hop_fix_M(wd_context *ctx, const wd_lattice *lat, const double2 *in, 
                      const int *stop)
 {
     const WdFixShared lock(wd_fix_mutex());
-    if (!lat->gauge_fix) return {};
+    if (!links_for(lat, ctx->stream)) return {};
     return store_fix<false>(ctx, ctx->stream, fix_args(lat, in, out, in, 0, -0.5, 4.0 + mass, stop), dag, true, 0,
                             lat->g.Vh);
 }
@@ -378,7 +388,7 @@ WdTried wd_hop_fix_residual(wd_context *ctx, const wd_lattice *lat, const double
                             double beta, const WdResSink &r)
 {
     const WdFixShared lock(wd_fix_mutex());
-    if (!lat->gauge_fix) return {};
+    if (!links_for(lat, ctx->stream)) return {};
     return run_fix<false>(ctx, fix_args(lat, in, nullptr, x, 0, alpha, beta), EpiRes{r.red, r});
 }
 
@@ -386,7 +396,7 @@ WdTried wd_hop_fix_norm(wd_context *ctx, const wd_lattice *lat, WdVec in, WdVec 
                         WdRed red)
 {
     const WdFixShared lock(wd_fix_mutex());
-    if (!lat->gauge_fix) return {};
+    if (!links_for(lat, ctx->stream)) return {};
     const double a = 4.0 + mass;
     return run_fix<false>(ctx, fix_args(lat, in.p, t.p, p.p, 0, -0.25 / a, a, &dev->stop), EpiNorm{dev, red});
 }
@@ -395,7 +405,7 @@ WdTried wd_hop_fix_update(wd_context *ctx, const wd_lattice *lat, WdVec in, WdVe
                           double mass, WdCgDev *dev, WdRed red)
 {
     const WdFixShared lock(wd_fix_mutex());
-    if (!lat->gauge_fix) return {};
+    if (!links_for(lat, ctx->stream)) return {};
     const double a = 4.0 + mass;
     return run_fix<true>(ctx, fix_args(lat, in.p, nullptr, t.p, 0, -0.25 / a, a, &dev->stop),
                          EpiUpdate{dev, red, (const double2 *)p.p, (double2 *)r.p, (double2 *)x.p});
@@ -405,7 +415,7 @@ WdTried wd_hop_fix_M_dot(wd_context *ctx, const wd_lattice *lat, WdVec in, WdVec
                          WdRed red)
 {
     const WdFixShared lock(wd_fix_mutex());
-    if (!lat->gauge_fix) return {};
+    if (!links_for(lat, ctx->stream)) return {};
     return run_fix<true>(ctx, fix_args(lat, in.p, q.p, in.p, 0, -0.5, 4.0 + mass, &dev->stop),
                          EpiDot{dev, red, (const double2 *)p.p}, true);
 }
@@ -414,7 +424,7 @@ WdTried wd_hop_fix_M_residual(wd_context *ctx, const wd_lattice *lat, const doub
                               WdRed red, double *result)
 {
     const WdFixShared lock(wd_fix_mutex());
-    if (!lat->gauge_fix) return {};
+    if (!links_for(lat, ctx->stream)) return {};
     return run_fix<false>(ctx, fix_args(lat, x, nullptr, x, 0, -0.5, 4.0 + mass),
                           EpiTrueRes{red, b, result}, true);
 }
@@ -424,6 +434,6 @@ WdTried wd_hop_fix_aos_range(wd_context *ctx, cudaStream_t stream, const wd_latt
                              int s_lo, int s_hi)
 {
     const WdFixShared lock(wd_fix_mutex());
-    if (!lat->gauge_fix) return {};
+    if (!links_for(lat, stream)) return {};
     return store_fix<true>(ctx, stream, fix_args(lat, in_aos, out_aos, x_aos, cb, alpha, beta), dag, false, s_lo, s_hi);
 }
