@@ -73,16 +73,114 @@ struct FixView {
     double2 *out;
 };
 
-// The FP64-pipe arithmetic for a site whose values do not fit a block scale
-template <bool DAG, bool AOS>
-__device__ __noinline__ void f64_route(const FixArgs &a, const FixView &w, int s, double2 *acc)
+// |v| 2^(1023 - E) as FP32, never rounded to zero
+__device__ __forceinline__ float size_of(double v, double scale)
 {
+    return v == 0.0 ? 0.f : fmaxf(fabsf((float)(v * scale)), 0x1p-50f);
+}
+
+// A closer look at a thread's components of a site in doubt: the sums S of
+// the sizes of the products that make up each real, from the FP64 operands.
+// Returns the reals whose S is zero as a bit mask (2k + {0: re, 1: im} for
+// component k of wd_fix::site's v): the fixed-point sum may be off zero by a unit.
+// Returns -1 if another S is below the share of the block scale that the
+// fixed-point sum is used for: the FP64 route.
+template <bool DAG, bool AOS>
+__device__ __forceinline__ int small_sums(const FixArgs &a, const double2 *in, int cb, int s, int half, uint32_t E)
+{
+    const wd_fix::Operands<AOS> p{a.g, cb, in, nullptr};
+    const WdSite c = wd_site(a.g, s, cb);
+    const double scale = __hiloint2double((int)(2046 - E) << 20, 0);
+    const float least = 2.f / (1 << wd_fix::kLeastExp);  // (the block scale is 2 here)
+    float sum[12] = {};  // own spin re, im per colour; spin 3 - half likewise
+#pragma unroll 1
+    for (int d = 0; d < 8; ++d) {
+        const int mu = d >> 1;
+        const bool fwd = !(d & 1), turn = mu == 0 || mu == 2;
+        const int nb = wd_neighbour(a.g, s, c, mu, fwd);
+        const double sg = (fwd ? -1.0 : 1.0) * (DAG ? -1.0 : 1.0);
+        float ur[9], ui[9];
+        const double2 *u = a.gauge + (size_t)((mu * 2 + (fwd ? cb : 1 - cb)) * 9) * a.g.Vh + (fwd ? s : nb);
+#pragma unroll
+        for (int k = 0; k < 9; ++k) {
+            const double2 e = u[(size_t)k * a.g.Vh];
+            ur[k] = size_of(e.x, 1.0);
+            ui[k] = size_of(e.y, 1.0);
+        }
+        // the lower spin's terms come from the same half for mu = 0, 1, from the other for mu = 2, 3
+#pragma unroll 1
+        for (int which = 0; which < (mu < 2 ? 1 : 2); ++which) {
+            const int h = half ^ which;
+            const double sigma = h ? -1.0 : 1.0, f = mu == 1 ? -sg * sigma : mu == 2 ? sg * sigma : sg;
+            const double2 *so = p.spin(nb, h), *sp = p.spin(nb, mu < 2 ? 3 - h : 2 + h);
+            float hr[3], hi[3];
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                const double2 x = so[k * p.colour_stride()], y = sp[k * p.colour_stride()];
+                hr[k] = size_of(turn ? fma(-f, y.y, x.x) : fma(f, y.x, x.x), scale);
+                hi[k] = size_of(turn ? fma(f, y.x, x.y) : fma(f, y.y, x.y), scale);
+            }
+#pragma unroll
+            for (int r = 0; r < 3; ++r) {
+                float re = 0.f, im = 0.f;
+#pragma unroll
+                for (int b = 0; b < 3; ++b) {
+                    const float ar = fwd ? ur[r * 3 + b] : ur[b * 3 + r], ai = fwd ? ui[r * 3 + b] : ui[b * 3 + r];
+                    re += ar * hr[b] + ai * hi[b];
+                    im += ar * hi[b] + ai * hr[b];
+                }
+                if (which == 0) {
+                    sum[2 * r] += re;
+                    sum[2 * r + 1] += im;
+                }
+                if (mu < 2 || which == 1) {
+                    sum[6 + 2 * r] += turn ? im : re;
+                    sum[7 + 2 * r] += turn ? re : im;
+                }
+            }
+        }
+        float m = sum[0];
+#pragma unroll
+        for (int k = 1; k < 12; ++k) m = fminf(m, sum[k]);
+        if (m >= least) return 0;
+    }
+    int zero = 0;
+#pragma unroll
+    for (int k = 0; k < 12; ++k) {
+        if (sum[k] == 0.f) zero |= 1 << k;
+        else if (sum[k] < least) return -1;
+    }
+    return zero;
+}
+
+// Sets right, where they need it, a thread's components t of a site that is in
+// doubt or out of range.  Out of line and on memory, so that the common path
+// keeps its registers (with the values alive across the call a hop took 11 %
+// longer).  A site in doubt of a dense field takes some 4 us.
+template <bool DAG, bool AOS>
+__device__ __noinline__ void rare_site(const FixArgs &a, const double2 *in, int cb, int s, int half, uint32_t E,
+                                       wd_fix::Judged state, double2 *t)
+{
+    if (state == wd_fix::kDoubt) {
+        const int zero = small_sums<DAG, AOS>(a, in, cb, s, half, E);
+        if (zero >= 0) {
+            for (int k = 0; k < 6; ++k) {
+                if (zero >> 2 * k & 1) t[k].x = 0.0;
+                if (zero >> 2 * k & 2) t[k].y = 0.0;
+            }
+            return;
+        }
+    }
     std::conditional_t<AOS, HopF64AoS<128>, HopF64<128>> p;
     p.g = a.g;
-    p.cb = w.cb;
-    p.in = w.in;
+    p.cb = cb;
+    p.in = in;
     p.gauge = a.gauge;
+    double2 acc[12];
     wd_hop_site<DAG>(p, s, acc);
+    const double pre = a.scaled ? 1.0 : a.alpha;
+#pragma unroll
+    for (int k = 0; k < 6; ++k) t[k] = c_scale(k < 3 ? acc[half * 3 + k] : acc[(3 - half) * 3 + k - 3], pre);
 }
 
 template <bool AOS>
@@ -256,22 +354,21 @@ __global__ void __launch_bounds__(block_threads(T), 512 / block_threads(T))
     const int s0 = s_lo + (T ? (int)(blockIdx.x * B + threadIdx.x) >> 1 : (int)blockIdx.x * 16 + (l >> 1));
     const int s = s0 < s_hi ? s0 : s_hi - 1;
     double2 v[6];
-    bool ok;
-    if constexpr (T > 0) ok = wd_fix::site<DAG>(p, *reinterpret_cast<wd_fix::Stage<B> *>(smem), s, half, a.pre, v);
-    else ok = wd_fix::site_split<DAG>(p, *reinterpret_cast<wd_fix::Split *>(smem), s, half, a.pre, v);
+    uint32_t E;
+    wd_fix::Judged state;
+    if constexpr (T > 0) state = wd_fix::site<DAG>(p, *reinterpret_cast<wd_fix::Stage<B> *>(smem), s, half, a.pre, v, E);
+    else state = wd_fix::site_split<DAG>(p, *reinterpret_cast<wd_fix::Split *>(smem), s, half, a.pre, v, E);
     typename Epi::Num n[Epi::N ? Epi::N : 1] = {};
     const int warp = threadIdx.x >> 5;  // split form: warps 0-2 hold colour `warp` of the two spins
-    if (s0 < s_hi && (T > 0 || warp < 3)) {
-        if (!ok) {
-            double2 acc[12];
-            f64_route<DAG, AOS>(a, w, s, acc);
-            const double pre = a.scaled ? 1.0 : a.alpha;
+    if (state != wd_fix::kGood && (T > 0 || warp < 3)) {
+        double2 t[6];
 #pragma unroll
-            for (int k = 0; k < (T ? 6 : 2); ++k) {
-                const int spin = k < (T ? 3 : 1) ? half : 3 - half;
-                v[k] = c_scale(acc[spin * 3 + (T ? k % 3 : warp)], pre);
-            }
-        }
+        for (int k = 0; k < (T ? 6 : 2); ++k) t[T ? k : 3 * k + warp] = v[k];
+        rare_site<DAG, AOS>(a, w.in, w.cb, s, half, E, state, t);
+#pragma unroll
+        for (int k = 0; k < (T ? 6 : 2); ++k) v[k] = t[T ? k : 3 * k + warp];
+    }
+    if (s0 < s_hi && (T > 0 || warp < 3)) {
 #pragma unroll
         for (int k = 0; k < (T ? 6 : 2); ++k) {
             const int spin = k < (T ? 3 : 1) ? half : 3 - half;

@@ -19,9 +19,13 @@
 // the FP64 form rounds each of its ~25 operations per component at
 // 2^-53 of the running sum.  Measured relative L2 error of one hop, Gaussian
 // fields: 1.4e-16 here, 2.0e-16 in FP64 (both against torch's own FP64 sums).
-// Values whose exponents do not fit (block exponents beyond 2^877, nonzero
-// values below 2^-895, NaN, infinity) are recomputed on the FP64 pipe by the
-// calling kernel, per site.
+// The unit is one for all colours, spins and neighbours of a site.  So that no
+// component loses digits beside larger ones, the sums stand only where every
+// component's own terms are large enough for it (kLeastExp below); other
+// sites, and those whose exponents do not fit (block exponents beyond 2^877,
+// nonzero values below 2^-894, NaN, infinity), are recomputed on the FP64 pipe
+// by the calling kernel.  The look at the terms is 48 of a thread's 3000
+// instructions (0.354 -> 0.371 ms at 32^3x64, 0.118 -> 0.120 at 24^3x48).
 //
 // Two threads share a site: each carries one of the two half-spinor
 // components through the eight link products and accumulates its own upper
@@ -32,12 +36,11 @@
 // are multiplied (0.472 -> 0.386 ms at 32^3x64); a row's links are read
 // from there when the row is due (0.377).  Complex products take three real
 // ones (Gauss): additions are cheaper than wide multiply-adds here.
-// Measured at 32^3x64: 0.354 ms (FP64 form 1.453 ms), 4.55 TB/s of
-// compulsory bytes, 68 % of measured HBM; 0.372 ms before the power-of-two
-// factor moved into the final conversion and the site coordinates lost their
-// divisions.  What bounds it now is issue and the integer pipes together
-// (fma-heavy 57 %, FP64 56 %, issue slots 46 % busy at 24^3x48); with every
-// load served by L1 it is no faster.  Dropped: converting with F2I.S64.F64
+// Measured at 32^3x64: 0.371 ms (FP64 form 1.453 ms), 4.34 TB/s of
+// compulsory bytes, 65 % of measured HBM.  What bounds it now is issue and
+// the integer pipes together (fma-heavy 60 %, FP64 56 %, ALU 34 %, issue slots
+// 44 % busy with 16 warps an SM at 32^4); with every load served by L1 it is
+// no faster.  Dropped: converting with F2I.S64.F64
 // (0.67 ms: it occupies the FP64 pipe), projecting after conversion on
 // integers (0.458 ms before staging), 20 warps per SM at 96 registers (0.395
 // ms against 0.372), the next direction's projection ahead of the current
@@ -52,9 +55,26 @@
 namespace wd_fix {
 
 constexpr int kUnit = 1080;        // x = T 2^(E - kUnit)
-constexpr int kExpTiny = 128;      // nonzero values with exponents below this need the FP64 route ...
+constexpr int kExpTiny = 128;      // nonzero values with exponents up to this need the FP64 route ...
 constexpr int kExpLow = 200;       // ... when the block exponent is below this
 constexpr int kExpHigh = 1900;     // block exponents above this (and NaN, infinity) take the FP64 route
+
+// What is known of a thread's components at a site
+enum Judged {
+    kGood,   // as good as FP64 arithmetic gives them
+    kDoubt,  // one may be too small beside the block scale
+    kFp64    // values that the block scale does not hold
+};
+// A component may be small because its terms cancel, or because they are all
+// small beside the block's largest value (one colour, spin or link entry beside
+// another); then the fixed unit, 2^-58 of the block scale, may be large beside it.
+// Let S be the sum of |U| |h| over the products behind a real of the result.
+// A row of a link's |re| and |im| adds up to at least 0.99 (checked when the
+// fixed-point links are made), so one direction whose half-spinor has its six
+// reals at 2^-7 of the block scale or more gives all reals that it enters S
+// >= 0.99 x 2^-7 of the scale: the unit is below 2^-50.9 S.  In a dense field the
+// eight directions miss that for two half-sites in ten million.
+constexpr int kLeastExp = 7;
 
 __device__ __forceinline__ float absmax3(float a, float b, float c)
 {
@@ -64,10 +84,11 @@ __device__ __forceinline__ float absmax3(float a, float b, float c)
 }
 
 // The FP64 number with words (hi, lo) as limbs l1 2^30 + l0 of trunc(x
-// 2^(1080-E)) (off by less than one unit below zero); ekey = E<<21 | 0x1fffff
-__device__ __forceinline__ void limbs(uint32_t hi, uint32_t lo, uint32_t ekey, int &l1, int &l0)
+// 2^(1080-E)) (off by less than one unit below zero); ekey = E<<21 | 0x1fffff.
+// sh: E less its exponent
+__device__ __forceinline__ void limbs(uint32_t hi, uint32_t lo, uint32_t ekey, int &l1, int &l0, uint32_t &sh)
 {
-    const uint32_t sh = (ekey - (hi << 1)) >> 21;  // E - exponent (the sign bit shifts out)
+    sh = (ekey - (hi << 1)) >> 21;  // E - exponent (the sign bit shifts out)
     const uint32_t h7 = (__funnelshift_l(lo, hi, 7) & 0x07ffffffu) | 0x08000000u;
     unsigned long long w = ((unsigned long long)h7 << 32) | (lo << 7);
     asm("shr.u64 %0, %0, %1;" : "+l"(w) : "r"(sh));
@@ -126,6 +147,9 @@ struct Acc {
     long long o[6], P[6], Q[6];
     uint32_t E;
     uint32_t tiny;  // OR of nonzero bits of values too small for the block scale
+    // of the half-spinors reached through mu = 0, 1 and through mu = 2, 3: the largest of the
+    // exponents of their smallest reals; at least 1 if one of them is not zero
+    uint32_t least[2];
 };
 
 // Two slots of one direction's operands for a block of T threads (T / 2 sites)
@@ -189,10 +213,11 @@ __device__ __forceinline__ void dir(const Stage<T> &sm, int slot, int half, doub
         else h[k] = make_double2(fma(cb_, sp[k].x, so[k].x), fma(cb_, sp[k].y, so[k].y));
         m = absmax3(m, __int_as_float(__double2hiint(h[k].x)), __int_as_float(__double2hiint(h[k].y)));
     }
+    const uint32_t some = min(__float_as_uint(m), 1u);
     m = absmax3(m, __shfl_xor_sync(0xffffffffu, m, 1), m);
     const uint32_t mb = __float_as_uint(m) & 0x7fffffffu;
     const uint32_t e = mb >> 20;
-    if (mb < ((uint32_t)kExpTiny << 20)) {
+    if (mb < ((uint32_t)(kExpTiny + 1) << 20)) {
 #pragma unroll
         for (int k = 0; k < 3; ++k)
             A.tiny |= (uint32_t)(__double2hiint(h[k].x) << 1) | (uint32_t)__double2loint(h[k].x) |
@@ -212,16 +237,20 @@ __device__ __forceinline__ void dir(const Stage<T> &sm, int slot, int half, doub
     }
     const uint32_t ekey = (A.E << 21) | 0x1fffffu;
     int x1[3], x0[3], q1[3], q0[3], v1[3], v0[3];
+    uint32_t sh = 0;
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
         int y1, y0;
-        limbs(__double2hiint(h[k].x), __double2loint(h[k].x), ekey, x1[k], x0[k]);
-        limbs(__double2hiint(h[k].y), __double2loint(h[k].y), ekey, y1, y0);
+        uint32_t sx, sy;
+        limbs(__double2hiint(h[k].x), __double2loint(h[k].x), ekey, x1[k], x0[k], sx);
+        limbs(__double2hiint(h[k].y), __double2loint(h[k].y), ekey, y1, y0, sy);
+        sh = k ? __vimax3_u32(sh, sx, sy) : max(sx, sy);
         q1[k] = FWD ? -(x1[k] + y1) : x1[k] + y1;
         q0[k] = FWD ? -(x0[k] + y0) : x0[k] + y0;
         v1[k] = y1 - x1[k];
         v0[k] = y0 - x0[k];
     }
+    A.least[MU / 2] = __vimax3_u32(A.least[MU / 2], A.E - sh, some);
     const long long hm64 = -(long long)half;  // sigma: all ones on the second half-spinor
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
@@ -287,8 +316,17 @@ __device__ __forceinline__ bool in_range(uint32_t E, uint32_t tiny)
     return E <= (uint32_t)kExpHigh && !(tiny && E < (uint32_t)kExpLow);
 }
 
+__device__ __forceinline__ Judged judged(uint32_t E, uint32_t tiny, bool good)
+{
+    return !in_range(E, tiny) ? kFp64 : good ? kGood : kDoubt;
+}
+// least reaches 2^-kLeastExp of the block scale 2^(E + 1), or nothing is there
+__device__ __forceinline__ bool good(uint32_t least, uint32_t E) { return least > E - kLeastExp || !least; }
+
 __device__ __forceinline__ void clear(Acc &A)
 {
+    A.least[0] = A.least[1] = 0;
+
 #pragma unroll
     for (int k = 0; k < 6; ++k) A.o[k] = A.P[k] = A.Q[k] = 0;
     A.tiny = 0;
@@ -296,10 +334,10 @@ __device__ __forceinline__ void clear(Acc &A)
 }
 
 // f times the hopping term at site s for the thread pair (half = 0, 1):
-// v[0..2] is spin `half`, v[3..5] spin 3 - half.  Returns false when the site's values
-// need the FP64 route (then v is not to be used).
+// v[0..2] is spin `half`, v[3..5] spin 3 - half, E the block exponent.
 template <bool DAG, int T, bool AOS>
-__device__ __forceinline__ bool site(const Operands<AOS> &p, Stage<T> &sm, int s, int half, Pow2 f, double2 *v)
+__device__ __forceinline__ Judged site(const Operands<AOS> &p, Stage<T> &sm, int s, int half, Pow2 f, double2 *v,
+                                       uint32_t &E)
 {
     const WdSite c = wd_site(p.g, s, p.cb);
     const double sigma = half ? -1.0 : 1.0;
@@ -328,6 +366,7 @@ __device__ __forceinline__ bool site(const Operands<AOS> &p, Stage<T> &sm, int s
     both(std::integral_constant<int, 3>());
     const uint32_t tiny = A.tiny | __shfl_xor_sync(0xffffffffu, A.tiny, 1);
     const int kexp = ((int)A.E - kUnit + f.shift) << 20;
+    E = A.E;
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
         const long long lr = A.P[2 * k] + __shfl_xor_sync(0xffffffffu, A.Q[2 * k], 1);
@@ -335,7 +374,17 @@ __device__ __forceinline__ bool site(const Operands<AOS> &p, Stage<T> &sm, int s
         v[k] = make_double2(value(A.o[2 * k], kexp, f.sign), value(A.o[2 * k + 1], kexp, f.sign));
         v[3 + k] = make_double2(value(lr, kexp, f.sign), value(li, kexp, f.sign));
     }
-    return in_range(A.E, tiny);
+    // (the lower spin's terms of mu = 2, 3 come from the partner's half)
+    const uint32_t own = max(A.least[0], A.least[1]), low = max(A.least[0], __shfl_xor_sync(0xffffffffu, A.least[1], 1));
+    // sums without terms are exactly zero, but for the missing units of negative zeros
+    if (__any_sync(0xffffffffu, !own || !low)) {
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            if (!own) v[k] = make_double2(0.0, 0.0);
+            if (!low) v[3 + k] = make_double2(0.0, 0.0);
+        }
+    }
+    return judged(E, tiny, good(own, E) && good(low, E));
 }
 
 // The same with a direction pair per warp, for lattices too small to fill the
@@ -344,7 +393,7 @@ __device__ __forceinline__ bool site(const Operands<AOS> &p, Stage<T> &sm, int s
 // colour 0-2 of the two spins: v[0] of spin `half`, v[1] of spin 3 - half.
 struct Split {
     Stage<128> st;
-    uint32_t E[4][32], tiny[4][32];
+    uint32_t E[4][32], tiny[4][32], least[4][32];
     // a thread's sums (re, im): of its own spin's colour c (k = c) and lower share (k = 3 + c), in
     // the place of its spinor copies once it has read them
     __device__ __forceinline__ longlong2 &sum(int warp, int k, int lane)
@@ -354,7 +403,8 @@ struct Split {
 };
 
 template <bool DAG, bool AOS>
-__device__ __forceinline__ bool site_split(const Operands<AOS> &p, Split &sm, int s, int half, Pow2 f, double2 *v)
+__device__ __forceinline__ Judged site_split(const Operands<AOS> &p, Split &sm, int s, int half, Pow2 f, double2 *v,
+                                             uint32_t &E)
 {
     const WdSite c = wd_site(p.g, s, p.cb);
     const double sigma = half ? -1.0 : 1.0;
@@ -377,15 +427,20 @@ __device__ __forceinline__ bool site_split(const Operands<AOS> &p, Split &sm, in
         }
         sm.E[MU][l] = A.E;
         sm.tiny[MU][l] = A.tiny;
+        sm.least[MU][l] = A.least[MU / 2];
     };
     if (w == 0) pair(std::integral_constant<int, 0>());
     else if (w == 1) pair(std::integral_constant<int, 1>());
     else if (w == 2) pair(std::integral_constant<int, 2>());
     else pair(std::integral_constant<int, 3>());
     __syncthreads();
-    uint32_t E = 0, tiny = 0;
+    uint32_t tiny = 0, own = 0, low = 0;
+    E = 0;
 #pragma unroll
     for (int m = 0; m < 4; ++m) {
+        const int j = m < 2 ? l : l ^ 1;  // the lower share of mu = 2, 3 is the partner's
+        own = max(own, sm.least[m][l]);
+        low = max(low, sm.least[m][j]);
         E = max(E, sm.E[m][l]);  // the pair's two lanes hold the same exponent
         tiny |= sm.tiny[m][l] | sm.tiny[m][l ^ 1];
     }
@@ -394,7 +449,7 @@ __device__ __forceinline__ bool site_split(const Operands<AOS> &p, Split &sm, in
 #pragma unroll
         for (int m = 0; m < 4; ++m) {
             const uint32_t d = min(E - sm.E[m][l], 63u);
-            const int j = m < 2 ? l : l ^ 1;  // the lower share of mu = 2, 3 is the partner's
+            const int j = m < 2 ? l : l ^ 1;
             const longlong2 a = sm.sum(m, w, l), b = sm.sum(m, 3 + w, j);
             t[0] += a.x >> d;
             t[1] += a.y >> d;
@@ -404,8 +459,10 @@ __device__ __forceinline__ bool site_split(const Operands<AOS> &p, Split &sm, in
         const int kexp = ((int)E - kUnit + f.shift) << 20;
         v[0] = make_double2(value(t[0], kexp, f.sign), value(t[1], kexp, f.sign));
         v[1] = make_double2(value(t[2], kexp, f.sign), value(t[3], kexp, f.sign));
+        if (!own) v[0] = make_double2(0.0, 0.0);
+        if (!low) v[1] = make_double2(0.0, 0.0);
     }
-    return in_range(E, tiny);
+    return judged(E, tiny, good(own, E) && good(low, E));
 }
 
 }  // namespace wd_fix
