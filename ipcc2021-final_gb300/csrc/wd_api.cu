@@ -1,6 +1,7 @@
 // wd_api.cu -- C ABI: contexts, resident lattices and fields, operators and
 // the host-buffer entry points that replace the reference's functions.
 #include <algorithm>
+#include <atomic>
 #include <cstring>
 #include <cstdio>
 #include <string>
@@ -74,8 +75,8 @@ extern "C" wd_status wd_context_create(int device, wd_context **out)
         e = cudaMalloc(&ctx->red_partial, sizeof(double2) * (WD_RED_BLOCKS + WD_RED_SLOTS));
     if (e == cudaSuccess) e = cudaHostAlloc(&ctx->red_result, sizeof(double2) * WD_RED_SLOTS, 0);
     if (e == cudaSuccess) e = cudaHostAlloc(&ctx->state_host, WD_STATE_HOST_BYTES, 0);
-    if (e == cudaSuccess) e = cudaMalloc(&ctx->dev_err, sizeof(int));
-    if (e == cudaSuccess) e = cudaMemset(ctx->dev_err, 0, sizeof(int));
+    if (e == cudaSuccess) e = cudaMalloc(&ctx->dev_err, 2 * sizeof(int));
+    if (e == cudaSuccess) e = cudaMemset(ctx->dev_err, 0, 2 * sizeof(int));
     if (e != cudaSuccess) {
         wd_context_destroy(ctx);
         cudaGetLastError();
@@ -98,6 +99,7 @@ static void host_cache_drop(wd_context *ctx)
 
 // ------------------------------------------- fixed-point links (wd_fix_links.h)
 static wd_lattice *fix_list = nullptr;
+static std::atomic<uint64_t> memory_epoch{1};
 
 std::shared_mutex &wd_fix_mutex()
 {
@@ -105,17 +107,13 @@ std::shared_mutex &wd_fix_mutex()
     return *m;
 }
 
-void wd_fix_enter(wd_lattice *lat, void *links)
-{
-    lat->gauge_fix = links;
-    lat->fix_prev = nullptr;
-    lat->fix_next = fix_list;
-    if (fix_list) fix_list->fix_prev = lat;
-    fix_list = lat;
-}
+void wd_memory_freed() { memory_epoch.fetch_add(1, std::memory_order_relaxed); }
 
-void wd_fix_free(wd_lattice *lat)
+// the caller holds the lock alone
+static void fix_free(wd_lattice *lat, wd_lattice::Fix state)
 {
+    lat->fix_state = state;
+    lat->fix_epoch = memory_epoch.load(std::memory_order_relaxed);
     if (!lat->gauge_fix) return;
     cudaDeviceSynchronize();  // launches of any context may still read them
     cudaFree(lat->gauge_fix);
@@ -125,10 +123,17 @@ void wd_fix_free(wd_lattice *lat)
     lat->fix_prev = lat->fix_next = nullptr;
 }
 
+void wd_fix_outdate(wd_lattice *lat)
+{
+    const WdFixAlone lock(wd_fix_mutex());
+    if (lat->fix_state == wd_lattice::kFixUnfit) lat->fix_was_unfit = true;
+    lat->fix_state = wd_lattice::kFixOpen;
+}
+
 void wd_drop_fix(wd_lattice *lat)
 {
     const WdFixAlone lock(wd_fix_mutex());
-    wd_fix_free(lat);
+    fix_free(lat, wd_lattice::kFixOpen);
 }
 
 bool wd_release_fix(int device)
@@ -138,7 +143,7 @@ bool wd_release_fix(int device)
     for (wd_lattice *lat = fix_list, *next; lat; lat = next) {
         next = lat->fix_next;
         if (lat->device != device) continue;
-        wd_fix_free(lat);
+        fix_free(lat, wd_lattice::kFixRefused);
         any = true;
     }
     return any;
@@ -148,6 +153,70 @@ size_t wd_fix_bytes(const wd_lattice *lat)
 {
     const WdFixShared lock(wd_fix_mutex());
     return lat->gauge_fix ? (size_t)lat->volume * 4 * 9 * sizeof(int4) : 0;
+}
+
+static bool fix_wanted(const wd_lattice *lat)
+{
+    return lat->use_fix && (lat->fix_state == wd_lattice::kFixOpen ||
+                            (lat->fix_state == wd_lattice::kFixRefused &&
+                             lat->fix_epoch != memory_epoch.load(std::memory_order_relaxed)));
+}
+
+// Memory for the copy, or false.  It only makes FP64 hops faster, so it is kept
+// where it leaves at least half of the device's memory free or in the context's
+// work-buffer cache (an eighth free); a small one, an eighth.
+static bool fix_alloc(wd_context *ctx, wd_lattice *lat)
+{
+    if (lat->gauge_fix) return true;
+    const size_t n = (size_t)lat->volume * 4 * 9 * sizeof(int4);
+    size_t free_b = 0, total_b = 0, cached = 0;
+    for (const auto &kv : ctx->pool_free) cached += kv.first;
+    if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess || free_b < n + total_b / 8 ||
+        (n >= (64u << 20) && free_b + cached < n + total_b / 2) || cudaMalloc(&lat->gauge_fix, n) != cudaSuccess) {
+        cudaGetLastError();
+        lat->gauge_fix = nullptr;
+        return false;
+    }
+    lat->fix_prev = nullptr;
+    lat->fix_next = fix_list;
+    if (fix_list) fix_list->fix_prev = lat;
+    fix_list = lat;
+    return true;
+}
+
+bool wd_fix_ensure(wd_context *ctx, const wd_lattice *lat_c)
+{
+    {
+        const WdFixShared lock(wd_fix_mutex());
+        if (lat_c->fix_state == wd_lattice::kFixReady) return true;
+        if (!fix_wanted(lat_c)) return false;
+    }
+    const WdFixAlone lock(wd_fix_mutex());
+    wd_lattice *lat = const_cast<wd_lattice *>(lat_c);
+    if (!fix_wanted(lat)) return lat->fix_state == wd_lattice::kFixReady;
+    // one pass converts the links and looks whether they fit (links that
+    // follow ones that did not are looked at before memory is asked for)
+    for (bool look = lat->fix_was_unfit && !lat->gauge_fix;; look = false) {
+        if (!look && !fix_alloc(ctx, lat)) {
+            fix_free(lat, wd_lattice::kFixRefused);
+            return false;
+        }
+        int bad = 0;
+        if (wd_gauge_to_fix(ctx, lat, look ? nullptr : lat->gauge_fix, ctx->dev_err + 1) != WD_OK ||
+            cudaMemcpyAsync(&bad, ctx->dev_err + 1, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream) != cudaSuccess ||
+            cudaStreamSynchronize(ctx->stream) != cudaSuccess) {
+            fix_free(lat, wd_lattice::kFixRefused);
+            return false;
+        }
+        if (bad) {
+            fix_free(lat, wd_lattice::kFixUnfit);
+            return false;
+        }
+        if (!look) break;
+    }
+    lat->fix_was_unfit = false;
+    lat->fix_state = wd_lattice::kFixReady;
+    return true;
 }
 
 cudaError_t wd_malloc(wd_context *ctx, void **p, size_t bytes)
@@ -204,6 +273,7 @@ void wd_pool_release(wd_context *ctx)
         ctx->pool_bytes -= kv.first;
     }
     ctx->pool_free.clear();
+    wd_memory_freed();
 }
 
 extern "C" void wd_context_destroy(wd_context *ctx)
@@ -331,30 +401,6 @@ static void *pinned_view(const void *p)
     return a.devicePointer;
 }
 
-// Allocates the lattice's fixed-point links if it has none: a copy that only
-// makes FP64 hops faster, so it is kept where it leaves at least half of the
-// device's memory free or in the context's work-buffer cache (an eighth free),
-// and given back when a later allocation needs its memory (wd_malloc).  The
-// caller holds the lock alone.  Returns the device flag behind the planes, or null.
-static int *want_fix(wd_context *ctx, wd_lattice *lat)
-{
-    const size_t n = (size_t)lat->volume * 4 * 9 * sizeof(int4);
-    if (!lat->gauge_fix && lat->use_fix) {
-        size_t free_b = 0, total_b = 0;
-        size_t cached = 0;
-        for (const auto &kv : ctx->pool_free) cached += kv.first;
-        const bool room = n < (64u << 20) || (cudaMemGetInfo(&free_b, &total_b) == cudaSuccess &&
-                                              free_b + cached >= n + total_b / 2 && free_b >= n + total_b / 8);
-        void *links = nullptr;
-        if (!room || cudaMalloc(&links, n + sizeof(int4)) != cudaSuccess) {
-            cudaGetLastError();
-            return nullptr;
-        }
-        wd_fix_enter(lat, links);
-    }
-    return lat->gauge_fix ? (int *)((char *)lat->gauge_fix + n) : nullptr;
-}
-
 static wd_status upload_gauge(wd_context *ctx, wd_lattice *lat, const double *const gauge[4])
 {
     const WdGeom &g = lat->g;
@@ -368,38 +414,31 @@ static wd_status upload_gauge(wd_context *ctx, wd_lattice *lat, const double *co
     }
     wd_status st = stage ? ensure_staging(ctx, bytes) : WD_OK;
     if (st != WD_OK) return st;
-    const WdFixAlone lock(wd_fix_mutex());  // no other context may take the copy while it is written
-    int *bad = want_fix(ctx, lat);
-    if (bad) WD_CUDA(ctx, cudaMemsetAsync(bad, 0, sizeof(int), ctx->stream));
+    wd_fix_outdate(lat);
     for (int mu = 0; mu < 4; ++mu) {
         const double2 *ref = view[mu];
         if (!ref) {
             WD_CUDA(ctx, cudaMemcpyAsync(ctx->staging, gauge[mu], bytes, cudaMemcpyHostToDevice, ctx->stream));
             ref = (const double2 *)ctx->staging;
         }
-        st = bad ? wd_gauge_ref_to_soa_fix(ctx, g, mu, ref, lat->gauge, lat->gauge_fix, bad)
-                 : wd_gauge_ref_to_soa(ctx, g, mu, ref, lat->gauge);
+        st = wd_gauge_ref_to_soa(ctx, g, mu, ref, lat->gauge);
         if (st != WD_OK) {
             cudaStreamSynchronize(ctx->stream);  // nothing reads the caller's arrays after the call
             return st;
         }
     }
     wd_lattice_invalidate_derived(lat);
-    int *host_bad = (int *)ctx->state_host;
-    *host_bad = 0;
-    if (bad) WD_CUDA(ctx, cudaMemcpyAsync(host_bad, bad, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
     WD_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-    if (*host_bad) wd_fix_free(lat);
     return WD_OK;
 }
 
-wd_status wd_lattice_make(wd_context *ctx, const int dims[4], const double *const gauge[4], bool fix, wd_lattice **out)
+extern "C" wd_status wd_lattice_create(wd_context *ctx, const int dims[4], const double *const gauge[4],
+                                       wd_lattice **out)
 {
     if (!ctx || !out || !gauge) return wd_fail(ctx, WD_ERR_BAD_ARG, "null argument");
     *out = nullptr;
     wd_lattice *lat = new wd_lattice();
     lat->device = ctx->device;
-    lat->use_fix = fix;
     wd_status st = make_geom(ctx, dims, &lat->g, &lat->volume);
     if (st != WD_OK) {
         delete lat;
@@ -419,12 +458,6 @@ wd_status wd_lattice_make(wd_context *ctx, const int dims[4], const double *cons
     return WD_OK;
 }
 
-extern "C" wd_status wd_lattice_create(wd_context *ctx, const int dims[4], const double *const gauge[4],
-                                       wd_lattice **out)
-{
-    return wd_lattice_make(ctx, dims, gauge, true, out);
-}
-
 extern "C" wd_status wd_lattice_update(wd_context *ctx, wd_lattice *lat, const double *const gauge[4])
 {
     if (!ctx || !lat || !gauge) return wd_fail(ctx, WD_ERR_BAD_ARG, "null argument");
@@ -438,6 +471,7 @@ extern "C" void wd_lattice_destroy(wd_lattice *lat)
     wd_drop_fix(lat);
     wd_lattice_invalidate_derived(lat);
     delete lat;
+    wd_memory_freed();
 }
 
 extern "C" int64_t wd_lattice_volume(const wd_lattice *lat) { return lat ? lat->volume : 0; }
@@ -505,7 +539,10 @@ extern "C" void wd_field_destroy(wd_field *f)
 {
     if (!f) return;
     if (f->pool) wd_dev_free(f->pool, f->data);
-    else cudaFree(f->data);  // cudaFree waits for work in flight on the device
+    else {
+        cudaFree(f->data);  // cudaFree waits for work in flight on the device
+        wd_memory_freed();
+    }
     delete f;
 }
 

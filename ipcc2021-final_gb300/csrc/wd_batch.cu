@@ -1104,9 +1104,30 @@ static double server_fix_bytes(const wd_server *sv)
 // the server accepts does not depend on them.
 static void server_make_room(wd_server *sv, double bytes)
 {
-    if (sv->gauge_bytes + sv->req_bytes + server_fix_bytes(sv) + bytes <= sv->cfg.hbm_budget_bytes) return;
-    for (wd_lattice *l : sv->lats)
+    double used = sv->gauge_bytes + sv->req_bytes + bytes;
+    for (const wd_lattice *l : sv->lats)
+        if (l->use_fix) used += (double)l->volume * 4 * 9 * sizeof(int4);
+    if (used <= sv->cfg.hbm_budget_bytes) return;
+    for (wd_lattice *l : sv->lats) {
+        l->use_fix = false;
         wd_drop_fix(l);
+    }
+}
+
+// Lets the lattices have them (again) where the budget has room.  FP64 hops run
+// in the plain FP64 server and in FP64 reliable updates only.
+static void server_allow_fix(wd_server *sv)
+{
+    if (sv->cfg.prec != WD_PREC_F64 && sv->cfg.prec_reliable == WD_PREC_DF64) return;
+    double used = sv->gauge_bytes + sv->req_bytes;
+    for (const wd_lattice *l : sv->lats)
+        if (l->use_fix) used += (double)l->volume * 4 * 9 * sizeof(int4);
+    for (wd_lattice *l : sv->lats) {
+        const double n = (double)l->volume * 4 * 9 * sizeof(int4);
+        if (l->use_fix || used + n > sv->cfg.hbm_budget_bytes) continue;
+        l->use_fix = true;
+        used += n;
+    }
 }
 
 static double request_bytes(const wd_server *sv, const wd_lattice *lat, int nsrc)
@@ -1163,10 +1184,9 @@ extern "C" wd_status wd_server_add_lattice(wd_server *sv, const int dims[4], con
 {
     if (!sv || !id) return WD_ERR_BAD_ARG;
     wd_lattice *lat = nullptr;
-    // FP64 hops run in the plain FP64 server and in FP64 reliable updates only
-    const bool fp64 = sv->cfg.prec == WD_PREC_F64 || sv->cfg.prec_reliable != WD_PREC_DF64;
-    wd_status st = wd_lattice_make(sv->ctx, dims, gauge, fp64, &lat);
+    wd_status st = wd_lattice_create(sv->ctx, dims, gauge, &lat);
     if (st != WD_OK) return st;
+    lat->use_fix = false;
     // derived link copies the server will use, built now so they count against the budget
     double bytes = (double)lat->volume * 4 * 9 * sizeof(double2);
     if (sv->cfg.prec != WD_PREC_F64) {
@@ -1188,6 +1208,8 @@ extern "C" wd_status wd_server_add_lattice(wd_server *sv, const int dims[4], con
     sv->gauge_bytes += bytes;
     sv->lats.push_back(lat);
     server_make_room(sv, 0);
+    server_allow_fix(sv);
+    wd_fix_ensure(sv->ctx, lat);
     *id = (int)sv->lats.size() - 1;
     return WD_OK;
 }
@@ -1331,6 +1353,7 @@ extern "C" wd_status wd_server_step(wd_server *sv, int *completed)
         if (completed) *completed = done;
         return st;
     }
+    server_allow_fix(sv);
     std::vector<int> fin;
     if (sv->eng) {
         sv->eng->take_retired(&fin);  // systems already solved at admission

@@ -9,46 +9,51 @@
 
 namespace {
 
-// One direction's links: reference AoS -> FP64 planes and fixed-point planes
-// (a tile of 64 sites through shared memory, each link read once).  *bad is
-// set when a link is outside what the fixed-point kernels are written for:
-// the integer ranges need |u| <= 1 and absolute row and column sums (columns:
-// the backward terms) of at most sqrt(6), and links much smaller than a
-// unitary matrix's would lose digits below the fixed 2^-60.
-__global__ void __launch_bounds__(256) k_gauge_in(const double2 *__restrict__ aos, double2 *__restrict__ soa,
-                                                  int4 *__restrict__ fix, int Vh, int *bad)
+// FP64 planes -> fixed-point planes (if fix is given).  *bad is set when a link
+// is outside what the fixed-point kernels are written for: the integer ranges
+// need |u| <= 1 and absolute row and column sums (columns: the backward terms)
+// of at most sqrt(6), the look at a component's terms needs such sums of 0.99,
+// and links much smaller than a unitary matrix's would lose digits below the
+// fixed 2^-60.  On integers and FP32, so that HBM bounds it (once for a set of
+// links), not the FP64 pipe.
+struct Fixed {
+    int hi, lo;   // round(x 2^60) in two limbs
+    float size;   // |x|
+};
+__device__ __forceinline__ Fixed fixed(double x)
 {
-    constexpr int kTile = 64;
-    __shared__ double2 tile[kTile * 9];
-    const int b = blockIdx.y, s0 = blockIdx.x * kTile, ns = min(kTile, Vh - s0);
-    const double2 *src = aos + ((size_t)b * Vh + s0) * 9;
-    soa += (size_t)b * 9 * Vh + s0;
-    fix += (size_t)b * 9 * Vh + s0;
-    for (int i = threadIdx.x; i < ns * 9; i += blockDim.x) tile[i] = src[i];
-    __syncthreads();
-    for (int i = threadIdx.x; i < ns * 9; i += blockDim.x) {
-        const int c = i / ns, s = i - c * ns;
-        const double2 v = tile[s * 9 + c];
-        soa[(size_t)c * Vh + s] = v;
-        const long long re = __double2ll_rn(v.x * 0x1p60), im = __double2ll_rn(v.y * 0x1p60);
-        const long long r1 = (re + (1ll << 29)) >> 30, i1 = (im + (1ll << 29)) >> 30;
-        fix[(size_t)c * Vh + s] = make_int4((int)r1, (int)(re - (r1 << 30)), (int)i1, (int)(im - (i1 << 30)));
-    }
-    for (int s = threadIdx.x; s < ns; s += blockDim.x) {
-        double row[3] = {0, 0, 0}, col[3] = {0, 0, 0};
-        bool ok = true;
+    const uint32_t hw = (uint32_t)__double2hiint(x), e = hw >> 20 & 0x7ff;
+    // |x| 2^60 = m 2^(e - 1015), m of 53 bits; e <= 1023 where the link fits
+    const uint64_t m = (uint64_t)(hw & 0xfffffu | (e ? 0x100000u : 0)) << 32 | (uint32_t)__double2loint(x);
+    const int n = min(1015 - (int)e, 62);
+    const uint64_t q = n > 0 ? (m + (1ull << (n - 1))) >> n : m << min(-n, 8);
+    const long long t = (int)hw < 0 ? -(long long)q : (long long)q, t1 = (t + (1ll << 29)) >> 30;
+    Fixed f{(int)t1, (int)(t - (t1 << 30)), 0.f};
+    if (e > 1100) f.size = __int_as_float(0x7f800000);  // too large, infinite, NaN
+    else if (e > 900) f.size = __uint_as_float((e - 896) << 23 | (uint32_t)(m >> 29 & 0x7fffffu));
+    return f;
+}
+
+__global__ void __launch_bounds__(128) k_gauge_fix(const double2 *__restrict__ gauge, int4 *__restrict__ fix, int Vh,
+                                                   int *bad)
+{
+    const int s = blockIdx.x * 128 + threadIdx.x;
+    if (s >= Vh) return;
+    const size_t i0 = (size_t)blockIdx.y * 9 * Vh + s;  // direction and parity
+    float row[3] = {0, 0, 0}, col[3] = {0, 0, 0};
+    bool ok = true;
 #pragma unroll
-        for (int k = 0; k < 9; ++k) {
-            const double ax = fabs(tile[s * 9 + k].x), ay = fabs(tile[s * 9 + k].y);
-            ok = ok && ax <= 1.0 + 0x1p-20 && ay <= 1.0 + 0x1p-20 && ax + ay <= 1.5;  // false for NaN too
-            row[k / 3] += ax + ay;
-            col[k % 3] += ax + ay;
-        }
-#pragma unroll
-        for (int k = 0; k < 3; ++k)
-            ok = ok && row[k] >= 0.99 && row[k] <= 2.46 && col[k] >= 0.99 && col[k] <= 2.46;
-        if (!ok) *bad = 1;
+    for (int k = 0; k < 9; ++k) {
+        const double2 v = gauge[i0 + (size_t)k * Vh];
+        const Fixed x = fixed(v.x), y = fixed(v.y);
+        if (fix) fix[i0 + (size_t)k * Vh] = make_int4(x.hi, x.lo, y.hi, y.lo);
+        ok = ok && x.size <= 1.f + 0x1p-20f && y.size <= 1.f + 0x1p-20f && x.size + y.size <= 1.5f;
+        row[k / 3] += x.size + y.size;
+        col[k % 3] += x.size + y.size;
     }
+#pragma unroll
+    for (int k = 0; k < 3; ++k) ok = ok && row[k] >= 0.99f && row[k] <= 2.46f && col[k] >= 0.99f && col[k] <= 2.46f;
+    if (!ok) *bad = 1;
 }
 
 struct FixArgs {
@@ -438,23 +443,33 @@ FixArgs fix_args(const wd_lattice *lat, const void *in, void *out, const void *x
                    (const int4 *)lat->gauge_fix, alpha, beta, pre, pow2 ? 1.0 : alpha, !pow2, stop, nullptr};
 }
 
-// Whether a launch on `stream` may use the lattice's fixed-point links (under
-// the lock).  A stream that is being captured may not: the graph would keep
-// their address past the moment they are freed or replaced, while the FP64
-// links stay where they are as long as the lattice.
-bool links_for(const wd_lattice *lat, cudaStream_t stream)
-{
-    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-    return lat->gauge_fix && cudaStreamIsCapturing(stream, &cs) == cudaSuccess && cs == cudaStreamCaptureStatusNone;
-}
+// A launch's hold on the lattice's fixed-point links: the lock shared, if they
+// are there or can be built.  A stream that is being captured may not use them:
+// the graph would keep their address past the moment they are freed or replaced,
+// while the FP64 links stay where they are as long as the lattice.
+struct Links {
+    WdFixShared lock;
+    Links(wd_context *ctx, const wd_lattice *lat, cudaStream_t stream)
+    {
+        cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+        if (cudaStreamIsCapturing(stream, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone) return;
+        lock = WdFixShared(wd_fix_mutex());
+        if (lat->fix_state == wd_lattice::kFixReady) return;
+        lock.unlock();
+        if (!wd_fix_ensure(ctx, lat)) return;
+        lock.lock();
+        if (lat->fix_state != wd_lattice::kFixReady) lock.unlock();  // taken back in between
+    }
+    explicit operator bool() const { return lock.owns_lock(); }
+};
 
 }  // namespace
 
-wd_status wd_gauge_ref_to_soa_fix(wd_context *ctx, const WdGeom &g, int mu, const double2 *ref, double2 *soa, void *fix,
-                                  int *bad)
+wd_status wd_gauge_to_fix(wd_context *ctx, const wd_lattice *lat, void *fix, int *bad)
 {
-    const size_t off = (size_t)mu * 2 * 9 * g.Vh;
-    k_gauge_in<<<dim3((g.Vh + 63) / 64, 2), 256, 0, ctx->stream>>>(ref, soa + off, (int4 *)fix + off, g.Vh, bad);
+    const int Vh = lat->g.Vh;
+    WD_CUDA(ctx, cudaMemsetAsync(bad, 0, sizeof(int), ctx->stream));
+    k_gauge_fix<<<dim3((Vh + 127) / 128, 8), 128, 0, ctx->stream>>>(lat->gauge, (int4 *)fix, Vh, bad);
     WD_LAUNCHED(ctx);
     return WD_OK;
 }
@@ -462,8 +477,8 @@ wd_status wd_gauge_ref_to_soa_fix(wd_context *ctx, const WdGeom &g, int mu, cons
 WdTried wd_hop_fix(wd_context *ctx, const wd_lattice *lat, const double2 *in, double2 *out, const double2 *x, int cb,
                    int dag, double alpha, double beta, const int *stop, double2 *zero)
 {
-    const WdFixShared lock(wd_fix_mutex());
-    if (!links_for(lat, ctx->stream)) return {};
+    const Links links(ctx, lat, ctx->stream);
+    if (!links) return {};
     FixArgs a = fix_args(lat, in, out, x, cb, alpha, beta, stop);
     a.zero = zero;
     // one shape (64 and 32 threads a block run within 0.3 % of 128): the
@@ -475,8 +490,8 @@ WdTried wd_hop_fix(wd_context *ctx, const wd_lattice *lat, const double2 *in, do
 WdTried wd_hop_fix_M(wd_context *ctx, const wd_lattice *lat, const double2 *in, double2 *out, double mass, int dag,
                      const int *stop)
 {
-    const WdFixShared lock(wd_fix_mutex());
-    if (!links_for(lat, ctx->stream)) return {};
+    const Links links(ctx, lat, ctx->stream);
+    if (!links) return {};
     return store_fix<false>(ctx, ctx->stream, fix_args(lat, in, out, in, 0, -0.5, 4.0 + mass, stop), dag, true, 0,
                             lat->g.Vh);
 }
@@ -484,16 +499,16 @@ WdTried wd_hop_fix_M(wd_context *ctx, const wd_lattice *lat, const double2 *in, 
 WdTried wd_hop_fix_residual(wd_context *ctx, const wd_lattice *lat, const double2 *in, const double2 *x, double alpha,
                             double beta, const WdResSink &r)
 {
-    const WdFixShared lock(wd_fix_mutex());
-    if (!links_for(lat, ctx->stream)) return {};
+    const Links links(ctx, lat, ctx->stream);
+    if (!links) return {};
     return run_fix<false>(ctx, fix_args(lat, in, nullptr, x, 0, alpha, beta), EpiRes{r.red, r});
 }
 
 WdTried wd_hop_fix_norm(wd_context *ctx, const wd_lattice *lat, WdVec in, WdVec t, WdVec p, double mass, WdCgDev *dev,
                         WdRed red)
 {
-    const WdFixShared lock(wd_fix_mutex());
-    if (!links_for(lat, ctx->stream)) return {};
+    const Links links(ctx, lat, ctx->stream);
+    if (!links) return {};
     const double a = 4.0 + mass;
     return run_fix<false>(ctx, fix_args(lat, in.p, t.p, p.p, 0, -0.25 / a, a, &dev->stop), EpiNorm{dev, red});
 }
@@ -501,8 +516,8 @@ WdTried wd_hop_fix_norm(wd_context *ctx, const wd_lattice *lat, WdVec in, WdVec 
 WdTried wd_hop_fix_update(wd_context *ctx, const wd_lattice *lat, WdVec in, WdVec t, WdVec p, WdVec r, WdVec x,
                           double mass, WdCgDev *dev, WdRed red)
 {
-    const WdFixShared lock(wd_fix_mutex());
-    if (!links_for(lat, ctx->stream)) return {};
+    const Links links(ctx, lat, ctx->stream);
+    if (!links) return {};
     const double a = 4.0 + mass;
     return run_fix<true>(ctx, fix_args(lat, in.p, nullptr, t.p, 0, -0.25 / a, a, &dev->stop),
                          EpiUpdate{dev, red, (const double2 *)p.p, (double2 *)r.p, (double2 *)x.p});
@@ -511,8 +526,8 @@ WdTried wd_hop_fix_update(wd_context *ctx, const wd_lattice *lat, WdVec in, WdVe
 WdTried wd_hop_fix_M_dot(wd_context *ctx, const wd_lattice *lat, WdVec in, WdVec q, WdVec p, double mass, WdCgDev *dev,
                          WdRed red)
 {
-    const WdFixShared lock(wd_fix_mutex());
-    if (!links_for(lat, ctx->stream)) return {};
+    const Links links(ctx, lat, ctx->stream);
+    if (!links) return {};
     return run_fix<true>(ctx, fix_args(lat, in.p, q.p, in.p, 0, -0.5, 4.0 + mass, &dev->stop),
                          EpiDot{dev, red, (const double2 *)p.p}, true);
 }
@@ -520,8 +535,8 @@ WdTried wd_hop_fix_M_dot(wd_context *ctx, const wd_lattice *lat, WdVec in, WdVec
 WdTried wd_hop_fix_M_residual(wd_context *ctx, const wd_lattice *lat, const double2 *b, const double2 *x, double mass,
                               WdRed red, double *result)
 {
-    const WdFixShared lock(wd_fix_mutex());
-    if (!links_for(lat, ctx->stream)) return {};
+    const Links links(ctx, lat, ctx->stream);
+    if (!links) return {};
     return run_fix<false>(ctx, fix_args(lat, x, nullptr, x, 0, -0.5, 4.0 + mass),
                           EpiTrueRes{red, b, result}, true);
 }
@@ -530,7 +545,7 @@ WdTried wd_hop_fix_aos_range(wd_context *ctx, cudaStream_t stream, const wd_latt
                              double2 *out_aos, const double2 *x_aos, int cb, int dag, double alpha, double beta,
                              int s_lo, int s_hi)
 {
-    const WdFixShared lock(wd_fix_mutex());
-    if (!links_for(lat, stream)) return {};
+    const Links links(ctx, lat, stream);
+    if (!links) return {};
     return store_fix<true>(ctx, stream, fix_args(lat, in_aos, out_aos, x_aos, cb, alpha, beta), dag, false, s_lo, s_hi);
 }

@@ -17,12 +17,17 @@ std::shared_mutex &wd_fix_mutex();
 using WdFixShared = std::shared_lock<std::shared_mutex>;
 using WdFixAlone = std::unique_lock<std::shared_mutex>;
 
-// Enters or removes (and frees) the copy; the caller holds the lock alone
-void wd_fix_enter(wd_lattice *lat, void *links);
-void wd_fix_free(wd_lattice *lat);
+// The lattice has its fixed-point links, built now if they fit, are wanted and
+// have room.  Not to be called under the lock (and the copy may be gone again
+// by the time the caller looks).
+bool wd_fix_ensure(wd_context *ctx, const wd_lattice *lat);
+// The lattice's links are about to change: the copy is no longer theirs
+void wd_fix_outdate(wd_lattice *lat);
 // Frees one lattice's copy, if it has one
 void wd_drop_fix(wd_lattice *lat);
 // Frees the copies of every lattice on a device; true if there were any
 bool wd_release_fix(int device);
-// Bytes of the copy the lattice holds now (0: none)
+// Bytes the lattice holds for its copy now (0: none)
 size_t wd_fix_bytes(const wd_lattice *lat);
+// Device memory was freed: copies that were refused are tried again
+void wd_memory_freed();

@@ -69,7 +69,8 @@ struct wd_context {
     void *red_partial = nullptr;  // WD_RED_BLOCKS double2 (+ result slots)
     void *red_result = nullptr;   // pinned host mirror of the reduction results
     void *state_host = nullptr;   // pinned host mirror of a solver's device scalars (WD_STATE_HOST_BYTES)
-    int *dev_err = nullptr;       // device flag: a kernel's bounded wait gave up (wd_context_device_check)
+    int *dev_err = nullptr;       // device flags: [0] a kernel's bounded wait gave up (wd_context_device_check),
+                                  // [1] links that the fixed-point copy does not hold
     void *staging = nullptr;      // device staging buffer for reference-layout copies
     size_t staging_bytes = 0;
     // cached host-buffer path state (wd_host_*): one lattice + fields
@@ -111,8 +112,6 @@ void wd_pool_release(wd_context *ctx);
 cudaError_t wd_malloc(wd_context *ctx, void **p, size_t bytes);
 // a library-internal FP64 field, from the work-buffer cache if it is small
 wd_status wd_field_create_work(wd_context *ctx, const wd_lattice *lat, wd_field **out);
-// wd_lattice_create; fix = false: without fixed-point links
-wd_status wd_lattice_make(wd_context *ctx, const int dims[4], const double *const gauge[4], bool fix, wd_lattice **out);
 
 struct wd_lattice {
     int device = 0;
@@ -120,12 +119,20 @@ struct wd_lattice {
     int64_t volume = 0;
     double2 *gauge = nullptr;     // FP64 [mu][parity][9][Vh]
     float4 *gauge_df = nullptr;   // double-float copy, same shape (lazily built)
-    // fixed-point copy, int4 {re hi, re lo, im hi, im lo}, same shape, written with the FP64 links at
-    // upload; null when they do not fit it or memory is short (FP64 hops then run on the FP64 pipe)
-    // (gauge_fix and the list are read and written under the lock of wd_fix_links.h only)
+    // fixed-point copy, int4 {re hi, re lo, im hi, im lo}, same shape, built on the first FP64 hop where the
+    // links fit it and memory is ample (else FP64 hops run on the FP64 pipe).  gauge_fix, its state and the
+    // list are read and written under the lock of wd_fix_links.h only.
     void *gauge_fix = nullptr;
-    wd_lattice *fix_prev = nullptr, *fix_next = nullptr;  // list of the lattices that hold one
-    bool use_fix = true;          // whether FP64 hops are expected on this lattice
+    enum Fix {
+        kFixOpen,     // not built for the present links (gauge_fix may hold memory for it)
+        kFixReady,
+        kFixUnfit,    // the present links do not fit it
+        kFixRefused   // no room when it was last tried, at fix_epoch
+    } fix_state = kFixOpen;
+    uint64_t fix_epoch = 0;
+    bool fix_was_unfit = false;   // earlier links did not fit: look before memory is asked for
+    bool use_fix = true;          // cleared by a server whose budget has no room for it
+    wd_lattice *fix_prev = nullptr, *fix_next = nullptr;  // list of the lattices that hold memory for one
     void *gauge_f32 = nullptr;    // FP32 12-real links [mu][parity][3][Vh] float4 (lazily built)
     void *gauge_h12 = nullptr;    // FP16 12-real links: uint4 [8][Vh] then uint2 [8][Vh] (lazily built)
 };

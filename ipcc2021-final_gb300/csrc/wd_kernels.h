@@ -15,10 +15,9 @@ wd_status wd_hop_f64(wd_context *ctx, const wd_lattice *lat, const double2 *in_b
                      double beta, const int *stop = nullptr);
 
 // ---- the FP64 hop in 64-bit fixed point (wd_dslash_fix.cu)
-// one direction's links from the reference layout into the FP64 planes and
-// the fixed-point planes; *bad (device) is set when they do not fit the latter
-wd_status wd_gauge_ref_to_soa_fix(wd_context *ctx, const WdGeom &g, int mu, const double2 *ref, double2 *soa, void *fix,
-                                  int *bad);
+// the fixed-point planes from the FP64 ones (fix null: only the look);
+// *bad (device) is set if the links do not fit them, else cleared
+wd_status wd_gauge_to_fix(wd_context *ctx, const wd_lattice *lat, void *fix, int *bad);
 // a residual hop's outputs: s32 = FP32(bhat - hop), |s32|^2
 struct WdResSink {
     const double2 *bhat;

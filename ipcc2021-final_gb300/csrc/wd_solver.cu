@@ -79,7 +79,7 @@ wd_status wd_true_residual(wd_context *ctx, const wd_lattice *lat, const double2
     const int64_t rb = wd_red_blocks(lat->g.Vh);
     WdVecBuf buf;
     WdTried one;
-    if (wd_fix_bytes(lat)) {  // (the allocation may give the links back)
+    if (wd_fix_ensure(ctx, lat)) {  // (the allocation may give the links back)
         if ((st = wd_vec_alloc(ctx, buf, WD_PREC_F64, (int64_t)wd_red_doubles(rb, 2) / 2 + 1)) != WD_OK) return st;
         const WdRed red = wd_red_view(buf.v.p, rb);
         double2 *res = (double2 *)ctx->red_partial + WD_RED_BLOCKS;
@@ -386,6 +386,7 @@ extern "C" wd_status wd_solve(wd_context *ctx, const wd_lattice *lat, const wd_f
     wd_solver_stats local;
     if (!stats) stats = &local;
     *stats = wd_solver_stats{};
+    wd_memory_freed();  // a program may have freed memory of its own since the links were last refused theirs
     const auto t0 = std::chrono::steady_clock::now();
     wd_status st;
     const bool mixed = params->prec == WD_PREC_F32 || params->prec == WD_PREC_F16;
