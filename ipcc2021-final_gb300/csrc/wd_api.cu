@@ -169,10 +169,9 @@ static bool fix_alloc(wd_context *ctx, wd_lattice *lat)
 {
     if (lat->gauge_fix) return true;
     const size_t n = (size_t)lat->volume * 4 * 9 * sizeof(int4);
-    size_t free_b = 0, total_b = 0, cached = 0;
-    for (const auto &kv : ctx->pool_free) cached += kv.first;
+    size_t free_b = 0, total_b = 0;
     if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess || free_b < n + total_b / 8 ||
-        (n >= (64u << 20) && free_b + cached < n + total_b / 2) || cudaMalloc(&lat->gauge_fix, n) != cudaSuccess) {
+        (n >= (64u << 20) && free_b + ctx->pool_free_bytes < n + total_b / 2) || cudaMalloc(&lat->gauge_fix, n) != cudaSuccess) {
         cudaGetLastError();
         lat->gauge_fix = nullptr;
         return false;
@@ -246,6 +245,7 @@ wd_status wd_dev_alloc(wd_context *ctx, void **p, size_t bytes)
     if (it != ctx->pool_free.end() && it->first <= 2 * bytes) {
         *p = it->second;
         ctx->pool_used[it->second] = it->first;
+        ctx->pool_free_bytes -= it->first;
         ctx->pool_free.erase(it);
         return WD_OK;
     }
@@ -256,12 +256,19 @@ wd_status wd_dev_alloc(wd_context *ctx, void **p, size_t bytes)
     return WD_OK;
 }
 
-void wd_dev_free(wd_context *ctx, void *p)
+void wd_dev_free(wd_context *ctx, void *p, size_t keep)
 {
     if (!p) return;
     auto it = ctx->pool_used.find(p);
     if (it == ctx->pool_used.end()) return;
-    ctx->pool_free.emplace(it->second, p);
+    if (ctx->pool_free_bytes + it->second > keep) {
+        cudaFree(p);
+        ctx->pool_bytes -= it->second;
+        wd_memory_freed();
+    } else {
+        ctx->pool_free.emplace(it->second, p);
+        ctx->pool_free_bytes += it->second;
+    }
     ctx->pool_used.erase(it);
 }
 
@@ -273,6 +280,7 @@ void wd_pool_release(wd_context *ctx)
         ctx->pool_bytes -= kv.first;
     }
     ctx->pool_free.clear();
+    ctx->pool_free_bytes = 0;
     wd_memory_freed();
 }
 
@@ -521,9 +529,11 @@ extern "C" wd_status wd_field_create_prec(wd_context *ctx, const wd_lattice *lat
 
 // A library-internal FP64 field, destroyed before ctx: up to 64 MB its memory
 // comes from the context's work-buffer cache, since a cudaMalloc and a
-// cudaFree (which waits for the device) per field cost
-// 70 us (a burst of 18 server systems 30.3 ms with them, 27.8 without; a
-// 12-column propagator at 16^3x32 30.1 and 28.9).
+// cudaFree (which waits for the device) per field cost 70 us (a burst of 18
+// server systems 30.3 ms with them, 27.8 without; a 12-column propagator at
+// 16^3x32 30.1 and 28.9).  It goes back there only while the cache holds 1 GB
+// or less: a program's burst of requests is not kept for good.
+constexpr size_t kFieldCache = (size_t)1 << 30;
 wd_status wd_field_create_work(wd_context *ctx, const wd_lattice *lat, wd_field **out)
 {
     return field_make(ctx, lat, WD_PREC_F64, field_bytes(lat, WD_PREC_F64) <= ((size_t)64 << 20), out);
@@ -538,7 +548,7 @@ extern "C" wd_precision wd_field_precision(const wd_field *f) { return f ? f->st
 extern "C" void wd_field_destroy(wd_field *f)
 {
     if (!f) return;
-    if (f->pool) wd_dev_free(f->pool, f->data);
+    if (f->pool) wd_dev_free(f->pool, f->data, kFieldCache);
     else {
         cudaFree(f->data);  // cudaFree waits for work in flight on the device
         wd_memory_freed();

@@ -83,6 +83,7 @@ struct wd_context {
     std::multimap<size_t, void *> pool_free;
     std::unordered_map<void *, size_t> pool_used;
     size_t pool_bytes = 0;
+    size_t pool_free_bytes = 0;  // of them in pool_free
     // host-side failure injection for tests: after this many more successful
     // field / work-buffer allocations the next ones fail with WD_ERR_OOM
     // (-1: off)
@@ -105,7 +106,8 @@ using WdTried = std::optional<wd_status>;
 
 // Work-buffer allocation through the context's cache (stream-ordered reuse)
 wd_status wd_dev_alloc(wd_context *ctx, void **p, size_t bytes);
-void wd_dev_free(wd_context *ctx, void *p);
+// keep: the block stays cached if the cache then holds at most this much, else it goes back to CUDA
+void wd_dev_free(wd_context *ctx, void *p, size_t keep = ~(size_t)0);
 void wd_pool_release(wd_context *ctx);
 // cudaMalloc that gives back the context's cached work buffers, then the
 // fixed-point links of the device's lattices, when memory runs out
