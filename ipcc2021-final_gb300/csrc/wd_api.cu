@@ -9,6 +9,7 @@
 #include "wd_kernels.h"
 #include "wd_precision.h"
 #include "wd_solver.h"
+#include "wd_tune.h"
 
 // ------------------------------------------------------------------ errors
 wd_status wd_fail(wd_context *ctx, wd_status s, const std::string &msg)
@@ -215,6 +216,7 @@ bool wd_fix_ensure(wd_context *ctx, const wd_lattice *lat_c)
     }
     lat->fix_was_unfit = false;
     lat->fix_state = wd_lattice::kFixReady;
+    wd_tune_note("hop_f64", kHopF64Variants);  // still what a pin chooses from
     return true;
 }
 

@@ -142,7 +142,7 @@ wd_status wd_hop_f64(wd_context *ctx, const wd_lattice *lat, const double2 *in_b
         return WD_OK;
     };
     // variants: 128, 64, 256 threads per block
-    return wd_tune_launch(ctx, "hop_f64", lat->g.Vh, 3, [&](int v) -> wd_status {
+    return wd_tune_launch(ctx, "hop_f64", lat->g.Vh, kHopF64Variants, [&](int v) -> wd_status {
         if (v == 1) return run(std::integral_constant<int, 64>());
         if (v == 2) return run(std::integral_constant<int, 256>());
         return run(std::integral_constant<int, 128>());

@@ -446,13 +446,15 @@ FixArgs fix_args(const wd_lattice *lat, const void *in, void *out, const void *x
 // A launch's hold on the lattice's fixed-point links: the lock shared, if they
 // are there or can be built.  A stream that is being captured may not use them:
 // the graph would keep their address past the moment they are freed or replaced,
-// while the FP64 links stay where they are as long as the lattice.
+// while the FP64 links stay where they are as long as the lattice.  Nor may a
+// lattice size whose FP64-pipe shape the caller has pinned: that kernel runs.
 struct Links {
     WdFixShared lock;
     Links(wd_context *ctx, const wd_lattice *lat, cudaStream_t stream)
     {
         cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
         if (cudaStreamIsCapturing(stream, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone) return;
+        if (wd_tune_pinned(ctx, "hop_f64", lat->g.Vh)) return;
         lock = WdFixShared(wd_fix_mutex());
         if (lat->fix_state == wd_lattice::kFixReady) return;
         lock.unlock();
@@ -481,9 +483,7 @@ WdTried wd_hop_fix(wd_context *ctx, const wd_lattice *lat, const double2 *in, do
     if (!links) return {};
     FixArgs a = fix_args(lat, in, out, x, cb, alpha, beta, stop);
     a.zero = zero;
-    // one shape (64 and 32 threads a block run within 0.3 % of 128): the
-    // tuner's variants are the FP64-pipe kernel's
-    wd_tune_note("hop_f64", 3);
+    // (one shape: 64 and 32 threads a block run within 0.3 % of 128)
     return store_fix<false>(ctx, ctx->stream, a, dag, false, 0, lat->g.Vh);
 }
 

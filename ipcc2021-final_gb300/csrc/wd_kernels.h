@@ -10,6 +10,7 @@
 #define WD_RED_SLOTS 16
 
 // ---- hopping term: out_cb = alpha * D_{cb,1-cb} in_{1-cb} + beta * x_cb
+constexpr int kHopF64Variants = 3;  // launch shapes of its FP64-pipe kernel
 wd_status wd_hop_f64(wd_context *ctx, const wd_lattice *lat, const double2 *in_block,
                      double2 *out_block, const double2 *x_block, int cb, int dag, double alpha,
                      double beta, const int *stop = nullptr);

@@ -8,6 +8,7 @@
 // out distinct from the inputs), which every hop launch is.  WD_TUNE=0
 // disables tuning (variant 0 everywhere); WD_TUNE_CACHE=<file> loads and
 // appends decisions so later processes skip the timing.
+#include <atomic>
 #include <cstdio>
 #include <cstdlib>
 #include <map>
@@ -18,11 +19,14 @@
 
 namespace {
 
+constexpr float kPinned = -1.0f;  // chosen by the caller, not timed
+
 struct Tuner {
     std::mutex mu;
     std::map<std::tuple<int, std::string, int>, int> best;  // (device, kernel, Vh) -> variant
     std::map<std::tuple<int, std::string, int>, float> best_ms;
     std::map<std::string, int> variants;  // kernel -> number of launch variants (seen at launch)
+    std::atomic<int> pins{0};  // entries of best_ms that are kPinned
     bool loaded = false;
     int enabled = -1;
 
@@ -140,6 +144,15 @@ void wd_tune_note(const char *kernel, int nvariants)
     T.variants[kernel] = nvariants;
 }
 
+bool wd_tune_pinned(wd_context *ctx, const char *kernel, int Vh)
+{
+    Tuner &T = tuner();
+    if (T.pins.load(std::memory_order_relaxed) == 0) return false;
+    std::lock_guard<std::mutex> lock(T.mu);
+    auto it = T.best_ms.find({ctx->device, kernel, Vh});
+    return it != T.best_ms.end() && it->second == kPinned;
+}
+
 extern "C" int wd_tune_report(char *buf, int len)
 {
     Tuner &T = tuner();
@@ -166,15 +179,18 @@ extern "C" int wd_tune_pin(int device, const char *kernel, int half_volume, int 
     std::lock_guard<std::mutex> lock(T.mu);
     T.load();
     const auto key = std::make_tuple(device, std::string(kernel), half_volume);
+    auto it = T.variants.find(kernel);
+    if (variant >= 0 && it != T.variants.end() && variant >= it->second) return -1;
+    auto old = T.best_ms.find(key);
+    if (old != T.best_ms.end() && old->second == kPinned) --T.pins;
     if (variant < 0) {
         T.best.erase(key);
         T.best_ms.erase(key);
         return 0;
     }
-    auto it = T.variants.find(kernel);
-    if (it != T.variants.end() && variant >= it->second) return -1;
     T.best[key] = variant;
-    T.best_ms[key] = -1.0f;  // pinned, not timed
+    T.best_ms[key] = kPinned;
+    ++T.pins;
     return 0;
 }
 

@@ -15,6 +15,10 @@ wd_status wd_tune_launch(wd_context *ctx, const char *kernel, int Vh, int nvaria
 // plain kernel's shape.
 int wd_tune_choice(wd_context *ctx, const char *kernel, int Vh);
 
-// Records that `kernel` has nvariants launch variants, for a launch whose
-// shape needs no timing.
+// Records that `kernel` has nvariants launch variants, where another kernel
+// stands in for it.
 void wd_tune_note(const char *kernel, int nvariants);
+
+// Whether a caller pinned (kernel, Vh) on this context's device (wd_tune_pin).
+// Without any pin in the process this is one load.
+bool wd_tune_pinned(wd_context *ctx, const char *kernel, int Vh);
