@@ -59,7 +59,7 @@ __device__ __forceinline__ typename V::R norm_acc(typename V::R s, typename V::C
 }
 
 template <class V>
-__global__ void __launch_bounds__(WD_RED_THREADS) k_cgd_norm(const typename V::E *__restrict__ t, int64_t n, WdCgDev *dev,
+__global__ void __launch_bounds__(WD_RED_THREADS) k_cgd_norm(const typename V::E *t, int64_t n, WdCgDev *dev,
                                                              WdRed red)
 {
     wd_pdl_wait(gridDim.x > 152);
@@ -71,8 +71,8 @@ __global__ void __launch_bounds__(WD_RED_THREADS) k_cgd_norm(const typename V::E
 }
 
 template <class V>
-__global__ void __launch_bounds__(WD_RED_THREADS) k_cgd_dot(const typename V::E *__restrict__ p,
-                                                            const typename V::E *__restrict__ q, int64_t n, WdCgDev *dev,
+__global__ void __launch_bounds__(WD_RED_THREADS) k_cgd_dot(const typename V::E *p,
+                                                            const typename V::E *q, int64_t n, WdCgDev *dev,
                                                             WdRed red)
 {
     wd_pdl_wait(gridDim.x > 152);
@@ -90,10 +90,10 @@ __global__ void __launch_bounds__(WD_RED_THREADS) k_cgd_dot(const typename V::E 
 }
 
 template <class V, bool CPLX>
-__global__ void __launch_bounds__(WD_RED_THREADS) k_cgd_update(const typename V::E *__restrict__ p,
-                                                               const typename V::E *__restrict__ q,
-                                                               typename V::E *__restrict__ x,
-                                                               typename V::E *__restrict__ r, int64_t n, WdCgDev *dev,
+__global__ void __launch_bounds__(WD_RED_THREADS) k_cgd_update(const typename V::E *p,
+                                                               const typename V::E *q,
+                                                               typename V::E *x,
+                                                               typename V::E *r, int64_t n, WdCgDev *dev,
                                                                WdRed red)
 {
     wd_pdl_wait(gridDim.x > 152);
@@ -115,7 +115,7 @@ __global__ void __launch_bounds__(WD_RED_THREADS) k_cgd_update(const typename V:
 }
 
 template <class V>
-__global__ void k_cgd_xpby(const typename V::E *__restrict__ r, typename V::E *__restrict__ p, int64_t n,
+__global__ void k_cgd_xpby(const typename V::E *r, typename V::E *p, int64_t n,
                            const WdCgDev *dev)
 {
     wd_pdl_wait(gridDim.x > 152);

@@ -43,10 +43,10 @@ constexpr int kSitesPerWarp = 10;
 struct SplitDF {
     WdGeom g;
     int cb;
-    const float4 *__restrict__ in;
-    const float4 *__restrict__ gauge;
-    const float4 *__restrict__ x;
-    float4 *__restrict__ out;
+    const float4 *in;
+    const float4 *gauge;
+    const float4 *x;
+    float4 *out;
     dfr alpha, beta;
     const int *stop = nullptr;  // device gate: the launch is a no-op while *stop != 0
 };

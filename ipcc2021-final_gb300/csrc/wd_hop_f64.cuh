@@ -51,7 +51,7 @@ struct HopF64 {
     static constexpr bool kPairDirs = true;  // FP64-pipe bound: fewest operations wins
     WdGeom g;
     int cb;
-    const double2 *__restrict__ in;     // parity 1-cb block [12][Vh]
+    const double2 *in;                  // parity 1-cb block [12][Vh] (kernels that start early read it too)
     const double2 *__restrict__ gauge;  // [4][2][9][Vh]
     const double2 *__restrict__ x;      // parity cb block or null
     double2 *__restrict__ out;          // parity cb block
