@@ -172,7 +172,7 @@ static bool fix_alloc(wd_context *ctx, wd_lattice *lat)
     const size_t n = (size_t)lat->volume * 4 * 9 * sizeof(int4);
     size_t free_b = 0, total_b = 0;
     if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess || free_b < n + total_b / 8 ||
-        (n >= (64u << 20) && free_b + ctx->pool_free_bytes < n + total_b / 2) || cudaMalloc(&lat->gauge_fix, n) != cudaSuccess) {
+        (n >= (64u << 20) && free_b + ctx->pool_free_bytes + ctx->fields->bytes < n + total_b / 2) || cudaMalloc(&lat->gauge_fix, n) != cudaSuccess) {
         cudaGetLastError();
         lat->gauge_fix = nullptr;
         return false;
@@ -226,7 +226,7 @@ cudaError_t wd_malloc(wd_context *ctx, void **p, size_t bytes)
     const bool full = ctx->exhaust_after == 0;
     if (ctx->exhaust_after >= 0) --ctx->exhaust_after;
     cudaError_t e = full ? cudaErrorMemoryAllocation : cudaMalloc(p, bytes);
-    if (e == cudaErrorMemoryAllocation && !ctx->pool_free.empty()) {
+    if (e == cudaErrorMemoryAllocation && !(ctx->pool_free.empty() && ctx->fields->free.empty())) {
         cudaGetLastError();
         wd_pool_release(ctx);
         if (!full) e = cudaMalloc(p, bytes);
@@ -258,19 +258,13 @@ wd_status wd_dev_alloc(wd_context *ctx, void **p, size_t bytes)
     return WD_OK;
 }
 
-void wd_dev_free(wd_context *ctx, void *p, size_t keep)
+void wd_dev_free(wd_context *ctx, void *p)
 {
     if (!p) return;
     auto it = ctx->pool_used.find(p);
     if (it == ctx->pool_used.end()) return;
-    if (ctx->pool_free_bytes + it->second > keep) {
-        cudaFree(p);
-        ctx->pool_bytes -= it->second;
-        wd_memory_freed();
-    } else {
-        ctx->pool_free.emplace(it->second, p);
-        ctx->pool_free_bytes += it->second;
-    }
+    ctx->pool_free.emplace(it->second, p);
+    ctx->pool_free_bytes += it->second;
     ctx->pool_used.erase(it);
 }
 
@@ -281,8 +275,10 @@ void wd_pool_release(wd_context *ctx)
         cudaFree(kv.second);
         ctx->pool_bytes -= kv.first;
     }
+    for (auto &kv : ctx->fields->free) cudaFree(kv.second);
     ctx->pool_free.clear();
-    ctx->pool_free_bytes = 0;
+    ctx->fields->free.clear();
+    ctx->pool_free_bytes = ctx->fields->bytes = 0;
     wd_memory_freed();
 }
 
@@ -292,6 +288,7 @@ extern "C" void wd_context_destroy(wd_context *ctx)
     cudaSetDevice(ctx->device);
     host_cache_drop(ctx);
     wd_pool_release(ctx);
+    ctx->fields->open = false;
     for (auto &kv : ctx->pool_used) cudaFree(kv.first);
     ctx->pool_used.clear();
     if (ctx->stream) cudaStreamSynchronize(ctx->stream);
@@ -494,15 +491,19 @@ static size_t field_bytes(const wd_lattice *lat, wd_precision prec)
     return b;
 }
 
-static wd_status field_make(wd_context *ctx, const wd_lattice *lat, wd_precision prec, bool pooled, wd_field **out)
+static wd_status field_make(wd_context *ctx, const wd_lattice *lat, wd_precision prec, bool cached, wd_field **out)
 {
     *out = nullptr;
     const size_t bytes = field_bytes(lat, prec);
     void *data = nullptr;
-    if (pooled) {
-        if (wd_status st = wd_dev_alloc(ctx, &data, bytes)) return st;
+    if (wd_alloc_fails(ctx)) return wd_fail(ctx, WD_ERR_OOM, "field: injected allocation failure");
+    WdFieldCache &cache = *ctx->fields;
+    const auto it = cached ? cache.free.find(bytes) : cache.free.end();
+    if (it != cache.free.end()) {
+        data = it->second;
+        cache.bytes -= bytes;
+        cache.free.erase(it);
     } else {
-        if (wd_alloc_fails(ctx)) return wd_fail(ctx, WD_ERR_OOM, "field: injected allocation failure");
         const cudaError_t e = wd_malloc(ctx, &data, bytes);
         if (e != cudaSuccess) return wd_cuda_check(ctx, e, "cudaMalloc(field)");
     }
@@ -510,7 +511,8 @@ static wd_status field_make(wd_context *ctx, const wd_lattice *lat, wd_precision
     f->lat = lat;
     f->storage = prec;
     f->data = data;
-    f->pool = pooled ? ctx : nullptr;
+    if (cached) f->cache = ctx->fields;
+    f->bytes = bytes;
     if (prec == WD_PREC_F64) f->d = (double2 *)f->data;
     if (prec == WD_PREC_F16) f->scale = (float *)((char *)f->data + (size_t)lat->volume * 12 * wd_entry_bytes(prec));
     const cudaError_t e = cudaMemsetAsync(f->data, 0, bytes, ctx->stream);
@@ -529,12 +531,12 @@ extern "C" wd_status wd_field_create_prec(wd_context *ctx, const wd_lattice *lat
     return field_make(ctx, lat, prec, false, out);
 }
 
-// A library-internal FP64 field, destroyed before ctx: up to 64 MB its memory
-// comes from the context's work-buffer cache, since a cudaMalloc and a
-// cudaFree (which waits for the device) per field cost 70 us (a burst of 18
-// server systems 30.3 ms with them, 27.8 without; a 12-column propagator at
-// 16^3x32 30.1 and 28.9).  It goes back there only while the cache holds 1 GB
-// or less: a program's burst of requests is not kept for good.
+// A library-internal FP64 field: up to 64 MB its memory
+// comes from a cache of such fields, since a cudaMalloc and a cudaFree (which
+// waits for the device) per field cost 70 us (a burst of 18 server systems
+// 30.3 ms with them, 27.8 without; a 12-column propagator at 16^3x32 30.1 and
+// 28.9).  The cache holds 1 GB at most: a program's burst of requests is not
+// kept for good.
 constexpr size_t kFieldCache = (size_t)1 << 30;
 wd_status wd_field_create_work(wd_context *ctx, const wd_lattice *lat, wd_field **out)
 {
@@ -550,8 +552,11 @@ extern "C" wd_precision wd_field_precision(const wd_field *f) { return f ? f->st
 extern "C" void wd_field_destroy(wd_field *f)
 {
     if (!f) return;
-    if (f->pool) wd_dev_free(f->pool, f->data, kFieldCache);
-    else {
+    WdFieldCache *c = f->cache.get();
+    if (c && c->open && c->bytes + f->bytes <= kFieldCache) {
+        c->free.emplace(f->bytes, f->data);
+        c->bytes += f->bytes;
+    } else {
         cudaFree(f->data);  // cudaFree waits for work in flight on the device
         wd_memory_freed();
     }

@@ -1287,8 +1287,8 @@ static wd_status server_admit(wd_server *sv, int *completed)
         if (sv->active_systems > 0 && sv->active_systems + p.nsrc > sv->cfg.max_systems) break;
         server_make_room(sv, bytes);
         // the budget bounds what is held, cached blocks of earlier requests too
-        if (sv->gauge_bytes + sv->req_bytes + server_fix_bytes(sv) + bytes + (double)sv->ctx->pool_free_bytes >
-            sv->cfg.hbm_budget_bytes)
+        const double cached = (double)(sv->ctx->pool_free_bytes + sv->ctx->fields->bytes);
+        if (sv->gauge_bytes + sv->req_bytes + server_fix_bytes(sv) + bytes + cached > sv->cfg.hbm_budget_bytes)
             wd_pool_release(sv->ctx);
         wd_server::Req &r = sv->reqs[p.id];
         wd_status st = WD_OK;

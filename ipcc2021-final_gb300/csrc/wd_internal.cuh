@@ -13,6 +13,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 #include <map>
+#include <memory>
 #include <optional>
 #include <string>
 #include <unordered_map>
@@ -53,6 +54,14 @@ struct WdGeom {
                        // instead of about twenty (the FP16 hop issues 1622 per site)
 };
 
+// Memory of the library's own FP64 fields (wd_field_create_work).  Fields share
+// it, so that one may be destroyed after its context, which closes it.
+struct WdFieldCache {
+    std::multimap<size_t, void *> free;
+    size_t bytes = 0;
+    bool open = true;
+};
+
 struct wd_context {
     int device = 0;
     cudaStream_t stream = nullptr;
@@ -84,6 +93,7 @@ struct wd_context {
     std::unordered_map<void *, size_t> pool_used;
     size_t pool_bytes = 0;
     size_t pool_free_bytes = 0;  // of them in pool_free
+    std::shared_ptr<WdFieldCache> fields = std::make_shared<WdFieldCache>();
     // host-side failure injection for tests: after this many more successful
     // field / work-buffer allocations the next ones fail with WD_ERR_OOM
     // (-1: off)
@@ -106,13 +116,12 @@ using WdTried = std::optional<wd_status>;
 
 // Work-buffer allocation through the context's cache (stream-ordered reuse)
 wd_status wd_dev_alloc(wd_context *ctx, void **p, size_t bytes);
-// keep: the block stays cached if the cache then holds at most this much, else it goes back to CUDA
-void wd_dev_free(wd_context *ctx, void *p, size_t keep = ~(size_t)0);
+void wd_dev_free(wd_context *ctx, void *p);
 void wd_pool_release(wd_context *ctx);
 // cudaMalloc that gives back the context's cached work buffers, then the
 // fixed-point links of the device's lattices, when memory runs out
 cudaError_t wd_malloc(wd_context *ctx, void **p, size_t bytes);
-// a library-internal FP64 field, from the work-buffer cache if it is small
+// a library-internal FP64 field, from a cache if it is small
 wd_status wd_field_create_work(wd_context *ctx, const wd_lattice *lat, wd_field **out);
 
 struct wd_lattice {
@@ -145,7 +154,8 @@ struct wd_field {
     void *data = nullptr;     // [parity][12][Vh] entries of the storage type
     float *scale = nullptr;   // FP16 storage: [parity][Vh] per-site scales (inside data)
     double2 *d = nullptr;     // == data for FP64 storage, else null
-    wd_context *pool = nullptr;  // owns data in its work-buffer cache, else null
+    std::shared_ptr<WdFieldCache> cache;  // takes data back, or null
+    size_t bytes = 0;                     // of data
 };
 
 // Work space of a grid reduction (wd_grid_sum_n): the blocks' partials, then

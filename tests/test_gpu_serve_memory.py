@@ -68,3 +68,20 @@ def test_budget_bounds_cached_blocks(wd):
         # beside the budget: the staging buffer of link uploads and small buffers
         assert peak - start <= budget + 9 * 16 * int(np.prod(large)) + (16 << 20)
         sv.close()
+
+
+def test_plain_server_outlives_its_context(wd):
+    """A server whose finished request was not collected, closed after its context."""
+    dims = (4, 4, 4, 4)
+    ctx = wd.Context(0)
+    sv = wd.Server(ctx, prec=wd.F64)
+    lat = sv.add_lattice(dims, wd.gen_gauge(dims, seed=93))
+    for seed in (1, 2):
+        sv.submit(lat, 1, mass=0.2, tol=1e-8, seeds=[seed])
+    for _ in range(4):
+        sv.step()
+    ctx.close()
+    sv.close()
+    with wd.Context(0) as other:
+        f = other.lattice(dims, wd.gen_gauge(dims, seed=93)).field(wd.gen_source(dims, seed=1))
+        assert abs(f.norm2() - 1.0) < 1e-12
