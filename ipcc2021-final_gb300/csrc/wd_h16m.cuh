@@ -193,14 +193,14 @@ __device__ __forceinline__ void h16_dir(const P &p, int s, const WdSite &c, floa
     unsigned sp[12], U[9];
 #pragma unroll
     for (int j = 0; j < 3; ++j) {
-        const uint4 v = __ldg(p.in.p + (size_t)j * Vh + nb);
+        const uint4 v = p.in.p[(size_t)j * Vh + nb];
         sp[4 * j] = v.x, sp[4 * j + 1] = v.y, sp[4 * j + 2] = v.z, sp[4 * j + 3] = v.w;
     }
-    const float sc = __ldg(p.in.scale + nb);
+    const float sc = p.in.scale[nb];
     // forward: U_mu(x) stored at this site (parity cb); backward: U_mu(x - mu) at the neighbour
     const size_t i = (size_t)(MU * 2 + (FWD ? p.cb : 1 - p.cb)) * Vh + (FWD ? s : nb);
-    const uint4 la = __ldg(p.link.a + i);
-    const uint2 lb = __ldg(p.link.b + i);
+    const uint4 la = p.link.a[i];
+    const uint2 lb = p.link.b[i];
     U[0] = la.x, U[1] = la.y, U[2] = la.z, U[3] = la.w, U[4] = lb.x, U[5] = lb.y;
     h16_dir_terms<MU, FWD, DAG>(sp, sc, U, acc);
 }
@@ -236,13 +236,13 @@ __device__ __forceinline__ void h16_dir_r2(const P &p, int s, const WdSite &c, c
     unsigned sp[12], U[9];
 #pragma unroll
     for (int j = 0; j < 3; ++j) {
-        const uint4 v = __ldg(p.in.p + (size_t)j * Vh + nb);
+        const uint4 v = p.in.p[(size_t)j * Vh + nb];
         sp[4 * j] = v.x, sp[4 * j + 1] = v.y, sp[4 * j + 2] = v.z, sp[4 * j + 3] = v.w;
     }
-    const float sc = __ldg(p.in.scale + nb);
+    const float sc = p.in.scale[nb];
     const size_t i = (size_t)(MU * 2 + (FWD ? p.cb : 1 - p.cb)) * Vh + (FWD ? s : nb);
-    const uint4 la = __ldg(p.link.a + i);
-    const uint2 lb = __ldg(p.link.b + i);
+    const uint4 la = p.link.a[i];
+    const uint2 lb = p.link.b[i];
     U[0] = la.x, U[1] = la.y, U[2] = la.z, U[3] = la.w, U[4] = lb.x, U[5] = lb.y;
     U[6] = r2[D][0][lane], U[7] = r2[D][1][lane], U[8] = r2[D][2][lane];
     h16_dir_terms<MU, FWD, DAG, false>(sp, sc, U, acc);
@@ -274,8 +274,8 @@ __device__ __forceinline__ void h16_fill_row2_dir(const WdGeom &g, int cb, const
     constexpr int MU = D / 2;
     constexpr bool FWD = (D % 2) == 0;
     const size_t i = (size_t)(MU * 2 + (FWD ? cb : 1 - cb)) * g.Vh + (FWD ? s : wd_neighbour(g, s, c, MU, false));
-    const uint4 la = __ldg(link.a + i);
-    const uint2 lb = __ldg(link.b + i);
+    const uint4 la = link.a[i];
+    const uint2 lb = link.b[i];
     unsigned U[9] = {la.x, la.y, la.z, la.w, lb.x, lb.y, 0u, 0u, 0u};
     h16_row2(U);
     r2[D][0][lane] = U[6], r2[D][1][lane] = U[7], r2[D][2][lane] = U[8];

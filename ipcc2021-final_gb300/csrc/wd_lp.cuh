@@ -45,7 +45,7 @@ struct SpF32 {
     {
 #pragma unroll
         for (int j = 0; j < 6; ++j) {
-            const float4 f = __ldg(p + (size_t)j * Vh + s);
+            const float4 f = p[(size_t)j * Vh + s];
             v[2 * j] = make_float2(f.x, f.y);
             v[2 * j + 1] = make_float2(f.z, f.w);
         }
@@ -67,8 +67,8 @@ struct SpF16 {
     __device__ __forceinline__ float load_raw(int s, float2 *v) const
     {
 #pragma unroll
-        for (int j = 0; j < 3; ++j) unpack4(__ldg(p + (size_t)j * Vh + s), v + 4 * j);
-        return __ldg(scale + s);
+        for (int j = 0; j < 3; ++j) unpack4(p[(size_t)j * Vh + s], v + 4 * j);
+        return scale[s];
     }
     __device__ __forceinline__ void load(int s, float2 *v) const
     {
@@ -130,7 +130,7 @@ struct LinkF32 {
         const float4 *b = g + (size_t)((mu * 2 + par) * 3) * Vh + s;
 #pragma unroll
         for (int j = 0; j < 3; ++j) {
-            const float4 f = __ldg(b + (size_t)j * Vh);
+            const float4 f = b[(size_t)j * Vh];
             U[2 * j] = make_float2(f.x, f.y);
             U[2 * j + 1] = make_float2(f.z, f.w);
         }
@@ -145,8 +145,8 @@ struct LinkF16 {
     __device__ __forceinline__ void load(int mu, int par, int s, float2 *U) const
     {
         const size_t i = (size_t)(mu * 2 + par) * Vh + s;
-        unpack4(__ldg(a + i), U);
-        const uint2 v = __ldg(b + i);
+        unpack4(a[i], U);
+        const uint2 v = b[i];
         U[4] = h2f(*reinterpret_cast<const __half2 *>(&v.x));
         U[5] = h2f(*reinterpret_cast<const __half2 *>(&v.y));
         su3_row2(U);

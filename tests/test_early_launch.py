@@ -45,3 +45,12 @@ def test_operands_are_not_promised_constant():
         assert "__restrict__" not in head, (name, head)
         for t in re.findall(r"\bconst\s+(\w+)\s+\w+", head):
             assert "__restrict__" not in defs.get(t, ""), (name, t)
+
+
+def test_no_loads_for_constant_data():
+    """Nor are they read with __ldg, which is the same promise; the one file
+    that does holds kernels that are launched in the ordinary way only."""
+    for f in sorted(CSRC.glob("*.cu*")):
+        text = re.sub(r"//[^\n]*", "", f.read_text())
+        if "__ldg(" in text or "ld.global.nc" in text:
+            assert f.name == "wd_h16_tma.cuh" and "wd_pdl_wait" not in text and "wd_launch" not in text, f.name
