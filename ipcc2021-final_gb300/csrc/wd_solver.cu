@@ -13,6 +13,7 @@
 // pipe).  Mixed precision (FP32 / FP16 inner) lives in wd_mixed.cu.
 #include <chrono>
 #include <cmath>
+#include <limits>
 #include "wd_fix_links.h"
 #include "wd_kernels.h"
 #include "wd_solver.h"
@@ -136,7 +137,8 @@ struct CgLoop {
         static_assert(sizeof(WdCgDev) <= 256 && 3 * sizeof(WdCgDev) <= WD_STATE_HOST_BYTES, "device scalars");
         host[2] = WdCgDev{};
         host[2].rr = rr;
-        host[2].target2 = target * target;
+        // (a square that underflows is still met by a residual of zero)
+        host[2].target2 = std::fmax(target * target, std::numeric_limits<double>::denorm_min());
         host[2].strict = strict;
         host[2].iters = iters;
         WD_CUDA(ctx, cudaMemcpyAsync(dev, &host[2], sizeof(WdCgDev), cudaMemcpyHostToDevice, ctx->stream));
