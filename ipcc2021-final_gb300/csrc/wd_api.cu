@@ -6,6 +6,7 @@
 #include <cstdio>
 #include <string>
 #include "wd_fix_links.h"
+#include "wd_pinned.h"
 #include "wd_kernels.h"
 #include "wd_precision.h"
 #include "wd_solver.h"
@@ -390,24 +391,6 @@ static bool host_pageable(const void *p)
     return a.type == cudaMemoryTypeUnregistered;
 }
 
-// The address at which kernels reach pinned host memory in 16-byte accesses,
-// or null.  The layout kernels then read or write it themselves, so the
-// conversion rides on the transfer instead of following or preceding it
-// through the staging buffer (32^3x64 on pinned arrays: field download 2.22
-// -> 2.09 ms, upload 2.05 -> 1.92, links 9.3 -> 7.8).  Pageable memory keeps
-// the copy: pages that were never touched fault one by one from the device
-// (118 ms for a fresh 403 MB array against 17).
-static void *pinned_view(const void *p)
-{
-    cudaPointerAttributes a;
-    if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
-        cudaGetLastError();
-        return nullptr;
-    }
-    if (a.type != cudaMemoryTypeHost || !a.devicePointer || ((uintptr_t)a.devicePointer & 15)) return nullptr;
-    return a.devicePointer;
-}
-
 static wd_status upload_gauge(wd_context *ctx, wd_lattice *lat, const double *const gauge[4])
 {
     const WdGeom &g = lat->g;
@@ -416,7 +399,7 @@ static wd_status upload_gauge(wd_context *ctx, wd_lattice *lat, const double *co
     bool stage = false;
     for (int mu = 0; mu < 4; ++mu) {
         if (!gauge[mu]) return wd_fail(ctx, WD_ERR_BAD_ARG, "gauge pointer is null");
-        view[mu] = (const double2 *)pinned_view(gauge[mu]);
+        view[mu] = (const double2 *)wd_pinned_view(gauge[mu], bytes);
         stage = stage || !view[mu];
     }
     wd_status st = stage ? ensure_staging(ctx, bytes) : WD_OK;
@@ -568,7 +551,7 @@ extern "C" wd_status wd_field_upload(wd_context *ctx, wd_field *f, const double 
 {
     if (!ctx || !f || !host) return wd_fail(ctx, WD_ERR_BAD_ARG, "null argument");
     const size_t bytes = (size_t)f->lat->volume * 12 * sizeof(double2);
-    const double2 *ref = f->storage == WD_PREC_F16 ? nullptr : (const double2 *)pinned_view(host);
+    const double2 *ref = f->storage == WD_PREC_F16 ? nullptr : (const double2 *)wd_pinned_view(host, bytes);
     wd_status st;
     if (!ref) {
         if ((st = ensure_staging(ctx, bytes)) != WD_OK) return st;
@@ -586,7 +569,7 @@ extern "C" wd_status wd_field_download(wd_context *ctx, const wd_field *f, doubl
 {
     if (!ctx || !f || !host) return wd_fail(ctx, WD_ERR_BAD_ARG, "null argument");
     const size_t bytes = (size_t)f->lat->volume * 12 * sizeof(double2);
-    double2 *ref = f->storage == WD_PREC_F16 ? nullptr : (double2 *)pinned_view(host);
+    double2 *ref = f->storage == WD_PREC_F16 ? nullptr : (double2 *)wd_pinned_view(host, bytes);
     const bool staged = !ref;
     wd_status st;
     if (staged) {
