@@ -283,6 +283,21 @@ void wd_pool_release(wd_context *ctx)
     wd_memory_freed();
 }
 
+void wd_fields_trim(wd_context *ctx, double bytes, size_t size, int keep)
+{
+    WdFieldCache &c = *ctx->fields;
+    keep = std::min(keep, (int)c.free.count(size));
+    bytes += (double)keep * size;
+    for (auto it = c.free.end(); (double)c.bytes > bytes && it != c.free.begin();) {
+        --it;
+        if (it->first == size && keep-- > 0) continue;
+        cudaFree(it->second);  // waits for work in flight on the device
+        c.bytes -= it->first;
+        it = c.free.erase(it);
+        wd_memory_freed();
+    }
+}
+
 extern "C" void wd_context_destroy(wd_context *ctx)
 {
     if (!ctx) return;

@@ -1286,10 +1286,13 @@ static wd_status server_admit(wd_server *sv, int *completed)
         if (sv->gauge_bytes + sv->req_bytes + keep + bytes > sv->cfg.hbm_budget_bytes) break;
         if (sv->active_systems > 0 && sv->active_systems + p.nsrc > sv->cfg.max_systems) break;
         server_make_room(sv, bytes);
-        // the budget bounds what is held, cached blocks of earlier requests too
-        const double cached = (double)(sv->ctx->pool_free_bytes + sv->ctx->fields->bytes);
-        if (sv->gauge_bytes + sv->req_bytes + server_fix_bytes(sv) + bytes + cached > sv->cfg.hbm_budget_bytes)
-            wd_pool_release(sv->ctx);
+        // The budget bounds the cached fields of earlier requests too.  (The solvers'
+        // cached work buffers stay outside: with them inside, a saturated
+        // server trades buffers of one lattice size for those of another at each
+        // admission: 204 solves/s, 199 if all are released, 215 without.)
+        wd_fields_trim(sv->ctx, std::max(0.0, sv->cfg.hbm_budget_bytes - sv->gauge_bytes - sv->req_bytes -
+                                                  server_fix_bytes(sv) - bytes),
+                       (size_t)field_bytes64(lat), 2 * p.nsrc);
         wd_server::Req &r = sv->reqs[p.id];
         wd_status st = WD_OK;
         for (int k = 0; k < p.nsrc && st == WD_OK; ++k) {

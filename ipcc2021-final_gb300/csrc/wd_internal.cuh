@@ -118,6 +118,8 @@ using WdTried = std::optional<wd_status>;
 wd_status wd_dev_alloc(wd_context *ctx, void **p, size_t bytes);
 void wd_dev_free(wd_context *ctx, void *p);
 void wd_pool_release(wd_context *ctx);
+// frees cached fields until at most `bytes` are cached beside up to `keep` of size `size`
+void wd_fields_trim(wd_context *ctx, double bytes, size_t size, int keep);
 // cudaMalloc that gives back the context's cached work buffers, then the
 // fixed-point links of the device's lattices, when memory runs out
 cudaError_t wd_malloc(wd_context *ctx, void **p, size_t bytes);
