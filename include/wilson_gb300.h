@@ -43,7 +43,9 @@ typedef enum wd_status {
 
 /* Arithmetic used by the hopping kernels. */
 typedef enum wd_precision {
-    WD_PREC_F64 = 0,  /* FP64 (links of unitary size: fixed point on the integer pipe, same accuracy) */
+    WD_PREC_F64 = 0,  /* FP64.  Links of unitary size: the hop sums in 64-bit fixed point on the integer pipe, where
+                       * every component's own terms reach 2^-7 of the site's largest neighbour component (error
+                       * below 2^-50 of them), else in FP64 operations */
     WD_PREC_DF64 = 1, /* double-float: FP32 hi/lo pairs, ~48-bit mantissa, FP64-class results */
     WD_PREC_F32 = 2,  /* FP32 storage and arithmetic */
     WD_PREC_F16 = 3   /* FP16 spinors with a per-site FP32 scale, 12-real links, FP32 arithmetic */

@@ -3,8 +3,11 @@
 // while they compute the current one.  Each copy moves one 4-, 8- or 16-byte
 // element; both addresses must be aligned to its size.  A thread's copies
 // become visible to that thread after cp.async.wait_group retires their
-// group; other threads would also need a barrier (the kernels using these
-// read back only their own copies).
+// group; other threads also need a barrier after that wait.  The FP16 and
+// double-float hops read back only their own copies.  The fixed-point hop
+// shares a site's link between the two threads of a pair: there the
+// __syncwarp after the wait makes the partner's copies visible, and keeps a
+// slot from being overwritten while the partner still reads it.
 #pragma once
 #include <cuda_runtime.h>
 

@@ -1,4 +1,6 @@
-// wd_dslash_f64.cu -- native FP64 hopping kernel (the plain drop-in arithmetic).
+// wd_dslash_f64.cu -- native FP64 hopping kernel (the plain drop-in arithmetic),
+// for lattices whose links the fixed-point hop (wd_dslash_fix.cu) does not hold
+// and launches that may not use its copy of them.
 //
 // Storage: double2 planes, spinor [12][Vh] per parity, links [mu][parity][9][Vh].
 // Algorithmic traffic per output site: 8 links x 144 B + 1 spinor in x 192 B

@@ -6,8 +6,8 @@
 // 32^3x64 however its 0.24 ms of memory traffic is arranged.  The integer
 // pipes take 24-28 wide multiply-adds (32 x 32 + 64 bits) per clock and SM, and
 // SU(3) links have entries within [-1, 1], so the matrix products are done on
-// integers: a link entry is round(u 2^60) in two 30-bit limbs (laid out once,
-// at upload), a projected half-spinor is brought to one exponent per output
+// integers: a link entry is round(u 2^60) in two 30-bit limbs (laid out
+// once, by the first hop on a set of links), a projected half-spinor is brought to one exponent per output
 // site (a block scale) in limbs of 28 and 30 bits, and a product costs three
 // wide multiply-adds (the low x low one is below the last place).  The sums
 // over colours and over the eight directions are exact integers and are
@@ -38,10 +38,10 @@
 // ones (Gauss): additions are cheaper than wide multiply-adds here.
 // Measured at 32^3x64: 0.371 ms (FP64 form 1.453 ms), 4.34 TB/s of
 // compulsory bytes, 65 % of measured HBM.  What bounds it now is issue and
-// the integer pipes together (fma-heavy 60 %, FP64 56 %, ALU 34 %, issue slots
-// 44 % busy with 16 warps an SM at 32^4); with every load served by L1 it is
-// no faster.  Dropped: converting with F2I.S64.F64
-// (0.67 ms: it occupies the FP64 pipe), projecting after conversion on
+// the integer pipes together (at 24^3x48 fma-heavy pipe 58 %, FP64 54 %, ALU
+// 37 %, issue slots 45 % busy with 15 warps an SM); with every load served by
+// L1 it is no faster.  Dropped: converting with F2I.S64.F64 (0.67 ms: it
+// occupies the FP64 pipe), projecting after conversion on
 // integers (0.458 ms before staging), 20 warps per SM at 96 registers (0.395
 // ms against 0.372), the next direction's projection ahead of the current
 // product (0.381 ms).

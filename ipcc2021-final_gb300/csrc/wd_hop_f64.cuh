@@ -89,7 +89,8 @@ struct HopF64 {
 // 32 neighbour sites are 6 KB of consecutive bytes, so every fetched line is
 // used, and the FP64 pipe (not the access pattern) still bounds the kernel.
 // The host-buffer path runs it on the staging buffers directly, with no
-// layout conversion between the copies and the arithmetic.
+// layout conversion between the copies and the arithmetic, where the
+// fixed-point hop (which reads both layouts) does not take the links.
 template <int THREADS>
 struct HopF64AoS : HopF64<THREADS> {
     __device__ __forceinline__ void load_in(int s, double2 *v) const

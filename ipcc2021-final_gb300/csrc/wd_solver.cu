@@ -9,8 +9,9 @@
 // iterations; it stops on the relative true residual |b - M x|/|b|.
 //
 // Both run in FP64 or in double-float (prec = WD_PREC_DF64: the same
-// recurrences on float-pair vectors, ~5x faster on GB300's narrow FP64
-// pipe).  Mixed precision (FP32 / FP16 inner) lives in wd_mixed.cu.
+// recurrences on float-pair vectors; on links that the fixed-point hop does
+// not hold, where FP64 runs on GB300's narrow FP64 pipe, about 4x faster).
+// Mixed precision (FP32 / FP16 inner) lives in wd_mixed.cu.
 #include <chrono>
 #include <cmath>
 #include <limits>
